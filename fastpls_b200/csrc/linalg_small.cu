@@ -2,6 +2,7 @@
 #include "context.cuh"
 #include "linalg_small.cuh"
 
+#include <algorithm>
 #include <vector>
 
 namespace fpls {
@@ -185,145 +186,287 @@ __device__ void round_robin_next(int* arr, int n) {
   arr[1] = last;
 }
 
-// With in_smem the working matrices W and V live in shared memory (after the
-// rotation tables): W is copied in first, and every rotation round touches
-// shared memory only.
-__global__ void jacobi_eig_kernel(int l, double* W, double* V, double* evals_out,
-                                  double* V_out, int ldv, const int max_sweeps, int in_smem) {
-  extern __shared__ double sm[];
-  const int npair = (l + 1) / 2;
-  const int le = 2 * npair;
-  double* cs = sm;              // [npair] cos
-  double* sn = sm + npair;      // [npair] sin
-  int* arr = reinterpret_cast<int*>(sm + 2 * npair);   // [le]
-  int* pp = arr + le;           // [npair]
-  int* qq = pp + npair;         // [npair]
-  __shared__ double scratch[32];
-  __shared__ int sweep_done;
-  if (in_smem) {
-    double* Ws = reinterpret_cast<double*>(reinterpret_cast<char*>(sm) + 32 * npair);
-    for (int t = threadIdx.x; t < l * l; t += blockDim.x) Ws[t] = W[t];
-    W = Ws;
-    V = Ws + (size_t)l * l;
+// Cyclic two-sided Jacobi on one CTA, for l <= kEigMax.  What bounds it is the
+// chain of rounds (le - 1 a sweep, six to nine sweeps), so a round is one
+// barrier long:
+//  * W is held by round-robin position, not by index (upper triangle), twice in
+//    shared memory: a round reads one copy and writes the other with every
+//    position moved on by one, so each thread's addresses are the same in
+//    every round and no barrier stands between the two halves of a rotation;
+//    one thread takes the 2 x 2 block of two pairs through both;
+//  * meanwhile one warp (two above 64) works out the next round's angles from
+//    the old blocks that its pairs come from, on a scheduler that the update
+//    warps leave to it: its chain of dependent FP64 operations is as long as
+//    the whole update;
+//  * V takes no part: the angles go to a log in global memory, and
+//    jacobi_apply_log_kernel runs V's rows through it, one warp a row, all
+//    rows at once over the GPU.
+// Measured: 0.66 us a round at 60 x 60 (the angles alone 0.47 us, the update
+// alone 0.37 us), 302 us + 50 us for V against 1600 us when W and V were updated
+// in place with three barriers a round; 110 x 110: 0.8 + 0.15 ms against 4.1 ms
+// of the whole-GPU one-sided Jacobi with its grid barrier a round.
+constexpr int kEigMax = 112;         // two copies of W in 227 KB of shared memory
+constexpr int kEigWarps = 32;
+constexpr int kEigSweeps = 60;
+constexpr int eig_blocks(int npair) { return npair * (npair / 2 + 1); }
+constexpr int kEigUpdate = 32 * (kEigWarps / 4) * 3;   // update threads, at most: schedulers 1 to 3
+constexpr int kEigBlocks = (eig_blocks(kEigMax / 2) + kEigUpdate - 1) / kEigUpdate;
+
+__device__ __forceinline__ int upper_at(int i, int j, int ld) { return i < j ? i + j * ld : j + i * ld; }
+
+struct Rot { double c, s; };   // top' = c top - s bot, bot' = s top + c bot
+
+// Whether the pair (p, q) is still coupled: |apq| above rounding of its diagonal.
+__device__ __forceinline__ bool coupled(double app, double apq, double aqq) {
+  return fabs(apq) > 1e-300 && fabs(apq) > kEps * sqrt(fabs(app * aqq));
+}
+
+// The rotation that decouples the pair (top, bot); a pair decoupled to rounding
+// is left alone.  tan solves wtb t^2 + (wbb - wtt) t - wtb = 0: its first value
+// comes from single precision (of numbers scaled by the larger one's power of
+// two) and one Newton step on that equation takes it to about 1e-13, which is
+// far below what the next sweep removes; the cosine is full double precision,
+// so the rotation is orthogonal to rounding whatever the angle.  `swap`: the
+// top index is the larger one (equal diagonals turn by +45 degrees from the
+// smaller index).
+__device__ __forceinline__ Rot decouple(bool swap, double wtt, double wtb, double wbb) {
+  const double d = wbb - wtt;
+  const int hid = __double2hiint(d) & 0x7ff00000, hiw = __double2hiint(wtb) & 0x7ff00000;
+  const int ex = max(hid, hiw);                      // exponent bits of the larger one
+  const bool plain = ex < 0x5d000000 && ex > 0x2b500000;   // about 1e-100 .. 1e140
+  const double scale = __hiloint2double(0x7fe00000 - (plain ? ex : 0x3ff00000), 0);   // 2^-exponent
+  const double ds = d * scale, es = wtb * scale;
+  const float df = static_cast<float>(ds), ef = static_cast<float>(es);
+  const float sq = fmaf(df, df, 4.0f * ef * ef);     // >= 1 (plain)
+  const float root = sq * rsqrtf(sq);
+  const float tf = __fdividef(2.0f * ef, df >= 0.0f ? df + root : df - root);
+  double t = static_cast<double>(tf);
+  t -= fma(es, fma(t, t, -1.0), ds * t) * static_cast<double>(__fdividef(1.0f, fmaf(2.0f * ef, tf, df)));
+  bool go = wtb * wtb > (kEps * kEps) * fabs(wtt * wbb) && hiw > 0x20b00000;   // above 1e-150
+  if (!plain) {
+    go = coupled(wtt, wtb, wbb);
+    const double tau = go ? d / (2.0 * wtb) : 0.0;
+    t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+  } else if (fabsf(tf) < 1e-18f) {
+    t = go ? wtb / d : 0.0;   // the small-angle limit
   }
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) V[t] = (t % l == t / l) ? 1.0 : 0.0;
-  __shared__ int rotated;
+  if (d == 0.0) t = swap ? -1.0 : 1.0;
+  t = go ? t : 0.0;
+  Rot r;
+  r.c = rsqrt(fma(t, t, 1.0));
+  r.s = t * r.c;
+  return r;
+}
+
+// Element (x, y) of the rotated block w of two pairs: x is the first pair's
+// top or bottom, y the second's.
+__device__ __forceinline__ double rotated_at(const double (&w)[4], Rot ra, bool x_top, Rot rb, bool y_top) {
+  const double u0 = x_top ? ra.c : ra.s, u1 = x_top ? -ra.s : ra.c;
+  const double v0 = y_top ? rb.c : rb.s, v1 = y_top ? -rb.s : rb.c;
+  return fma(v0, fma(u0, w[0], u1 * w[2]), v1 * fma(u0, w[1], u1 * w[3]));
+}
+
+// Round-robin: position 0 keeps its index, the others move on by one a round;
+// pair k is the positions k (top) and le - 1 - k (bottom).
+__device__ __forceinline__ int next_position(int i, int le) { return i == 0 ? 0 : i == le - 1 ? 1 : i + 1; }
+__device__ __forceinline__ int ring_prev(int i, int le) { return i == 1 ? le - 1 : i - 1; }
+
+// Offsets of the block of pairs a and b in W (from), and of where its elements
+// go (to).
+__device__ __forceinline__ void block_offsets(int a, int b, int le, int ld, int (&from)[4], int (&to)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = e & 2 ? le - 1 - a : a, j = e & 1 ? le - 1 - b : b;
+    from[e] = upper_at(i, j, ld);
+    to[e] = upper_at(next_position(i, le), next_position(j, le), ld);
+  }
+}
+
+template <int NB>   // blocks of the pair grid per update thread
+__global__ void __launch_bounds__(32 * kEigWarps)
+jacobi_eig_kernel(int l, const double* __restrict__ G, int ldg, double* __restrict__ evals, int* __restrict__ rank_of,
+                  double2* __restrict__ log, int* __restrict__ rounds_out, int max_sweeps) {
+  extern __shared__ double sm[];
+  // Along a warp the two positions of a block move by one each, so an even
+  // leading dimension makes every step odd: no bank conflicts.
+  const int le = l + (l & 1), npair = le / 2, ld = le, half = le * ld;
+  Rot* rots = reinterpret_cast<Rot*>(sm + 2 * half);   // [2][npair]
+  __shared__ double scratch[32];
+  __shared__ int open;
+  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
+  for (int t = tid; t < le * le; t += nt) {
+    const int i = t % le, j = t / le;
+    sm[i + j * ld] = (i < l && j < l) ? G[i + (size_t)j * ldg] : 0.0;
+  }
   __syncthreads();
-  // Frobenius norm for the convergence test.
   double fro = 0.0;
-  for (int t = threadIdx.x; t < l * l; t += blockDim.x) fro += W[t] * W[t];
-  fro = block_sum(fro, scratch);
-  const double thresh = kEps * kEps * fro;
+  for (int t = tid; t < l * l; t += nt) {
+    const double w = sm[t % l + (t / l) * ld];
+    fro += w * w;
+  }
+  const double thresh = kEps * kEps * block_sum(fro, scratch);
+  // Warps 0 and 4 work out the angles (pair k); the warps of schedulers 1 to 3
+  // update, each thread the block of a pair a (fastest) with pair a + delta
+  // around the ring, delta up to half of it: one thread for each couple of pairs.
+  const int k = warp == 0 ? lane : lane + 32;
+  const bool angles = (warp == 0 || warp == 4) && k < npair;
+  const int update = 32 * 3 * (nt / 128), uid = 32 * (3 * (warp >> 2) + (warp & 3) - 1) + lane;
+  int pa[NB], pb[NB], from[NB][4], to[NB][4];
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    pa[u] = -1;
+    const int t = uid + u * update, a = t % npair, delta = t / npair;
+    if ((warp & 3) == 0 || 2 * delta > npair || (2 * delta == npair && a >= npair / 2)) continue;
+    pa[u] = a;
+    pb[u] = a + delta < npair ? a + delta : a + delta - npair;
+    block_offsets(pa[u], pb[u], le, ld, from[u], to[u]);
+  }
+  // the current pairs whose indices pair k has next: its top is the top of
+  // k - 1 (the bottom of 0 for k = 1), its bottom the bottom of k + 1 (the top
+  // of the last pair for the last)
+  const int A = k == 0 ? 0 : k - 1, B = min(k + 1, npair - 1);
+  const bool a_top = k != 1, b_top = k == npair - 1 && npair > 1;
+  int faa[4], fab[4], fbb[4], unused[4];
+  int top = k, bot = le - 1 - k;   // pair k's indices
+  if (angles) {
+    block_offsets(A, A, le, ld, faa, unused);
+    block_offsets(A, B, le, ld, fab, unused);
+    block_offsets(B, B, le, ld, fbb, unused);
+    rots[k] = decouple(top > bot, sm[top + top * ld], sm[upper_at(top, bot, ld)], sm[bot + bot * ld]);
+  }
+  int cur = 0, round = 0;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    // converged when the off-diagonal part is at rounding of the whole, or no
+    // pair is coupled any more (which a sweep without a rotation would show)
+    if (tid == 0) open = 0;
+    const double* Wc = sm + cur * half;
     double off = 0.0;
-    for (int t = threadIdx.x; t < l * l; t += blockDim.x) {
-      const int i = t % l, j = t / l;
-      if (i != j) off += W[t] * W[t];
-    }
-    off = block_sum(off, scratch);
-    if (threadIdx.x == 0) {
-      sweep_done = (off <= thresh) ? 1 : 0;
-      rotated = 0;
-    }
+    bool mine = false;
     __syncthreads();
-    if (sweep_done) break;
-    for (int r = 0; r < le - 1; ++r) {
-      // round-robin pairing of round r: position 0 stays, positions 1..le-1
-      // have turned r places (position i holds 1 + (i - 1 - r) mod (le - 1))
-      for (int k = threadIdx.x; k < npair; k += blockDim.x) {
-        const int ik = le - 1 - k;
-        int p = k == 0 ? 0 : 1 + ((k - 1 - r) % (le - 1) + (le - 1)) % (le - 1);
-        int q = 1 + ((ik - 1 - r) % (le - 1) + (le - 1)) % (le - 1);
-        if (p > q) { const int t = p; p = q; q = t; }
-        pp[k] = p; qq[k] = q;
-        double c = 1.0, s = 0.0;
-        if (q < l) {
-          const double apq = W[p + (size_t)q * l];
-          const double app = W[p + (size_t)p * l];
-          const double aqq = W[q + (size_t)q * l];
-          // a rotation is skipped once the pair is decoupled to rounding
-          if (apq != 0.0 && fabs(apq) > 1e-300 && fabs(apq) > kEps * sqrt(fabs(app * aqq))) {
-            const double tau = (aqq - app) / (2.0 * apq);
-            const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-            c = 1.0 / sqrt(1.0 + t * t);
-            s = t * c;
-            rotated = 1;
+    for (int t = tid; t < l * l; t += nt) {
+      const int i = t % l, j = t / l;
+      if (i < j) {
+        const double w = Wc[i + j * ld];
+        off += 2.0 * w * w;
+        mine = mine || coupled(Wc[i + i * ld], w, Wc[j + j * ld]);
+      }
+    }
+    if (mine) open = 1;
+    off = block_sum(off, scratch);
+    if (off <= thresh || !open) break;
+    for (int r = 0; r < le - 1; ++r, ++round) {
+      const double* W = sm + cur * half;
+      double* Wn = sm + (cur ^ 1) * half;
+      const Rot* rc = rots + cur * npair;
+      if (angles) {
+        const Rot rA = rc[A], rB = rc[B];
+        double waa[4], wab[4], wbb[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          waa[e] = W[faa[e]];
+          wab[e] = W[fab[e]];
+          wbb[e] = W[fbb[e]];
+        }
+        if (k != 0) top = ring_prev(top, le);
+        bot = ring_prev(bot, le);
+        rots[(cur ^ 1) * npair + k] = decouple(top > bot, rotated_at(waa, rA, a_top, rA, a_top),
+                                               rotated_at(wab, rA, a_top, rB, b_top),
+                                               rotated_at(wbb, rB, b_top, rB, b_top));
+        log[(size_t)round * npair + k] = make_double2(rc[k].c, rc[k].s);
+      }
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        if (pa[u] < 0) continue;
+        const Rot ra = rc[pa[u]], rb = rc[pb[u]];
+        const double w00 = W[from[u][0]], w01 = W[from[u][1]], w10 = W[from[u][2]], w11 = W[from[u][3]];
+        const double r00 = ra.c * w00 - ra.s * w10, r01 = ra.c * w01 - ra.s * w11;
+        const double r10 = ra.s * w00 + ra.c * w10, r11 = ra.s * w01 + ra.c * w11;
+        Wn[to[u][0]] = rb.c * r00 - rb.s * r01;
+        Wn[to[u][1]] = rb.s * r00 + rb.c * r01;
+        if (pa[u] != pb[u]) Wn[to[u][2]] = rb.c * r10 - rb.s * r11;
+        Wn[to[u][3]] = rb.s * r10 + rb.c * r11;
+      }
+      cur ^= 1;
+      __syncthreads();
+    }
+  }
+  // a whole number of sweeps: every position holds its own index again
+  if (tid == 0) *rounds_out = round;
+  const double* Wc = sm + cur * half;
+  for (int i = tid; i < l; i += nt) {
+    const double ev = Wc[i + i * ld], v = isnan(ev) ? -INFINITY : ev;
+    int rank = 0;
+    for (int j = 0; j < l; ++j) {
+      const double wj = Wc[j + j * ld], w = isnan(wj) ? -INFINITY : wj;
+      rank += (w > v) || (w == v && j < i);
+    }
+    rank_of[i] = rank;
+    evals[rank] = ev;
+  }
+}
+
+// Row i of V = e_i through the logged rotations, written in the eigenvalues'
+// order.  One warp a row (lane = pair, and pair + 32), the row in shared
+// memory, kStage rounds of angles loaded ahead: bound by the latency of one
+// round's shared-memory update, for all rows at once.
+constexpr int kApplyWarps = 4;
+template <int PP>   // pairs per lane
+__global__ void __launch_bounds__(32 * kApplyWarps)
+jacobi_apply_log_kernel(int l, const double2* __restrict__ log, const int* __restrict__ rounds,
+                        const int* __restrict__ rank_of, double* __restrict__ V, int ldv) {
+  __shared__ double rows[kApplyWarps][kEigMax + 2];
+  constexpr int kStage = 16 / PP;
+  const int le = l + (l & 1), npair = le / 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kApplyWarps + warp;
+  if (i >= l) return;   // whole warps; no block-wide barrier below
+  double* row = rows[warp];
+  for (int j = lane; j < le; j += 32) row[j] = j == i ? 1.0 : 0.0;
+  __syncwarp();
+  int top[PP], bot[PP];
+#pragma unroll
+  for (int u = 0; u < PP; ++u) {
+    const int k = lane + 32 * u;
+    top[u] = k;
+    bot[u] = le - 1 - k;
+  }
+  const int R = *rounds;
+  double2 now[kStage][PP], next[kStage][PP];
+  auto fetch = [&](int r0, double2 (&d)[kStage][PP]) {
+#pragma unroll
+    for (int g = 0; g < kStage; ++g)
+#pragma unroll
+      for (int u = 0; u < PP; ++u) {
+        const int k = lane + 32 * u;
+        d[g][u] = (r0 + g < R && k < npair) ? __ldg(log + (size_t)(r0 + g) * npair + k) : make_double2(1.0, 0.0);
+      }
+  };
+  fetch(0, now);
+  for (int r0 = 0; r0 < R; r0 += kStage) {
+    fetch(r0 + kStage, next);
+#pragma unroll
+    for (int g = 0; g < kStage; ++g) {
+      if (r0 + g < R) {
+#pragma unroll
+        for (int u = 0; u < PP; ++u) {
+          if (lane + 32 * u < npair) {
+            const double c = now[g][u].x, s = now[g][u].y;
+            const double x = row[top[u]], y = row[bot[u]];
+            row[top[u]] = c * x - s * y;
+            row[bot[u]] = s * x + c * y;
+            if (lane + 32 * u != 0) top[u] = ring_prev(top[u], le);
+            bot[u] = ring_prev(bot[u], le);
           }
         }
-        cs[k] = c; sn[k] = s;
+        __syncwarp();
       }
-      __syncthreads();
-      if (npair <= 32) {
-        // lane = pair, warps stride over the rows / columns (no index division)
-        const int k = threadIdx.x & 31, w0 = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        const bool act = k < npair && qq[k] < l && sn[k] != 0.0;
-        const int p = act ? pp[k] : 0, q = act ? qq[k] : 0;
-        const double c = act ? cs[k] : 1.0, sv = act ? sn[k] : 0.0;
-        // rows: W <- J^T W
-        if (act)
-          for (int j = w0; j < l; j += nw) {
-            const double wp = W[p + j * l], wq = W[q + j * l];
-            W[p + j * l] = c * wp - sv * wq;
-            W[q + j * l] = sv * wp + c * wq;
-          }
-        __syncthreads();
-        // columns: W <- W J, V <- V J
-        if (act)
-          for (int i = w0; i < l; i += nw) {
-            const double wp = W[i + p * l], wq = W[i + q * l];
-            W[i + p * l] = c * wp - sv * wq;
-            W[i + q * l] = sv * wp + c * wq;
-            const double vp = V[i + p * l], vq = V[i + q * l];
-            V[i + p * l] = c * vp - sv * vq;
-            V[i + q * l] = sv * vp + c * vq;
-          }
-        __syncthreads();
-        continue;
-      }
-      // rows: W <- J^T W
-      for (int t = threadIdx.x; t < npair * l; t += blockDim.x) {
-        const int k = t % npair, j = t / npair;
-        const int p = pp[k], q = qq[k];
-        if (q >= l || sn[k] == 0.0) continue;
-        const double c = cs[k], s = sn[k];
-        const double wp = W[p + (size_t)j * l], wq = W[q + (size_t)j * l];
-        W[p + (size_t)j * l] = c * wp - s * wq;
-        W[q + (size_t)j * l] = s * wp + c * wq;
-      }
-      __syncthreads();
-      // columns: W <- W J, V <- V J
-      for (int t = threadIdx.x; t < npair * l; t += blockDim.x) {
-        const int k = t % npair, i = t / npair;
-        const int p = pp[k], q = qq[k];
-        if (q >= l || sn[k] == 0.0) continue;
-        const double c = cs[k], s = sn[k];
-        const double wp = W[i + (size_t)p * l], wq = W[i + (size_t)q * l];
-        W[i + (size_t)p * l] = c * wp - s * wq;
-        W[i + (size_t)q * l] = s * wp + c * wq;
-        const double vp = V[i + (size_t)p * l], vq = V[i + (size_t)q * l];
-        V[i + (size_t)p * l] = c * vp - s * vq;
-        V[i + (size_t)q * l] = s * vp + c * vq;
-      }
-      __syncthreads();
     }
-    if (!rotated) break;   // a whole sweep without a rotation: converged
+#pragma unroll
+    for (int g = 0; g < kStage; ++g)
+#pragma unroll
+      for (int u = 0; u < PP; ++u) now[g][u] = next[g][u];
   }
-  // Sort eigenvalues descending (selection order kept in arr).
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < l; ++i) arr[i] = i;
-    for (int i = 0; i < l; ++i) {
-      int best = i;
-      for (int j = i + 1; j < l; ++j)
-        if (W[arr[j] + (size_t)arr[j] * l] > W[arr[best] + (size_t)arr[best] * l]) best = j;
-      const int t = arr[i]; arr[i] = arr[best]; arr[best] = t;
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < l; i += blockDim.x) evals_out[i] = W[arr[i] + (size_t)arr[i] * l];
-  for (long long t = threadIdx.x; t < (long long)l * l; t += blockDim.x) {
-    const int i = static_cast<int>(t % l), j = static_cast<int>(t / l);
-    V_out[i + (size_t)j * ldv] = V[i + (size_t)arr[j] * l];
-  }
+  for (int j = lane; j < l; j += 32) V[i + (size_t)rank_of[j] * ldv] = row[j];
 }
 
 // ---------------------------------------------------------- one-sided Jacobi ---
@@ -515,24 +658,37 @@ void qr_orthonormalize(int rows, int cols, const double* Y, int ldy, double* Q, 
   cgs2_orthonormalize(rows, cols, Y, ldy, Q, ldq);
 }
 
+bool eig_sym_fits(int l) { return l <= kEigMax; }
+
 void eig_sym_desc(int l, const double* G, int ldg, double* evals, double* V, int ldv) {
   if (l <= 0) return;
+  FPLS_REQUIRE(eig_sym_fits(l), "eig_sym_desc: the matrix does not fit in shared memory");
   Context& ctx = Context::get();
-  double* W = ctx.arena.alloc_n<double>((size_t)l * l);
-  double* Vw = ctx.arena.alloc_n<double>((size_t)l * l);
-  copy_matrix(W, l, G, ldg, l, l);
-  const int npair = (l + 1) / 2;
-  const size_t tables = (size_t)npair * 2 * sizeof(double) + (size_t)(2 * npair + 2 * npair) * sizeof(int);
-  const size_t with_mats = tables + 2 * (size_t)l * l * sizeof(double) + 64;
-  constexpr size_t kEigSmemMax = 200 * 1024;
-  const bool in_smem = with_mats <= kEigSmemMax;
+  const int le = l + (l & 1), npair = le / 2;
+  const size_t smem = 2 * (size_t)le * le * sizeof(double) + 2 * (size_t)npair * sizeof(Rot);
+  // whole groups of four warps (one of each scheduler); the warp pair 0 and 4
+  // is there from 65 on
+  const int groups = std::min(kEigWarps / 4, std::max(npair > 32 ? 2 : 1, ceil_div(eig_blocks(npair), 96)));
+  const int blocks = ceil_div(eig_blocks(npair), 96 * groups);
+  auto kernel = blocks == 1 ? jacobi_eig_kernel<1> : blocks == 2 ? jacobi_eig_kernel<2> : jacobi_eig_kernel<kEigBlocks>;
   static bool attr_set = false;
   if (!attr_set) {
-    FPLS_CUDA(cudaFuncSetAttribute(jacobi_eig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEigSmemMax));
+    FPLS_CUDA(cudaFuncSetAttribute(jacobi_eig_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    FPLS_CUDA(cudaFuncSetAttribute(jacobi_eig_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    FPLS_CUDA(cudaFuncSetAttribute(jacobi_eig_kernel<kEigBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     attr_set = true;
   }
-  const size_t smem = in_smem ? with_mats : tables + 64;
-  jacobi_eig_kernel<<<1, 1024, smem, ctx.stream>>>(l, W, Vw, evals, V, ldv, 60, in_smem ? 1 : 0);
+  double2* log = ctx.arena.alloc_n<double2>((size_t)kEigSweeps * (le - 1) * npair);
+  int* rank_of = ctx.arena.alloc_n<int>(l + 1);
+  int* rounds = rank_of + l;
+  kernel<<<1, 128 * groups, smem, ctx.stream>>>(l, G, ldg, evals, rank_of, log, rounds, kEigSweeps);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+  const int grid = ceil_div(l, kApplyWarps);
+  if (npair <= 32)
+    jacobi_apply_log_kernel<1><<<grid, 32 * kApplyWarps, 0, ctx.stream>>>(l, log, rounds, rank_of, V, ldv);
+  else
+    jacobi_apply_log_kernel<2><<<grid, 32 * kApplyWarps, 0, ctx.stream>>>(l, log, rounds, rank_of, V, ldv);
   ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }

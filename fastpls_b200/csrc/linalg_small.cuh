@@ -21,12 +21,14 @@ void spd_solve(int k, const double* G, int ldg, int nrhs, const double* B, int l
 // Q equals that of Householder QR; column signs follow R_jj > 0.
 void qr_orthonormalize(int rows, int cols, const double* Y, int ldy, double* Q, int ldq);
 
-// Symmetric eigen-decomposition (cyclic Jacobi), eigenvalues in descending
-// order.  G (l x l) is read only; evals[l], V (l x l).
+// Symmetric eigen-decomposition (cyclic Jacobi on one CTA), eigenvalues in
+// descending order.  G (l x l) is read only; evals[l], V (l x l).  l up to
+// what fits in shared memory (eig_sym_fits).
+bool eig_sym_fits(int l);
 void eig_sym_desc(int l, const double* G, int ldg, double* evals, double* V, int ldv);
 
 // Eigen-decomposition of a symmetric positive semi-definite G (l x l),
-// eigenvalues descending: the single-CTA Jacobi for small l, else the
+// eigenvalues descending: the single-CTA Jacobi where it fits, else the
 // whole-GPU one-sided Jacobi SVD of G (singular values = eigenvalues).
 void eig_psd_desc(int l, const double* G, int ldg, double* evals, double* V, int ldv);
 

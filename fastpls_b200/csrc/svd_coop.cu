@@ -326,7 +326,7 @@ void svd_jacobi_coop(int rows, int cols, const double* A, int lda, double* U, in
 }
 
 void eig_psd_desc(int l, const double* G, int ldg, double* evals, double* V, int ldv) {
-  if (l <= 64) {
+  if (eig_sym_fits(l)) {
     eig_sym_desc(l, G, ldg, evals, V, ldv);
     return;
   }
