@@ -3,6 +3,7 @@
 #include "linalg_small.cuh"
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 namespace fpls {
@@ -37,51 +38,13 @@ __device__ void chol_lower_inplace(double* A, int k, int lda, int* ok) {
   __syncthreads();
 }
 
-__global__ void spd_solve_kernel(int k, const double* __restrict__ G, int ldg, int nrhs,
-                                 const double* __restrict__ B, int ldb, double* __restrict__ X,
-                                 int ldx, double* W, int* d_flag, double ridge_rel) {
-  __shared__ int ok;
-  __shared__ double ridge;
-  __shared__ double scratch[32];
-  // Copy G (+ ridge) into W.
+// X = G^{-1} B by LU with partial pivoting on [G | B] (k x (k + nrhs)) in the
+// global workspace W, for one CTA; raises *d_flag when G is singular.
+__device__ void lu_solve(int k, const double* __restrict__ G, int ldg, double ridge, int nrhs,
+                         const double* __restrict__ B, int ldb, double* __restrict__ X, int ldx, double* W,
+                         int* d_flag) {
+  __shared__ int piv, ok;
   if (threadIdx.x == 0) ok = 1;
-  double dsum = 0.0;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) dsum += G[i + (size_t)i * ldg];
-  dsum = block_sum(dsum, scratch);
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    if (ridge_rel > 0.0) {
-      r = ridge_rel * dsum / static_cast<double>(k);
-      if (!isfinite(r) || r <= 0.0) r = ridge_rel;
-    }
-    ridge = r;
-  }
-  __syncthreads();
-  for (long long t = threadIdx.x; t < (long long)k * k; t += blockDim.x) {
-    const int i = static_cast<int>(t % k), j = static_cast<int>(t / k);
-    W[i + (size_t)j * k] = G[i + (size_t)j * ldg] + (i == j ? ridge : 0.0);
-  }
-  __syncthreads();
-  chol_lower_inplace(W, k, k, &ok);
-  if (ok) {
-    // Forward and back substitution, one thread per right-hand side.
-    for (int c = threadIdx.x; c < nrhs; c += blockDim.x) {
-      double* x = X + (size_t)c * ldx;
-      const double* b = B + (size_t)c * ldb;
-      for (int i = 0; i < k; ++i) {
-        double s = b[i];
-        for (int l = 0; l < i; ++l) s -= W[i + (size_t)l * k] * x[l];
-        x[i] = s / W[i + (size_t)i * k];
-      }
-      for (int i = k - 1; i >= 0; --i) {
-        double s = x[i];
-        for (int l = i + 1; l < k; ++l) s -= W[l + (size_t)i * k] * x[l];
-        x[i] = s / W[i + (size_t)i * k];
-      }
-    }
-    return;
-  }
-  // LU with partial pivoting on [G | B] (k x (k + nrhs)) in W.
   __syncthreads();
   const int ncol = k + nrhs;
   for (long long t = threadIdx.x; t < (long long)k * ncol; t += blockDim.x) {
@@ -89,7 +52,6 @@ __global__ void spd_solve_kernel(int k, const double* __restrict__ G, int ldg, i
     W[i + (size_t)j * k] = (j < k) ? G[i + (size_t)j * ldg] + (i == j ? ridge : 0.0)
                                    : B[i + (size_t)(j - k) * ldb];
   }
-  __shared__ int piv;
   for (int j = 0; j < k; ++j) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -136,33 +98,238 @@ __global__ void spd_solve_kernel(int k, const double* __restrict__ G, int ldg, i
   }
 }
 
-// --------------------------------------------------------------- CholeskyQR ---
-// Upper Cholesky of the Gram in place (G = R^T R stored in the upper triangle).
-__global__ void chol_upper_kernel(double* G, int k, int* d_flag) {
-  __shared__ int ok;
-  if (threadIdx.x == 0) ok = 1;
-  __syncthreads();
-  // Lower Cholesky of G equals the transpose of the upper factor.
-  chol_lower_inplace(G, k, k, &ok);
-  if (!ok && threadIdx.x == 0) atomicExch(d_flag, 1);
+// ridge_rel mean(diag G) (ridge_rel itself when that is not a positive number).
+__device__ double ridge_of(int k, const double* __restrict__ G, int ldg, double ridge_rel) {
+  __shared__ double scratch[32];
+  if (!(ridge_rel > 0.0)) return 0.0;
+  double dsum = 0.0;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) dsum += G[i + (size_t)i * ldg];
+  dsum = block_sum(dsum, scratch);
+  const double r = ridge_rel * dsum / static_cast<double>(k);
+  return (!isfinite(r) || r <= 0.0) ? ridge_rel : r;
 }
 
-// Q[i, :] = Y[i, :] * R^{-1}, R upper given as L^T (lower factor L in G).
-__global__ void trsm_rows_kernel(int rows, int k, const double* __restrict__ Y, int ldy,
-                                 const double* __restrict__ L, double* __restrict__ Q, int ldq) {
-  extern __shared__ double Ls[];
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) Ls[t] = L[t];
+// Systems too large for shared memory: one CTA, the factor in global memory.
+__global__ void spd_solve_large_kernel(int k, const double* __restrict__ G, int ldg, int nrhs,
+                                       const double* __restrict__ B, int ldb, double* __restrict__ X,
+                                       int ldx, double* W, int* d_flag, double ridge_rel) {
+  __shared__ int ok;
+  if (threadIdx.x == 0) ok = 1;
+  const double ridge = ridge_of(k, G, ldg, ridge_rel);
+  for (long long t = threadIdx.x; t < (long long)k * k; t += blockDim.x) {
+    const int i = static_cast<int>(t % k), j = static_cast<int>(t / k);
+    W[i + (size_t)j * k] = G[i + (size_t)j * ldg] + (i == j ? ridge : 0.0);
+  }
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows) return;
-  // Row solve: q_j = (y_j - sum_{l<j} q_l R[l][j]) / R[j][j], R[l][j] = L[j][l].
-  for (int j = 0; j < k; ++j) {
-    double s = Y[i + (size_t)j * ldy];
-    for (int l = 0; l < j; ++l) s -= Q[i + (size_t)l * ldq] * Ls[j + l * k];
-    Q[i + (size_t)j * ldq] = s / Ls[j + j * k];
+  chol_lower_inplace(W, k, k, &ok);
+  if (!ok) {
+    __syncthreads();
+    lu_solve(k, G, ldg, ridge, nrhs, B, ldb, X, ldx, W, d_flag);
+    return;
+  }
+  // Forward and back substitution, one thread per right-hand side.
+  for (int c = threadIdx.x; c < nrhs; c += blockDim.x) {
+    double* x = X + (size_t)c * ldx;
+    const double* b = B + (size_t)c * ldb;
+    for (int i = 0; i < k; ++i) {
+      double s = b[i];
+      for (int l = 0; l < i; ++l) s -= W[i + (size_t)l * k] * x[l];
+      x[i] = s / W[i + (size_t)i * k];
+    }
+    for (int i = k - 1; i >= 0; --i) {
+      double s = x[i];
+      for (int l = i + 1; l < k; ++l) s -= W[l + (size_t)i * k] * x[l];
+      x[i] = s / W[i + (size_t)i * k];
+    }
   }
 }
 
+// ---- Cholesky factor and triangular solves in shared memory (k <= kCholMax) ---
+// The factor is held column-major with an odd leading dimension of at least
+// 8 NR (zero rows below k); eight lanes share one right-hand side, lane g with
+// its entries g, g + 8, ... in NR registers, so a solved entry reaches the
+// others by one shuffle and the update needs no barrier.  Every CTA factors
+// its own copy (a few us, bound by the chain of k pivots) and then takes 64
+// right-hand sides at a time: one launch instead of a factor launch and a solve
+// launch, and no CTA waits for another.
+constexpr int kCholMax = 160;
+constexpr int kCholThreads = 512;
+constexpr int kCholGroups = kCholThreads / 8;
+constexpr int chol_ld(int nr) { return 8 * nr + 1; }
+constexpr size_t chol_smem(int nr) { return (size_t)(8 * nr) * (chol_ld(nr) + 1) * sizeof(double); }
+
+// Up to 16 columns (NR = 2) the factor takes roots and divisions in the order
+// of the plain right-looking loop, as it always did: the OPLS filter's
+// subspace iteration runs on eight columns, and the split-precision products
+// behind it turn a different last bit into 1e-5 of the trailing components.
+// Larger ones multiply by reciprocal roots.
+template <int NR>
+constexpr bool kCholDivides = NR <= 2;
+template <int NR>
+__device__ __forceinline__ double over_diag(double v, double d) { return kCholDivides<NR> ? v / d : v * d; }
+
+// Factors G (+ ridge) into L; diag[j] = L[j][j], or its reciprocal where the
+// solves multiply.  False (in every thread) when a pivot is not positive.  The
+// trailing matrix stays in registers (lane = rows lane, lane + 32, ..., warp =
+// columns warp, warp + 16, ...); a column reaches shared memory, scaled by its
+// owning warp, just before it is used, so a column costs one barrier and its
+// chain is barrier, load, multiply-add, shuffle, root.
+template <int NR>
+__device__ bool chol_factor(int k, const double* __restrict__ G, int ldg, double ridge, double* L, double* diag) {
+  constexpr int ld = chol_ld(NR), kWarps = kCholThreads / 32;
+  constexpr int U = (8 * NR + 31) / 32, M = (8 * NR + kWarps - 1) / kWarps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double a[U][M];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int i = lane + 32 * u, c = warp + kWarps * m;
+      a[u][m] = (i < k && c <= i) ? G[i + (size_t)c * ldg] + (i == c ? ridge : 0.0) : 0.0;
+    }
+  for (int j = 0; j < k; ++j) {
+    if (warp == j % kWarps) {
+      const int mj = j / kWarps, uj = j / 32;
+      double v[U], pivot = 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        v[u] = 0.0;
+#pragma unroll
+        for (int m = 0; m < M; ++m) v[u] = m == mj ? a[u][m] : v[u];
+        pivot = u == uj ? v[u] : pivot;
+      }
+      pivot = __shfl_sync(0xffffffffu, pivot, j & 31);
+      const bool good = pivot > 0.0 && isfinite(pivot);
+      const double d = !good ? -1.0 : kCholDivides<NR> ? sqrt(pivot) : rsqrt(pivot);
+      if (lane == 0) diag[j] = d;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = lane + 32 * u;
+        if (i < 8 * NR) L[i + j * ld] = i > j ? over_diag<NR>(v[u], d) : 0.0;
+      }
+    }
+    __syncthreads();
+    if (diag[j] < 0.0) return false;
+    double f[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) f[m] = warp + kWarps * m < 8 * NR ? L[warp + kWarps * m + j * ld] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double li = lane + 32 * u < 8 * NR ? L[lane + 32 * u + j * ld] : 0.0;
+#pragma unroll
+      for (int m = 0; m < M; ++m) a[u][m] -= li * f[m];
+    }
+  }
+  return true;
+}
+
+// y <- L^{-1} y for the group's right-hand side.
+template <int NR>
+__device__ __forceinline__ void solve_lower(double (&y)[NR], int k, int g, const double* L, const double* diag) {
+  constexpr int ld = chol_ld(NR);
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    if (8 * r >= k) break;
+#pragma unroll 2
+    for (int jl = 0; jl < 8; ++jl) {
+      const int j = 8 * r + jl;
+      if (j >= k) break;
+      const double q = __shfl_sync(0xffffffffu, over_diag<NR>(y[r], diag[j]), jl, 8);
+      const double* col = L + g + j * ld;
+      y[r] = g == jl ? q : g > jl ? y[r] - col[8 * r] * q : y[r];
+#pragma unroll
+      for (int u = r + 1; u < NR; ++u) y[u] -= col[8 * u] * q;
+    }
+  }
+}
+
+// y <- L^{-T} y.
+template <int NR>
+__device__ __forceinline__ void solve_lower_t(double (&y)[NR], int k, int g, const double* L, const double* diag) {
+  constexpr int ld = chol_ld(NR);
+#pragma unroll
+  for (int r = NR - 1; r >= 0; --r) {
+    if (8 * r >= k) continue;
+#pragma unroll 2
+    for (int jl = 7; jl >= 0; --jl) {
+      const int j = 8 * r + jl;
+      if (j >= k) continue;
+      const double q = __shfl_sync(0xffffffffu, over_diag<NR>(y[r], diag[j]), jl, 8);
+      const double* row = L + j + g * ld;
+      y[r] = g == jl ? q : g < jl ? y[r] - row[8 * r * ld] * q : y[r];
+#pragma unroll
+      for (int u = 0; u < r; ++u) y[u] -= row[8 * u * ld] * q;
+    }
+  }
+}
+
+template <int NR>
+__global__ void __launch_bounds__(kCholThreads)
+spd_solve_kernel(int k, const double* __restrict__ G, int ldg, int nrhs, const double* __restrict__ B, int ldb,
+                 double* __restrict__ X, int ldx, double* W, int* d_flag, double ridge_rel) {
+  extern __shared__ double L[];
+  double* diag = L + 8 * NR * chol_ld(NR);
+  const double ridge = ridge_of(k, G, ldg, ridge_rel);
+  if (!chol_factor<NR>(k, G, ldg, ridge, L, diag)) {
+    if (blockIdx.x == 0) lu_solve(k, G, ldg, ridge, nrhs, B, ldb, X, ldx, W, d_flag);
+    return;
+  }
+  const int g = threadIdx.x & 7, group = threadIdx.x >> 3;
+  for (int c0 = blockIdx.x * kCholGroups; c0 < nrhs; c0 += gridDim.x * kCholGroups) {
+    const int c = c0 + group;
+    double y[NR];
+#pragma unroll
+    for (int u = 0; u < NR; ++u) y[u] = (c < nrhs && g + 8 * u < k) ? B[g + 8 * u + (size_t)c * ldb] : 0.0;
+    solve_lower<NR>(y, k, g, L, diag);
+    solve_lower_t<NR>(y, k, g, L, diag);
+#pragma unroll
+    for (int u = 0; u < NR; ++u)
+      if (c < nrhs && g + 8 * u < k) X[g + 8 * u + (size_t)c * ldx] = y[u];
+  }
+}
+
+// One CholeskyQR pass: Q = Y R^{-1} with G = Y^T Y = R^T R (each row of Q solves
+// R^T q = y).  Raises *d_flag when G is not positive definite.
+template <int NR>
+__global__ void __launch_bounds__(kCholThreads)
+chol_qr_kernel(int k, const double* __restrict__ G, int rows, const double* Y, int ldy, double* Q, int ldq,
+               int* d_flag) {
+  extern __shared__ double L[];
+  double* diag = L + 8 * NR * chol_ld(NR);
+  if (!chol_factor<NR>(k, G, k, 0.0, L, diag)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(d_flag, 1);
+    return;
+  }
+  const int g = threadIdx.x & 7, group = threadIdx.x >> 3;
+  for (int i0 = blockIdx.x * kCholGroups; i0 < rows; i0 += gridDim.x * kCholGroups) {
+    const int i = i0 + group;
+    double y[NR];
+#pragma unroll
+    for (int u = 0; u < NR; ++u) y[u] = (i < rows && g + 8 * u < k) ? Y[i + (size_t)(g + 8 * u) * ldy] : 0.0;
+    solve_lower<NR>(y, k, g, L, diag);
+#pragma unroll
+    for (int u = 0; u < NR; ++u)
+      if (i < rows && g + 8 * u < k) Q[i + (size_t)(g + 8 * u) * ldq] = y[u];
+  }
+}
+
+// The register count of a size: f(std::integral_constant<int, NR>).
+template <typename F>
+void with_chol_size(int k, F&& f) {
+  if (k <= 16) f(std::integral_constant<int, 2>{});
+  else if (k <= 32) f(std::integral_constant<int, 4>{});
+  else if (k <= 64) f(std::integral_constant<int, 8>{});
+  else if (k <= 104) f(std::integral_constant<int, 13>{});
+  else if (k <= 128) f(std::integral_constant<int, 16>{});
+  else f(std::integral_constant<int, 20>{});
+}
+
+template <typename K>
+void allow_smem(K kernel, size_t bytes) {
+  FPLS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+}
+
+// ------------------------------------------------- Gram-Schmidt fallback ---
 __global__ void normalize_col_kernel(double* q, int rows, const double* nrm2) {
   const double nr = sqrt(*nrm2);
   const double inv = (nr > 0.0 && isfinite(nr)) ? 1.0 / nr : 0.0;
@@ -184,6 +351,120 @@ __device__ void round_robin_next(int* arr, int n) {
   const int last = arr[n - 1];
   for (int i = n - 1; i > 1; --i) arr[i] = arr[i - 1];
   arr[1] = last;
+}
+
+// Up to kEigTiny the rotations are applied in place, rows then columns, V along
+// with W.  The OPLS filter takes its leading vectors through 8 x 8 cores of
+// this size; the split-precision products behind it turn a different last bit
+// here into 1e-5 of the trailing components, so this arithmetic stays.
+constexpr int kEigTiny = 16;
+__global__ void jacobi_eig_tiny_kernel(int l, const double* __restrict__ G, int ldg, double* evals_out,
+                                       double* V_out, int ldv, const int max_sweeps) {
+  extern __shared__ double sm[];
+  const int npair = (l + 1) / 2;
+  const int le = 2 * npair;
+  double* cs = sm;              // [npair] cos
+  double* sn = sm + npair;      // [npair] sin
+  int* arr = reinterpret_cast<int*>(sm + 2 * npair);   // [le]
+  int* pp = arr + le;           // [npair]
+  int* qq = pp + npair;         // [npair]
+  __shared__ double scratch[32];
+  __shared__ int sweep_done;
+  double* W = sm + 4 * npair;
+  double* V = W + (size_t)l * l;
+  for (int t = threadIdx.x; t < l * l; t += blockDim.x) W[t] = G[t % l + (size_t)(t / l) * ldg];
+  for (int t = threadIdx.x; t < l * l; t += blockDim.x) V[t] = (t % l == t / l) ? 1.0 : 0.0;
+  __shared__ int rotated;
+  __syncthreads();
+  // Frobenius norm for the convergence test.
+  double fro = 0.0;
+  for (int t = threadIdx.x; t < l * l; t += blockDim.x) fro += W[t] * W[t];
+  fro = block_sum(fro, scratch);
+  const double thresh = kEps * kEps * fro;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    double off = 0.0;
+    for (int t = threadIdx.x; t < l * l; t += blockDim.x) {
+      const int i = t % l, j = t / l;
+      if (i != j) off += W[t] * W[t];
+    }
+    off = block_sum(off, scratch);
+    if (threadIdx.x == 0) {
+      sweep_done = (off <= thresh) ? 1 : 0;
+      rotated = 0;
+    }
+    __syncthreads();
+    if (sweep_done) break;
+    for (int r = 0; r < le - 1; ++r) {
+      // round-robin pairing of round r: position 0 stays, positions 1..le-1
+      // have turned r places (position i holds 1 + (i - 1 - r) mod (le - 1))
+      for (int k = threadIdx.x; k < npair; k += blockDim.x) {
+        const int ik = le - 1 - k;
+        int p = k == 0 ? 0 : 1 + ((k - 1 - r) % (le - 1) + (le - 1)) % (le - 1);
+        int q = 1 + ((ik - 1 - r) % (le - 1) + (le - 1)) % (le - 1);
+        if (p > q) { const int t = p; p = q; q = t; }
+        pp[k] = p; qq[k] = q;
+        double c = 1.0, s = 0.0;
+        if (q < l) {
+          const double apq = W[p + (size_t)q * l];
+          const double app = W[p + (size_t)p * l];
+          const double aqq = W[q + (size_t)q * l];
+          // a rotation is skipped once the pair is decoupled to rounding
+          if (apq != 0.0 && fabs(apq) > 1e-300 && fabs(apq) > kEps * sqrt(fabs(app * aqq))) {
+            const double tau = (aqq - app) / (2.0 * apq);
+            const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+            c = 1.0 / sqrt(1.0 + t * t);
+            s = t * c;
+            rotated = 1;
+          }
+        }
+        cs[k] = c; sn[k] = s;
+      }
+      __syncthreads();
+      {
+        // lane = pair, warps stride over the rows / columns (no index division)
+        const int k = threadIdx.x & 31, w0 = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        const bool act = k < npair && qq[k] < l && sn[k] != 0.0;
+        const int p = act ? pp[k] : 0, q = act ? qq[k] : 0;
+        const double c = act ? cs[k] : 1.0, sv = act ? sn[k] : 0.0;
+        // rows: W <- J^T W
+        if (act)
+          for (int j = w0; j < l; j += nw) {
+            const double wp = W[p + j * l], wq = W[q + j * l];
+            W[p + j * l] = c * wp - sv * wq;
+            W[q + j * l] = sv * wp + c * wq;
+          }
+        __syncthreads();
+        // columns: W <- W J, V <- V J
+        if (act)
+          for (int i = w0; i < l; i += nw) {
+            const double wp = W[i + p * l], wq = W[i + q * l];
+            W[i + p * l] = c * wp - sv * wq;
+            W[i + q * l] = sv * wp + c * wq;
+            const double vp = V[i + p * l], vq = V[i + q * l];
+            V[i + p * l] = c * vp - sv * vq;
+            V[i + q * l] = sv * vp + c * vq;
+          }
+        __syncthreads();
+      }
+    }
+    if (!rotated) break;   // a whole sweep without a rotation: converged
+  }
+  // Sort eigenvalues descending (selection order kept in arr).
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < l; ++i) arr[i] = i;
+    for (int i = 0; i < l; ++i) {
+      int best = i;
+      for (int j = i + 1; j < l; ++j)
+        if (W[arr[j] + (size_t)arr[j] * l] > W[arr[best] + (size_t)arr[best] * l]) best = j;
+      const int t = arr[i]; arr[i] = arr[best]; arr[best] = t;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < l; i += blockDim.x) evals_out[i] = W[arr[i] + (size_t)arr[i] * l];
+  for (long long t = threadIdx.x; t < (long long)l * l; t += blockDim.x) {
+    const int i = static_cast<int>(t % l), j = static_cast<int>(t / l);
+    V_out[i + (size_t)j * ldv] = V[i + (size_t)arr[j] * l];
+  }
 }
 
 // Cyclic two-sided Jacobi on one CTA, for l <= kEigMax.  What bounds it is the
@@ -603,9 +884,21 @@ void spd_solve(int k, const double* G, int ldg, int nrhs, const double* B, int l
                int ldx, int* d_flag, double ridge_rel) {
   if (k <= 0 || nrhs <= 0) return;
   Context& ctx = Context::get();
-  double* W = ctx.arena.alloc_n<double>((size_t)k * (k + nrhs));
-  spd_solve_kernel<<<1, 512, 0, ctx.stream>>>(k, G, ldg, nrhs, B, ldb, X, ldx, W,
-                                              d_flag ? d_flag : ctx.d_status + 1, ridge_rel); ::fpls::note_launch();
+  double* W = ctx.arena.alloc_n<double>((size_t)k * (k + nrhs));   // the factor, or the LU fallback's
+  int* flag = d_flag ? d_flag : ctx.d_status + 1;
+  if (k > kCholMax) {
+    spd_solve_large_kernel<<<1, 512, 0, ctx.stream>>>(k, G, ldg, nrhs, B, ldb, X, ldx, W, flag, ridge_rel);
+  } else {
+    const int grid = std::min(ceil_div(nrhs, kCholGroups), 2 * ctx.sm_count);
+    with_chol_size(k, [&](auto nr) {
+      constexpr int NR = decltype(nr)::value;
+      static const bool once = (allow_smem(spd_solve_kernel<NR>, chol_smem(NR)), true);
+      (void)once;
+      spd_solve_kernel<NR><<<grid, kCholThreads, chol_smem(NR), ctx.stream>>>(k, G, ldg, nrhs, B, ldb, X, ldx, W,
+                                                                              flag, ridge_rel);
+    });
+  }
+  ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 
@@ -634,18 +927,17 @@ void qr_orthonormalize(int rows, int cols, const double* Y, int ldy, double* Q, 
   dzero(flag, sizeof(int));
   const double* src = Y;
   int lds = ldy;
-  const size_t smem = (size_t)cols * cols * sizeof(double);
-  const bool fits = smem <= 200 * 1024;
-  if (fits) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      FPLS_CUDA(cudaFuncSetAttribute(trsm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_set = true;
-    }
+  if (cols <= kCholMax) {
     for (int pass = 0; pass < 2; ++pass) {
       gemm(true, false, cols, cols, rows, 1.0, src, lds, src, lds, 0.0, G, cols);
-      chol_upper_kernel<<<1, 512, 0, ctx.stream>>>(G, cols, flag); ::fpls::note_launch();
-      trsm_rows_kernel<<<ceil_div(rows, 128), 128, smem, ctx.stream>>>(rows, cols, src, lds, G, Q, ldq); ::fpls::note_launch();
+      const int grid = std::min(ceil_div(rows, kCholGroups), 2 * ctx.sm_count);
+      with_chol_size(cols, [&](auto nr) {
+        constexpr int NR = decltype(nr)::value;
+        static const bool once = (allow_smem(chol_qr_kernel<NR>, chol_smem(NR)), true);
+        (void)once;
+        chol_qr_kernel<NR><<<grid, kCholThreads, chol_smem(NR), ctx.stream>>>(cols, G, rows, src, lds, Q, ldq, flag);
+      });
+      ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
       src = Q;
       lds = ldq;
@@ -664,6 +956,13 @@ void eig_sym_desc(int l, const double* G, int ldg, double* evals, double* V, int
   if (l <= 0) return;
   FPLS_REQUIRE(eig_sym_fits(l), "eig_sym_desc: the matrix does not fit in shared memory");
   Context& ctx = Context::get();
+  if (l <= kEigTiny) {
+    const size_t smem = (2 * (size_t)l * l + 4 * (size_t)((l + 1) / 2)) * sizeof(double);
+    jacobi_eig_tiny_kernel<<<1, 64, smem, ctx.stream>>>(l, G, ldg, evals, V, ldv, kEigSweeps);
+    ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
+    return;
+  }
   const int le = l + (l & 1), npair = le / 2;
   const size_t smem = 2 * (size_t)le * le * sizeof(double) + 2 * (size_t)npair * sizeof(Rot);
   // whole groups of four warps (one of each scheduler); the warp pair 0 and 4

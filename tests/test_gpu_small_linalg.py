@@ -37,3 +37,35 @@ def test_randomized_svd_core_sizes(lib, k):
     approx = (got["u"] * got["d"]) @ got["vt"]
     want = (ref.U * ref.s) @ ref.Vt
     assert np.linalg.norm(approx - want) <= 1000 * tol * np.linalg.norm(want)
+
+
+# Cholesky solves: the lane groups' register counts change at 32, 64, 104, 128
+# and 160 unknowns (161: the global-memory kernel); 64 right-hand sides a CTA pass
+@pytest.mark.parametrize("d,q", [(1, 5), (7, 63), (8, 64), (16, 65), (17, 66), (32, 129), (33, 129), (64, 200), (65, 200),
+                                 (104, 300), (105, 300), (128, 330), (129, 330), (160, 400), (161, 400)])
+def test_spd_solve_sizes(lib, d, q):
+    from oracle import gaussian_y as ogy
+    rng = np.random.default_rng(d)
+    Y = rng.standard_normal((450, q))
+    G = rng.standard_normal((q, d)) / np.sqrt(d)
+    got = lib.gaussian_y_encode(Y, G)
+    ref = ogy.prepare_regression(Y, G)
+    # condition of Z^T Z below 1e5 at every size: rounding 1e-16 stays below 1e-9
+    assert np.linalg.norm(got["Z"] - ref["Z"]) < 1e-9 * np.linalg.norm(ref["Z"])
+    assert np.linalg.norm(got["decoder"] - ref["decoder"]) < 1e-9 * np.linalg.norm(ref["decoder"])
+
+
+# CholeskyQR2 at the same register counts (l = k + 10 columns; 161: Gram-Schmidt)
+# and around whole groups of 64 rows
+@pytest.mark.parametrize("rows,l", [(90, 16), (91, 17), (127, 22), (128, 32), (129, 33), (300, 64), (301, 65), (320, 104), (321, 105),
+                                    (400, 128), (401, 129), (449, 160), (450, 161)])
+def test_cholesky_qr_sizes(lib, rows, l):
+    k, cols = l - 10, min(rows, l + 40)
+    A = _matrix(rows, cols, l, 0.98)
+    got = lib.truncated_svd(A, k, svd_method=4, oversample=10, power_iters=1, seed=5)
+    assert np.linalg.norm(got["u"].T @ got["u"] - np.eye(k)) < 1000 * EPS * k
+    ref = osvd.truncated_svd(A, k, svd_method=4, oversample=10, power_iters=1, seed=5)
+    # one power iteration cubes the decay: the sample's smallest direction is
+    # 0.98^(3 l) of the largest, which is how far rounding is amplified
+    tol = 1000 * EPS / 0.98 ** (3 * l)
+    assert np.max(np.abs(got["d"] - ref.s)) <= tol * ref.s[0]
