@@ -346,13 +346,6 @@ __global__ void dot_self_kernel(const double* x, int n, double* out) {
 }
 
 // ------------------------------------------------------------- Jacobi eigen ---
-__device__ void round_robin_next(int* arr, int n) {
-  // keep arr[0]; rotate arr[1..n-1] right by one
-  const int last = arr[n - 1];
-  for (int i = n - 1; i > 1; --i) arr[i] = arr[i - 1];
-  arr[1] = last;
-}
-
 // Up to kEigTiny the rotations are applied in place, rows then columns, V along
 // with W.  The OPLS filter takes its leading vectors through 8 x 8 cores of
 // this size; the split-precision products behind it turn a different last bit
@@ -751,27 +744,186 @@ jacobi_apply_log_kernel(int l, const double2* __restrict__ log, const int* __res
 }
 
 // ---------------------------------------------------------- one-sided Jacobi ---
-// W (r x c, r >= c) is overwritten; V (c x c) accumulates the rotations.
-__global__ void jacobi_svd_kernel(int r, int c, double* W, double* V, int max_sweeps,
+// ---- Thin SVD of up to kThinMax columns: QR first, one-sided Jacobi on R ----
+// The rotations of one-sided Jacobi depend on the columns' inner products only,
+// and those of A = Q R are those of R; so A is reduced to its c x c triangle by
+// Householder QR over row blocks (one CTA a block, the blocks' triangles stacked
+// and reduced again), the sweeps run on R, and U = A V / s is one product.
+// A sweep over A itself moves its columns three times through shared (or global)
+// memory: 375 x 22 took 340 us that way, 5000 x 22 several ms.
+constexpr int kThinMax = 96;
+
+// R (c x c, upper) of rows [b rb, b rb + rb) of A into rows [b c, b c + c) of
+// out.  Every warp works out the reflector of a column for itself and applies it
+// to its own columns, so a column costs one barrier.
+__global__ void __launch_bounds__(512) qr_block_kernel(const double* __restrict__ A, int rows, int c, int lda, int rb,
+                                                       double* __restrict__ out, int ldo) {
+  extern __shared__ double sm[];
+  double* X = sm;                       // [rb][c], column-major
+  double* diag = sm + (size_t)rb * c;   // [c]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int r0 = blockIdx.x * rb, nr = min(rb, rows - r0), steps = min(c, nr);
+  for (int j = warp; j < c; j += nw)
+    for (int i = lane; i < nr; i += 32) X[i + j * rb] = A[r0 + i + (size_t)j * lda];
+  __syncthreads();
+  for (int j = 0; j < steps; ++j) {
+    const double* x = X + j * rb;
+    double sigma = 0.0;
+    for (int i = j + 1 + lane; i < nr; i += 32) sigma += x[i] * x[i];
+    sigma = warp_sum(sigma);
+    const double alpha = x[j], norm = sqrt(alpha * alpha + sigma);
+    const double beta = alpha >= 0.0 ? -norm : norm, head = alpha - beta;
+    if (threadIdx.x == 0) diag[j] = beta;
+    if (norm > 0.0) {
+      const double inv = 1.0 / (norm * (norm + fabs(alpha)));   // 2 / v.v, v = (head, x below)
+      for (int col = j + 1 + warp; col < c; col += nw) {
+        double* y = X + col * rb;
+        double d = 0.0;
+        for (int i = j + 1 + lane; i < nr; i += 32) d += x[i] * y[i];
+        const double yj = y[j], w = (warp_sum(d) + head * yj) * inv;
+        for (int i = j + 1 + lane; i < nr; i += 32) y[i] -= w * x[i];
+        __syncwarp();
+        if (lane == 0) y[j] = yj - w * head;
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = warp; j < c; j += nw)
+    for (int i = lane; i < c; i += 32) {
+      const double v = i < j ? (i < nr ? X[i + j * rb] : 0.0) : i == j && j < steps ? diag[j] : 0.0;
+      out[blockIdx.x * c + i + (size_t)j * ldo] = v;
+    }
+}
+
+// One-sided Jacobi on R (c x c, column-major), one CTA, one warp a column pair,
+// the pairs turning as in the symmetric solver: singular values and V,
+// descending.  A column of R and the one of V below it sit in NE registers a
+// lane each while their rotation is worked out.
+template <int NE>
+__global__ void __launch_bounds__(1024) jacobi_core_kernel(const double* __restrict__ R, int c, int max_sweeps, double null_rel,
+                                                           double* __restrict__ s_out, double* __restrict__ V_out) {
+  extern __shared__ double sm[];
+  double* W = sm;                       // [c][c]
+  double* V = W + c * c;
+  double* norms = V + c * c;
+  __shared__ double scratch[32];
+  __shared__ int rotated;
+  const int npair = (c + 1) / 2, ce = 2 * npair;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  double fro = 0.0;
+  for (int t = threadIdx.x; t < c * c; t += blockDim.x) {
+    const double w = R[t];
+    W[t] = w;
+    V[t] = t % c == t / c ? 1.0 : 0.0;
+    fro += w * w;
+  }
+  // A column below this squared norm is a null direction (U's column is
+  // replaced): its angle to the others is rounding, which no rotation removes,
+  // so a rank-deficient matrix (every centred class response) would never
+  // converge.
+  const double null2 = block_sum(fro, scratch) / c * null_rel * null_rel;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    if (threadIdx.x == 0) rotated = 0;
+    __syncthreads();
+    for (int rr = 0; rr < ce - 1; ++rr) {
+      for (int k = warp; k < npair; k += nw) {
+        const int u = k - 1 - rr, v = ce - 2 - k - rr;   // positions k and ce - 1 - k, turned rr places
+        int p = k == 0 ? 0 : 1 + (u < 0 ? u + ce - 1 : u), q = 1 + (v < 0 ? v + ce - 1 : v);
+        if (p > q) { const int t = p; p = q; q = t; }
+        if (q >= c) continue;
+        double x[NE], y[NE], vx[NE], vy[NE];
+        double a = 0.0, b = 0.0, g = 0.0;
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+          const int i = lane + 32 * e;
+          const bool in = i < c;
+          x[e] = in ? W[i + p * c] : 0.0;
+          y[e] = in ? W[i + q * c] : 0.0;
+          vx[e] = in ? V[i + p * c] : 0.0;
+          vy[e] = in ? V[i + q * c] : 0.0;
+          a += x[e] * x[e];
+          b += y[e] * y[e];
+          g += x[e] * y[e];
+        }
+        a = warp_sum(a); b = warp_sum(b); g = warp_sum(g);
+        if (fmin(a, b) <= null2) continue;
+        const Rot t = decouple(false, a, g, b);
+        if (t.s == 0.0) continue;
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+          const int i = lane + 32 * e;
+          if (i < c) {
+            W[i + p * c] = t.c * x[e] - t.s * y[e];
+            W[i + q * c] = t.s * x[e] + t.c * y[e];
+            V[i + p * c] = t.c * vx[e] - t.s * vy[e];
+            V[i + q * c] = t.s * vx[e] + t.c * vy[e];
+          }
+        }
+        if (lane == 0) rotated = 1;
+      }
+      __syncthreads();
+    }
+    if (!rotated) break;
+    __syncthreads();   // every thread has read the flag before it is cleared
+  }
+  for (int k = warp; k < c; k += nw) {
+    double a = 0.0;
+    for (int i = lane; i < c; i += 32) a += W[i + k * c] * W[i + k * c];
+    a = warp_sum(a);
+    if (lane == 0) norms[k] = sqrt(a);
+  }
+  __syncthreads();
+  for (int k = warp; k < c; k += nw) {   // rank of column k, then its place in the outputs
+    const double v = isnan(norms[k]) ? -INFINITY : norms[k];
+    int rank = 0;
+    for (int j = lane; j < c; j += 32) {
+      const double w = isnan(norms[j]) ? -INFINITY : norms[j];
+      rank += (w > v) || (w == v && j < k);
+    }
+    rank = __reduce_add_sync(0xffffffffu, rank);
+    if (lane == 0) s_out[rank] = norms[k];
+    for (int i = lane; i < c; i += 32) V_out[i + rank * c] = V[i + k * c];
+  }
+}
+
+// U[:, j] /= s[j] where s[j] is no null direction (else zero; completed below).
+__global__ void scale_left_kernel(double* U, int rows, int c, int ldu, const double* __restrict__ s, double tol_rel) {
+  const double tol = tol_rel * s[0];
+  const int j = blockIdx.y;
+  const double sj = s[j];
+  const bool ok = sj > tol && sj > 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+    double* u = U + i + (size_t)j * ldu;
+    *u = ok ? *u / sj : 0.0;
+  }
+}
+
+// More columns than kThinMax: W (r x c, r >= c) is overwritten in global memory,
+// V (c x c) accumulates the rotations; one CTA, one warp a pair.
+__global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* W, double* V, int max_sweeps,
                                   double* U_out, int ldu, double* s_out, double* V_out, int ldv,
                                   int transpose_out) {
   extern __shared__ double sm[];
   const int npair = (c + 1) / 2;
   const int ce = 2 * npair;
-  int* arr = reinterpret_cast<int*>(sm);
-  int* order = arr + ce;
-  double* norms = sm + (2 * ce + 1) / 2 + 1;
+  double* norms = sm;
+  int* order = reinterpret_cast<int*>(sm + c);
   __shared__ int rotated;
+  __shared__ double scratch0[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int t = threadIdx.x; t < c * c; t += blockDim.x) V[t] = (t % c == t / c) ? 1.0 : 0.0;
-  if (threadIdx.x == 0) for (int i = 0; i < ce; ++i) arr[i] = i;
   __syncthreads();
+  double null2 = 0.0;   // as in jacobi_core_kernel
+  for (int j = warp; j < c; j += nwarps)
+    for (int i = lane; i < r; i += 32) null2 += W[i + (size_t)j * r] * W[i + (size_t)j * r];
+  null2 = block_sum(null2, scratch0) / c * (kEps * r) * (kEps * r);
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
     for (int rr = 0; rr < ce - 1; ++rr) {
       for (int k = warp; k < npair; k += nwarps) {
-        int p = arr[k], q = arr[ce - 1 - k];
+        const int u = k - 1 - rr, v = ce - 2 - k - rr;
+        int p = k == 0 ? 0 : 1 + (u < 0 ? u + ce - 1 : u), q = 1 + (v < 0 ? v + ce - 1 : v);
         if (p > q) { const int t = p; p = q; q = t; }
         if (q >= c) continue;
         double* wp = W + (size_t)p * r;
@@ -782,29 +934,26 @@ __global__ void jacobi_svd_kernel(int r, int c, double* W, double* V, int max_sw
           a += x * x; b += y * y; g += x * y;
         }
         a = warp_sum(a); b = warp_sum(b); g = warp_sum(g);
-        if (fabs(g) > kEps * sqrt(a * b) && fabs(g) > 1e-300) {
-          const double zeta = (b - a) / (2.0 * g);
-          const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-          const double cs = 1.0 / sqrt(1.0 + t * t);
-          const double sn = cs * t;
+        if (fmin(a, b) <= null2) continue;
+        const Rot t = decouple(false, a, g, b);
+        if (t.s != 0.0) {
           for (int i = lane; i < r; i += 32) {
             const double x = wp[i], y = wq[i];
-            wp[i] = cs * x - sn * y;
-            wq[i] = sn * x + cs * y;
+            wp[i] = t.c * x - t.s * y;
+            wq[i] = t.s * x + t.c * y;
           }
           for (int i = lane; i < c; i += 32) {
             const double x = V[i + (size_t)p * c], y = V[i + (size_t)q * c];
-            V[i + (size_t)p * c] = cs * x - sn * y;
-            V[i + (size_t)q * c] = sn * x + cs * y;
+            V[i + (size_t)p * c] = t.c * x - t.s * y;
+            V[i + (size_t)q * c] = t.s * x + t.c * y;
           }
           if (lane == 0) rotated = 1;
         }
       }
       __syncthreads();
-      if (threadIdx.x == 0) round_robin_next(arr, ce);
-      __syncthreads();
     }
     if (!rotated) break;
+    __syncthreads();
   }
   // Column norms and descending order.
   for (int k = warp; k < c; k += nwarps) {
@@ -814,13 +963,14 @@ __global__ void jacobi_svd_kernel(int r, int c, double* W, double* V, int max_sw
     if (lane == 0) norms[k] = sqrt(a);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < c; ++i) order[i] = i;
-    for (int i = 0; i < c; ++i) {
-      int best = i;
-      for (int j = i + 1; j < c; ++j) if (norms[order[j]] > norms[order[best]]) best = j;
-      const int t = order[i]; order[i] = order[best]; order[best] = t;
+  for (int i = threadIdx.x; i < c; i += blockDim.x) {
+    const double v = isnan(norms[i]) ? -INFINITY : norms[i];
+    int rank = 0;
+    for (int j = 0; j < c; ++j) {
+      const double w = isnan(norms[j]) ? -INFINITY : norms[j];
+      rank += (w > v) || (w == v && j < i);
     }
+    order[rank] = i;
   }
   __syncthreads();
   const double smax = norms[order[0]];
@@ -992,27 +1142,81 @@ void eig_sym_desc(int l, const double* G, int ldg, double* evals, double* V, int
   FPLS_CHECK_LAUNCH();
 }
 
+namespace {
+
+// R of A (rows x c, lda) by blocks of rows until one block holds it all.
+const double* reduce_to_triangle(const double* A, int rows, int c, int lda) {
+  Context& ctx = Context::get();
+  const int rb_max = std::min(512, static_cast<int>((200 * 1024 / sizeof(double) - c) / c));
+  static const bool once = (allow_smem(qr_block_kernel, 201 * 1024), true);
+  (void)once;
+  while (true) {
+    // blocks of 256 rows (three times the columns, at least) keep the first pass on many SMs
+    const int rb = rows <= rb_max ? rows : std::min(rb_max, std::max(256, 3 * c));
+    const int nb = ceil_div(rows, rb);
+    double* out = ctx.arena.alloc_n<double>((size_t)nb * c * c);
+    const size_t smem = ((size_t)rb * c + c) * sizeof(double);
+    qr_block_kernel<<<nb, 512, smem, ctx.stream>>>(A, rows, c, lda, rb, out, nb * c); ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
+    if (nb == 1) return out;
+    A = out;
+    rows = nb * c;
+    lda = rows;
+  }
+}
+
+}  // namespace
+
 void svd_thin(int rows, int cols, const double* A, int lda, double* U, int ldu, double* s,
-              double* V, int ldv) {
+              double* V, int ldv, int need) {
   if (rows <= 0 || cols <= 0) return;
   Context& ctx = Context::get();
   const bool tall = rows >= cols;
   const int r = tall ? rows : cols;
   const int c = tall ? cols : rows;
-  double* W = ctx.arena.alloc_n<double>((size_t)r * c);
-  double* Vw = ctx.arena.alloc_n<double>((size_t)c * c);
-  if (tall) {
-    copy_matrix(W, r, A, lda, rows, cols);
-  } else {
-    transpose_kernel<<<256, 256, 0, ctx.stream>>>(A, rows, cols, lda, W); ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
+  const double* M = A;   // the tall form, r x c
+  int ldm = lda;
+  double* W = nullptr;
+  if (!tall || c > kThinMax) {
+    W = ctx.arena.alloc_n<double>((size_t)r * c);
+    if (tall) {
+      copy_matrix(W, r, A, lda, rows, cols);
+    } else {
+      transpose_kernel<<<256, 256, 0, ctx.stream>>>(A, rows, cols, lda, W); ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+    }
+    M = W;
+    ldm = r;
   }
-  const int ce = c + (c & 1);
-  const size_t smem = (size_t)(2 * ce + 2) * sizeof(int) + (size_t)(c + 2) * sizeof(double) + 64;
-  // tall: U (rows x c) <- normalised W, V (cols x c) <- rotations.
+  // tall: U (rows x c) is M's side, V (cols x c) the rotations.
   // wide: A^T = U' S V'^T, so U (rows x c) <- V', V (cols x c) <- U'.
-  jacobi_svd_kernel<<<1, 1024, smem, ctx.stream>>>(r, c, W, Vw, 60, U, ldu, s, V, ldv, tall ? 0 : 1); ::fpls::note_launch();
+  if (c > kThinMax) {
+    double* Vw = ctx.arena.alloc_n<double>((size_t)c * c);
+    const size_t lists = (size_t)(c + (c + 1) / 2) * sizeof(double);
+    jacobi_svd_kernel<<<1, 1024, lists, ctx.stream>>>(r, c, W, Vw, 60, U, ldu, s, V, ldv, tall ? 0 : 1);
+    ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
+    return;
+  }
+  const double* R = reduce_to_triangle(M, r, c, ldm);
+  double* Vs = ctx.arena.alloc_n<double>((size_t)c * c);
+  const double tol_rel = kEps * static_cast<double>(r);
+  const size_t smem = (2 * (size_t)c * c + c) * sizeof(double);
+  const int threads = 32 * std::min(32, std::max(4, (c + 1) / 2));
+  auto core = c <= 32 ? jacobi_core_kernel<1> : c <= 64 ? jacobi_core_kernel<2> : jacobi_core_kernel<3>;
+  static const bool once = (allow_smem(jacobi_core_kernel<1>, 160 * 1024), allow_smem(jacobi_core_kernel<2>, 160 * 1024),
+                            allow_smem(jacobi_core_kernel<3>, 160 * 1024), true);
+  (void)once;
+  core<<<1, threads, smem, ctx.stream>>>(R, c, 60, tol_rel, s, Vs); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
+  double* left = tall ? U : V;    // M's side
+  const int ldl = tall ? ldu : ldv;
+  copy_matrix(tall ? V : U, tall ? ldv : ldu, Vs, c, c, need);
+  gemm(false, false, r, need, c, 1.0, M, ldm, Vs, c, 0.0, left, ldl);
+  scale_left_kernel<<<dim3(std::min(ceil_div(r, 256), 64), need), 256, 0, ctx.stream>>>(left, r, need, ldl, s, tol_rel);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+  complete_null_columns(r, need, s, 1e-4, left, ldl);
 }
 
 }  // namespace fpls

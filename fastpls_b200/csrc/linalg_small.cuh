@@ -34,9 +34,15 @@ void eig_psd_desc(int l, const double* G, int ldg, double* evals, double* V, int
 
 // Thin SVD A = U diag(s) V^T of a rows x cols matrix by one-sided Jacobi,
 // singular values descending, U rows x r, V cols x r with r = min(rows, cols).
-// Null directions are completed to an orthonormal set.
+// Null directions are completed to an orthonormal set.  All r values are
+// written, of U and V the first `need` columns at least.
 void svd_thin(int rows, int cols, const double* A, int lda, double* U, int ldu, double* s,
-              double* V, int ldv);
+              double* V, int ldv, int need);
+
+// Columns j < cols of U (L rows) whose s[j] is negligible against s[0]: unit
+// vectors made orthogonal to the columns before them; columns whose s[j] is
+// below weak_rel s[0]: made orthogonal to them as they are.
+void complete_null_columns(int L, int cols, const double* s, double weak_rel, double* U, int ldu);
 
 // Same contract as svd_thin, computed by a cooperative one-sided Jacobi over
 // the whole GPU (one CTA per column pair, grid barrier per round); for

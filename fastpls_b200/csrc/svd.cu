@@ -41,7 +41,7 @@ SvdResult exact_svd(const double* A, int rows, int cols, int lda, int k, bool le
   double* sw = ctx.arena.alloc_n<double>(max_rank);
   double* Vw = ctx.arena.alloc_n<double>((size_t)cols * max_rank);
   if (max_rank > kCoopSvdMin) svd_jacobi_coop(rows, cols, A, lda, Uw, rows, sw, Vw, cols);
-  else svd_thin(rows, cols, A, lda, Uw, rows, sw, Vw, cols);
+  else svd_thin(rows, cols, A, lda, Uw, rows, sw, Vw, cols, rank);
   copy_matrix(U, ldu, Uw, rows, rows, rank);
   d2d(s, sw, rank * sizeof(double));
   if (!left_only && V) copy_matrix(V, ldv, Vw, cols, cols, rank);
@@ -132,8 +132,8 @@ SvdResult truncated_svd_device(const double* A, int rows, int cols, int lda, int
   double* Ub = ctx.arena.alloc_n<double>((size_t)l * bmr);
   double* sb = ctx.arena.alloc_n<double>(bmr);
   double* Vb = ctx.arena.alloc_n<double>((size_t)cols * bmr);
-  svd_thin(l, cols, B, l, Ub, l, sb, Vb, cols);
   const int r2 = std::min(rank, bmr);
+  svd_thin(l, cols, B, l, Ub, l, sb, Vb, cols, r2);
   gemm(false, false, rows, r2, l, 1.0, Q, rows, Ub, l, 0.0, U, ldu);
   d2d(s, sb, r2 * sizeof(double));
   if (!left_only && V) copy_matrix(V, ldv, Vb, cols, cols, r2);

@@ -134,7 +134,7 @@ SvdResult truncated_rsvd_crossprod_device(const double* X, int n, int p, const d
   double* sb = ctx.arena.alloc_n<double>(r);
   double* Vb = ctx.arena.alloc_n<double>((size_t)m * r);
   if (r > 96) svd_jacobi_coop(l, m, B, l, Ub, l, sb, Vb, m);
-  else svd_thin(l, m, B, l, Ub, l, sb, Vb, m);
+  else svd_thin(l, m, B, l, Ub, l, sb, Vb, m, std::min(target, r));
   const int actual = std::min(target, r);
   gemm(false, false, p, actual, l, 1.0, Qp, p, Ub, l, 0.0, U, ldu);
   d2d(s, sb, actual * sizeof(double));

@@ -69,3 +69,25 @@ def test_cholesky_qr_sizes(lib, rows, l):
     # 0.98^(3 l) of the largest, which is how far rounding is amplified
     tol = 1000 * EPS / 0.98 ** (3 * l)
     assert np.max(np.abs(got["d"] - ref.s)) <= tol * ref.s[0]
+
+
+# Exact thin SVD through QR: one block of rows, several, a ragged last one shorter
+# than the columns, two levels, wide inputs, one / two / three registers a lane,
+# the largest column count of this route, the first of the whole-GPU one
+@pytest.mark.parametrize("rows,cols", [(5, 1), (8, 5), (32, 32), (375, 22), (512, 22), (513, 22), (522, 22), (5000, 22),
+                                       (40, 4000), (400, 33), (300, 64), (700, 65), (260, 96), (2000, 96), (200, 97)])
+@pytest.mark.parametrize("deficient", [False, True])
+def test_exact_svd_shapes(lib, rows, cols, deficient):
+    r = min(rows, cols)
+    A = _matrix(rows, cols, rows + cols, 0.95)
+    if deficient and r > 1:     # a centred class response: one exact null direction
+        A = A - A.mean(axis=1 if cols <= rows else 0, keepdims=True)
+    got = lib.truncated_svd(A, r, svd_method=3)
+    s = np.linalg.svd(A, compute_uv=False)
+    # backward stable: eps times the size, of the largest singular value
+    tol = 20 * EPS * max(rows, cols) * s[0]
+    assert np.max(np.abs(got["d"] - s)) < tol
+    assert np.linalg.norm((got["u"] * got["d"]) @ got["vt"] - A) < 10 * r * tol
+    assert np.linalg.norm(got["vt"] @ got["vt"].T - np.eye(r)) < 1e3 * EPS * r
+    # U = A V / s amplifies rounding by up to 1e4, weaker columns are made orthogonal
+    assert np.linalg.norm(got["u"].T @ got["u"] - np.eye(r)) < 1e4 * EPS * max(rows, cols)
