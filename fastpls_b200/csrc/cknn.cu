@@ -30,6 +30,7 @@
 #include "capi_util.cuh"
 #include "cknn.cuh"
 #include "context.cuh"
+#include "row_topk.cuh"
 #include "tc_util.cuh"
 
 namespace fpls {
@@ -1070,8 +1071,13 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const double* dT
   gemm(false, true, ntest, C, kdim, 1.0, dTt, ntest, dC, C, 0.0, base, ntest);
   int* cand = ctx.arena.alloc_n<int>((size_t)npairs);
   double* cbase = ctx.arena.alloc_n<double>((size_t)npairs);
-  select_candidates_kernel<<<ceil_div(ntest, 128), 128, 0, ctx.stream>>>(base, ntest, C, tm, cand, cbase); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  if (tm <= kRowTopkMax) {
+    row_topk_launch(base, ntest, C, nullptr, tm, -1, false, cand, cbase);
+  } else {   // longer candidate lists than the register lists hold
+    select_candidates_kernel<<<ceil_div(ntest, 128), 128, 0, ctx.stream>>>(base, ntest, C, tm, cand, cbase);
+    ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
+  }
 
   // training rows grouped by class (row-major), test rows row-major
   pt.mark("base scores + candidates");

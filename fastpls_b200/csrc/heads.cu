@@ -3,6 +3,7 @@
 #include "context.cuh"
 #include "heads.cuh"
 #include "linalg_small.cuh"
+#include "row_topk.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -11,46 +12,6 @@
 
 namespace fpls {
 namespace {
-
-__global__ void argmax_kernel(const double* __restrict__ S, int w, int C, const double* bias,
-                              int* labels) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= w) return;
-  int best = 0;
-  double bv = S[i] + (bias ? bias[0] : 0.0);
-  for (int c = 1; c < C; ++c) {
-    const double v = S[i + (size_t)c * w] + (bias ? bias[c] : 0.0);
-    if (v > bv) { bv = v; best = c; }
-  }
-  labels[i] = best + 1;
-}
-
-// Insertion into a descending top list: strict '>' keeps the earlier class on
-// ties (candidate_insert_top, src/fastPLS.cpp:1249-1267).
-__global__ void topk_kernel(const double* __restrict__ S, int w, int C, const double* bias,
-                            int top_k, int* idx, double* score) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= w) return;
-  double vals[32];
-  int ids[32];
-  const int k = min(top_k, 32);
-  for (int j = 0; j < k; ++j) { vals[j] = -INFINITY; ids[j] = 0; }
-  for (int c = 0; c < C; ++c) {
-    const double v = S[i + (size_t)c * w] + (bias ? bias[c] : 0.0);
-    for (int j = 0; j < k; ++j) {
-      if (v > vals[j]) {
-        for (int h = k - 1; h > j; --h) { vals[h] = vals[h - 1]; ids[h] = ids[h - 1]; }
-        vals[j] = v;
-        ids[j] = c + 1;
-        break;
-      }
-    }
-  }
-  for (int j = 0; j < k; ++j) {
-    idx[i + (size_t)j * w] = ids[j];
-    score[i + (size_t)j * w] = vals[j];
-  }
-}
 
 // Class sums of the score columns (T n x kmax into sums C x kmax) in a fixed
 // order: warp w takes (class c, column j) = (w % C, w / C) and walks that
@@ -152,16 +113,15 @@ void lowrank_predict(const double* Xs, int w, int p, const double* R, int kmax, 
 
 void row_argmax(const double* S, int w, int C, const double* bias, int* labels) {
   if (w <= 0) return;
-  argmax_kernel<<<ceil_div(w, 256), 256, 0, Context::get().stream>>>(S, w, C, bias, labels); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  // first maximum; a NaN first score, or no finite one, leaves class 1
+  row_topk_launch(S, w, C, bias, 1, 1, true, labels, nullptr);
 }
 
 void row_topk(const double* S, int w, int C, const double* bias, int top_k, int* idx,
               double* score) {
-  FPLS_REQUIRE(top_k >= 1 && top_k <= 32, "top-k supports 1..32 classes per row");
+  FPLS_REQUIRE(top_k >= 1 && top_k <= kRowTopkMax, "top-k supports 1..32 classes per row");
   if (w <= 0) return;
-  topk_kernel<<<ceil_div(w, 128), 128, 0, Context::get().stream>>>(S, w, C, bias, top_k, idx, score); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  row_topk_launch(S, w, C, bias, top_k, 0, false, idx, score);
 }
 
 void lda_train_prefix(const double* T, int n, int kmax, const int* y_host, int C,
