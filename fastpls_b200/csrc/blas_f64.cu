@@ -1,143 +1,14 @@
 #include "blas_f64.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+
 #include "context.cuh"
+#include "gemm_f64.cuh"
 
 namespace fpls {
 namespace {
-
-constexpr int BM = 64;
-constexpr int BN = 64;
-constexpr int BK = 16;
-constexpr int PAD = 4;  // row stride of 68 doubles keeps the DMMA fragment loads conflict-free
-constexpr int GEMM_THREADS = 128;
-
-// Tile loader: fetches the BK x BM slice of op(A) (or BK x BN of op(B)) for the
-// k-block starting at k0 into registers; out-of-range elements read as zero.
-template <bool KContig>
-__device__ __forceinline__ void load_tile(double (&r)[8], const double* __restrict__ P, int ld,
-                                          int mn0, int k0, int MN, int K, int kend) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int mn, k;
-    if (KContig) {  // element (mn, k) at P[k + mn*ld]
-      k = t & 15;
-      mn = (t >> 4) + 8 * i;
-    } else {        // element (mn, k) at P[mn + k*ld]
-      mn = t & 63;
-      k = (t >> 6) + 2 * i;
-    }
-    const int gm = mn0 + mn;
-    const int gk = k0 + k;
-    double v = 0.0;
-    if (gm < MN && gk < kend && gk < K) {
-      v = KContig ? __ldg(P + (size_t)gm * ld + gk) : __ldg(P + gm + (size_t)gk * ld);
-    }
-    r[i] = v;
-  }
-}
-
-template <bool KContig>
-__device__ __forceinline__ void store_tile(double (*S)[BM + PAD], const double (&r)[8]) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int mn, k;
-    if (KContig) {
-      k = t & 15;
-      mn = (t >> 4) + 8 * i;
-    } else {
-      mn = t & 63;
-      k = (t >> 6) + 2 * i;
-    }
-    S[k][mn] = r[i];
-  }
-}
-
-// op(A) (m,k): transA ? A[k + m*lda] : A[m + k*lda]   -> K-contiguous when transA
-// op(B) (k,n): transB ? B[n + k*ldb] : B[k + n*ldb]   -> K-contiguous when !transB
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(GEMM_THREADS)
-gemm_f64_dmma(int M, int N, int K, double alpha, const double* __restrict__ A, int lda,
-              const double* __restrict__ B, int ldb, double beta, double* __restrict__ C, int ldc,
-              int k_per_split, long long split_stride, int upper) {
-  __shared__ double As[2][BK][BM + PAD];
-  __shared__ double Bs[2][BK][BN + PAD];
-  const int bm = blockIdx.x * BM;
-  const int bn = blockIdx.y * BN;
-  if (upper && bm >= bn + BN) return;  // tile entirely below the diagonal
-  const int kbeg = blockIdx.z * k_per_split;
-  const int kend = min(K, kbeg + k_per_split);
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int gid = lane >> 2;
-  const int tig = lane & 3;
-  const int wm = (warp & 1) * 32;
-  const int wn = (warp >> 1) * 32;
-
-  double acc[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-  double ra[8], rb[8];
-  if (kbeg < kend) {
-    load_tile<TA>(ra, A, lda, bm, kbeg, M, K, kend);
-    load_tile<!TB>(rb, B, ldb, bn, kbeg, N, K, kend);
-    store_tile<TA>(As[0], ra);
-    store_tile<!TB>(Bs[0], rb);
-  }
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    const bool has_next = (k0 + BK) < kend;
-    if (has_next) {
-      load_tile<TA>(ra, A, lda, bm, k0 + BK, M, K, kend);
-      load_tile<!TB>(rb, B, ldb, bn, k0 + BK, N, K, kend);
-    }
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk + tig][wm + i * 8 + gid];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk + tig][wn + j * 8 + gid];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-    }
-    if (has_next) {
-      store_tile<TA>(As[buf ^ 1], ra);
-      store_tile<!TB>(Bs[buf ^ 1], rb);
-    }
-    __syncthreads();
-    buf ^= 1;
-  }
-
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = bm + wm + i * 8 + gid;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int n = bn + wn + j * 8 + tig * 2 + e;
-        if (n >= N) continue;
-        // split-K: each K range stores its own partial (summed in range order
-        // by splitk_reduce_kernel, so runs repeat bit for bit)
-        double* cp = C + (size_t)blockIdx.z * split_stride + m + (size_t)n * ldc;
-        const double v = alpha * acc[i][j][e];
-        if (split_stride) {
-          *cp = v;
-        } else {
-          *cp = (beta == 0.0) ? v : (v + beta * *cp);
-        }
-      }
-    }
-  }
-}
 
 __global__ void scale_matrix_kernel(double* C, int M, int N, int ldc, double beta) {
   const size_t total = (size_t)M * N;
@@ -185,14 +56,17 @@ __global__ void gemv_n_kernel(int M, int K, double alpha, const double* __restri
 // C (M x N, ldc) = beta C + sum_{z < splits} W_z, W_z = W + z stride (ld ldw):
 // the split-K partials added in K-range order.
 __global__ void splitk_reduce_kernel(const double* __restrict__ W, int splits, long long stride, int M, int N,
-                                     int ldw, double beta, double* __restrict__ C, int ldc) {
+                                     int ldw, double beta, double* __restrict__ C, int ldc,
+                                     const double* __restrict__ row_add) {
   const size_t total = (size_t)M * N;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     const int m = static_cast<int>(t % M), n = static_cast<int>(t / M);
     double acc = 0.0;
     for (int z = 0; z < splits; ++z) acc += W[(size_t)z * stride + m + (size_t)n * ldw];
     double* cp = C + m + (size_t)n * ldc;
-    *cp = (beta == 0.0) ? acc : acc + beta * *cp;
+    double v = (beta == 0.0) ? acc : acc + beta * *cp;
+    if (row_add) v += row_add[n];
+    *cp = v;
   }
 }
 
@@ -388,53 +262,96 @@ int grid_for(size_t total, int threads) {
 
 }  // namespace
 
+namespace {
+
+using gemm64::kBK;
+using gemm64::kBM;
+
+// K ranges of a product of `tiles` 64 x 64 output tiles: enough for two tiles an
+// SM, at least 128 terms each.  The ranges set the order of the sum, so this rule
+// does not look at the tile width.
+int split_count(int tiles, int K, int sm_count) {
+  const int target = 2 * sm_count;
+  if (tiles >= target || K < 4 * kBK) return 1;
+  return std::max(1, std::min(ceil_div(target, tiles), ceil_div(K, 8 * kBK)));
+}
+
+struct GemmPlan { int nt, splits, kps; };
+
+// Tile width and K ranges by modelled time.  An SM's FP64 tensor pipe takes
+// 8 nt cycles a contraction step and tile whatever shares it, so the time is
+// that of the SM with the most tiles; the tiles' operands come from L2 at about
+// 2900 bytes a clock (all SMs), a tile's start and end cost about 2500 cycles,
+// partials are written, read and summed once more.  Products below 2^28
+// multiply-adds keep the ranges of split_count (only their width is chosen):
+// they are over in tens of microseconds, and iterations that feed the split
+// precisions need their last bits unchanged.  50000 x 768 x 100 (S = X^T Y):
+// 551 us on 64 x 64 tiles in 13 ranges (312 tiles on 148 SMs).
+GemmPlan plan_gemm(int M, int N, int K, int sm_count) {
+  const double steps_min = 8 * kBK;
+  const bool large = static_cast<double>(M) * N * K >= 268435456.0;
+  const int base = split_count(ceil_div(M, kBM) * ceil_div(N, 64), K, sm_count);
+  const int smax = large ? std::max(1, std::min(64, static_cast<int>(K / steps_min))) : base;
+  GemmPlan best{8, base, 0};
+  double best_cost = 1e300;
+  for (int nt : gemm64::kWidths) {
+    const long long tiles = (long long)ceil_div(M, kBM) * ceil_div(N, 8 * nt);
+    if (ceil_div(N, 8 * nt) > 65535) continue;
+    for (int want = large ? 1 : base; want <= smax; ++want) {
+      const int kps = ceil_div(ceil_div(K, want), kBK) * kBK, splits = ceil_div(K, kps);
+      const double units = static_cast<double>(tiles) * splits, waves = std::ceil(units / sm_count);
+      const double tensor = waves * kps * 8.0 * nt, overhead = 2500.0 * std::ceil(waves / 2.0);
+      const double bytes = units * kps * (kBM + 8.0 * nt) * 8.0;
+      double cost = std::max(tensor, bytes / 2900.0) + overhead;
+      if (splits > 1) cost += 3000.0 + (2.0 * splits + 1.0) * M * N * 8.0 / 2900.0;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = GemmPlan{nt, splits, kps};
+      }
+    }
+  }
+  return best;
+}
+
+void gemm_run(bool transA, bool transB, int nt, const gemm64::Args& g, int splits, cudaStream_t st) {
+  const dim3 grid(ceil_div(g.M, kBM), ceil_div(g.N, 8 * nt), splits);
+  // 16-byte copies need both operands' columns on 16-byte boundaries
+  auto aligned = [](const double* p, int ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 2 == 0; };
+  const bool vec = aligned(g.A, g.lda) && aligned(g.B, g.ldb);
+  if (!transA && !transB) gemm64::launch<false, false>(g, nt, vec, grid, st);
+  else if (transA && !transB) gemm64::launch<true, false>(g, nt, vec, grid, st);
+  else if (!transA) gemm64::launch<false, true>(g, nt, vec, grid, st);
+  else gemm64::launch<true, true>(g, nt, vec, grid, st);
+}
+
+}  // namespace
+
 void gemm(bool transA, bool transB, int M, int N, int K, double alpha, const double* A, int lda,
-          const double* B, int ldb, double beta, double* C, int ldc) {
+          const double* B, int ldb, double beta, double* C, int ldc, const double* row_add) {
   if (M <= 0 || N <= 0) return;
-  cudaStream_t st = Context::get().stream;
+  Context& ctx = Context::get();
+  cudaStream_t st = ctx.stream;
   if (K <= 0) {
     scale_matrix_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(C, M, N, ldc, beta); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
+    if (row_add) add_row_vector(C, M, N, ldc, row_add);
     return;
   }
-  const int gm = ceil_div(M, BM);
-  const int gn = ceil_div(N, BN);
-  // Split K so that the grid covers the SMs at least twice for skinny outputs.
-  int splits = 1;
-  const int tiles = gm * gn;
-  const int target = 2 * Context::get().sm_count;
-  if (tiles < target && K >= 4 * BK) {
-    splits = std::min(ceil_div(target, tiles), ceil_div(K, 8 * BK));
-    if (splits < 1) splits = 1;
-  }
-  int kps = ceil_div(K, splits);
-  kps = ceil_div(kps, BK) * BK;
-  splits = ceil_div(K, kps);
+  const GemmPlan plan = plan_gemm(M, N, K, ctx.sm_count);
+  gemm64::Args g{M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, plan.kps, 0, 0, row_add};
   // split-K partials go to a per-stream workspace and are summed in order
-  double* dst = C;
-  int ldd = ldc;
-  long long stride = 0;
-  if (splits > 1) {
-    stride = (long long)M * N;
-    dst = Context::get().splitk_workspace(st, (size_t)splits * M * N);
-    ldd = M;
+  if (plan.splits > 1) {
+    g.split_stride = (long long)M * N;
+    g.C = ctx.splitk_workspace(st, (size_t)plan.splits * M * N);
+    g.ldc = M;
+    g.beta = 0.0;
+    g.row_add = nullptr;
   }
-  const double beta_k = splits > 1 ? 0.0 : beta;
-  dim3 grid(gm, gn, splits);
-  Context& ctx = Context::get();
   const int slot = ctx.prof_begin("gemm_f64_dmma", st);
-  if (!transA && !transB)
-    gemm_f64_dmma<false, false><<<grid, GEMM_THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta_k, dst, ldd, kps, stride, 0);
-  else if (transA && !transB)
-    gemm_f64_dmma<true, false><<<grid, GEMM_THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta_k, dst, ldd, kps, stride, 0);
-  else if (!transA && transB)
-    gemm_f64_dmma<false, true><<<grid, GEMM_THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta_k, dst, ldd, kps, stride, 0);
-  else
-    gemm_f64_dmma<true, true><<<grid, GEMM_THREADS, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta_k, dst, ldd, kps, stride, 0);
-  ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
-  if (splits > 1) {
-    splitk_reduce_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(dst, splits, stride, M, N, ldd, beta, C, ldc);
+  gemm_run(transA, transB, plan.nt, g, plan.splits, st);
+  if (plan.splits > 1) {
+    splitk_reduce_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(g.C, plan.splits, g.split_stride, M, N, M, beta,
+                                                                      C, ldc, row_add);
     ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
   }
@@ -459,35 +376,28 @@ void gram_tiles_f64(const double* X, int n, int p, int ldx, double* K, int ldk) 
   if (n <= 0) return;
   Context& ctx = Context::get();
   cudaStream_t st = ctx.stream;
-  const int g = ceil_div(n, BM);
-  int splits = 1;
-  const int tiles = g * (g + 1) / 2;
-  const int target = 2 * ctx.sm_count;
-  if (tiles < target && p >= 4 * BK) splits = std::max(1, std::min(ceil_div(target, tiles), ceil_div(p, 8 * BK)));
-  int kps = ceil_div(ceil_div(p, splits), BK) * BK;
+  const int g = ceil_div(n, kBM);
+  int splits = split_count(g * (g + 1) / 2, p, ctx.sm_count);
+  const int kps = ceil_div(ceil_div(p, splits), kBK) * kBK;
   splits = ceil_div(p, kps);
   if (p <= 0) {
     scale_matrix_kernel<<<grid_for((size_t)n * n, 256), 256, 0, st>>>(K, n, n, ldk, 0.0); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
   }
   if (p > 0) {
-    double* dst = K;
-    int ldd = ldk;
-    long long stride = 0;
+    gemm64::Args a{n, n, p, 1.0, X, ldx, X, ldx, 0.0, K, ldk, kps, 0, 1, nullptr};
     if (splits > 1) {  // partials of the K ranges, summed in order (lower tiles stay unused)
-      stride = (long long)n * n;
-      dst = ctx.splitk_workspace(st, (size_t)splits * n * n);
-      ldd = n;
+      a.split_stride = (long long)n * n;
+      a.C = ctx.splitk_workspace(st, (size_t)splits * n * n);
+      a.ldc = n;
     }
     const int slot = ctx.prof_begin("gemm_f64_dmma", st);
-    gemm_f64_dmma<TX, !TX><<<dim3(g, g, splits), GEMM_THREADS, 0, st>>>(n, n, p, 1.0, X, ldx, X, ldx, 0.0, dst,
-                                                                       ldd, kps, stride, 1); ::fpls::note_launch();
+    gemm_run(TX, !TX, 8, a, splits, st);   // square tiles, as the diagonal cuts them
     // algorithmic work: the upper tiles' share of 2 n^2 p flops
-    ctx.prof_end(slot, st, 8.0 * ((double)n * p + (double)n * n), (double)n * (n + BM) * p);
-    FPLS_CHECK_LAUNCH();
+    ctx.prof_end(slot, st, 8.0 * ((double)n * p + (double)n * n), (double)n * (n + kBM) * p);
     if (splits > 1) {
-      splitk_reduce_kernel<<<grid_for((size_t)n * n, 256), 256, 0, st>>>(dst, splits, stride, n, n, ldd, 0.0, K,
-                                                                        ldk);
+      splitk_reduce_kernel<<<grid_for((size_t)n * n, 256), 256, 0, st>>>(a.C, splits, a.split_stride, n, n, n, 0.0, K,
+                                                                        ldk, nullptr);
       ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
     }
@@ -562,7 +472,8 @@ void gemv(bool trans, int rows, int cols, double alpha, const double* A, int lda
       gemv_n_kernel<<<dim3(gx, splits), 256, 0, st>>>(rows, cols, alpha, A, lda, x, ws, kps, (long long)rows, 0.0);
       ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
-      splitk_reduce_kernel<<<grid_for(rows, 256), 256, 0, st>>>(ws, splits, rows, rows, 1, rows, beta, y, rows);
+      splitk_reduce_kernel<<<grid_for(rows, 256), 256, 0, st>>>(ws, splits, rows, rows, 1, rows, beta, y, rows,
+                                                               nullptr);
     } else {
       gemv_n_kernel<<<dim3(gx, splits), 256, 0, st>>>(rows, cols, alpha, A, lda, x, y, kps, 0ll, beta);
     }

@@ -9,10 +9,11 @@
 
 namespace fpls {
 
-// C = alpha * op(A) * op(B) + beta * C, op(A): M x K, op(B): K x N.
+// C = alpha * op(A) * op(B) + beta * C, op(A): M x K, op(B): K x N; row_add
+// (N values, or null) is then added to every row.
 void gemm(bool transA, bool transB, int M, int N, int K, double alpha,
           const double* A, int lda, const double* B, int ldb, double beta,
-          double* C, int ldc);
+          double* C, int ldc, const double* row_add = nullptr);
 
 // K (n x n) = X X^T for X n x p: the upper-triangle tiles by FP64 tensor-core
 // MMA, the lower triangle mirrored (K exactly symmetric).

@@ -106,8 +106,7 @@ void lowrank_predict(const double* Xs, int w, int p, const double* R, int kmax, 
   for (int a = 0; a < L; ++a) {
     const int mc = ncomp_host[a];
     double* Ya = Ypred + (size_t)a * w * m;
-    gemm(false, false, w, m, mc, 1.0, T, w, W + (size_t)a * kmax * m, kmax, 0.0, Ya, w);
-    add_row_vector(Ya, w, m, w, mY);
+    gemm(false, false, w, m, mc, 1.0, T, w, W + (size_t)a * kmax * m, kmax, 0.0, Ya, w, mY);
   }
 }
 

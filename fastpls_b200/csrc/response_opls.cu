@@ -199,8 +199,7 @@ int fpls_gaussian_y_decode(const double* Z, int w, int d, const double* decoder,
     const double* dD = upload(decoder, (size_t)d * q);
     const double* dmu = upload(y_center, q);
     double* dY = ctx.arena.alloc_n<double>((size_t)w * q);
-    gemm(false, false, w, q, d, 1.0, dZ, w, dD, d, 0.0, dY, w);
-    add_row_vector(dY, w, q, w, dmu);
+    gemm(false, false, w, q, d, 1.0, dZ, w, dD, d, 0.0, dY, w, dmu);
     d2h(Y, dY, (size_t)w * q * sizeof(double));
     ctx.sync();
   });
