@@ -281,8 +281,7 @@ struct GemmPlan { int nt, splits, kps; };
 // Tile width and K ranges by modelled time.  An SM's FP64 tensor pipe takes
 // 8 nt cycles a contraction step and tile whatever shares it, so the time is
 // that of the SM with the most tiles; the tiles' operands come from L2 at about
-// 2900 bytes a clock (all SMs), a tile's start and end cost about 2500 cycles,
-// partials are written, read and summed once more.  Products below 2^28
+// 2900 bytes a clock (all SMs), partials are written, read and summed once more.  Products below 2^28
 // multiply-adds keep the ranges of split_count (only their width is chosen):
 // they are over in tens of microseconds, and iterations that feed the split
 // precisions need their last bits unchanged.  50000 x 768 x 100 (S = X^T Y):
@@ -300,9 +299,12 @@ GemmPlan plan_gemm(int M, int N, int K, int sm_count) {
     for (int want = large ? 1 : base; want <= smax; ++want) {
       const int kps = ceil_div(ceil_div(K, want), kBK) * kBK, splits = ceil_div(K, kps);
       const double units = static_cast<double>(tiles) * splits, waves = std::ceil(units / sm_count);
-      const double tensor = waves * kps * 8.0 * nt, overhead = 2500.0 * std::ceil(waves / 2.0);
+      // a tile alone: its tensor time at the pace one warp a scheduler holds, plus
+      // its first loads and its stores, which the SM's other tiles hide
+      const double work = kps * 8.0 * nt, alone = work / 0.85 + 4000.0;
+      const double resident = std::min(waves, nt >= 13 ? 2.0 : nt >= 8 ? 3.0 : 4.0);
       const double bytes = units * kps * (kBM + 8.0 * nt) * 8.0;
-      double cost = std::max(tensor, bytes / 2900.0) + overhead;
+      double cost = std::max(waves * std::max(work / 0.95, alone / resident), bytes / 2900.0);
       if (splits > 1) cost += 3000.0 + (2.0 * splits + 1.0) * M * N * 8.0 / 2900.0;
       if (cost < best_cost) {
         best_cost = cost;

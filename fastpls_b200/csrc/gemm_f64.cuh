@@ -127,18 +127,33 @@ __global__ void __launch_bounds__(kThreads) gemm_f64_dmma(Args g) {
     const double* a_s = As + (b % S) * TileA::kSize;
     const double* b_s = Bs + (b % S) * TileB::kSize;
     const int kleft = kend - (kbeg + b * kBK);
+    double fa[2][2], fb[2][NT];
+    auto load_step = [&](int s4, int buf) {
 #pragma unroll
-    for (int kk = 0; kk < kBK; kk += 4) {
-      if (kk >= kleft) break;   // the range's last tile: nothing but zeros from here on
-      double a[2], bf[NT];
+      for (int i = 0; i < 2; ++i) fa[buf][i] = a_s[TileA::at(wm + i * 8 + gid, 4 * s4 + tig)];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) a[i] = a_s[TileA::at(wm + i * 8 + gid, kk + tig)];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) bf[j] = b_s[TileB::at(j * 8 + gid, kk + tig)];
+      for (int j = 0; j < NT; ++j) fb[buf][j] = b_s[TileB::at(j * 8 + gid, 4 * s4 + tig)];
+    };
+    auto multiply = [&](int buf) {
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], bf[j]);
+        for (int i = 0; i < 2; ++i) dmma_8x8x4(acc[i][j][0], acc[i][j][1], fa[buf][i], fb[buf][j]);
+    };
+    if (kleft >= kBK) {
+      // the next step's fragments load under this step's products: one warp a
+      // scheduler is enough to keep the tensor pipe busy
+      load_step(0, 0);
+#pragma unroll
+      for (int s4 = 0; s4 < kBK / 4; ++s4) {
+        if (s4 + 1 < kBK / 4) load_step(s4 + 1, (s4 + 1) & 1);
+        multiply(s4 & 1);
+      }
+    } else {   // the range's last tile: nothing but zeros after kleft
+      for (int s4 = 0; 4 * s4 < kleft; ++s4) {
+        load_step(s4, 0);
+        multiply(0);
+      }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
