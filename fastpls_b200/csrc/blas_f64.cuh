@@ -36,8 +36,10 @@ void col_sd_centered(const double* X, int n, int p, int ldx, double* out);
 void col_sum(const double* X, int n, int p, int ldx, double* out);
 void col_sqdev(const double* X, int n, int p, int ldx, const double* mu, double* out);
 void div_vec(const double* in, size_t count, double d, bool root, double* out);
-// X[:, j] = (X[:, j] - mean[j]) / scale[j]   (mean or scale may be null).
-void center_scale(double* X, int n, int p, int ldx, const double* mean, const double* scale);
+// dst[:, j] = (src[:, j] - mean[j]) / scale[j] (mean or scale may be null); n x p,
+// ld n, dst may be src.
+void center_scale(const double* src, double* dst, int n, int p, const double* mean, const double* scale);
+void center_scale(const float* src, double* dst, int n, int p, const double* mean, const double* scale);
 // dst (n x p, ldd) = src (n x p, lds)
 void copy_matrix(double* dst, int ldd, const double* src, int lds, int n, int p);
 // X[i, j] += v[j] for all i (row broadcast)

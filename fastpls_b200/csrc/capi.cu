@@ -51,21 +51,10 @@ __global__ void scale_column_kernel(const double* src, int n, double inv, double
   if (i < n) dst[i] = src[i] * inv;
 }
 
-__global__ void center_copy_kernel(const double* X, int w, int p, const double* mX,
-                                   const double* vX, double* out) {
-  const size_t total = (size_t)w * p;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    const int j = static_cast<int>(t / w);
-    out[t] = (X[t] - mX[j]) / vX[j];
-  }
-}
-
 double* centered_test_copy(const double* Xh, int w, int p, const double* mX_d, const double* vX_d) {
-  Context& ctx = Context::get();
-  double* X = upload(Xh, (size_t)w * p);
-  center_copy_kernel<<<2 * ctx.sm_count, 256, 0, ctx.stream>>>(X, w, p, mX_d, vX_d, X); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  const MatrixSource src(Xh, false, (size_t)w * p);
+  double* X = src.centred((size_t)w * p);
+  center_scale(src.f64(), X, w, p, mX_d, vX_d);
   return X;
 }
 
@@ -252,12 +241,13 @@ int pls_model1_impl(const double* X, int n, int p, const double* Y, int m, const
     std::vector<int> nc(ncomp, ncomp + L);
     for (int& c : nc) c = std::max(1, std::min(c, max_rank));
     const int K0 = std::min(max_of(nc.data(), L), max_rank);
-    double* dX = upload(X, (size_t)n * p);
-    double* dY = upload(Y, (size_t)n * m);
+    const MatrixSource sX(X, false, (size_t)n * p), sY(Y, false, (size_t)n * m);
+    double* dX = sX.centred((size_t)n * p);
+    double* dY = sY.centred((size_t)n * m);
     double* dmX = ctx.arena.alloc_n<double>(p);
     double* dvX = ctx.arena.alloc_n<double>(p);
     double* dmY = ctx.arena.alloc_n<double>(m);
-    center_scale_xy(dX, n, p, dY, m, scaling, dmX, dvX, dmY);
+    center_scale_xy(sX, dX, n, p, sY, dY, m, scaling, dmX, dvX, dmY);
     FitOptions opt;
     opt.scaling = scaling;
     opt.fit = fit != 0;
@@ -349,12 +339,13 @@ int fpls_pls_model2_fast_xprod(const double* X, int n, int p, const double* Y, i
     std::vector<int> nc(ncomp, ncomp + L);
     for (int& c : nc) c = std::max(1, c);
     const int K = max_of(nc.data(), L);
-    double* dX = upload(X, (size_t)n * p);
-    double* dY = upload(Y, (size_t)n * m);
+    const MatrixSource sX(X, false, (size_t)n * p), sY(Y, false, (size_t)n * m);
+    double* dX = sX.centred((size_t)n * p);
+    double* dY = sY.centred((size_t)n * m);
     double* dmX = ctx.arena.alloc_n<double>(p);
     double* dvX = ctx.arena.alloc_n<double>(p);
     double* dmY = ctx.arena.alloc_n<double>(m);
-    center_scale_xy(dX, n, p, dY, m, scaling, dmX, dvX, dmY);
+    center_scale_xy(sX, dX, n, p, sY, dY, m, scaling, dmX, dvX, dmY);
     double* dR = ctx.arena.alloc_n<double>((size_t)p * K);
     double* dQ = ctx.arena.alloc_n<double>((size_t)m * K);
     double* dB = B ? ctx.arena.alloc_n<double>((size_t)p * m * L) : nullptr;
@@ -375,9 +366,10 @@ int fpls_pls_model2_fast_xprod(const double* X, int n, int p, const double* Y, i
   });
 }
 
-// Fast SIMPLS (pls_model2_fast) on device copies of X (n x p) and Y (n x m),
-// both centred / scaled in place; host outputs as fpls_pls_model2_fast.
-static void simpls_fast_on_device(double* dX, int n, int p, double* dYc, int m, const int* ncomp, int L,
+// Fast SIMPLS (pls_model2_fast): centred / scaled copies of X (n x p) and Y
+// (n x m) go to dX and dYc; host outputs as fpls_pls_model2_fast.
+static void simpls_fast_on_device(const MatrixSource& sX, double* dX, int n, int p, const MatrixSource& sY, double* dYc,
+                                  int m, const int* ncomp, int L,
                                   int scaling, int fit, int seed, double* R, double* Q, double* mX, double* vX,
                                   double* mY, double* B, double* Yfit, double* R2Y, int* n_components) {
     FPLS_REQUIRE(n > 0 && p > 0 && m > 0, "pls_model2_fast requires non-empty X and Y");
@@ -393,7 +385,7 @@ static void simpls_fast_on_device(double* dX, int n, int p, double* dYc, int m, 
     double* dmX = ctx.arena.alloc_n<double>(p);
     double* dvX = ctx.arena.alloc_n<double>(p);
     double* dmY = ctx.arena.alloc_n<double>(m);
-    center_scale_xy(dX, n, p, dYc, m, scaling, dmX, dvX, dmY);
+    center_scale_xy(sX, dX, n, p, sY, dYc, m, scaling, dmX, dvX, dmY);
     // Single fit on all rows: S = Xc^T Yc as the reference (fastPLS.cpp:2499);
     // the two predictor passes per component run FP64 or, in the mixed
     // session precision, as BF16x3 tensor-core products.
@@ -490,9 +482,8 @@ int fpls_pls_model2_fast(const double* X, int n, int p, const double* Y, int m, 
     FPLS_REQUIRE(n > 0 && p > 0 && m > 0, "pls_model2_fast requires non-empty X and Y");
     Context& ctx = Context::get();
     ctx.begin_call();
-    double* dX = upload(X, (size_t)n * p);
-    double* dYc = upload(Y, (size_t)n * m);
-    simpls_fast_on_device(dX, n, p, dYc, m, ncomp, L, scaling, fit, seed, R, Q, mX, vX, mY, B, Yfit, R2Y,
+    const MatrixSource sX(X, false, (size_t)n * p), sY(Y, false, (size_t)n * m);
+    simpls_fast_on_device(sX, sX.centred((size_t)n * p), n, p, sY, sY.centred((size_t)n * m), m, ncomp, L, scaling, fit, seed, R, Q, mX, vX, mY, B, Yfit, R2Y,
                           n_components);
   });
 }
@@ -507,9 +498,8 @@ int fpls_pls_model2_fast_rows(const double* X, int n, int p, const double* Y, in
     Context& ctx = Context::get();
     ctx.begin_call();
     RowShardScope shards(ctx, allreduce, user, n);
-    double* dX = upload(X, (size_t)n * p);
-    double* dYc = upload(Y, (size_t)n * m);
-    simpls_fast_on_device(dX, n, p, dYc, m, ncomp, L, scaling, fit, seed, R, Q, mX, vX, mY, B, Yfit, R2Y,
+    const MatrixSource sX(X, false, (size_t)n * p), sY(Y, false, (size_t)n * m);
+    simpls_fast_on_device(sX, sX.centred((size_t)n * p), n, p, sY, sY.centred((size_t)n * m), m, ncomp, L, scaling, fit, seed, R, Q, mX, vX, mY, B, Yfit, R2Y,
                           n_components);
   });
 }
@@ -606,9 +596,10 @@ int fpls_kernel_pls_model2_fast(const double* X, int n, int p, const double* Y, 
     download(col_means, dcm, n);
     download(grand_mean, dg, 1);
     if (gamma_used) *gamma_used = g;
-    double* dY = upload(Y, (size_t)n * m);
+    const MatrixSource sY(Y, false, (size_t)n * m);
+    const MatrixSource sK(dK);
     // The inner fit runs on the centred kernel with scaling "none" (R/main.R:2875-2891).
-    simpls_fast_on_device(dK, n, n, dY, m, ncomp, L, 3, fit, seed, R, Q, mK, vK, mY, B, Yfit, R2Y, n_components);
+    simpls_fast_on_device(sK, dK, n, n, sY, sY.centred((size_t)n * m), m, ncomp, L, 3, fit, seed, R, Q, mK, vK, mY, B, Yfit, R2Y, n_components);
   });
 }
 
@@ -625,14 +616,14 @@ int fpls_pls_model2(const double* X, int n, int p, const double* Y, int m, const
     ctx.begin_call();
     const int K = max_of(ncomp, L);
     FPLS_REQUIRE(K >= 1, "ncomp must be >= 1");
-    double* dX = upload(X, (size_t)n * p);
-    double* dYraw = upload(Y, (size_t)n * m);
+    const MatrixSource sX(X, false, (size_t)n * p), sY(Y, false, (size_t)n * m);
+    const double* dYraw = sY.f64();
+    double* dX = sX.centred((size_t)n * p);
     double* dY = ctx.arena.alloc_n<double>((size_t)n * m);
-    d2d(dY, dYraw, (size_t)n * m * sizeof(double));
     double* dmX = ctx.arena.alloc_n<double>(p);
     double* dvX = ctx.arena.alloc_n<double>(p);
     double* dmY = ctx.arena.alloc_n<double>(m);
-    center_scale_xy(dX, n, p, dY, m, scaling, dmX, dvX, dmY);
+    center_scale_xy(sX, dX, n, p, sY, dY, m, scaling, dmX, dvX, dmY);
     FitOptions opt;
     opt.scaling = scaling;
     opt.fit = fit != 0;
@@ -750,9 +741,7 @@ int fpls_predict_classes(const double* Xtest, int w, int p, const double* mX, co
         const int r0 = blk * B, rb = std::min(B, w - r0), b = blk & 1;
         if (blk + 1 < nblk) issue_copy(blk + 1);
         FPLS_CUDA(cudaStreamWaitEvent(ctx.stream, ctx.copy_event(b), 0));
-        center_copy_kernel<<<2 * ctx.sm_count, 256, 0, ctx.stream>>>(xb[b], rb, p, dmX, dvX, xb[b]);
-        ::fpls::note_launch();
-        FPLS_CHECK_LAUNCH();
+        center_scale(xb[b], xb[b], rb, p, dmX, dvX);
         lowrank_predict(xb[b], rb, p, dR, kmax, dW, m, ncomp, L, dmY, dT, dYp);
         FPLS_CUDA(cudaEventRecord(ctx.copy_event(2 + b), ctx.stream));   // xb[b] read by now
         for (int a = 0; a < L; ++a) {
@@ -892,29 +881,12 @@ void lda_project_scores_device(const double* dX, int w, int p, const double* dR,
   if (dS_out) add_row_vector(dS, w, C, w, dc);
 }
 
-__global__ void widen_f32_kernel(const float* __restrict__ src, size_t total, double* __restrict__ dst) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x)
-    dst[t] = static_cast<double>(src[t]);
-}
-
 // An FP32 device matrix widened exactly into a fresh FP64 copy.
-double* widen_on_device(const float* d32, size_t count) {
-  Context& ctx = Context::get();
-  double* d = ctx.arena.alloc_n<double>(count ? count : 1);
-  if (count) {
-    widen_f32_kernel<<<4 * ctx.sm_count, 256, 0, ctx.stream>>>(d32, count, d);
-    ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-  }
+double* widen_on_device(const float* d32, int rows, int cols) {
+  double* d = Context::get().arena.alloc_n<double>(std::max<size_t>((size_t)rows * cols, 1));
+  center_scale(d32, d, rows, cols, nullptr, nullptr);
   return d;
 }
-
-// A caller's matrix (FP64, or FP32 widened exactly) as a fresh FP64 device copy.
-double* upload_widened(const void* X, bool f32, size_t count) {
-  if (!f32) return upload(static_cast<const double*>(X), count);
-  return widen_on_device(upload(static_cast<const float*>(X), count), count);
-}
-
 
 }  // namespace
 
@@ -942,12 +914,13 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
     PhaseTimer pt("PLS + LDA call");
     std::vector<int> nc(ncomp, ncomp + L);
     for (int& c : nc) c = std::max(1, c);
-    // one upload of each matrix for the whole pipeline
-    double* dX = upload_widened(Xtrain, f32, (size_t)n * p);
-    double* dY = upload(Ytrain, (size_t)n * m);
+    // one upload of each matrix for the whole pipeline (none of device memory)
+    const MatrixSource sX(Xtrain, f32, (size_t)n * p), sY(Ytrain, false, (size_t)n * m);
+    double* dX = sX.centred((size_t)n * p);
+    double* dY = sY.centred((size_t)n * m);
     // the test rows cross the link while the fit runs
     capi::SideUpload xt_up(Xtest, ntest > 0 ? (size_t)ntest * p * (f32 ? sizeof(float) : sizeof(double)) : 0);
-    pt.mark("X, Y to FP64");
+    pt.mark("upload");
     int K0 = 0;
     double* dR = nullptr;
     double* dT = nullptr;   // training scores (X - mX) / vX R, n x K0
@@ -959,7 +932,7 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
       double* dmX = ctx.arena.alloc_n<double>(p);
       double* dvX = ctx.arena.alloc_n<double>(p);
       double* dmY = ctx.arena.alloc_n<double>(m);
-      center_scale_xy(dX, n, p, dY, m, scaling, dmX, dvX, dmY);
+      center_scale_xy(sX, dX, n, p, sY, dY, m, scaling, dmX, dvX, dmY);
       pt.mark("centre / scale");
       FitOptions opt;
       opt.scaling = scaling;
@@ -1000,7 +973,7 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
       std::vector<double> hQ((size_t)m * K0), hmY(m);
       int done = 0;
       // centres / scales dX in place (the fit's own copy) and fits on it
-      simpls_fast_on_device(dX, n, p, dY, m, nc.data(), L, scaling, fit, seed, hR.data(), hQ.data(), hmX.data(),
+      simpls_fast_on_device(sX, dX, n, p, sY, dY, m, nc.data(), L, scaling, fit, seed, hR.data(), hQ.data(), hmX.data(),
                             hvX.data(), hmY.data(), B, Yfit, R2Y, &done);
       if (done < K0) throw Error(FPLS_ERR_NUMERICAL, "pls_lda has invalid effective component count");
       if (Q) std::copy(hQ.begin(), hQ.end(), Q);
@@ -1046,7 +1019,7 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
     pt.mark("LDA outputs to host");
     if (ntest > 0) {
       xt_up.wait();
-      const double* dXt = f32 ? widen_on_device(static_cast<const float*>(xt_up.dst), (size_t)ntest * p)
+      const double* dXt = f32 ? widen_on_device(static_cast<const float*>(xt_up.dst), ntest, p)
                               : static_cast<const double*>(xt_up.dst);
       const double* dRp = upload(hRp.data(), (size_t)p * K0);
       const double* doff = upload(hoff.data(), K0);

@@ -21,18 +21,31 @@ inline void set_err(char* err, size_t errlen, const char* msg) {
 template <typename Fn>
 int guarded(char* err, size_t errlen, Fn&& fn) {
   if (err && errlen) err[0] = '\0';
+  // Kernels of a call that leaves early may still read the caller's matrices:
+  // they end before the error is returned.
+  auto settle = [] {
+    try {
+      Context& ctx = Context::get();
+      cudaStreamSynchronize(ctx.stream);
+      cudaStreamSynchronize(ctx.side);
+    } catch (...) {   // no device
+    }
+  };
   try {
     fn();
     Context::get().end_call();
     return FPLS_OK;
   } catch (const Error& e) {
     set_err(err, errlen, e.what());
+    settle();
     return e.code;
   } catch (const std::exception& e) {
     set_err(err, errlen, e.what());
+    settle();
     return FPLS_ERR_INTERNAL;
   } catch (...) {
     set_err(err, errlen, "fastpls_b200: unknown internal error");
+    settle();
     return FPLS_ERR_INTERNAL;
   }
 }
@@ -49,10 +62,10 @@ void download(T* host, const T* dev, size_t n) {
   if (host && n) d2h(host, dev, n * sizeof(T));
 }
 
-// A copy of a caller's matrix (host or device) on the copy stream, queued
+// A caller's matrix for a later step of the same call: the caller's own device
+// memory, or a copy of it on the copy stream, queued
 // behind the work the main stream has enqueued so far (so that an earlier
-// upload keeps the whole link), for a later step of the same call; wait()
-// makes the main stream wait for it.  A call that leaves early (an error)
+// upload keeps the whole link); wait() makes the main stream wait for it.  A call that leaves early (an error)
 // waits for the copy on the host, so that no copy still writes into arena
 // memory the next call reuses.  Uses copy events 0 and 1 of the context.
 struct SideUpload {
@@ -60,6 +73,10 @@ struct SideUpload {
   bool pending = false;
   SideUpload(const void* src, size_t bytes) {
     if (!bytes) return;
+    if (device_readable(src, sizeof(double))) {   // nothing to copy
+      dst = const_cast<void*>(src);
+      return;
+    }
     Context& ctx = Context::get();
     dst = ctx.arena.alloc_n<char>(bytes);
     FPLS_CUDA(cudaEventRecord(ctx.copy_event(0), ctx.stream));

@@ -195,6 +195,33 @@ void dzero(void* dst, size_t bytes) {
   FPLS_CUDA(cudaMemsetAsync(dst, 0, bytes, Context::get().stream));
 }
 
+bool device_readable(const void* p, size_t align) {
+  if (!p || reinterpret_cast<uintptr_t>(p) % align) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == Context::get().device;
+}
+
+MatrixSource::MatrixSource(const void* caller, bool is_f32, size_t count) : f32(is_f32) {
+  const size_t es = is_f32 ? sizeof(float) : sizeof(double);
+  if (device_readable(caller, es)) {
+    ptr = caller;
+    return;
+  }
+  void* copy = Context::get().arena.alloc(std::max<size_t>(count, 1) * es);
+  h2d(copy, caller, count * es);
+  ptr = copy;
+  own = true;
+}
+
+double* MatrixSource::centred(size_t count) const {
+  if (own && !f32) return static_cast<double*>(const_cast<void*>(ptr));
+  return Context::get().arena.alloc_n<double>(std::max<size_t>(count, 1));
+}
+
 void shard_sum(double* buf, size_t count) {
   Context& ctx = Context::get();
   if (!ctx.shards || count == 0) return;

@@ -146,6 +146,23 @@ struct RowShardScope {
   RowShardScope& operator=(const RowShardScope&) = delete;
 };
 
+// A caller's matrix as device memory to read from during the call: the caller's
+// own when it already is (device memory of the library's device, aligned for its
+// elements), else an arena copy.  `own`: the copy, which the call may overwrite.
+struct MatrixSource {
+  const void* ptr = nullptr;
+  bool f32 = false;
+  bool own = false;
+  MatrixSource() {}
+  // The library's own FP64 buffer, centred in place.
+  explicit MatrixSource(double* buffer) : ptr(buffer), own(true) {}
+  MatrixSource(const void* caller, bool is_f32, size_t count);
+  const double* f64() const { return static_cast<const double*>(ptr); }
+  // FP64 storage for a centred copy of `count` values: the own copy, or fresh.
+  double* centred(size_t count) const;
+};
+bool device_readable(const void* p, size_t align);
+
 // Host <-> device copies on the context stream (synchronous w.r.t. the caller
 // once sync() is called).
 void h2d(void* dst, const void* src, size_t bytes);

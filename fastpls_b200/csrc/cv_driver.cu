@@ -653,7 +653,7 @@ void run_sequential(const CvFitSet& fs, const double* X, const int* y, const int
     gather_rows_kernel<<<2 * ctx.sm_count, 256, 0, ctx.stream>>>(X, n, p, d_idx, nf, Xf); ::fpls::note_launch();
     onehot_kernel<<<2 * ctx.sm_count, 256, 0, ctx.stream>>>(d_lab, nf, m, Yf); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
-    center_scale_xy(Xf, nf, p, Yf, m, opt.scaling, mX, vX, mY);
+    center_scale_xy(MatrixSource(Xf), Xf, nf, p, MatrixSource(Yf), Yf, m, opt.scaling, mX, vX, mY);
     gemm(true, false, p, m, nf, 1.0, Xf, nf, Yf, nf, 0.0, S, p);
     device_gaussian(om, p, fs.seeds[f]);
     XOperatorF64 xop(Xf, nf, p);
@@ -678,7 +678,7 @@ void run_sequential(const CvFitSet& fs, const double* X, const int* y, const int
     h2d(d_idx, trows.data(), nt * sizeof(int));
     gather_rows_kernel<<<2 * ctx.sm_count, 256, 0, ctx.stream>>>(X, n, p, d_idx, nt, Xt); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
-    center_scale(Xt, nt, p, nt, mX, opt.scaling == 2 ? vX : nullptr);
+    center_scale(Xt, Xt, nt, p, mX, opt.scaling == 2 ? vX : nullptr);
     lowrank_predict(Xt, nt, p, R, K, W, m, ncomp, L, mY, T, Yp);
     for (int s = 0; s < L; ++s) row_argmax(Yp + (size_t)s * nt * m, nt, m, nullptr, lab + (size_t)s * nt);
     scatter_pred_kernel<<<ceil_div((long long)nt * L, 256), 256, 0, ctx.stream>>>(lab, nt, L, d_idx, n, fs.group[f], res.d_pred); ::fpls::note_launch();

@@ -143,13 +143,13 @@ static void center_scale_xy_sharded(double* X, int n, int p, double* Y, int m, i
   shard_sum(buf, (size_t)p + my);
   if (scaling < 3) {
     div_vec(buf, p, nt, false, mX);
-    center_scale(X, n, p, n, mX, nullptr);
+    center_scale(X, X, n, p, mX, nullptr);
   } else {
     fill(mX, p, 0.0);
   }
   if (Y) {
     div_vec(buf + p, m, nt, false, mY);
-    center_scale(Y, n, m, n, mY, nullptr);
+    center_scale(Y, Y, n, m, mY, nullptr);
   }
   if (scaling == 2) {
     // sd of the centred columns: their mean (zero up to rounding), then the
@@ -161,34 +161,42 @@ static void center_scale_xy_sharded(double* X, int n, int p, double* Y, int m, i
     col_sqdev(X, n, p, n, mu, vX);
     shard_sum(vX, p);
     div_vec(vX, p, nt - 1.0, true, vX);
-    center_scale(X, n, p, n, nullptr, vX);
+    center_scale(X, X, n, p, nullptr, vX);
   } else {
     fill(vX, p, 1.0);
   }
 }
 
-void center_scale_xy(double* X, int n, int p, double* Y, int m, int scaling, double* mX,
-                     double* vX, double* mY) {
+void center_scale_xy(const MatrixSource& Xs, double* X, int n, int p, const MatrixSource& Ys, double* Y, int m,
+                     int scaling, double* mX, double* vX, double* mY) {
+  auto copy_in = [](const MatrixSource& s, double* d, int rows, int cols, const double* mean) {
+    if (s.f32) center_scale(static_cast<const float*>(s.ptr), d, rows, cols, mean, nullptr);
+    else if (mean || s.ptr != d) center_scale(s.f64(), d, rows, cols, mean, nullptr);
+  };
   if (sharded()) {
+    copy_in(Xs, X, n, p, nullptr);
+    if (Y) copy_in(Ys, Y, n, m, nullptr);
     center_scale_xy_sharded(X, n, p, Y, m, scaling, mX, vX, mY);
     return;
   }
   // src/fastPLS.cpp:4817-4834: mX = mean, X -= mX, vX = sd(X centred), X /= vX
   if (scaling < 3) {
-    col_mean(X, n, p, n, mX);
-    center_scale(X, n, p, n, mX, nullptr);
+    if (Xs.f32) col_mean(static_cast<const float*>(Xs.ptr), n, p, n, mX);
+    else col_mean(Xs.f64(), n, p, n, mX);
+    copy_in(Xs, X, n, p, mX);
   } else {
+    copy_in(Xs, X, n, p, nullptr);
     fill(mX, p, 0.0);
   }
   if (scaling == 2) {
     col_sd_centered(X, n, p, n, vX);
-    center_scale(X, n, p, n, nullptr, vX);
+    center_scale(X, X, n, p, nullptr, vX);
   } else {
     fill(vX, p, 1.0);
   }
   if (Y) {
-    col_mean(Y, n, m, n, mY);
-    center_scale(Y, n, m, n, mY, nullptr);
+    col_mean(Ys.f64(), n, m, n, mY);
+    copy_in(Ys, Y, n, m, mY);
   }
 }
 

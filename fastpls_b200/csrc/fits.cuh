@@ -3,6 +3,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "context.cuh"
 
 namespace fpls {
 
@@ -18,9 +19,10 @@ struct FitOptions {
   bool xprod = false;     // PLSSVD: matrix-free X^T Y (src/fastPLS.cpp:5518-5690)
 };
 
-// Centres / scales X (n x p) and Y (n x m) in place, writing mX, vX (p) and mY (m).
-void center_scale_xy(double* X, int n, int p, double* Y, int m, int scaling, double* mX,
-                     double* vX, double* mY);
+// X (n x p) and Y (n x m) = the sources centred / scaled (either may be its own
+// source's copy), writing mX, vX (p) and mY (m).
+void center_scale_xy(const MatrixSource& Xs, double* X, int n, int p, const MatrixSource& Ys, double* Y, int m,
+                     int scaling, double* mX, double* vX, double* mY);
 
 struct PlssvdOut {
   double* C_latent;  // K0 x K0 x L (zeroed by the callee)

@@ -150,7 +150,7 @@ void preprocess_kernel_x_device(double* X, int n, int p, int scaling, double* mX
   Context& ctx = Context::get();
   if (scaling < 3) {
     col_mean(X, n, p, n, mX);
-    center_scale(X, n, p, n, mX, nullptr);
+    center_scale(X, X, n, p, mX, nullptr);
   } else {
     fill(mX, p, 0.0);
   }
@@ -158,7 +158,7 @@ void preprocess_kernel_x_device(double* X, int n, int p, int scaling, double* mX
     col_sd_centered(X, n, p, n, vX);
     fix_scale_kernel<<<grid_of(p, 256, ctx.sm_count), 256, 0, ctx.stream>>>(vX, p); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
-    center_scale(X, n, p, n, nullptr, vX);
+    center_scale(X, X, n, p, nullptr, vX);
   } else {
     fill(vX, p, 1.0);
   }

@@ -20,13 +20,32 @@
 namespace fpls {
 namespace {
 
-__global__ void opls_rank1_update_kernel(double* X, int n, int p, const double* t, const double* pv) {
-  const size_t total = (size_t)n * p;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
-       k += (size_t)gridDim.x * blockDim.x) {
-    const int i = static_cast<int>(k % n), j = static_cast<int>(k / n);
-    X[k] -= t[i] * pv[j];
+// X (n x p) -= t pv^T; a block takes 2048 rows of a column (reads and writes X
+// once: 20000 x 8000 in 0.43 ms at 6 TB/s, with index divisions 0.6 ms).
+constexpr int kRank1Rows = 2048;
+__global__ void __launch_bounds__(256) opls_rank1_update_kernel(double* X, int n, int p, const double* __restrict__ t,
+                                                                const double* __restrict__ pv) {
+  const int i0 = blockIdx.x * kRank1Rows + threadIdx.x;
+  for (int j = blockIdx.y; j < p; j += gridDim.y) {
+    double* x = X + (size_t)j * n;
+    const double q = pv[j];
+    double v[8], w[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int i = i0 + 256 * u;
+      v[u] = i < n ? x[i] : 0.0;
+      w[u] = i < n ? t[i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i0 + 256 * u < n) x[i0 + 256 * u] = v[u] - w[u] * q;
   }
+}
+
+void opls_rank1_update(double* X, int n, int p, const double* t, const double* pv) {
+  const dim3 grid(ceil_div(n, kRank1Rows), std::min(p, 65535));
+  opls_rank1_update_kernel<<<grid, 256, 0, Context::get().stream>>>(X, n, p, t, pv); ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
 }
 
 __global__ void dot2_kernel(const double* x, const double* y, int n, double* out) {
@@ -81,6 +100,17 @@ double scalar_d2h(const double* d) {
 __global__ void unit_vector_kernel(double* u, int p) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p; i += gridDim.x * blockDim.x)
     u[i] = (i == 0) ? 1.0 : 0.0;
+}
+
+// Where the filtered matrix (count values) is built: in the caller's output when
+// that is device memory apart from the inputs, else in the library's storage.
+double* filtered_storage(double* Xf, const MatrixSource& X, size_t count, const MatrixSource& Y, size_t y_count) {
+  auto apart = [&](const MatrixSource& s, size_t c) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(Xf), b = reinterpret_cast<uintptr_t>(s.ptr);
+    return a + count * sizeof(double) <= b || b + c * sizeof(double) <= a;
+  };
+  if (device_readable(Xf, sizeof(double)) && apart(X, count) && apart(Y, y_count)) return Xf;
+  return X.centred(count);
 }
 
 // Leading left singular vector u (p) of S (p x q), to rounding, as the first
@@ -165,11 +195,12 @@ int fpls_gaussian_y_encode(const double* Y, int n, int q, const double* projecti
     FPLS_REQUIRE(n > 0 && q > 0 && d > 0, "gaussian_y_encode: empty input");
     Context& ctx = Context::get();
     ctx.begin_call();
-    double* dY = upload(Y, (size_t)n * q);
+    const MatrixSource sY(Y, false, (size_t)n * q);
+    double* dY = sY.centred((size_t)n * q);
     const double* dG = upload(projection, (size_t)q * d);
     double* dmu = ctx.arena.alloc_n<double>(q);
-    col_mean(dY, n, q, n, dmu);
-    center_scale(dY, n, q, n, dmu, nullptr);
+    col_mean(sY.f64(), n, q, n, dmu);
+    center_scale(sY.f64(), dY, n, q, dmu, nullptr);
     double* dZ = ctx.arena.alloc_n<double>((size_t)n * d);
     xgemm(false, n, d, q, dY, n, dG, q, dZ, n);
     // decoder = (Z^T Z + 1e-8 mean(diag) I)^{-1} Z^T Yc
@@ -234,28 +265,30 @@ int fpls_opls_filter(const double* X, int n, int p, const double* Y, int q, int 
     FPLS_REQUIRE(north >= 0, "north must be >= 0");
     Context& ctx = Context::get();
     ctx.begin_call();
-    double* dX = upload(X, (size_t)n * p);
-    double* dY = upload(Y, (size_t)n * q);
+    const MatrixSource sX(X, false, (size_t)n * p), sY(Y, false, (size_t)n * q);
+    double* dX = filtered_storage(Xf, sX, (size_t)n * p, sY, (size_t)n * q);
+    double* dY = sY.centred((size_t)n * q);
     double* dmX = ctx.arena.alloc_n<double>(p);
     double* dvX = ctx.arena.alloc_n<double>(p);
     double* dmY = ctx.arena.alloc_n<double>(q);
     // Centre / scale (scaling 2 uses the (n-1) standard deviation, zeros -> 1).
     if (scaling < 3) {
-      col_mean(dX, n, p, n, dmX);
-      center_scale(dX, n, p, n, dmX, nullptr);
+      col_mean(sX.f64(), n, p, n, dmX);
+      center_scale(sX.f64(), dX, n, p, dmX, nullptr);
     } else {
+      center_scale(sX.f64(), dX, n, p, nullptr, nullptr);
       fill(dmX, p, 0.0);
     }
     if (scaling == 2) {
       col_sd_centered(dX, n, p, n, dvX);
       sd_fix_kernel<<<ceil_div(p, 256), 256, 0, ctx.stream>>>(dvX, p); ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
-      center_scale(dX, n, p, n, nullptr, dvX);
+      center_scale(dX, dX, n, p, nullptr, dvX);
     } else {
       fill(dvX, p, 1.0);
     }
-    col_mean(dY, n, q, n, dmY);
-    center_scale(dY, n, q, n, dmY, nullptr);
+    col_mean(sY.f64(), n, q, n, dmY);
+    center_scale(sY.f64(), dY, n, q, dmY, nullptr);
     double* S = ctx.arena.alloc_n<double>((size_t)p * q);
     double* u = ctx.arena.alloc_n<double>(p);
     double* t = ctx.arena.alloc_n<double>(n);
@@ -295,13 +328,12 @@ int fpls_opls_filter(const double* X, int n, int p, const double* Y, int q, int 
       const double toss = scalar_d2h(sc + 3);
       if (!(toss > 0.0) || !std::isfinite(toss)) break;
       gemv(true, n, p, 1.0 / toss, dX, n, to, 0.0, po);
-      opls_rank1_update_kernel<<<4 * ctx.sm_count, 256, 0, ctx.stream>>>(dX, n, p, to, po); ::fpls::note_launch();
-      FPLS_CHECK_LAUNCH();
+      opls_rank1_update(dX, n, p, to, po);
       d2d(dW + (size_t)k * p, wo, p * sizeof(double));
       d2d(dP + (size_t)k * p, po, p * sizeof(double));
       ++k;
     }
-    d2h(Xf, dX, (size_t)n * p * sizeof(double));
+    if (dX != Xf) d2h(Xf, dX, (size_t)n * p * sizeof(double));
     d2h(mX, dmX, p * sizeof(double));
     d2h(vX, dvX, p * sizeof(double));
     if (k > 0) {
@@ -320,21 +352,21 @@ int fpls_opls_apply_filter(const double* X, int w, int p, const double* mX, cons
     FPLS_REQUIRE(w > 0 && p > 0 && north >= 0, "opls_apply_filter: empty input");
     Context& ctx = Context::get();
     ctx.begin_call();
-    double* dX = upload(X, (size_t)w * p);
+    const MatrixSource sX(X, false, (size_t)w * p);
+    double* dX = filtered_storage(Xf, sX, (size_t)w * p, sX, (size_t)w * p);
     const double* dm = upload(mX, p);
     const double* dv = upload(vX, p);
-    center_scale(dX, w, p, w, dm, dv);
+    center_scale(sX.f64(), dX, w, p, dm, dv);
     if (north > 0) {
       const double* dW = upload(W_orth, (size_t)p * north);
       const double* dP = upload(P_orth, (size_t)p * north);
       double* t = ctx.arena.alloc_n<double>(w);
       for (int a = 0; a < north; ++a) {
         gemv(false, w, p, 1.0, dX, w, dW + (size_t)a * p, 0.0, t);
-        opls_rank1_update_kernel<<<4 * ctx.sm_count, 256, 0, ctx.stream>>>(dX, w, p, t, dP + (size_t)a * p); ::fpls::note_launch();
-        FPLS_CHECK_LAUNCH();
+        opls_rank1_update(dX, w, p, t, dP + (size_t)a * p);
       }
     }
-    d2h(Xf, dX, (size_t)w * p * sizeof(double));
+    if (dX != Xf) d2h(Xf, dX, (size_t)w * p * sizeof(double));
     ctx.sync();
   });
 }

@@ -15,8 +15,13 @@
 namespace fpls {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
+// Threads a block.  The order of every sum is that of kSumThreads lanes (and
+// kSumThreads / 32 warps), whatever the block: larger blocks only bring more
+// loads in flight and more columns at a time.
+constexpr int kMaxThreads = 1024;
+constexpr int kSumThreads = 256;
+constexpr int kSumWarps = kSumThreads / 32;
+constexpr int kAhead = 16;    // loads of one thread that go out before they are used
 
 struct Eng {
   int n, p, m, F, K, cp, cn, szp, szn;
@@ -64,71 +69,78 @@ __device__ __forceinline__ void chunk_range(int chunk, int sz, int total, int& b
   e = min(total, b + sz);
 }
 
+// parts[0] + parts[stride] + ... in order, kAhead loads at a time (each kernel of
+// the loop starts with such a sum, and its loads one after another were a third
+// of the launch).
 __device__ __forceinline__ double sum_parts(const double* parts, int count, int stride) {
   double s = 0.0;
-  for (int c = 0; c < count; ++c) s += parts[(size_t)c * stride];
+  for (int c0 = 0; c0 < count; c0 += kAhead) {
+    double v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) v[u] = c0 + u < count ? parts[(size_t)(c0 + u) * stride] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (c0 + u < count) s += v[u];
+  }
   return s;
 }
 
-// Block-wide sums of the first `count` entries of a per-thread vector; the
-// result is written to out[0..count) by threads 0..count-1.  One pass of warp
-// shuffles per entry and a single shared-memory exchange for all entries.
-template <int NV>
-__device__ __forceinline__ void block_sum_vec(double (&v)[NV], int count, double* out, int out_stride) {
-  __shared__ double sm[kWarps][NV];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    if (j < count) {
-      const double w = warp_sum(v[j]);
-      if (lane == 0) sm[warp][j] = w;
-    }
-  }
-  __syncthreads();
-  for (int j = threadIdx.x; j < count; j += blockDim.x) {
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) s += sm[w][j];
-    out[(size_t)j * out_stride] = s;
-  }
-  __syncthreads();
+// Block-wide sum of term(r) over r < rows, in kSumThreads lanes; all threads.
+template <typename F>
+__device__ __forceinline__ double chunk_sum(int rows, double* scratch, F term) {
+  double s = 0.0;
+  if (threadIdx.x < kSumThreads)
+    for (int r = threadIdx.x; r < rows; r += kSumThreads) s = term(r, s);
+  return block_sum(s, scratch);
 }
 
-constexpr int NV = 16;      // register block of per-thread partial sums
 constexpr int kMaxChunk = 4096;  // rows of a chunk staged in shared memory
 
 // out[j * out_stride] = sum_{r < rows} M[r + j*ld] * xs[r] for j < ncols, with xs
 // (the chunk's vector) in shared memory.  Warps take columns; when there are
-// fewer columns than warps, several warps split the rows of one column.  Each
-// lane streams consecutive rows, so every column read is coalesced.
+// fewer columns than kSumWarps, several warps split the rows of one column.  Each
+// lane streams consecutive rows, so every column read is coalesced, and takes
+// the eight rows of a 256-row stretch at once: a column is one wait for memory,
+// not one for each 64 rows (8000 x 100 in chunks of 250 rows: 19 us of a 45 us
+// launch went there).
 __device__ void chunk_dots(const double* __restrict__ M, size_t ld, int ncols,
                            const double* xs, int rows, double* out, int out_stride) {
-  __shared__ double red[kWarps];
+  __shared__ double red[kSumWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (ncols >= kWarps) {
-    for (int j = warp; j < ncols; j += kWarps) {
+  if (ncols >= kSumWarps) {
+    for (int j = warp; j < ncols; j += blockDim.x >> 5) {
       const double* col = M + (size_t)j * ld;
       double a0 = 0.0, a1 = 0.0;
-      int r = lane;
-      for (; r + 32 < rows; r += 64) {
-        a0 += col[r] * xs[r];
-        a1 += col[r + 32] * xs[r + 32];
+      for (int r0 = lane; r0 < rows; r0 += 256) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = r0 + 32 * u < rows ? col[r0 + 32 * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          const int r = r0 + 32 * u;
+          if (r + 32 < rows) {
+            a0 += v[u] * xs[r];
+            a1 += v[u + 1] * xs[r + 32];
+          } else if (r < rows) {
+            a0 += v[u] * xs[r];
+          }
+        }
       }
-      if (r < rows) a0 += col[r] * xs[r];
       const double acc = warp_sum(a0 + a1);
       if (lane == 0) out[(size_t)j * out_stride] = acc;
     }
     return;
   }
-  const int g = kWarps / max(ncols, 1);   // warps per column
+  const int g = kSumWarps / max(ncols, 1);   // warps per column
   const int j = warp / g, sub = warp % g;
   double acc = 0.0;
-  if (j < ncols) {
+  if (warp < kSumWarps && j < ncols) {
     const double* col = M + (size_t)j * ld;
+#pragma unroll 4
     for (int r = sub * 32 + lane; r < rows; r += 32 * g) acc += col[r] * xs[r];
   }
   acc = warp_sum(acc);
-  if (lane == 0) red[warp] = acc;
+  if (lane == 0 && warp < kSumWarps) red[warp] = acc;
   __syncthreads();
   if (threadIdx.x < ncols) {
     double t = 0.0;
@@ -144,9 +156,7 @@ __device__ __forceinline__ void chunk_StY(const Eng& e, int f, int chunk, const 
                                           bool norm_only) {
   if (norm_only) {
     __shared__ double scratch[32];
-    double s2 = 0.0;
-    for (int r = threadIdx.x; r < en - b; r += blockDim.x) s2 += ys[r] * ys[r];
-    s2 = block_sum(s2, scratch);
+    const double s2 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + ys[r] * ys[r]; });
     if (threadIdx.x == 0) e.npart[(size_t)f * e.cp + chunk] = s2;
     return;
   }
@@ -154,7 +164,7 @@ __device__ __forceinline__ void chunk_StY(const Eng& e, int f, int chunk, const 
 }
 
 // First component's refresh start: y = Omega (or the single column of S).
-__global__ void k_refresh_start(Eng e) {
+__global__ void __launch_bounds__(kMaxThreads) k_refresh_start(Eng e) {
   __shared__ double ys[kMaxChunk];
   const int f = blockIdx.y, chunk = blockIdx.x;
   if (e.status[f]) return;
@@ -172,7 +182,7 @@ __global__ void k_refresh_start(Eng e) {
 }
 
 // y <- S z with z = sum of the partials of S^T y; then the next partials (or ||y||^2).
-__global__ void k_refresh_apply(Eng e, const double* zin, double* zout, int last) {
+__global__ void __launch_bounds__(kMaxThreads) k_refresh_apply(Eng e, const double* zin, double* zout, int last) {
   extern __shared__ double zs[];
   __shared__ double ys[kMaxChunk];
   const int f = blockIdx.y, chunk = blockIdx.x;
@@ -186,7 +196,14 @@ __global__ void k_refresh_apply(Eng e, const double* zin, double* zout, int last
   double* yf = e.y + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     double acc = 0.0;
-    for (int j = 0; j < e.m; ++j) acc += Sf[i + (size_t)j * e.p] * zs[j];
+    for (int j0 = 0; j0 < e.m; j0 += kAhead) {
+      double v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) v[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.p] : 0.0;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (j0 + u < e.m) acc += v[u] * zs[j0 + u];
+    }
     yf[i] = acc;
     ys[i - b] = acc;
   }
@@ -196,7 +213,8 @@ __global__ void k_refresh_apply(Eng e, const double* zin, double* zout, int last
 
 // r = -sign(y0) y / ||y|| (Householder QR of a single column; the 1 x m core
 // SVD from gesvd keeps U = 1).  Rhat = colscale * r; cpart = delta . Rhat.
-__global__ void k_refresh_finish(Eng e) {
+__global__ void __launch_bounds__(kMaxThreads) k_refresh_finish(Eng e) {
+  __shared__ double rhs[kMaxChunk];
   __shared__ double scratch[32];
   const int f = blockIdx.y, chunk = blockIdx.x;
   if (e.status[f]) return;
@@ -212,22 +230,22 @@ __global__ void k_refresh_finish(Eng e) {
   const double sgn = (yf[0] >= 0.0) ? -1.0 : 1.0;
   const double* sc = e.colscale ? e.colscale + (size_t)f * e.p : nullptr;
   const double* dl = e.delta ? e.delta + (size_t)f * e.p : nullptr;
-  double c = 0.0;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     const double ri = sgn * yf[i] / nrm;
     e.r[(size_t)f * e.p + i] = ri;
     const double rh = sc ? ri * sc[i] : ri;
     e.Rhat[(size_t)f * e.p + i] = rh;
-    if (dl) c += dl[i] * rh;
+    rhs[i - b] = rh;
   }
   if (dl) {
-    c = block_sum(c, scratch);
+    __syncthreads();
+    const double c = chunk_sum(en - b, scratch, [&](int r, double s) { return s + dl[b + r] * rhs[r]; });
     if (threadIdx.x == 0) e.cpart[(size_t)f * e.cp + chunk] = c;
   }
 }
 
 // t = mask * (U - delta.rhat); partial sums of t^2, t and q = Y^T t.
-__global__ void k_scores(Eng e, int a) {
+__global__ void __launch_bounds__(kMaxThreads) k_scores(Eng e, int a) {
   extern __shared__ double qs[];
   __shared__ double ts[kMaxChunk];
   __shared__ double scratch[32];
@@ -244,19 +262,17 @@ __global__ void k_scores(Eng e, int a) {
     for (int j = threadIdx.x; j < e.m; j += blockDim.x) qs[j] = 0.0;
     __syncthreads();
   }
-  double s2 = 0.0, s1 = 0.0;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     const double u = Uf[i] - c;
     const double t = (mk && !mk[i]) ? 0.0 : u;
     Tf[i] = t;
     ts[i - b] = t;
     if (keep) keep[i] = u;
-    s2 += t * t;
-    s1 += t;
     if (e.labels && t != 0.0) atomicAdd(&qs[e.labels[i]], t);
   }
-  s2 = block_sum(s2, scratch);
-  s1 = block_sum(s1, scratch);
+  __syncthreads();
+  const double s2 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + ts[r] * ts[r]; });
+  const double s1 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + ts[r]; });
   if (threadIdx.x == 0) {
     e.tpart[((size_t)f * e.cn + chunk) * 2 + 0] = s2;
     e.tpart[((size_t)f * e.cn + chunk) * 2 + 1] = s1;
@@ -270,18 +286,13 @@ __global__ void k_scores(Eng e, int a) {
 }
 
 __device__ __forceinline__ void t_stats(const Eng& e, int f, double& tn, double& st) {
-  double s2 = 0.0, s1 = 0.0;
   const double* tp = e.tpart + (size_t)f * e.cn * 2;
-  for (int c = 0; c < e.cn; ++c) {
-    s2 += tp[2 * c];
-    s1 += tp[2 * c + 1];
-  }
-  tn = sqrt(s2);
-  st = s1;
+  tn = sqrt(sum_parts(tp, e.cn, 2));
+  st = sum_parts(tp + 1, e.cn, 2);
 }
 
 // p = colscale * (P - delta * sum(t)) / ||t||; partial w = V^T p.
-__global__ void k_loading(Eng e, int a) {
+__global__ void __launch_bounds__(kMaxThreads) k_loading(Eng e, int a) {
   __shared__ double ps[kMaxChunk];
   const int f = blockIdx.y, chunk = blockIdx.x;
   if (e.status[f]) return;
@@ -312,7 +323,7 @@ __global__ void k_loading(Eng e, int a) {
 }
 
 // v = p - V (V^T p); partials of ||v||^2 and of S^T v.
-__global__ void k_orth(Eng e, int a) {
+__global__ void __launch_bounds__(kMaxThreads) k_orth(Eng e, int a) {
   extern __shared__ double ws[];
   __shared__ double vsh[kMaxChunk];
   __shared__ double scratch[32];
@@ -326,21 +337,30 @@ __global__ void k_orth(Eng e, int a) {
   const double* Vf = e.V + (size_t)f * e.p * e.K;
   const double* pf = e.pv + (size_t)f * e.p;
   double* vf = e.v + (size_t)f * e.p;
-  double s2 = 0.0;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     double x = pf[i];
-    int l = 0;
-    for (; l + 4 <= a; l += 4) {
-      const double v0 = Vf[i + (size_t)l * e.p], v1 = Vf[i + (size_t)(l + 1) * e.p];
-      const double v2 = Vf[i + (size_t)(l + 2) * e.p], v3 = Vf[i + (size_t)(l + 3) * e.p];
-      x -= v0 * ws[l] + v1 * ws[l + 1] + v2 * ws[l + 2] + v3 * ws[l + 3];
+    for (int l0 = 0; l0 < a; l0 += kAhead) {
+      double v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) v[u] = l0 + u < a ? Vf[i + (size_t)(l0 + u) * e.p] : 0.0;
+#pragma unroll
+      for (int u = 0; u < kAhead; u += 4) {
+        const int l = l0 + u;
+        const double v0 = v[u], v1 = v[u + 1], v2 = v[u + 2], v3 = v[u + 3];
+        if (l + 4 <= a) {
+          x -= v0 * ws[l] + v1 * ws[l + 1] + v2 * ws[l + 2] + v3 * ws[l + 3];
+        } else {   // the last one to three columns one by one
+          if (l < a) x -= v0 * ws[l];
+          if (l + 1 < a) x -= v1 * ws[l + 1];
+          if (l + 2 < a) x -= v2 * ws[l + 2];
+        }
+      }
     }
-    for (; l < a; ++l) x -= Vf[i + (size_t)l * e.p] * ws[l];
     vf[i] = x;
     vsh[i - b] = x;
-    s2 += x * x;
   }
-  s2 = block_sum(s2, scratch);
+  __syncthreads();
+  const double s2 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + vsh[r] * vsh[r]; });
   if (threadIdx.x == 0) e.vpart[(size_t)f * e.cp + chunk] = s2;
   // S^T v (unnormalised) for the deflation.
   chunk_dots(e.S + (size_t)f * e.p * e.m + b, e.p, e.m, vsh, en - b,
@@ -350,7 +370,7 @@ __global__ void k_orth(Eng e, int a) {
 // v /= ||v||; V[:, a] = v; S -= v (v^T S); R[:, a] = r / ||t||; Q[:, a] = q / ||t||;
 // then the next component's refresh start (partials of S^T r_a over the
 // deflated S, or ||S[:,0]||^2 when m == 1).
-__global__ void k_deflate(Eng e, int a, int next) {
+__global__ void __launch_bounds__(kMaxThreads) k_deflate(Eng e, int a, int next) {
   extern __shared__ double vs[];
   __shared__ double ysh[kMaxChunk];
   const int f = blockIdx.y, chunk = blockIdx.x;
@@ -377,7 +397,25 @@ __global__ void k_deflate(Eng e, int a, int next) {
     const double vi = vf[i] / vn;
     vf[i] = vi;
     Vcol[i] = vi;
-    for (int j = 0; j < e.m; ++j) Sf[i + (size_t)j * e.p] -= vi * vs[j];
+    ysh[i - b] = vi;
+  }
+  __syncthreads();
+  // the rank-1 update, elementwise: one column group for each kSumThreads, side by
+  // side, eight columns of a row loaded before any is stored
+  const int group = threadIdx.x / kSumThreads, groups = blockDim.x / kSumThreads;
+  for (int i = b + threadIdx.x % kSumThreads; i < en; i += kSumThreads) {
+    const double vi = ysh[i - b];
+    for (int j0 = 8 * group; j0 < e.m; j0 += 8 * groups) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.p] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (j0 + u < e.m) Sf[i + (size_t)(j0 + u) * e.p] = x[u] - vi * vs[j0 + u];
+    }
+  }
+  __syncthreads();
+  for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     const double ri = rf[i] / tn;
     Rcol[i] = ri;
     if (next) {
@@ -521,10 +559,10 @@ void simpls_batch_crosscov(const SimplsBatch& b, const double* /*Xc*/, const int
   Eng e = make_eng(b);
   double* M = ctx.arena.alloc_n<double>((size_t)b.n * b.F * b.m);
   double* P = ctx.arena.alloc_n<double>((size_t)b.p * b.F * b.m);
-  k_masked_response<<<2 * ctx.sm_count, kThreads, 0, ctx.stream>>>(e, M); ::fpls::note_launch();
+  k_masked_response<<<8 * ctx.sm_count, 256, 0, ctx.stream>>>(e, M); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
   b.X->t_times(M, b.F * b.m, P);
-  k_crosscov_finish<<<2 * ctx.sm_count, kThreads, 0, ctx.stream>>>(e, P); ::fpls::note_launch();
+  k_crosscov_finish<<<8 * ctx.sm_count, 256, 0, ctx.stream>>>(e, P); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 
@@ -630,6 +668,13 @@ void simpls_batch_run(const SimplsBatch& b) {
   dzero(b.V, F * b.p * b.K * sizeof(double));
   dzero(b.tnorm, F * b.K * sizeof(double));
   const dim3 gp(e.cp, b.F), gn(e.cn, b.F);
+  // Four warp columns at a time for every block of columns a kernel multiplies:
+  // 256 threads up to 32 columns (60 fits of a grid fill the SMs with blocks as
+  // it is, and 1024-thread ones took 35 us instead of 10 for their class scores),
+  // then 512, then 1024.
+  auto block = [](int cols) { return cols <= 32 ? 256 : cols <= 64 ? 512 : kMaxThreads; };
+  const int tm = block(b.m), tq = b.labels ? 256 : tm;
+  constexpr int kThreads = 256;   // elementwise kernels
   // all-reduce buffer of a row-sharded fit: [P (F x p) | t^T t, sum t (F x 2) | Y^T t (F x m)]
   const size_t shard_count = sharded() ? F * ((size_t)b.p + 2 + b.m) : 0;
   double* shard_red = shard_count ? ar.alloc_n<double>(shard_count) : nullptr;
@@ -660,7 +705,7 @@ void simpls_batch_run(const SimplsBatch& b) {
   const bool eligible = simpls_graph_enabled() && !trace && !ctx.profile && !shard_red;
   const bool graph = eligible && simpls_seen().count(key) > 0;
   auto loop = [&]() {
-  k_refresh_start<<<gp, kThreads, 0, st>>>(e); ::fpls::note_launch();
+  k_refresh_start<<<gp, tm, 0, st>>>(e); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
   for (int a = 0; a < b.K; ++a) {
     // Refresh: y <- S (S^T y) `iters` times from the warm start, then normalise.
@@ -668,7 +713,7 @@ void simpls_batch_run(const SimplsBatch& b) {
     double* zout = e.zB;
     for (int it = 0; it < e.iters; ++it) {
       const int last = (it == e.iters - 1) ? 1 : 0;
-      k_refresh_apply<<<gp, kThreads, sm_m, st>>>(e, zin, zout, last); ::fpls::note_launch();
+      k_refresh_apply<<<gp, tm, sm_m, st>>>(e, zin, zout, last); ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
       std::swap(zin, zout);
     }
@@ -677,7 +722,7 @@ void simpls_batch_run(const SimplsBatch& b) {
     mark("refresh");
     b.X->times(e.Rhat, b.F, e.U);
     mark("X*R");
-    k_scores<<<gn, kThreads, b.labels ? sm_m : 0, st>>>(e, a); ::fpls::note_launch();
+    k_scores<<<gn, tq, b.labels ? sm_m : 0, st>>>(e, a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("scores");
     b.X->t_times(e.T, b.F, e.P);
@@ -689,13 +734,13 @@ void simpls_batch_run(const SimplsBatch& b) {
       FPLS_CHECK_LAUNCH();
     }
     mark("X^T*T");
-    k_loading<<<gp, kThreads, 0, st>>>(e, a); ::fpls::note_launch();
+    k_loading<<<gp, block(a), 0, st>>>(e, a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("loading");
-    k_orth<<<gp, kThreads, sm_k, st>>>(e, a); ::fpls::note_launch();
+    k_orth<<<gp, tm, sm_k, st>>>(e, a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("orth");
-    k_deflate<<<gp, kThreads, sm_m, st>>>(e, a, a + 1 < b.K ? 1 : 0); ::fpls::note_launch();
+    k_deflate<<<gp, tm, sm_m, st>>>(e, a, a + 1 < b.K ? 1 : 0); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("deflate");
   }
