@@ -6,6 +6,7 @@
 
 #include "context.cuh"
 #include "gemm_f64.cuh"
+#include "gemv_f64.cuh"
 
 namespace fpls {
 namespace {
@@ -21,15 +22,12 @@ __global__ void scale_matrix_kernel(double* C, int M, int N, int ldc, double bet
   }
 }
 
-// Matrix-vector products: kGemvAhead loads of the matrix go out before they are
-// multiplied (in order).  Four at a time, a 400 x 2000 product waited 63 times
-// for L2 (69 us); 32 at a time it waits eight times.
 constexpr int kGemvAhead = 32;
 
 // y[m] = alpha * sum_k A[m + k*lda] x[k] (+ beta y); grid.y splits K into partials.
-__global__ void gemv_n_kernel(int M, int K, double alpha, const double* __restrict__ A, int lda,
-                              const double* __restrict__ x, double* __restrict__ y,
-                              int k_per_split, long long split_stride, double beta) {
+__global__ void __launch_bounds__(kGemvRows) gemv_n_kernel(int M, int K, double alpha, const double* __restrict__ A, int lda,
+                                                           const double* __restrict__ x, double* __restrict__ y,
+                                                           int k_per_split, long long split_stride, double beta) {
   __shared__ double xs[256];
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   const int kbeg = blockIdx.y * k_per_split;
@@ -40,17 +38,7 @@ __global__ void gemv_n_kernel(int M, int K, double alpha, const double* __restri
     __syncthreads();
     if (threadIdx.x < kn) xs[threadIdx.x] = x[kc + threadIdx.x];
     __syncthreads();
-    if (m < M) {
-      const double* ap = A + m + (size_t)kc * lda;
-      for (int k = 0; k < kn; k += kGemvAhead) {
-        double v[kGemvAhead];
-#pragma unroll
-        for (int u = 0; u < kGemvAhead; ++u) v[u] = k + u < kn ? __ldg(ap + (size_t)(k + u) * lda) : 0.0;
-#pragma unroll
-        for (int u = 0; u < kGemvAhead; ++u)
-          if (k + u < kn) acc = fma(v[u], xs[k + u], acc);
-      }
-    }
+    if (m < M) acc = gemv_row<kGemvAhead>(A + m + (size_t)kc * lda, lda, xs, kn, acc);
   }
   if (m < M) {
     if (split_stride) y[(size_t)blockIdx.y * split_stride + m] = alpha * acc;
@@ -76,24 +64,12 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ W, int splits, l
 }
 
 // y[n] = alpha * sum_k A[k + n*lda] x[k] + beta y[n] ; one warp per column.
-__global__ void gemv_t_kernel(int K, int N, double alpha, const double* __restrict__ A, int lda,
-                              const double* __restrict__ x, double beta, double* __restrict__ y) {
-  const int warps_per_block = blockDim.x >> 5;
-  const int n = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(128) gemv_t_kernel(int K, int N, double alpha, const double* __restrict__ A, int lda,
+                                                     const double* __restrict__ x, double beta, double* __restrict__ y) {
+  const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= N) return;
-  const double* ap = A + (size_t)n * lda;
-  double acc = 0.0;
-  for (int k0 = lane; k0 < K; k0 += 32 * kGemvAhead) {
-    double v[kGemvAhead];
-#pragma unroll
-    for (int u = 0; u < kGemvAhead; ++u) v[u] = k0 + 32 * u < K ? __ldg(ap + k0 + 32 * u) : 0.0;
-#pragma unroll
-    for (int u = 0; u < kGemvAhead; ++u)
-      if (k0 + 32 * u < K) acc = fma(v[u], __ldg(x + k0 + 32 * u), acc);
-  }
-  acc = warp_sum(acc);
-  if (lane == 0) y[n] = (beta == 0.0) ? alpha * acc : alpha * acc + beta * y[n];
+  const double acc = gemv_column<kGemvAhead>(A + (size_t)n * lda, x, K);
+  if ((threadIdx.x & 31) == 0) y[n] = (beta == 0.0) ? alpha * acc : alpha * acc + beta * y[n];
 }
 
 // Per-column sums over rows: one warp a column, lane l adds the rows l, l + 32, ...
@@ -489,12 +465,8 @@ void gemv(bool trans, int rows, int cols, double alpha, const double* A, int lda
       FPLS_CHECK_LAUNCH();
       return;
     }
-    const int gx = ceil_div(rows, 256);
-    int splits = 1;
-    const int target = 4 * Context::get().sm_count;
-    if (gx < target) splits = std::max(1, std::min(ceil_div(target, gx), ceil_div(cols, 256)));
-    int kps = ceil_div(cols, splits);
-    splits = ceil_div(cols, kps);
+    const GemvRanges gr = gemv_ranges(rows, cols, ctx.sm_count);
+    const int gx = gr.row_blocks, splits = gr.splits, kps = gr.kps;
     if (splits > 1) {
       // partials of the column ranges, summed in order (runs repeat bit for bit)
       double* ws = ctx.splitk_workspace(st, (size_t)splits * rows);

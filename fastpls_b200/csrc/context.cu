@@ -83,6 +83,8 @@ Context& Context::get() {
     FPLS_CUDA(cudaStreamCreateWithFlags(&ctx.copy, cudaStreamNonBlocking));
     FPLS_CUDA(cudaMalloc(&ctx.d_status, 64 * sizeof(int)));
     FPLS_CUDA(cudaMemset(ctx.d_status, 0, 64 * sizeof(int)));
+    FPLS_CUDA(cudaHostAlloc(&ctx.host_fail, sizeof(int), cudaHostAllocMapped));
+    *ctx.host_fail = 0;
     ctx.device = dev;
   }
   return ctx;
@@ -97,6 +99,7 @@ long long launch_count() { return g_launches; }
 
 void Context::begin_call() {
   arena.reset();
+  *host_fail = 0;
   if (!call_start) {
     FPLS_CUDA(cudaEventCreate(&call_start));
     FPLS_CUDA(cudaEventCreate(&call_stop));
@@ -114,6 +117,7 @@ void Context::end_call() {
   float ms = 0.f;
   FPLS_CUDA(cudaEventElapsedTime(&ms, call_start, call_stop));
   last_call_ms = ms;
+  if (*static_cast<volatile int*>(host_fail)) throw Error(kErrCuda, "a grid barrier wait exceeded its limit");
 }
 
 int Context::read_status() {

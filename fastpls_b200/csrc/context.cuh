@@ -47,6 +47,7 @@ struct Context {
   cudaEvent_t copy_event(int i);   // i-th event of the copy stream (created on first use)
   Arena arena;
   int* d_status = nullptr;     // device-side failure flag (0 = ok)
+  int* host_fail = nullptr;    // mapped host flag: a bounded grid-barrier wait of this call gave up
   int sm_count = kSMCount;
   int precision = 0;           // session precision of single fits: 0 FP64, 1 BF16x3 (predictor GEMMs)
   // Timing of the last ABI call (events on `stream`, bracketing the whole call).

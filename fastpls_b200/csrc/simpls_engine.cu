@@ -1,5 +1,6 @@
 #include "blas_f64.cuh"
 #include "context.cuh"
+#include "gemv_f64.cuh"
 #include "simpls_engine.cuh"
 
 #include <algorithm>
@@ -25,6 +26,7 @@ constexpr int kAhead = 16;    // loads of one thread that go out before they are
 
 struct Eng {
   int n, p, m, F, K, cp, cn, szp, szn;
+  int lds;         // leading dimension of S and V: p, or a chunk's own copy
   const double* Yg;
   const int* labels;
   const double* mY_all;
@@ -62,6 +64,8 @@ struct Eng {
   double* v;       // F x p
   double* vpart;   // F x cp
   double* vSpart;  // F x cp x m
+  double* upart;   // usplits x n partials of U (one-launch loop)
+  int usplits;     // 0: U holds the sums
 };
 
 __device__ __forceinline__ void chunk_range(int chunk, int sz, int total, int& b, int& e) {
@@ -85,13 +89,22 @@ __device__ __forceinline__ double sum_parts(const double* parts, int count, int 
   return s;
 }
 
-// Block-wide sum of term(r) over r < rows, in kSumThreads lanes; all threads.
+// Block-wide sum of term(r) over r < rows, in kSumThreads lanes and warp order;
+// all threads.
 template <typename F>
 __device__ __forceinline__ double chunk_sum(int rows, double* scratch, F term) {
   double s = 0.0;
-  if (threadIdx.x < kSumThreads)
+  if (threadIdx.x < kSumThreads) {
     for (int r = threadIdx.x; r < rows; r += kSumThreads) s = term(r, s);
-  return block_sum(s, scratch);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = s;
+  }
+  __syncthreads();
+  double r = 0.0;
+#pragma unroll
+  for (int i = 0; i < kSumWarps; ++i) r += scratch[i];
+  __syncthreads();
+  return r;
 }
 
 constexpr int kMaxChunk = 4096;  // rows of a chunk staged in shared memory
@@ -103,7 +116,7 @@ constexpr int kMaxChunk = 4096;  // rows of a chunk staged in shared memory
 // the eight rows of a 256-row stretch at once: a column is one wait for memory,
 // not one for each 64 rows (8000 x 100 in chunks of 250 rows: 19 us of a 45 us
 // launch went there).
-__device__ void chunk_dots(const double* __restrict__ M, size_t ld, int ncols,
+__device__ void chunk_dots(const double* M, size_t ld, int ncols,
                            const double* xs, int rows, double* out, int out_stride) {
   __shared__ double red[kSumWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -136,8 +149,14 @@ __device__ void chunk_dots(const double* __restrict__ M, size_t ld, int ncols,
   double acc = 0.0;
   if (warp < kSumWarps && j < ncols) {
     const double* col = M + (size_t)j * ld;
-#pragma unroll 4
-    for (int r = sub * 32 + lane; r < rows; r += 32 * g) acc += col[r] * xs[r];
+    for (int r0 = sub * 32 + lane; r0 < rows; r0 += 256 * g) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = r0 + 32 * g * u < rows ? col[r0 + 32 * g * u] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r0 + 32 * g * u < rows) acc += v[u] * xs[r0 + 32 * g * u];
+    }
   }
   acc = warp_sum(acc);
   if (lane == 0 && warp < kSumWarps) red[warp] = acc;
@@ -160,17 +179,14 @@ __device__ __forceinline__ void chunk_StY(const Eng& e, int f, int chunk, const 
     if (threadIdx.x == 0) e.npart[(size_t)f * e.cp + chunk] = s2;
     return;
   }
-  chunk_dots(Sf + b, e.p, e.m, ys, en - b, zout + ((size_t)f * e.cp + chunk) * e.m, 1);
+  chunk_dots(Sf + b, e.lds, e.m, ys, en - b, zout + ((size_t)f * e.cp + chunk) * e.m, 1);
 }
 
 // First component's refresh start: y = Omega (or the single column of S).
-__global__ void __launch_bounds__(kMaxThreads) k_refresh_start(Eng e) {
-  __shared__ double ys[kMaxChunk];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+__device__ __forceinline__ void refresh_start_chunk(const Eng& e, int f, int chunk, double* ys) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
-  const double* Sf = e.S + (size_t)f * e.p * e.m;
+  const double* Sf = e.S + (size_t)f * e.lds * e.m;
   const double* y0 = e.m1_mode ? Sf : e.omega + (size_t)f * e.p;
   double* yf = e.y + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
@@ -181,25 +197,35 @@ __global__ void __launch_bounds__(kMaxThreads) k_refresh_start(Eng e) {
   chunk_StY(e, f, chunk, Sf, ys, b, en, e.zA, e.iters == 0);
 }
 
+__global__ void __launch_bounds__(kMaxThreads) k_refresh_start(Eng e) {
+  __shared__ double vec[kMaxChunk];
+  if (e.status[blockIdx.y]) return;
+  refresh_start_chunk(e, blockIdx.y, blockIdx.x, vec);
+}
+
 // y <- S z with z = sum of the partials of S^T y; then the next partials (or ||y||^2).
-__global__ void __launch_bounds__(kMaxThreads) k_refresh_apply(Eng e, const double* zin, double* zout, int last) {
-  extern __shared__ double zs[];
-  __shared__ double ys[kMaxChunk];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+__device__ __forceinline__ void refresh_apply_chunk(const Eng& e, const double* zin, double* zout, int last, int f, int chunk, double* zs, double* ys) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
+  const double* Sf = e.S + (size_t)f * e.lds * e.m;
+  double* yf = e.y + (size_t)f * e.p;
+  // the first columns of this thread's row are on their way while z is summed
+  double v[kAhead];
+  {
+    const int i = b + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) v[u] = i < en && u < e.m ? Sf[i + (size_t)u * e.lds] : 0.0;
+  }
   for (int j = threadIdx.x; j < e.m; j += blockDim.x)
     zs[j] = sum_parts(zin + (size_t)f * e.cp * e.m + j, e.cp, e.m);
   __syncthreads();
-  const double* Sf = e.S + (size_t)f * e.p * e.m;
-  double* yf = e.y + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     double acc = 0.0;
     for (int j0 = 0; j0 < e.m; j0 += kAhead) {
-      double v[kAhead];
+      if (j0 > 0 || i >= b + (int)blockDim.x) {
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) v[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.p] : 0.0;
+        for (int u = 0; u < kAhead; ++u) v[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.lds] : 0.0;
+      }
 #pragma unroll
       for (int u = 0; u < kAhead; ++u)
         if (j0 + u < e.m) acc += v[u] * zs[j0 + u];
@@ -211,13 +237,16 @@ __global__ void __launch_bounds__(kMaxThreads) k_refresh_apply(Eng e, const doub
   chunk_StY(e, f, chunk, Sf, ys, b, en, zout, last != 0);
 }
 
+__global__ void __launch_bounds__(kMaxThreads) k_refresh_apply(Eng e, const double* zin, double* zout, int last) {
+  extern __shared__ double coef[];
+  __shared__ double vec[kMaxChunk];
+  if (e.status[blockIdx.y]) return;
+  refresh_apply_chunk(e, zin, zout, last, blockIdx.y, blockIdx.x, coef, vec);
+}
+
 // r = -sign(y0) y / ||y|| (Householder QR of a single column; the 1 x m core
 // SVD from gesvd keeps U = 1).  Rhat = colscale * r; cpart = delta . Rhat.
-__global__ void __launch_bounds__(kMaxThreads) k_refresh_finish(Eng e) {
-  __shared__ double rhs[kMaxChunk];
-  __shared__ double scratch[32];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+__device__ __forceinline__ void refresh_finish_chunk(const Eng& e, int f, int chunk, double* rhs, double* scratch) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
   const double nrm = sqrt(sum_parts(e.npart + (size_t)f * e.cp, e.cp, 1));
@@ -244,13 +273,15 @@ __global__ void __launch_bounds__(kMaxThreads) k_refresh_finish(Eng e) {
   }
 }
 
-// t = mask * (U - delta.rhat); partial sums of t^2, t and q = Y^T t.
-__global__ void __launch_bounds__(kMaxThreads) k_scores(Eng e, int a) {
-  extern __shared__ double qs[];
-  __shared__ double ts[kMaxChunk];
+__global__ void __launch_bounds__(kMaxThreads) k_refresh_finish(Eng e) {
+  __shared__ double vec[kMaxChunk];
   __shared__ double scratch[32];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+  if (e.status[blockIdx.y]) return;
+  refresh_finish_chunk(e, blockIdx.y, blockIdx.x, vec, scratch);
+}
+
+// t = mask * (U - delta.rhat); partial sums of t^2, t and q = Y^T t.
+__device__ __forceinline__ void scores_chunk(const Eng& e, int a, int f, int chunk, double* qs, double* ts, double* scratch) {
   int b, en;
   chunk_range(chunk, e.szn, e.n, b, en);
   const double c = e.delta ? sum_parts(e.cpart + (size_t)f * e.cp, e.cp, 1) : 0.0;
@@ -263,7 +294,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_scores(Eng e, int a) {
     __syncthreads();
   }
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    const double u = Uf[i] - c;
+    const double u = (e.usplits > 1 ? sum_parts(e.upart + i, e.usplits, e.n) : Uf[i]) - c;
     const double t = (mk && !mk[i]) ? 0.0 : u;
     Tf[i] = t;
     ts[i - b] = t;
@@ -285,31 +316,50 @@ __global__ void __launch_bounds__(kMaxThreads) k_scores(Eng e, int a) {
   chunk_dots(e.Yg + b, e.n, e.m, ts, en - b, qp, 1);
 }
 
+__global__ void __launch_bounds__(kMaxThreads) k_scores(Eng e, int a) {
+  extern __shared__ double coef[];
+  __shared__ double vec[kMaxChunk];
+  __shared__ double scratch[32];
+  if (e.status[blockIdx.y]) return;
+  scores_chunk(e, a, blockIdx.y, blockIdx.x, coef, vec, scratch);
+}
+
 __device__ __forceinline__ void t_stats(const Eng& e, int f, double& tn, double& st) {
-  const double* tp = e.tpart + (size_t)f * e.cn * 2;
-  tn = sqrt(sum_parts(tp, e.cn, 2));
-  st = sum_parts(tp + 1, e.cn, 2);
+  const double2* tp = reinterpret_cast<const double2*>(e.tpart) + (size_t)f * e.cn;
+  double s2 = 0.0, s1 = 0.0;
+  for (int c0 = 0; c0 < e.cn; c0 += kAhead / 2) {
+    double2 v[kAhead / 2];
+#pragma unroll
+    for (int u = 0; u < kAhead / 2; ++u) v[u] = c0 + u < e.cn ? tp[c0 + u] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < kAhead / 2; ++u) {
+      if (c0 + u < e.cn) {
+        s2 += v[u].x;
+        s1 += v[u].y;
+      }
+    }
+  }
+  tn = sqrt(s2);
+  st = s1;
 }
 
 // p = colscale * (P - delta * sum(t)) / ||t||; partial w = V^T p.
-__global__ void __launch_bounds__(kMaxThreads) k_loading(Eng e, int a) {
-  __shared__ double ps[kMaxChunk];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+__device__ __forceinline__ void loading_chunk(const Eng& e, int a, int f, int chunk, double* ps) {
+  int b, en;
+  chunk_range(chunk, e.szp, e.p, b, en);
+  const double* Pf = e.P + (size_t)f * e.p;
+  const double p0 = b + (int)threadIdx.x < en ? Pf[b + threadIdx.x] : 0.0;   // on its way during the sums
   double tn, st;
   t_stats(e, f, tn, st);
   if (!(tn > 0.0) || !isfinite(tn)) {
     if (chunk == 0 && threadIdx.x == 0) e.status[f] = 1;
     return;
   }
-  int b, en;
-  chunk_range(chunk, e.szp, e.p, b, en);
   const double* sc = e.colscale ? e.colscale + (size_t)f * e.p : nullptr;
   const double* dl = e.delta ? e.delta + (size_t)f * e.p : nullptr;
-  const double* Pf = e.P + (size_t)f * e.p;
   double* pf = e.pv + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    double v = Pf[i];
+    double v = i < b + (int)blockDim.x ? p0 : Pf[i];
     if (dl) v -= dl[i] * st;
     if (sc) v *= sc[i];
     v /= tn;
@@ -318,31 +368,42 @@ __global__ void __launch_bounds__(kMaxThreads) k_loading(Eng e, int a) {
   }
   __syncthreads();
   if (a > 0)
-    chunk_dots(e.V + (size_t)f * e.p * e.K + b, e.p, a, ps, en - b,
+    chunk_dots(e.V + (size_t)f * e.lds * e.K + b, e.lds, a, ps, en - b,
                e.wpart + ((size_t)f * e.cp + chunk) * e.K, 1);
 }
 
+__global__ void __launch_bounds__(kMaxThreads) k_loading(Eng e, int a) {
+  __shared__ double vec[kMaxChunk];
+  if (e.status[blockIdx.y]) return;
+  loading_chunk(e, a, blockIdx.y, blockIdx.x, vec);
+}
+
 // v = p - V (V^T p); partials of ||v||^2 and of S^T v.
-__global__ void __launch_bounds__(kMaxThreads) k_orth(Eng e, int a) {
-  extern __shared__ double ws[];
-  __shared__ double vsh[kMaxChunk];
-  __shared__ double scratch[32];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+__device__ __forceinline__ void orth_chunk(const Eng& e, int a, int f, int chunk, double* ws, double* vsh, double* scratch) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
+  const double* Vf = e.V + (size_t)f * e.lds * e.K;
+  const double* pf = e.pv + (size_t)f * e.p;
+  double* vf = e.v + (size_t)f * e.p;
+  // this thread's row is on its way while w is summed
+  double v[kAhead], x0 = 0.0;
+  {
+    const int i = b + threadIdx.x;
+    if (i < en) x0 = pf[i];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) v[u] = i < en && u < a ? Vf[i + (size_t)u * e.lds] : 0.0;
+  }
   for (int l = threadIdx.x; l < a; l += blockDim.x)
     ws[l] = sum_parts(e.wpart + (size_t)f * e.cp * e.K + l, e.cp, e.K);
   __syncthreads();
-  const double* Vf = e.V + (size_t)f * e.p * e.K;
-  const double* pf = e.pv + (size_t)f * e.p;
-  double* vf = e.v + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    double x = pf[i];
+    const bool first = i < b + (int)blockDim.x;
+    double x = first ? x0 : pf[i];
     for (int l0 = 0; l0 < a; l0 += kAhead) {
-      double v[kAhead];
+      if (l0 > 0 || !first) {
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) v[u] = l0 + u < a ? Vf[i + (size_t)(l0 + u) * e.p] : 0.0;
+        for (int u = 0; u < kAhead; ++u) v[u] = l0 + u < a ? Vf[i + (size_t)(l0 + u) * e.lds] : 0.0;
+      }
 #pragma unroll
       for (int u = 0; u < kAhead; u += 4) {
         const int l = l0 + u;
@@ -363,60 +424,71 @@ __global__ void __launch_bounds__(kMaxThreads) k_orth(Eng e, int a) {
   const double s2 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + vsh[r] * vsh[r]; });
   if (threadIdx.x == 0) e.vpart[(size_t)f * e.cp + chunk] = s2;
   // S^T v (unnormalised) for the deflation.
-  chunk_dots(e.S + (size_t)f * e.p * e.m + b, e.p, e.m, vsh, en - b,
+  chunk_dots(e.S + (size_t)f * e.lds * e.m + b, e.lds, e.m, vsh, en - b,
              e.vSpart + ((size_t)f * e.cp + chunk) * e.m, 1);
+}
+
+__global__ void __launch_bounds__(kMaxThreads) k_orth(Eng e, int a) {
+  extern __shared__ double coef[];
+  __shared__ double vec[kMaxChunk];
+  __shared__ double scratch[32];
+  if (e.status[blockIdx.y]) return;
+  orth_chunk(e, a, blockIdx.y, blockIdx.x, coef, vec, scratch);
 }
 
 // v /= ||v||; V[:, a] = v; S -= v (v^T S); R[:, a] = r / ||t||; Q[:, a] = q / ||t||;
 // then the next component's refresh start (partials of S^T r_a over the
 // deflated S, or ||S[:,0]||^2 when m == 1).
-__global__ void __launch_bounds__(kMaxThreads) k_deflate(Eng e, int a, int next) {
-  extern __shared__ double vs[];
-  __shared__ double ysh[kMaxChunk];
-  const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;
+__device__ __forceinline__ void deflate_chunk(const Eng& e, int a, int next, int f, int chunk, double* vs, double* ysh) {
+  int b, en;
+  chunk_range(chunk, e.szp, e.p, b, en);
+  double* Sf = e.S + (size_t)f * e.lds * e.m;
+  double* vf = e.v + (size_t)f * e.p;
+  double* Vcol = e.V + ((size_t)f * e.K + a) * e.lds;
+  double* Rcol = e.R + ((size_t)f * e.K + a) * e.p;
+  const double* rf = e.r + (size_t)f * e.p;
+  double* yf = e.y + (size_t)f * e.p;
+  // The rows' own values are on their way while the partials are summed: v and r
+  // of row threadIdx.x, and the first eight columns of S that this thread updates
+  // (one column group for each kSumThreads).
+  const int group = threadIdx.x / kSumThreads, groups = blockDim.x / kSumThreads;
+  const int i0 = b + threadIdx.x, s0 = b + threadIdx.x % kSumThreads;
+  const double v0 = i0 < en ? vf[i0] : 0.0, r0 = i0 < en ? rf[i0] : 0.0;
+  double x[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) x[u] = s0 < en && 8 * group + u < e.m ? Sf[s0 + (size_t)(8 * group + u) * e.lds] : 0.0;
+  for (int j = threadIdx.x; j < e.m; j += blockDim.x) vs[j] = sum_parts(e.vSpart + (size_t)f * e.cp * e.m + j, e.cp, e.m);
+  double tn, st;
+  t_stats(e, f, tn, st);
   const double vn = sqrt(sum_parts(e.vpart + (size_t)f * e.cp, e.cp, 1));
   if (!(vn > 0.0) || !isfinite(vn)) {
     if (chunk == 0 && threadIdx.x == 0) e.status[f] = 1;
     return;
   }
-  int b, en;
-  chunk_range(chunk, e.szp, e.p, b, en);
-  for (int j = threadIdx.x; j < e.m; j += blockDim.x)
-    vs[j] = sum_parts(e.vSpart + (size_t)f * e.cp * e.m + j, e.cp, e.m) / vn;
-  __syncthreads();
-  double tn, st;
-  t_stats(e, f, tn, st);
-  double* Sf = e.S + (size_t)f * e.p * e.m;
-  double* vf = e.v + (size_t)f * e.p;
-  double* Vcol = e.V + ((size_t)f * e.K + a) * e.p;
-  double* Rcol = e.R + ((size_t)f * e.K + a) * e.p;
-  const double* rf = e.r + (size_t)f * e.p;
-  double* yf = e.y + (size_t)f * e.p;
-  for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    const double vi = vf[i] / vn;
+  for (int j = threadIdx.x; j < e.m; j += blockDim.x) vs[j] /= vn;
+  for (int i = i0; i < en; i += blockDim.x) {
+    const double vi = (i == i0 ? v0 : vf[i]) / vn;
     vf[i] = vi;
     Vcol[i] = vi;
     ysh[i - b] = vi;
   }
   __syncthreads();
-  // the rank-1 update, elementwise: one column group for each kSumThreads, side by
-  // side, eight columns of a row loaded before any is stored
-  const int group = threadIdx.x / kSumThreads, groups = blockDim.x / kSumThreads;
-  for (int i = b + threadIdx.x % kSumThreads; i < en; i += kSumThreads) {
+  // the rank-1 update, elementwise, eight columns of a row loaded before any is stored
+  for (int i = s0; i < en; i += kSumThreads) {
     const double vi = ysh[i - b];
     for (int j0 = 8 * group; j0 < e.m; j0 += 8 * groups) {
-      double x[8];
+      if (i > s0 || j0 > 8 * group) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) x[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.p] : 0.0;
+        for (int u = 0; u < 8; ++u) x[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.lds] : 0.0;
+      }
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        if (j0 + u < e.m) Sf[i + (size_t)(j0 + u) * e.p] = x[u] - vi * vs[j0 + u];
+        if (j0 + u < e.m) Sf[i + (size_t)(j0 + u) * e.lds] = x[u] - vi * vs[j0 + u];
     }
   }
   __syncthreads();
-  for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    const double ri = rf[i] / tn;
+  for (int i = i0; i < en; i += blockDim.x) {
+    const double ri = (i == i0 ? r0 : rf[i]) / tn;
     Rcol[i] = ri;
     if (next) {
       const double y0 = e.m1_mode ? Sf[i] : ri;
@@ -442,6 +514,187 @@ __global__ void __launch_bounds__(kMaxThreads) k_deflate(Eng e, int a, int next)
   if (next) {
     __syncthreads();
     chunk_StY(e, f, chunk, Sf, ysh, b, en, e.zA, e.iters == 0);
+  }
+}
+
+__global__ void __launch_bounds__(kMaxThreads) k_deflate(Eng e, int a, int next) {
+  extern __shared__ double coef[];
+  __shared__ double vec[kMaxChunk];
+  if (e.status[blockIdx.y]) return;
+  deflate_chunk(e, a, next, blockIdx.y, blockIdx.x, coef, vec);
+}
+
+// ---- The component loop of one small fit in one launch -----------------------
+// A fit of a few hundred samples spends its time between kernels: eleven launches
+// a component, 5.2 us each inside a graph, for phases that move a few hundred
+// kilobytes of L2.  Here the phases are the same chunk bodies (sums in the same
+// order: the results are those of the launches bit for bit) with a grid barrier
+// between them, eight a component: the split sums of X r and the normalisation of
+// r are folded into the phases that read them, and a block keeps its chunk of S,
+// V and the p-vectors in shared memory.  400 x 2000, 5 responses: 57 us a component
+// as a graph of launches, 40 us now (1.2 us a barrier, about 3.5 us a phase).
+struct LoopArgs {
+  Eng e;
+  const double* X;    // n x p
+  GemvRanges xr;      // ranges of X r
+  int coef_len;       // doubles of dynamic shared memory before the X tile
+  unsigned* barrier;  // zero at the start
+  unsigned* stop;     // barrier after which a stopped fit leaves (all ones: none)
+  int* fail;          // a barrier wait gave up
+  int* host_fail;     // the same for the host (mapped)
+};
+
+// Threads of a block: a chunk has 250 rows or so, and more warps only add issue
+// slots spent on predicated-off loads (1024 threads: 48 us a component).
+constexpr int kLoopThreads = 256;
+constexpr int kLoopWarps = kLoopThreads / 32;
+constexpr size_t kLoopSmem = 190 * 1024;             // beside the static arrays
+constexpr long long kBarrierClocks = 4000000000ll;   // about two seconds
+
+// Every CTA of the (cooperative) grid has arrived `count` times; false when a
+// wait ran out, in every thread of every CTA sooner or later.
+__device__ bool grid_barrier(const LoopArgs& g, unsigned count) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(g.barrier, 1u);
+    const long long t0 = clock64();
+    ok = 1;
+    while (true) {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(g.barrier) : "memory");
+      if (seen >= count * gridDim.x) break;
+      if (*(volatile int*)g.fail || clock64() - t0 > kBarrierClocks) {
+        atomicExch(g.fail, 1);
+        *(volatile int*)g.host_fail = 1;
+        ok = 0;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+__global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
+  extern __shared__ double coef[];   // max(m, K)
+  __shared__ double vec[kMaxChunk];
+  __shared__ double scratch[32];
+  const Eng& e = g.e;
+  unsigned arrived = 0;
+  // The block's own chunk of S, V and the p-vectors stays in shared memory for the
+  // whole loop (a chunk a block): what a phase waits for in L2 is other blocks'
+  // partials only.
+  double* tile = coef + g.coef_len;            // [256][32]
+  double* own = tile + 256 * 32;
+  Eng l = e;
+  int b = 0, en = 0;
+  if (blockIdx.x < e.cp) chunk_range(blockIdx.x, e.szp, e.p, b, en);
+  l.lds = e.szp;
+  l.S = own - b;
+  l.V = own + (size_t)e.szp * e.m - b;
+  double* vecs = own + (size_t)e.szp * (e.m + e.K);
+  l.y = vecs - b;
+  l.r = vecs + e.szp - b;
+  l.pv = vecs + 2 * e.szp - b;
+  l.v = vecs + 3 * e.szp - b;
+  for (int j = threadIdx.x >> 5; j < e.m; j += kLoopThreads / 32)
+    for (int i = b + (threadIdx.x & 31); i < en; i += 32) l.S[i + (size_t)j * l.lds] = e.S[i + (size_t)j * e.p];
+  __syncthreads();
+  // A phase over `count` chunks; false: leave (a wait gave up, or the fit stopped).
+  // Block 0 has chunk 0, which raises the status: it names the barrier that ends
+  // this phase, so that a block still on its way from the one before does not
+  // leave early.
+  auto phase = [&](int count, auto body) {
+    for (int c = blockIdx.x; c < count; c += gridDim.x) {
+      body(c);
+      __syncthreads();   // the next chunk reuses the shared arrays
+    }
+    ++arrived;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && e.status[0] != 0) *(volatile unsigned*)g.stop = arrived;
+    if (!grid_barrier(g, arrived)) return false;
+    return *(volatile unsigned*)g.stop > arrived;
+  };
+  if (!phase(e.cp, [&](int c) { refresh_start_chunk(l, 0, c, vec);
+                             if (e.iters == 0)
+                               for (int i = b + threadIdx.x; i < en; i += blockDim.x) e.y[i] = l.y[i];
+                           }))
+    return;
+  for (int a = 0; a < e.K; ++a) {
+    double *zin = e.zA, *zout = e.zB;
+    for (int it = 0; it < e.iters; ++it) {
+      const int last = it == e.iters - 1 ? 1 : 0;
+      if (!phase(e.cp, [&](int c) {
+            refresh_apply_chunk(l, zin, zout, last, 0, c, coef, vec);
+            if (last)   // every block reads it for X r
+              for (int i = b + threadIdx.x; i < en; i += blockDim.x) e.y[i] = l.y[i];
+          }))
+        return;
+      double* t = zin;
+      zin = zout;
+      zout = t;
+    }
+    // r = +-y / ||y|| and X r: an item is 32 rows of one column range.  Its X tile
+    // comes in by all threads at once (one wait for L2, 148 SMs sharing X); one
+    // warp then takes the rows' chains, 256 dependent multiply-adds each at most.
+    {
+      const double nrm = sqrt(sum_parts(e.npart, e.cp, 1));
+      if (!(nrm > 0.0) || !isfinite(nrm)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) e.status[0] = 1;
+      } else {
+        const double sgn = (e.y[0] >= 0.0) ? -1.0 : 1.0;
+        const int row_groups = (e.n + 31) / 32, items = row_groups * g.xr.splits;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int i = b + threadIdx.x; i < en; i += blockDim.x) l.r[i] = sgn * l.y[i] / nrm;
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+          const int rg = item % row_groups, z = item / row_groups, row = 32 * rg + lane;
+          const int kbeg = z * g.xr.kps, kend = min(e.p, kbeg + g.xr.kps);
+          double acc = 0.0;
+          for (int kc = kbeg; kc < kend; kc += 256) {
+            const int kn = min(256, kend - kc);
+            double x[256 / kLoopWarps];
+#pragma unroll
+            for (int u = 0; u < 256 / kLoopWarps; ++u) {
+              const int k = warp + kLoopWarps * u;
+              x[u] = k < kn && row < e.n ? __ldg(g.X + row + (size_t)(kc + k) * e.n) : 0.0;
+            }
+            if (threadIdx.x < kn) {
+              const double r = sgn * e.y[kc + threadIdx.x] / nrm;
+              vec[threadIdx.x] = r;
+            }
+#pragma unroll
+            for (int u = 0; u < 256 / kLoopWarps; ++u) tile[(warp + kLoopWarps * u) * 32 + lane] = x[u];
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll 8
+              for (int k = 0; k < kn; ++k) acc = fma(tile[k * 32 + lane], vec[k], acc);
+            }
+            __syncthreads();
+          }
+          if (warp == 0 && row < e.n) {
+            if (e.usplits > 1) e.upart[(size_t)z * e.n + row] = acc;
+            else e.U[row] = acc;
+          }
+        }
+      }
+    }
+    if (!phase(0, [](int) {})) return;
+    if (!phase(e.cn, [&](int c) { scores_chunk(e, a, 0, c, coef, vec, scratch); })) return;
+    for (int j = blockIdx.x * (kLoopThreads / 32) + (threadIdx.x >> 5); j < e.p; j += gridDim.x * (kLoopThreads / 32)) {
+      const double acc = gemv_column<32>(g.X + (size_t)j * e.n, e.T, e.n);
+      if ((threadIdx.x & 31) == 0) e.P[j] = acc;
+    }
+    if (!phase(0, [](int) {})) return;
+    if (!phase(e.cp, [&](int c) { loading_chunk(l, a, 0, c, vec); })) return;
+    if (!phase(e.cp, [&](int c) { orth_chunk(l, a, 0, c, coef, vec, scratch); })) return;
+    if (!phase(e.cp, [&](int c) {
+          deflate_chunk(l, a, a + 1 < e.K ? 1 : 0, 0, c, coef, vec);
+          if (e.iters == 0)
+            for (int i = b + threadIdx.x; i < en; i += blockDim.x) e.y[i] = l.y[i];
+        }))
+      return;
   }
 }
 
@@ -522,6 +775,7 @@ __global__ void k_shard_unpack(Eng e, const double* __restrict__ red) {
 Eng make_eng(const SimplsBatch& b) {
   Eng e{};
   e.n = b.n; e.p = b.p; e.m = b.m; e.F = b.F; e.K = b.K;
+  e.lds = b.p;
   const int target = 4 * Context::get().sm_count;
   e.cp = std::max(1, std::min(ceil_div(target, b.F), ceil_div(b.p, 256)));
   e.cp = std::max(e.cp, ceil_div(b.p, kMaxChunk));
@@ -697,6 +951,42 @@ void simpls_batch_run(const SimplsBatch& b) {
     marks.emplace_back(name, ev);
   };
   mark("start");
+  // One small fit on its own: the whole loop in one launch (not while a trace or
+  // the profiler times the kernels, nor for row-sharded fits, whose all-reduce is
+  // the caller's).  Above 4 M matrix elements the products are the time and have
+  // more loads in flight as kernels of their own.
+  auto* op64 = dynamic_cast<XOperatorF64*>(b.X);
+  const int coef_len = std::max(std::max(b.m, 1), std::max(b.K, 1));
+  const size_t loop_smem = (coef_len + 256 * 32 + (size_t)e.szp * (b.m + b.K + 4)) * sizeof(double);
+  if (simpls_graph_enabled() && !trace && !ctx.profile && !shard_red && op64 && b.F == 1 && !b.labels && !b.mask &&
+      !b.delta && !b.colscale && !b.dY && (size_t)b.n * b.p <= ((size_t)1 << 22) && e.cp <= ctx.sm_count &&
+      loop_smem <= kLoopSmem) {
+    LoopArgs g;
+    g.xr = gemv_ranges(b.n, b.p, ctx.sm_count);
+    e.usplits = g.xr.splits;
+    e.upart = e.usplits > 1 ? ar.alloc_n<double>((size_t)e.usplits * b.n) : nullptr;
+    g.e = e;
+    g.X = op64->Xc;
+    unsigned* ctl = ar.alloc_n<unsigned>(128);   // each on a line of its own
+    dzero(ctl, 64 * sizeof(unsigned));
+    FPLS_CUDA(cudaMemsetAsync(ctl + 64, 0xff, sizeof(unsigned), st));
+    g.barrier = ctl;
+    g.fail = reinterpret_cast<int*>(ctl + 32);
+    g.stop = ctl + 64;
+    g.host_fail = ctx.host_fail;
+    g.coef_len = coef_len;
+    const int want = std::max({e.cp, e.cn, ceil_div(b.n, 32) * g.xr.splits, ceil_div(b.p, kLoopWarps)});
+    static const bool once = [] {
+      FPLS_CUDA(cudaFuncSetAttribute(simpls_loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLoopSmem));
+      return true;
+    }();
+    (void)once;
+    void* args[] = {&g};
+    FPLS_CUDA(cudaLaunchCooperativeKernel((const void*)simpls_loop_kernel, dim3(std::min(std::max(want, e.cp), ctx.sm_count)),
+                                          dim3(kLoopThreads), args, loop_smem, st));
+    ::fpls::note_launch();
+    return;   // a wait that gave up ends the call with an error (Context::end_call)
+  }
   // The component loop as one CUDA graph once its shape has run (not while a
   // trace or the kernel-class profiler records events, nor for row-sharded
   // fits, whose all-reduce callback is the caller's).
