@@ -331,20 +331,16 @@ void gemm_run(bool transA, bool transB, int nt, const gemm64::Args& g, int split
 
 }  // namespace
 
-void gemm(bool transA, bool transB, int M, int N, int K, double alpha, const double* A, int lda,
-          const double* B, int ldb, double beta, double* C, int ldc, const double* row_add) {
-  if (M <= 0 || N <= 0) return;
+namespace {
+
+// The tiles of a product: into C (beta, row_add applied) or, with several K
+// ranges, into partials that the caller adds.
+Partials gemm_tiles(bool transA, bool transB, int M, int N, int K, double alpha, const double* A, int lda,
+                    const double* B, int ldb, double beta, double* C, int ldc, const double* row_add) {
   Context& ctx = Context::get();
   cudaStream_t st = ctx.stream;
-  if (K <= 0) {
-    scale_matrix_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(C, M, N, ldc, beta); ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-    if (row_add) add_row_vector(C, M, N, ldc, row_add);
-    return;
-  }
   const GemmPlan plan = plan_gemm(M, N, K, ctx.sm_count);
   gemm64::Args g{M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, plan.kps, 0, 0, row_add};
-  // split-K partials go to a per-stream workspace and are summed in order
   if (plan.splits > 1) {
     g.split_stride = (long long)M * N;
     g.C = ctx.splitk_workspace(st, (size_t)plan.splits * M * N);
@@ -354,14 +350,40 @@ void gemm(bool transA, bool transB, int M, int N, int K, double alpha, const dou
   }
   const int slot = ctx.prof_begin("gemm_f64_dmma", st);
   gemm_run(transA, transB, plan.nt, g, plan.splits, st);
-  if (plan.splits > 1) {
-    splitk_reduce_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(g.C, plan.splits, g.split_stride, M, N, M, beta,
-                                                                      C, ldc, row_add);
+  // algorithmic work: 2MNK flops; each operand and the result once
+  ctx.prof_end(slot, st, 8.0 * ((double)M * K + (double)K * N + (double)M * N), 2.0 * (double)M * N * K);
+  return Partials{g.C, plan.splits, (size_t)M * N};
+}
+
+}  // namespace
+
+Partials gemm_partials(bool transA, bool transB, int M, int N, int K, const double* A, int lda, const double* B,
+                       int ldb, double* C) {
+  if (M <= 0 || N <= 0 || K <= 0) {
+    gemm(transA, transB, M, N, K, 1.0, A, lda, B, ldb, 0.0, C, M);
+    return Partials{C, 1, 0};
+  }
+  return gemm_tiles(transA, transB, M, N, K, 1.0, A, lda, B, ldb, 0.0, C, M, nullptr);
+}
+
+void gemm(bool transA, bool transB, int M, int N, int K, double alpha, const double* A, int lda,
+          const double* B, int ldb, double beta, double* C, int ldc, const double* row_add) {
+  if (M <= 0 || N <= 0) return;
+  cudaStream_t st = Context::get().stream;
+  if (K <= 0) {
+    scale_matrix_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(C, M, N, ldc, beta); ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
+    if (row_add) add_row_vector(C, M, N, ldc, row_add);
+    return;
+  }
+  const Partials p = gemm_tiles(transA, transB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, row_add);
+  // split-K partials are summed in order
+  if (p.splits > 1) {
+    splitk_reduce_kernel<<<grid_for((size_t)M * N, 256), 256, 0, st>>>(p.w, p.splits, p.stride, M, N, M, beta, C, ldc,
+                                                                      row_add);
     ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
   }
-  // algorithmic work: 2MNK flops; each operand and the result once
-  ctx.prof_end(slot, st, 8.0 * ((double)M * K + (double)K * N + (double)M * N), 2.0 * (double)M * N * K);
 }
 
 __global__ void mirror_upper_f64_kernel(double* K, int n, int ldk) {
@@ -451,6 +473,24 @@ void gram_t_f64(const double* S, int p, int q, int lds, double* G, int ldg) {
   ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
   gram_tiles_f64<false>(St, q, p, q, G, ldg);
+}
+
+Partials gemv_partials(int rows, int cols, const double* A, int lda, const double* x, double* y) {
+  Context& ctx = Context::get();
+  const GemvRanges gr = gemv_ranges(rows, std::max(cols, 1), ctx.sm_count);
+  if (rows <= 0 || cols <= 0 || gr.splits == 1) {
+    gemv(false, rows, cols, 1.0, A, lda, x, 0.0, y);
+    return Partials{y, 1, 0};
+  }
+  cudaStream_t st = ctx.stream;
+  const int slot = ctx.prof_begin("gemv_f64", st);
+  double* ws = ctx.splitk_workspace(st, (size_t)gr.splits * rows);
+  gemv_n_kernel<<<dim3(gr.row_blocks, gr.splits), kGemvRows, 0, st>>>(rows, cols, 1.0, A, lda, x, ws, gr.kps,
+                                                                      (long long)rows, 0.0);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+  ctx.prof_end(slot, st, 8.0 * ((double)rows * cols + rows + cols), 2.0 * (double)rows * cols);
+  return Partials{ws, gr.splits, (size_t)rows};
 }
 
 void gemv(bool trans, int rows, int cols, double alpha, const double* A, int lda, const double* x,

@@ -15,6 +15,20 @@ void gemm(bool transA, bool transB, int M, int N, int K, double alpha,
           const double* A, int lda, const double* B, int ldb, double beta,
           double* C, int ldc, const double* row_add = nullptr);
 
+// A product left as partial sums: entry t is w[t] + w[t + stride] + ... (splits
+// terms, in that order; one: the product itself).  Valid until the next product
+// on the same stream.
+struct Partials {
+  const double* w;
+  int splits;
+  size_t stride;
+};
+// gemm (alpha 1, beta 0, ldc = M) whose K ranges the reader adds up.
+Partials gemm_partials(bool transA, bool transB, int M, int N, int K, const double* A, int lda, const double* B,
+                       int ldb, double* C);
+// gemv (no transpose, alpha 1, beta 0) whose column ranges the reader adds up.
+Partials gemv_partials(int rows, int cols, const double* A, int lda, const double* x, double* y);
+
 // K (n x n) = X X^T for X n x p: the upper-triangle tiles by FP64 tensor-core
 // MMA, the lower triangle mirrored (K exactly symmetric).
 void gram_f64(const double* X, int n, int p, int ldx, double* K, int ldk);

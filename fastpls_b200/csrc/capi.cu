@@ -116,22 +116,38 @@ __global__ void select_ncomp_kernel(const long long* __restrict__ counts, int S,
                                     int Ko, const int* __restrict__ nc, const int* __restrict__ fb, int nc_min,
                                     double* __restrict__ acc_out, int* __restrict__ best_slice,
                                     int* __restrict__ best_comp) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  // one warp a slot, a lane a slice (one thread a slot read its slices one after
+  // another: 14 us for 10 x 30)
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= S) return;
   const int o = ids[s];
   int bi = 0;
   double bv = -1.0;
-  bool any = false;
-  for (int l = 0; l < L; ++l) {
-    const long long ok = counts[2 * ((size_t)s * L + l)], tot = counts[2 * ((size_t)s * L + l) + 1];
-    const double acc = tot ? static_cast<double>(ok) / static_cast<double>(tot) : nan("");
-    acc_out[o + (size_t)l * Ko] = acc;
-    if (isfinite(acc) && (!any || acc > bv)) {
-      bv = acc;
-      bi = l;
-      any = true;
+  for (int l0 = 0; l0 < L; l0 += 32) {
+    const int l = l0 + lane;
+    double v = -1.0;   // below every accuracy
+    if (l < L) {
+      const long long ok = counts[2 * ((size_t)s * L + l)], tot = counts[2 * ((size_t)s * L + l) + 1];
+      const double acc = tot ? static_cast<double>(ok) / static_cast<double>(tot) : nan("");
+      acc_out[o + (size_t)l * Ko] = acc;
+      if (isfinite(acc)) v = acc;
+    }
+    int at = l;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {   // the largest, the first of equals
+      const double w = __shfl_xor_sync(0xffffffffu, v, d);
+      const int wa = __shfl_xor_sync(0xffffffffu, at, d);
+      if (w > v || (w == v && wa < at)) {
+        v = w;
+        at = wa;
+      }
+    }
+    if (v > bv) {
+      bv = v;
+      bi = at;
     }
   }
+  if (lane != 0) return;
   best_slice[s] = bi;
   best_comp[o] = fb[s] ? nc_min : nc[bi];
 }
@@ -1385,7 +1401,7 @@ static void double_cv_impl(const void* X, int x_is_float32, bool x_on_device, in
     double* d_acc = ctx.arena.alloc_n<double>((size_t)Ko * L);
     int* d_best = ctx.arena.alloc_n<int>(S);
     int* d_bcomp = ctx.arena.alloc_n<int>(Ko);
-    select_ncomp_kernel<<<ceil_div(S, 128), 128, 0, ctx.stream>>>(d_cnt, S, L, d_ids, Ko, d_nc, d_fb,
+    select_ncomp_kernel<<<ceil_div(S, 4), 128, 0, ctx.stream>>>(d_cnt, S, L, d_ids, Ko, d_nc, d_fb,
                                                                   *std::min_element(nc.begin(), nc.end()), d_acc,
                                                                   d_best, d_bcomp);
     ::fpls::note_launch();

@@ -143,12 +143,22 @@ __global__ void pred_counts_kernel(const int* __restrict__ pred, int L, int n, c
   const int g = gs / L;
   const int* pr = pred + (size_t)gs * n;
   double ok = 0.0, tot = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    if (exclude && exclude[i] == g) continue;
-    const int v = pr[i];
-    if (v < 1) continue;
-    tot += 1.0;
-    ok += (v == y[i]) ? 1.0 : 0.0;
+  // four rows a thread at a time, their three loads each together
+  for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {
+    int p[4], t[4], x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * blockDim.x;
+      p[u] = i < n ? pr[i] : 0;
+      t[u] = i < n ? y[i] : 0;
+      x[u] = i < n && exclude ? exclude[i] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (p[u] < 1 || (exclude && x[u] == g)) continue;
+      tot += 1.0;
+      ok += p[u] == t[u] ? 1.0 : 0.0;
+    }
   }
   ok = block_sum(ok, scratch);
   tot = block_sum(tot, scratch);
@@ -184,15 +194,16 @@ __global__ void cv_predict_kernel(int F, int n, int m, int K, int L, const int* 
   const double* mf = mYf + (size_t)f * m;
   const double* tk = Tkeep + (size_t)f * K * n + i;
   // the slices in increasing ncomp (order), each written once y holds its
-  // components; the scores of four components are loaded together
+  // components; the scores of kAhead components are loaded together
+  constexpr int kAhead = MB <= 8 ? 16 : 4;
   int next = 0;
   int nc_next = L > 0 ? ncomp[order[0]] : 0;
-  for (int a0 = 0; a0 < K; a0 += 4) {
-    double t[4];
+  for (int a0 = 0; a0 < K; a0 += kAhead) {
+    double t[kAhead];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) t[u] = a0 + u < done ? tk[(size_t)(a0 + u) * n] : 0.0;
+    for (int u = 0; u < kAhead; ++u) t[u] = a0 + u < done ? tk[(size_t)(a0 + u) * n] : 0.0;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < kAhead; ++u) {
       const int a = a0 + u;
       if (a >= K) break;
       if (a < done) {

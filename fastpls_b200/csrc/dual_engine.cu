@@ -39,7 +39,9 @@ struct DualEng {
   double* KCV;   // F x n x K
   double* Kcy;   // F x n   K image of the warm start r / ||t|| of the last component
   double* cp;    // n x F   loading coefficients (input of the K product)
-  double* Gp;    // n x F   K cp
+  const double* Gp;   // n x F   K cp, or its partial sums: gsplits of them, gstride apart
+  int gsplits;
+  size_t gstride;
   // K cp as INT8-product partials (when kpart is set): entry (i, f) is the sum
   // over segments s of tile (i / 128) * kntn + f / 64 of
   // kpart[(s * 64 + f % 64) * 128 + i % 128], in segment order.
@@ -556,7 +558,17 @@ static __device__ bool dual_b(const DualEng& e, int a, ClusterRed& R, const Rows
       }
       kv[k] = v;
     } else {
-      kv[k] = e.Gp[(size_t)f * n + i];
+      const double* gp = e.Gp + (size_t)f * n + i;
+      double v = gp[0];
+      for (int s0 = 1; s0 < e.gsplits; s0 += 8) {
+        double t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = s0 + u < e.gsplits ? gp[(s0 + u) * e.gstride] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (s0 + u < e.gsplits) v += t[u];
+      }
+      kv[k] = v;
     }
   }
   if (a > 0) {
@@ -933,7 +945,7 @@ void dual_simpls_run(const DualBatch& b) {
   e.KCV = ar.alloc_n<double>(F * n * K);
   e.Kcy = ar.alloc_n<double>(F * n);
   e.cp = ar.alloc_n<double>(F * n);
-  e.Gp = ar.alloc_n<double>(F * n);
+  double* Gp = ar.alloc_n<double>(F * n);
   e.scal = ar.alloc_n<double>(2 * F);
   e.qs = ar.alloc_n<double>(F * m);
   e.ntrain = b.ntrain;
@@ -1000,7 +1012,11 @@ void dual_simpls_run(const DualBatch& b) {
       ctx.prof_end(ks, st, S * nd * nd + S * nd * Fd + 16.0 * nd * Fd, 0.5 * S * (S + 1.0) * 2.0 * nd * nd * Fd);
     } else {
       const int ks = ctx.prof_begin("k_products_f64", st);
-      b.Kop->times(e.cp, b.F, e.Gp);
+      // its ranges' partial sums are added by the next step as it reads K c_p
+      const Partials gp = b.Kop->times_partials(e.cp, b.F, Gp);
+      e.Gp = gp.w;
+      e.gsplits = gp.splits;
+      e.gstride = gp.stride;
       ctx.prof_end(ks, st, 8.0 * (nd * nd + 2.0 * nd * Fd), 2.0 * nd * nd * Fd);
     }
     pt.mark("K products");

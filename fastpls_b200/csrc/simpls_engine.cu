@@ -64,8 +64,11 @@ struct Eng {
   double* v;       // F x p
   double* vpart;   // F x cp
   double* vSpart;  // F x cp x m
-  double* upart;   // usplits x n partials of U (one-launch loop)
-  int usplits;     // 0: U holds the sums
+  // U and P as partial sums of the products' ranges (Partials), added in order
+  // where they are read: the separate reductions were 8 % of a grid's component
+  double* upart;
+  const double* ppart;
+  int usplits, psplits;   // up to 1: U, P hold the sums
 };
 
 __device__ __forceinline__ void chunk_range(int chunk, int sz, int total, int& b, int& e) {
@@ -76,12 +79,12 @@ __device__ __forceinline__ void chunk_range(int chunk, int sz, int total, int& b
 // parts[0] + parts[stride] + ... in order, kAhead loads at a time (each kernel of
 // the loop starts with such a sum, and its loads one after another were a third
 // of the launch).
-__device__ __forceinline__ double sum_parts(const double* parts, int count, int stride) {
+__device__ __forceinline__ double sum_parts(const double* parts, int count, size_t stride) {
   double s = 0.0;
   for (int c0 = 0; c0 < count; c0 += kAhead) {
     double v[kAhead];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) v[u] = c0 + u < count ? parts[(size_t)(c0 + u) * stride] : 0.0;
+    for (int u = 0; u < kAhead; ++u) v[u] = c0 + u < count ? parts[(c0 + u) * stride] : 0.0;
 #pragma unroll
     for (int u = 0; u < kAhead; ++u)
       if (c0 + u < count) s += v[u];
@@ -294,7 +297,7 @@ __device__ __forceinline__ void scores_chunk(const Eng& e, int a, int f, int chu
     __syncthreads();
   }
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    const double u = (e.usplits > 1 ? sum_parts(e.upart + i, e.usplits, e.n) : Uf[i]) - c;
+    const double u = (e.usplits > 1 ? sum_parts(e.upart + (size_t)f * e.n + i, e.usplits, (size_t)e.n * e.F) : Uf[i]) - c;
     const double t = (mk && !mk[i]) ? 0.0 : u;
     Tf[i] = t;
     ts[i - b] = t;
@@ -348,7 +351,10 @@ __device__ __forceinline__ void loading_chunk(const Eng& e, int a, int f, int ch
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
   const double* Pf = e.P + (size_t)f * e.p;
-  const double p0 = b + (int)threadIdx.x < en ? Pf[b + threadIdx.x] : 0.0;   // on its way during the sums
+  auto p_at = [&](int i) {
+    return e.psplits > 1 ? sum_parts(e.ppart + (size_t)f * e.p + i, e.psplits, (size_t)e.p * e.F) : Pf[i];
+  };
+  const double p0 = b + (int)threadIdx.x < en ? p_at(b + threadIdx.x) : 0.0;   // on its way during the sums
   double tn, st;
   t_stats(e, f, tn, st);
   if (!(tn > 0.0) || !isfinite(tn)) {
@@ -359,7 +365,7 @@ __device__ __forceinline__ void loading_chunk(const Eng& e, int a, int f, int ch
   const double* dl = e.delta ? e.delta + (size_t)f * e.p : nullptr;
   double* pf = e.pv + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
-    double v = i < b + (int)blockDim.x ? p0 : Pf[i];
+    double v = i < b + (int)blockDim.x ? p0 : p_at(i);
     if (dl) v -= dl[i] * st;
     if (sc) v *= sc[i];
     v /= tn;
@@ -806,6 +812,19 @@ void XOperatorF64::t_times(const double* T, int F, double* P) {
   else gemm(true, false, p, F, n, 1.0, Xc, n, T, n, 0.0, P, p);
 }
 
+Partials XOperatorF64::times_partials(const double* Rhat, int F, double* U) {
+  if (F == 1) return gemv_partials(n, p, Xc, n, Rhat, U);
+  return gemm_partials(false, false, n, F, p, Xc, n, Rhat, p, U);
+}
+
+Partials XOperatorF64::t_times_partials(const double* T, int F, double* P) {
+  if (F == 1) {
+    t_times(T, F, P);
+    return Partials{P, 1, 0};
+  }
+  return gemm_partials(true, false, p, F, n, Xc, n, T, n, P);
+}
+
 void XOperatorF64::gram(double* K) { gram_f64(Xc, n, p, n, K, n); }
 
 void simpls_batch_crosscov(const SimplsBatch& b, const double* /*Xc*/, const int* /*n_train*/) {
@@ -1010,12 +1029,20 @@ void simpls_batch_run(const SimplsBatch& b) {
     k_refresh_finish<<<gp, kThreads, 0, st>>>(e); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("refresh");
-    b.X->times(e.Rhat, b.F, e.U);
+    const Partials up = b.X->times_partials(e.Rhat, b.F, e.U);
+    e.upart = const_cast<double*>(up.w);
+    e.usplits = up.splits;
     mark("X*R");
     k_scores<<<gn, tq, b.labels ? sm_m : 0, st>>>(e, a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("scores");
-    b.X->t_times(e.T, b.F, e.P);
+    if (shard_red) {
+      b.X->t_times(e.T, b.F, e.P);   // the all-reduce takes the sums
+    } else {
+      const Partials pp = b.X->t_times_partials(e.T, b.F, e.P);
+      e.ppart = pp.w;
+      e.psplits = pp.splits;
+    }
     if (shard_red) {
       k_shard_pack<<<shard_grid, kThreads, 0, st>>>(e, shard_red); ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();

@@ -16,6 +16,7 @@
 
 #include <cstdint>
 
+#include "blas_f64.cuh"
 #include "common.cuh"
 
 namespace fpls {
@@ -27,6 +28,16 @@ struct XOperator {
   virtual ~XOperator() {}
   virtual void times(const double* Rhat, int F, double* U) = 0;
   virtual void t_times(const double* T, int F, double* P) = 0;
+  // The same products, possibly left as partial sums for the reader to add (U, P
+  // then stay unwritten).
+  virtual Partials times_partials(const double* Rhat, int F, double* U) {
+    times(Rhat, F, U);
+    return Partials{U, 1, 0};
+  }
+  virtual Partials t_times_partials(const double* T, int F, double* P) {
+    t_times(T, F, P);
+    return Partials{P, 1, 0};
+  }
   // K (n x n) = Xc Xc^T, the row Gram of the predictors.
   virtual void gram(double* K) = 0;
   int n = 0, p = 0;
@@ -38,6 +49,8 @@ struct XOperatorF64 : public XOperator {
   XOperatorF64(const double* X, int n_, int p_) : Xc(X) { n = n_; p = p_; }
   void times(const double* Rhat, int F, double* U) override;
   void t_times(const double* T, int F, double* P) override;
+  Partials times_partials(const double* Rhat, int F, double* U) override;
+  Partials t_times_partials(const double* T, int F, double* P) override;
   void gram(double* K) override;
 };
 
