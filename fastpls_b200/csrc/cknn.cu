@@ -22,9 +22,11 @@
 #include <cstdlib>
 #include <cmath>
 #include <limits>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "blas_f64.cuh"
 #include "capi_util.cuh"
@@ -490,11 +492,10 @@ knn_tile_kernel_v2(const KnnItem* __restrict__ items, KnnClassInfo ci, const int
 }
 
 // ----------------------------------------------------- tensor-core filter
-// The same (class, pair tile, training chunk) items on the BF16 tensor cores,
-// with results equal to the FP64 tiles':
-//   pass 1  128 pairs x 128 training rows of approximate similarities per
-//           tile: both score rows split into BF16 planes hi = bf16(x),
-//           lo = bf16(x - hi), three products hi.hi + hi.lo + lo.hi
+// The same (class, pair tile, training chunk) items on the 16-bit tensor
+// cores, with results equal to the FP64 tiles': the products below only choose
+// which training rows are scored, the scores and lists are FP64.
+//   pass 1  128 pairs x 128 training rows of approximate similarities per tile
 //           (tcgen05.mma kind::f16, M128 N128 K16, FP32 accumulation in TMEM,
 //           double-buffered so the epilogue overlaps the next tile); each pair
 //           row keeps running maxima of 64 disjoint buckets of its values and
@@ -502,58 +503,118 @@ knn_tile_kernel_v2(const KnnItem* __restrict__ items, KnnClassInfo ci, const int
 //   bar     per pair, theta = the k-th largest of those values over all its
 //           chunks.  They are approximate values of distinct training rows, so
 //           theta is at most the k-th largest approximate value of the class.
-//           Every approximate value is within eps = 2^-14 |x| max|y| of the
-//           exact dot: the split leaves x - hi - lo below 2^-18 |x| and drops
-//           terms below 3 2^-18 |x||y| in all (1.2e-5 |x||y|); the BF16
-//           products are exact in FP32 and the FP32 accumulation of the 3 x 128
-//           products loses at most 384 2^-23 sum|x_k y_k| <= 4.6e-5 |x||y|
-//           even with every addition truncated; 5.7e-5 < 2^-14.  So each row
-//           of the pair's exact top k has an approximate value of at least
+//           Every approximate value is within eps of the exact dot, so each
+//           row of the pair's exact top k has an approximate value of at least
 //           theta - 2 eps;
 //   pass 2  the same products again; every training row whose approximate
 //           value reaches that bar is scored exactly (FP64 dot of the two score
-//           rows) and folded into the pair's top-k list, which is what the
-//           FP64 tiles write and knn_merge_kernel reads.
+//           rows, knn_exact_kernel) and the pair's k largest go to the list
+//           that knn_merge_kernel reads.
+// Two forms of the products, by PLANES:
+//   1  one FP16 product of rows scaled by powers of two: each test row into
+//      norm [1/2, 1), the training rows by one power so that their largest
+//      norm is in [1/2, 1].  Rounding each factor to FP16 leaves
+//      2^-11 |x_k| + 2^-25 a factor, so (2^-10 + 2^-22) |x||y| and at most
+//      2 sqrt(128) 2^-25 a dot, which is below 2^-18.5 |x| max|y|; the 128
+//      products are exact in FP32, and their accumulation loses at most
+//      128 2^-23 |x||y| even with every addition truncated.  In all below
+//      1.02 2^-10 |x| max|y|; eps = 17/16 2^-10 |x| max|y|.
+//   2  both rows split into BF16 planes hi = bf16(x), lo = bf16(x - hi), three
+//      products hi.hi + hi.lo + lo.hi: the split leaves x - hi - lo below
+//      2^-18 |x| and drops terms below 3 2^-18 |x||y| in all (1.2e-5 |x||y|),
+//      the accumulation of 3 x 128 products loses at most 4.6e-5 |x||y|;
+//      5.7e-5 < eps = 2^-14 |x| max|y|.
+// The FP16 form runs first: a third of the MMA work, half the bytes through L2
+// and shared memory, and two CTAs on an SM.  Its wider bar costs a few more
+// exact scores; a class whose similarities to a test row crowd within it fills
+// the candidate slots of a pair, and then the products run again as split BF16,
+// and after that on the FP64 tiles.
+// What bounds it: a 128 x 128 tile brings 32 KB out of L2, 16384 values out of
+// TMEM, one max or compare a value, and 128 x 128 x 112 products, each a third
+// to a half of the tile's time; two CTAs overlap them.  1,200,000 training rows
+// of 100 scores, 10^6 pairs, 7.9e9 similarities: pass 1 1.84 ms, pass 2
+// 1.64 ms (1.06 ms is the MMA work of one pass at the measured 1670 TFLOP/s);
+// with split BF16 throughout, a search of the maxima in shared memory and an
+// atomic a hit, one CTA an SM: 5.65 and 7.55 ms.
 // Score rows up to 128 wide, neighbour lists up to 16 long, up to 2^24
-// training rows.  Warp 0 loads (TMA, SWIZZLE_128B boxes of 64 x 128 BF16: the
-// A tile once, the B tiles through two stages), warp 1 issues the MMAs,
+// training rows.  Warp 0 loads (TMA, SWIZZLE_128B boxes of 64 x 128 values:
+// the A tile once, the B tiles through two stages), warp 1 issues the MMAs,
 // warps 2..9 are the epilogue (two per TMEM lane quarter).  Every mbarrier
 // wait is bounded; no cluster multicast.
 constexpr int kFT = 128;                  // pairs per tile = training rows per tile
-constexpr int kFK = 128;                  // contraction width (rows zero padded)
-constexpr int kFBox = 64 * kFT * 2;       // one 64-wide box of 128 BF16 rows: 16 KB
-constexpr int kFOperand = 4 * kFBox;      // two planes x two boxes: 64 KB
+constexpr int kFK = 128;                  // widest score row
+constexpr int kFBox = 64 * kFT * 2;       // one 64-wide box of 128 16-bit rows: 16 KB
 constexpr int kFEpiWarps = 8;             // two per TMEM lane quarter, half the columns each
 constexpr int kFThreads = 64 + 32 * kFEpiWarps;
-constexpr int kFBarOff = 3 * kFOperand;   // A, then two B stages
 constexpr int kFList = 16;                // longest neighbour list of the filter
 constexpr int kFBuckets = 32;             // pass 1: running maxima per thread
 constexpr int kFCap = 128;                // pass 2: candidate rows kept per pair
-constexpr int kFSmem = kFBarOff + 256 + 1024;
-constexpr uint32_t kFIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kFT >> 3) << 17) |
-                             (uint32_t(kFT >> 4) << 24);
-static_assert(kFSmem <= 227 * 1024, "filter tiles exceed shared memory");
+template <int PLANES>
+struct FilterTile {
+  static constexpr int kOperand = PLANES * 2 * kFBox;   // planes x two boxes
+  static constexpr int kBarOff = 3 * kOperand;          // A, then two B stages
+  static constexpr int kSmem = kBarOff + 256 + 1024;
+  static constexpr int kCtas = PLANES == 1 ? 2 : 1;     // per SM
+  // D FP32; A and B FP16 (one plane) or BF16 (two)
+  static constexpr uint32_t kIdesc = (1u << 4) | (PLANES == 1 ? 0u : (1u << 7) | (1u << 10)) |
+                                     (uint32_t(kFT >> 3) << 17) | (uint32_t(kFT >> 4) << 24);
+};
+static_assert(FilterTile<2>::kSmem <= 227 * 1024 && 2 * (FilterTile<1>::kSmem + 1024) <= 228 * 1024,
+              "filter tiles exceed shared memory");
 
-__device__ __forceinline__ void umma_bf16_f32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t acc) {
+__device__ __forceinline__ void umma_16bit_f32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(kFIdesc), "r"(acc)
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
       : "memory");
 }
 
-template <int PASS>
-__global__ void __launch_bounds__(kFThreads, 1)
-knn_filter_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
-                  const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl,
-                  const KnnItem* __restrict__ items, KnnClassInfo ci, const int* __restrict__ pairs, int ntest,
-                  const double* __restrict__ Tq, const double* __restrict__ Ts, int K, int use_k,
-                  float* __restrict__ apart, const float* __restrict__ bar, int* __restrict__ ccount,
-                  int* __restrict__ crow, int* err) {
+// Compare-exchange steps of a bitonic merge of N values into descending order.
+template <int N>
+__device__ __forceinline__ void bitonic_merge_desc(float (&x)[N]) {
+#pragma unroll
+  for (int d = N / 2; d > 0; d >>= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((i & d) == 0) {
+        const float a = x[i], b = x[i + d];
+        x[i] = fmaxf(a, b);
+        x[i + d] = fminf(a, b);
+      }
+}
+
+// The kFList values of x[OFF ..] in descending order (bitonic network).
+template <int OFF, int M>
+__device__ __forceinline__ void sort16_desc(const float (&x)[M], float (&out)[kFList]) {
+#pragma unroll
+  for (int i = 0; i < kFList; ++i) out[i] = x[OFF + i];
+#pragma unroll
+  for (int size = 2; size <= kFList; size <<= 1)
+#pragma unroll
+    for (int d = size / 2; d > 0; d >>= 1)
+#pragma unroll
+      for (int i = 0; i < kFList; ++i)
+        if ((i & d) == 0) {
+          const bool desc = (i & size) == 0;
+          const float a = out[i], b = out[i + d];
+          out[i] = desc ? fmaxf(a, b) : fminf(a, b);
+          out[i + d] = desc ? fminf(a, b) : fmaxf(a, b);
+        }
+}
+
+template <int PASS, int PLANES>
+__global__ void __launch_bounds__(kFThreads, FilterTile<PLANES>::kCtas)
+knn_filter_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ CUtensorMap mA1,
+                  const __grid_constant__ CUtensorMap mB0, const __grid_constant__ CUtensorMap mB1,
+                  const KnnItem* __restrict__ items, KnnClassInfo ci, int K, int use_k, float* __restrict__ apart,
+                  const float* __restrict__ bar, int* __restrict__ ccount, int* __restrict__ crow, int* err) {
+  using Tile = FilterTile<PLANES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kFBarOff);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Tile::kBarOff);
   uint64_t* fullA = bars;
   uint64_t* full = bars + 1;     // [2]
   uint64_t* empty = bars + 3;    // [2]
@@ -570,6 +631,8 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant
   const int r0 = ci.row_offs[c] + it.chunk * ci.chunk_rows[c];
   const int r1 = min(ci.row_offs[c + 1], r0 + ci.chunk_rows[c]);
   const int ntiles = (r1 - r0 + kFT - 1) / kFT;
+  const int nbox = (K + 63) / 64;        // 64-wide boxes a plane holds
+  const int ksteps = (K + 15) / 16;      // columns past K are zero: their steps add nothing
 
   if (threadIdx.x == 0) {
     tc::mbar_init(tc::smem_u32(fullA), 1);
@@ -596,23 +659,19 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant
   if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------- producer
     const uint32_t sa = tc::smem_u32(smem);
-    tc::mbar_expect_tx(tc::smem_u32(fullA), kFOperand);
-    tc::tma_load_2d(&mAh, sa, tc::smem_u32(fullA), 0, p0);
-    tc::tma_load_2d(&mAh, sa + kFBox, tc::smem_u32(fullA), 64, p0);
-    tc::tma_load_2d(&mAl, sa + 2 * kFBox, tc::smem_u32(fullA), 0, p0);
-    tc::tma_load_2d(&mAl, sa + 3 * kFBox, tc::smem_u32(fullA), 64, p0);
+    auto load = [&](const CUtensorMap* m0, const CUtensorMap* m1, uint32_t dst, uint32_t fb, int row) {
+      tc::mbar_expect_tx(fb, PLANES * nbox * kFBox);
+      for (int x = 0; x < nbox; ++x) {
+        tc::tma_load_2d(m0, dst + x * kFBox, fb, x * 64, row);
+        if (PLANES == 2) tc::tma_load_2d(m1, dst + (2 + x) * kFBox, fb, x * 64, row);
+      }
+    };
+    load(&mA0, &mA1, sa, tc::smem_u32(fullA), p0);
     int issued = 0;
     for (int t = 0; t < ntiles; ++t) {
       const int s = t & 1;
       if (!tc::mbar_wait(tc::smem_u32(&empty[s]), ((t >> 1) & 1) ^ 1, err)) break;
-      const uint32_t fb = tc::smem_u32(&full[s]);
-      const uint32_t sb = tc::smem_u32(smem + (1 + s) * kFOperand);
-      const int row = r0 + t * kFT;
-      tc::mbar_expect_tx(fb, kFOperand);
-      tc::tma_load_2d(&mBh, sb, fb, 0, row);
-      tc::tma_load_2d(&mBh, sb + kFBox, fb, 64, row);
-      tc::tma_load_2d(&mBl, sb + 2 * kFBox, fb, 0, row);
-      tc::tma_load_2d(&mBl, sb + 3 * kFBox, fb, 64, row);
+      load(&mB0, &mB1, sa + (1 + s) * Tile::kOperand, tc::smem_u32(&full[s]), r0 + t * kFT);
       issued = t + 1;
     }
     // the copies in flight land before the CTA exits (bounded waits)
@@ -631,16 +690,19 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant
       if (!tc::mbar_wait(tc::smem_u32(&tempty[b]), ((t >> 1) & 1) ^ 1, err)) { ok = false; break; }
       if (!tc::mbar_wait(tc::smem_u32(&full[b]), (t >> 1) & 1, err)) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sb = tc::smem_u32(smem + (1 + b) * kFOperand);
+      const uint32_t sb = sa + (1 + b) * Tile::kOperand;
       const uint32_t acc = tmem + static_cast<uint32_t>(b * kFT);
 #pragma unroll
       for (int kk = 0; kk < kFK / 16; ++kk) {
+        if (kk >= ksteps) break;
         const uint32_t off = (kk >> 2) * kFBox + (kk & 3) * 32;   // box, then 32 bytes per K16 step
-        const uint64_t ah = tc::sw128_desc(sa + off), al = tc::sw128_desc(sa + 2 * kFBox + off);
-        const uint64_t bh = tc::sw128_desc(sb + off), bl = tc::sw128_desc(sb + 2 * kFBox + off);
-        umma_bf16_f32(acc, ah, bh, kk > 0 ? 1u : 0u);
-        umma_bf16_f32(acc, ah, bl, 1u);
-        umma_bf16_f32(acc, al, bh, 1u);
+        const uint64_t a0 = tc::sw128_desc(sa + off), b0 = tc::sw128_desc(sb + off);
+        umma_16bit_f32(acc, a0, b0, Tile::kIdesc, kk > 0 ? 1u : 0u);
+        if (PLANES == 2) {
+          const uint64_t a1 = tc::sw128_desc(sa + 2 * kFBox + off), b1 = tc::sw128_desc(sb + 2 * kFBox + off);
+          umma_16bit_f32(acc, a0, b1, Tile::kIdesc, 1u);
+          umma_16bit_f32(acc, a1, b0, Tile::kIdesc, 1u);
+        }
       }
       tc::umma_commit(tc::smem_u32(&empty[b]));
       tc::umma_commit(tc::smem_u32(&tfull[b]));
@@ -648,142 +710,263 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant
     // every MMA issued has completed before TMEM is released
     tc::umma_commit(tc::smem_u32(done));
     tc::mbar_wait(tc::smem_u32(done), 0, err, false);
-  } else if (warp >= 2) {
-    // ---------------------------------------------------------- epilogue
-    // Two warps per TMEM lane quarter, each with half of the tile's columns:
-    // thread (row r, half h) loads its 64 values in one round and releases
-    // the accumulator before using them.
-    //   pass 1: 32 running maxima of disjoint buckets of the half row's
-    //           values (one max per value).  They are values of distinct
-    //           training rows, so the k-th largest of them is at most the
-    //           k-th largest approximate value, which is all the bar needs;
-    //   pass 2: the rows whose value reaches the bar are noted in the pair's
-    //           candidate slots (scored exactly by knn_exact_kernel, outside
-    //           this pipeline).
-    // The two halves of a pair row's bucket maxima are merged at the end.
-    const int q = warp & 3;
-    const int h = (warp - 2) / 4;
-    const int r = q * 32 + lane;          // pair row of the tile (TMEM lane)
+  }
+  // ------------------------------------------------------------ epilogue
+  // Two warps per TMEM lane quarter, each with half of the tile's columns:
+  // thread (row r, half h) loads its 64 values in two rounds and releases the
+  // accumulator before it uses the second.
+  //   pass 1: 32 running maxima of disjoint buckets of the half row's values
+  //           (one max per value).  They are values of distinct training rows,
+  //           so the k-th largest of them is at most the k-th largest
+  //           approximate value, which is all the bar needs.  A sorting
+  //           network in registers orders them at the end, and the two halves
+  //           of a pair row meet in shared memory;
+  //   pass 2: the columns that reach the bar become bits of a mask; one atomic
+  //           a tile reserves their places in the pair's candidate slots, and
+  //           the rows are written while the next tile is compared (with an
+  //           atomic a hit, waited for, pass 2 took 1.3 times pass 1).
+  const int q = warp & 3;
+  const int h = (warp - 2) / 4;
+  const int r = q * 32 + lane;          // pair row of the tile (TMEM lane)
+  float top[kFList];
+  if (warp >= 2) {
     const bool row_ok = r < np;
-    const int tr = row_ok ? pairs[p0 + r] % ntest : 0;
     float M[kFBuckets];
 #pragma unroll
     for (int e = 0; e < kFBuckets; ++e) M[e] = -INFINITY;
+    // the rows past np are other pairs' or padding: their maxima are not
+    // written, and no finite value reaches their bar
     const float thr = (PASS == 2 && row_ok) ? bar[p0 + r] : INFINITY;
-    for (int t = 0; t < ntiles; ++t) {
-      const int b = t & 1;
-      const bool ok = tc::mbar_wait(tc::smem_u32(&tfull[b]), (t >> 1) & 1, err);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int n0 = r0 + t * kFT;
-      const int ncol = min(kFT, r1 - n0);
-      const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * kFT + h * 64);
-      uint32_t v[4][16];
-      __syncwarp();
+    uint32_t held[2] = {0u, 0u};   // the last tile's hits, not yet written
+    int slot = 0, hbase = 0;
+    auto write_hits = [&]() {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tc::tmem_ld16_raw(base + c * 16, v[c]);
-      tc::tmem_wait_ld();
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      tc::mbar_arrive(tc::smem_u32(&tempty[b]));
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        // values past the class's last training row (or of an absent pair
-        // row) are NaN: they fail every comparison, so they neither raise a
-        // bucket maximum nor become candidates (not even for a bar of -inf)
-        float f[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const bool in = ok && row_ok && h * 64 + g * 16 + i < ncol;
-          f[i] = in ? __uint_as_float(v[g][i]) : __int_as_float(0x7fc00000);
-        }
-        if (PASS == 1) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) M[(g * 16 + i) % kFBuckets] = fmaxf(M[(g * 16 + i) % kFBuckets], f[i]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (f[i] >= thr) {
-              const int slot = atomicAdd(ccount + p0 + r, 1);
-              if (slot < kFCap) crow[(size_t)(p0 + r) * kFCap + slot] = n0 + h * 64 + g * 16 + i;
-            }
+      for (int x = 0; x < 2; ++x) {
+        while (held[x]) {
+          const int i = __ffs(held[x]) - 1;
+          held[x] &= held[x] - 1;
+          if (slot < kFCap) crow[(size_t)(p0 + r) * kFCap + slot] = hbase + 32 * x + i;
+          ++slot;
         }
       }
-      if (!ok) break;
-    }
-    // the two halves meet in the (now idle) A-tile buffer after the closing
-    // barrier below
-    if (PASS == 1) {
-      float* ls = reinterpret_cast<float*>(smem);
+    };
+    for (int t = 0; t < ntiles; ++t) {
+      const int b = t & 1;
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&tfull[b]), (t >> 1) & 1, err))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int n0 = r0 + t * kFT + h * 64;
+      const int ncol = min(64, r1 - n0);   // columns of this half that are rows of the class (may be <= 0)
+      const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * kFT + h * 64);
+      uint32_t hits[2] = {0u, 0u};
 #pragma unroll
-      for (int e = 0; e < kFBuckets; ++e) ls[(h * kFBuckets + e) * kFT + r] = M[e];
+      for (int x = 0; x < 2; ++x) {
+        uint32_t v[2][16];
+        tc::tmem_ld16_raw(base + x * 32, v[0]);
+        tc::tmem_ld16_raw(base + x * 32 + 16, v[1]);
+        tc::tmem_wait_ld();
+        if (x == 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          tc::mbar_arrive(tc::smem_u32(&tempty[b]));
+        }
+        if (PASS == 1) {
+          if (ncol == 64) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) M[i] = fmaxf(M[i], __uint_as_float(v[i >> 4][i & 15]));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (x * 32 + i < ncol) M[i] = fmaxf(M[i], __uint_as_float(v[i >> 4][i & 15]));
+          }
+        } else {
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            float mx = __uint_as_float(v[g][0]);
+#pragma unroll
+            for (int i = 1; i < 16; ++i) mx = fmaxf(mx, __uint_as_float(v[g][i]));
+            if (mx >= thr) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (__uint_as_float(v[g][i]) >= thr) hits[x] |= 1u << (g * 16 + i);
+            }
+          }
+        }
+      }
+      if (PASS == 2) {
+        if (ncol < 64) {   // columns past the class's last training row
+          hits[0] = ncol <= 0 ? 0u : (ncol >= 32 ? hits[0] : hits[0] & ((1u << ncol) - 1u));
+          hits[1] = ncol <= 32 ? 0u : hits[1] & ((1u << (ncol - 32)) - 1u);
+        }
+        write_hits();
+        held[0] = hits[0];
+        held[1] = hits[1];
+        hbase = n0;
+        const int n = __popc(hits[0]) + __popc(hits[1]);
+        if (n) slot = atomicAdd(ccount + p0 + r, n);
+      }
+    }
+    if (PASS == 2) write_hits();
+    if (PASS == 1) {
+      // the kFList largest of this half's maxima, descending
+      float other[kFList];
+      sort16_desc<0>(M, top);
+      sort16_desc<16>(M, other);
+#pragma unroll
+      for (int e = 0; e < kFList; ++e) top[e] = fmaxf(top[e], other[kFList - 1 - e]);
+      bitonic_merge_desc(top);
+      // every MMA that reads the A tile has completed (the last accumulator
+      // was waited for), so its buffer takes the second half's list
+      float* ls = reinterpret_cast<float*>(smem);
+      if (h == 1) {
+#pragma unroll
+        for (int e = 0; e < kFList; ++e) ls[e * kFT + r] = top[e];
+      }
     }
   }
   // every MMA has completed (the issuer waited for them) and every epilogue
   // thread has stored its values: one thread per pair row writes its list
-  __syncthreads();
-  if (PASS == 1 && warp >= 2 && warp < 6) {
-    const int r = (warp & 3) * 32 + lane;
-    if (r < np) {
-      const int qi = p0 + r - ci.pair_offs[c];
-      const long long o = ci.part_base[c] + ((long long)qi * ci.nchunks[c] + it.chunk) * use_k;
-      // the use_k largest of the row's 64 bucket maxima, in descending order
-      float* ls = reinterpret_cast<float*>(smem);
-      for (int e = 0; e < use_k; ++e) {
-        int best = 0;
-        float bv = ls[r];
-        for (int x = 1; x < 2 * kFBuckets; ++x) {
-          const float vx = ls[x * kFT + r];
-          if (vx > bv) { bv = vx; best = x; }
-        }
-        apart[o + e] = bv;
-        ls[best * kFT + r] = -INFINITY;
-      }
-    }
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PASS == 1 && warp >= 2 && h == 0 && r < np) {
+    const float* ls = reinterpret_cast<const float*>(smem);
+#pragma unroll
+    for (int e = 0; e < kFList; ++e) top[e] = fmaxf(top[e], ls[(kFList - 1 - e) * kFT + r]);
+    bitonic_merge_desc(top);
+    const int qi = p0 + r - ci.pair_offs[c];
+    const long long o = ci.part_base[c] + ((long long)qi * ci.nchunks[c] + it.chunk) * use_k;
+#pragma unroll
+    for (int e = 0; e < kFList; ++e)
+      if (e < use_k) apart[o + e] = top[e];
+  }
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kFT) : "memory");
   }
 }
 
-// Row i of the BF16 planes (rows_pad x kFK, zero padded) = the hi / lo split
-// of row src(i) of S (row-major, K doubles per row): src(i) = pairs[i] % ntest
-// when pairs is given (the test row of class-sorted pair i), else i.
-__global__ void knn_split_rows_kernel(const double* __restrict__ S, int rows, int K, const int* __restrict__ pairs,
-                                      int ntest, int rows_pad, __nv_bfloat16* __restrict__ hi,
-                                      __nv_bfloat16* __restrict__ lo) {
-  const size_t total = (size_t)rows_pad * kFK;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int i = static_cast<int>(t / kFK), k = static_cast<int>(t % kFK);
-    double x = 0.0;
-    if (i < rows && k < K) {
-      const int src = pairs ? pairs[i] % ntest : i;
-      x = S[(size_t)src * K + k];
+// Row i of the FP16 plane (rows_pad x kw, zero padded) = row src(i) of S
+// (row-major, K doubles a row) times a power of two, one warp a row: src(i) =
+// pairs[i] % ntest when pairs is given (the test row of class-sorted pair i;
+// the power takes its norm into [1/2, 1), and slack[i] = 2 eps in the scaled
+// units, rounded up), else i (the power takes the largest norm of the rows,
+// *ymax_bits, into [1/2, 1]).  A norm that is not finite raises *flag to 2 and
+// leaves zeros, except that of a test row with a NaN, which has no similarity
+// to anything: zeros, and a slack of -inf that lets no row through.
+__global__ void __launch_bounds__(256)
+knn_half_rows_kernel(const double* __restrict__ S, int rows, int K, const int* __restrict__ pairs, int ntest,
+                     int rows_pad, int kw, const unsigned* __restrict__ ymax_bits, __half* __restrict__ plane,
+                     float* __restrict__ slack, int* flag) {
+  const int lane = threadIdx.x & 31;
+  const double ymax = static_cast<double>(__uint_as_float(*ymax_bits));
+  int ey = 0;
+  const bool y_ok = isfinite(ymax);
+  if (y_ok) frexp(ymax, &ey);
+  const int nq = kw / 64;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < rows_pad; i += gridDim.x * 8) {
+    double x[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    if (i < rows) {
+      const double* row = S + (size_t)(pairs ? pairs[i] % ntest : i) * K;
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (m * 64 + lane * 2 + u < K) x[m][u] = row[m * 64 + lane * 2 + u];
     }
-    const __nv_bfloat16 h = __double2bfloat16(x);
-    hi[t] = h;
-    lo[t] = __double2bfloat16(x - static_cast<double>(__bfloat162float(h)));
+    int e = ey;
+    bool ok = y_ok;
+    if (pairs) {
+      double s2 = 0.0;
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) s2 = fma(x[m][u], x[m][u], s2);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      const double norm = sqrt(s2);
+      ok = isfinite(norm);
+      e = 0;
+      if (ok) frexp(norm, &e);
+      if (lane == 0 && i < rows) {
+        // 2 (17/16 2^-10) |x| max|y|
+        slack[i] = ok ? __double2float_ru(ldexp(norm, -e) * ldexp(ymax, -ey) * (17.0 / 8192.0))
+                      : (norm != norm ? -INFINITY : INFINITY);
+        if (!ok && norm == norm) atomicMax(flag, 2);
+      }
+    }
+    if (!y_ok && i == 0 && lane == 0) atomicMax(flag, 2);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      if (m < nq) {
+        const __half2 v = ok ? __halves2half2(__double2half(ldexp(x[m][0], -e)), __double2half(ldexp(x[m][1], -e)))
+                             : __halves2half2(__half(0.0f), __half(0.0f));
+        *reinterpret_cast<__half2*>(plane + (size_t)i * kw + m * 64 + lane * 2) = v;
+      }
   }
 }
 
-// Largest row norm of S (rows x K, row-major) as float bits (non-negative
-// floats order as their bit patterns; a NaN norm wins and disables the filter).
-__global__ void knn_row_norm_max_kernel(const double* __restrict__ S, int rows, int K, unsigned* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows) return;
-  double s = 0.0;
-  for (int k = 0; k < K; ++k) s = fma(S[(size_t)i * K + k], S[(size_t)i * K + k], s);
-  atomicMax(out, __float_as_uint(__double2float_ru(sqrt(s))));
+// Row i of the BF16 planes (rows_pad x kw, zero padded) = the hi / lo split
+// of row src(i) of S (row-major, K doubles per row): src(i) = pairs[i] % ntest
+// when pairs is given (the test row of class-sorted pair i; slack[i] = 2 eps,
+// rounded up), else i.
+__global__ void __launch_bounds__(256)
+knn_split_rows_kernel(const double* __restrict__ S, int rows, int K, const int* __restrict__ pairs, int ntest,
+                      int rows_pad, int kw, const unsigned* __restrict__ ymax_bits, __nv_bfloat16* __restrict__ hi,
+                      __nv_bfloat16* __restrict__ lo, float* __restrict__ slack) {
+  const int lane = threadIdx.x & 31;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < rows_pad; i += gridDim.x * 8) {
+    const double* row = S + (size_t)(i < rows ? (pairs ? pairs[i] % ntest : i) : 0) * K;
+    double s2 = 0.0;
+    for (int k = lane; k < kw; k += 32) {
+      const double x = (i < rows && k < K) ? row[k] : 0.0;
+      s2 = fma(x, x, s2);
+      const __nv_bfloat16 h = __double2bfloat16(x);
+      hi[(size_t)i * kw + k] = h;
+      lo[(size_t)i * kw + k] = __double2bfloat16(x - static_cast<double>(__bfloat162float(h)));
+    }
+    if (pairs && i < rows) {
+      for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      if (lane == 0)
+        slack[i] = __double2float_ru(ldexp(sqrt(s2) * static_cast<double>(__uint_as_float(*ymax_bits)), -13));
+    }
+  }
+}
+
+// Largest row norm of S (rows x K, row-major), rounded up, as float bits
+// (non-negative floats order as their bit patterns; a NaN norm wins): one warp
+// a row, four rows' loads in flight.
+__global__ void __launch_bounds__(256)
+knn_row_norm_max_kernel(const double* __restrict__ S, int rows, int K, unsigned* out) {
+  const int lane = threadIdx.x & 31;
+  const int stride = gridDim.x * 8;
+  unsigned best = 0u;
+  for (int i0 = blockIdx.x * 8 + (threadIdx.x >> 5); i0 < rows; i0 += 4 * stride) {
+    double x[4][kFK / 32];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int m = 0; m < kFK / 32; ++m) {
+        const long long i = i0 + (long long)u * stride;
+        x[u][m] = (i < rows && lane + 32 * m < K) ? S[(size_t)i * K + lane + 32 * m] : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      double s2 = 0.0;
+#pragma unroll
+      for (int m = 0; m < kFK / 32; ++m) s2 = fma(x[u][m], x[u][m], s2);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      best = max(best, __float_as_uint(__double2float_ru(sqrt(s2))) & 0x7fffffffu);
+    }
+  }
+  if (lane == 0 && best) atomicMax(out, best);
 }
 
 // Per class-sorted pair: theta = the k-th largest approximate similarity over
 // all its chunk lists, bar = theta - 2 eps (rounded down), -inf when the
-// class has fewer than k rows.
-__global__ void knn_filter_bar_kernel(const float* __restrict__ apart, KnnClassInfo ci, int C,
-                                      const int* __restrict__ pairs, long long total_pairs, int ntest,
-                                      const double* __restrict__ Tq, int K, int use_k,
-                                      const unsigned* __restrict__ ymax_bits, float* __restrict__ bar) {
+// class has fewer than k rows.  The running list stays in registers: a sorted
+// chunk list merges into it as max against the reverse, then a bitonic merge.
+__global__ void __launch_bounds__(256)
+knn_filter_bar_kernel(const float* __restrict__ apart, KnnClassInfo ci, int C, long long total_pairs, int use_k,
+                      const float* __restrict__ slack, float* __restrict__ bar) {
   const long long P = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (P >= total_pairs) return;
   int lo = 0, hi = C - 1;   // the last class whose pair offset is <= P
@@ -795,26 +978,25 @@ __global__ void knn_filter_bar_kernel(const float* __restrict__ apart, KnnClassI
   const int c = lo;
   const long long qi = P - ci.pair_offs[c];
   const int nch = ci.nchunks[c];
-  float lst[kKnnMax];
-  for (int e = 0; e < use_k; ++e) lst[e] = -INFINITY;
+  float lst[kFList];
+#pragma unroll
+  for (int e = 0; e < kFList; ++e) lst[e] = -INFINITY;
   for (int s = 0; s < nch; ++s) {
     const float* l = apart + ci.part_base[c] + (qi * nch + s) * use_k;
-    for (int e = 0; e < use_k; ++e) {
-      const float v = l[e];
-      if (!(v > lst[use_k - 1])) break;   // chunk lists are sorted
-      insert_desc<float, int>(lst, nullptr, use_k, 1, v, 0);
-    }
+    float in[kFList];
+#pragma unroll
+    for (int e = 0; e < kFList; ++e) in[e] = e < use_k ? l[e] : -INFINITY;
+#pragma unroll
+    for (int e = 0; e < kFList; ++e) lst[e] = fmaxf(lst[e], in[kFList - 1 - e]);
+    bitonic_merge_desc(lst);
   }
-  const float theta = lst[use_k - 1];
-  if (theta == -INFINITY) {
-    bar[P] = -INFINITY;
-    return;
-  }
-  const double* x = Tq + (size_t)(pairs[P] % ntest) * K;
-  double s2 = 0.0;
-  for (int k = 0; k < K; ++k) s2 = fma(x[k], x[k], s2);
-  const double eps = ldexp(sqrt(s2) * static_cast<double>(__uint_as_float(*ymax_bits)), -14);
-  bar[P] = __double2float_rd(static_cast<double>(theta) - 2.0 * eps);
+  float theta = lst[0];
+#pragma unroll
+  for (int e = 1; e < kFList; ++e)
+    if (e == use_k - 1) theta = lst[e];
+  // a slack of -inf marks a test row with a NaN: no row reaches its bar
+  const float sl = slack[P];
+  bar[P] = sl == -INFINITY ? INFINITY : (theta == -INFINITY ? -INFINITY : __fadd_rd(theta, -sl));
 }
 
 // Exact scores of the candidates of every pair (one warp per class-sorted
@@ -822,7 +1004,7 @@ __global__ void knn_filter_bar_kernel(const float* __restrict__ apart, KnnClassI
 // takes candidates lane, lane + 32, ... and forms their dots (k in order).  The
 // use_k largest go to plist[P * use_k ..] in descending order (-inf when there
 // are fewer).  A pair with more than kFCap
-// candidates raises *overflow (its list would be incomplete).
+// candidates raises *overflow to 1 (its list would be incomplete).
 __global__ void knn_exact_kernel(const int* __restrict__ ccount, const int* __restrict__ crow,
                                  const int* __restrict__ pairs, long long total_pairs, int ntest,
                                  const double* __restrict__ Tq, const double* __restrict__ Ts, int K, int use_k,
@@ -832,7 +1014,7 @@ __global__ void knn_exact_kernel(const int* __restrict__ ccount, const int* __re
   if (P >= total_pairs) return;   // whole warps
   int cnt = ccount[P];
   if (cnt > kFCap) {
-    if (lane == 0) atomicExch(overflow, 1);
+    if (lane == 0) atomicMax(overflow, 1);
     cnt = kFCap;
   }
   const double* xr = Tq + (size_t)(pairs[P] % ntest) * K;
@@ -906,13 +1088,14 @@ __global__ void knn_exact_kernel(const int* __restrict__ ccount, const int* __re
   }
 }
 
-CUtensorMap make_bf16_rows_map(const __nv_bfloat16* p, int rows_pad) {
+// A plane of 16-bit score rows, kw (64 or 128) wide, in boxes of 64 x 128.
+CUtensorMap make_rows_map(CUtensorMapDataType type, const void* p, int rows_pad, int kw) {
   CUtensorMap m;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(kFK), static_cast<cuuint64_t>(rows_pad)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(kFK) * 2};
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(kw), static_cast<cuuint64_t>(rows_pad)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(kw) * 2};
   cuuint32_t box[2] = {64, static_cast<cuuint32_t>(kFT)};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = tc::encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p), dims, strides,
+  CUresult r = tc::encode_fn()(&m, type, 2, const_cast<void*>(p), dims, strides,
                                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed (cKNN score planes)");
@@ -1049,8 +1232,7 @@ void candidate_centroids_device(const double* dTn, int n, int k, const int* dy, 
 
 void candidate_knn_predict_device(const double* dTt, int ntest, const double* dTr, int ntrain, int kdim,
                                   const int* dy, const double* dC, int C, const double* dbias, int top_k,
-                                  int top_m, int knn_k, double tau, double alpha, int* d_ti, double* d_ts,
-                                  bool allow_filter) {
+                                  int top_m, int knn_k, double tau, double alpha, int* d_ti, double* d_ts) {
   Context& ctx = Context::get();
   const int tk = std::max(1, std::min(top_k, C));
   const int tm = std::max(tk, std::min(std::max(1, top_m), C));
@@ -1100,38 +1282,44 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const double* dT
   std::vector<int> hp(C);
   d2h(hp.data(), pcount, C * sizeof(int));
   ctx.sync();
-  // Tile kernel (FASTPLS_CKNN_TILES): 4 or unset the BF16 tensor-core filter
-  // with exact FP64 rescoring (score rows up to 128 wide), 1 the 16-wide
-  // k-step FP64 kernel, 2 / 3 the staged FP64 kernels with two / one
-  // training-row buffers.
+  // Tile kernel (FASTPLS_CKNN_TILES): 4 or unset the tensor-core filter with
+  // exact FP64 rescoring (score rows up to 128 wide), 1 the 16-wide k-step FP64
+  // kernel, 2 / 3 the staged FP64 kernels with two / one training-row buffers.
   const char* tv = std::getenv("FASTPLS_CKNN_TILES");
   const char sel = (tv && tv[0]) ? tv[0] : '4';
-  const bool use_filter = allow_filter && sel == '4' && kdim <= kFK && use_k <= kFList;
-  const int tile_m = use_filter ? kFT : kTileM;   // pairs per item
-  const int gran = use_filter ? kFT : kTileN;     // chunk rows are a multiple of this
-  std::vector<int> poffs(C + 1, 0), chunk_rows(C, 0), nchunks(C, 0);
-  std::vector<long long> part_base(C, 0);
+  const bool use_filter = sel == '4' && kdim <= kFK && use_k <= kFList;
+  std::vector<int> poffs(C + 1, 0);
+  for (int c = 0; c < C; ++c) poffs[c + 1] = poffs[c] + hp[c];
+  // the (class, pair tile, row chunk) items of a tile kernel and the places of
+  // their lists: tile_m pairs an item, chunks of a multiple of gran rows
+  std::vector<int> chunk_rows(C), nchunks(C);
+  std::vector<long long> part_base(C);
   std::vector<KnnItem> items;
   long long part_total = 0;
-  for (int c = 0; c < C; ++c) {
-    poffs[c + 1] = poffs[c] + hp[c];
-    const int rows = cr.offs[c + 1] - cr.offs[c];
-    int S = 0, cr_rows = 0;
-    if (rows > 0) {
-      S = std::min(kMaxChunks, std::max(1, ceil_div(rows, kMinChunkRows)));
-      cr_rows = ceil_div(ceil_div(rows, S), gran) * gran;
-      S = ceil_div(rows, cr_rows);
+  auto make_items = [&](int tile_m, int gran) {
+    items.clear();
+    part_total = 0;
+    for (int c = 0; c < C; ++c) {
+      const int rows = cr.offs[c + 1] - cr.offs[c];
+      int S = 0, cr_rows = 0;
+      if (rows > 0) {
+        S = std::min(kMaxChunks, std::max(1, ceil_div(rows, kMinChunkRows)));
+        cr_rows = ceil_div(ceil_div(rows, S), gran) * gran;
+        S = ceil_div(rows, cr_rows);
+      }
+      chunk_rows[c] = cr_rows;
+      nchunks[c] = S;
+      part_base[c] = part_total;
+      part_total += (long long)hp[c] * S * use_k;
+      if (rows > 0 && hp[c] > 0) {
+        const int tiles = ceil_div(hp[c], tile_m);
+        for (int t = 0; t < tiles; ++t)
+          for (int s = 0; s < S; ++s) items.push_back(KnnItem{c, t, s, 0});
+      }
     }
-    chunk_rows[c] = cr_rows;
-    nchunks[c] = S;
-    part_base[c] = part_total;
-    part_total += (long long)hp[c] * S * use_k;
-    if (rows > 0 && hp[c] > 0) {
-      const int tiles = ceil_div(hp[c], tile_m);
-      for (int t = 0; t < tiles; ++t)
-        for (int s = 0; s < S; ++s) items.push_back(KnnItem{c, t, s, 0});
-    }
-  }
+    FPLS_REQUIRE(items.size() < (1u << 31), "candidate-kNN: too many work items");
+  };
+  make_items(use_filter ? kFT : kTileM, use_filter ? kFT : kTileN);
   const long long total_pairs = poffs[C];
   if (pt.enabled()) {
     double work = 0.0;
@@ -1148,116 +1336,154 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const double* dT
   KnnClassInfo ci;
   ci.row_offs = cr.d_offs;
   ci.pair_offs = d_poffs;
-  ci.chunk_rows = upload(chunk_rows.data(), C);
-  ci.nchunks = upload(nchunks.data(), C);
-  ci.part_base = upload(part_base.data(), C);
-  double* part = ctx.arena.alloc_n<double>((size_t)std::max<long long>(part_total, 1));
+  auto upload_items = [&] {
+    ci.chunk_rows = upload(chunk_rows.data(), C);
+    ci.nchunks = upload(nchunks.data(), C);
+    ci.part_base = upload(part_base.data(), C);
+  };
+  upload_items();
   double* cscore = ctx.arena.alloc_n<double>((size_t)npairs);
   pt.mark("class rows + pair lists");
-  // the lists the merge reads: (pair, chunk) lists of the FP64 tiles, or one
-  // exact list per pair from the filter
+  // the lists the merge reads: one exact list per pair from the filter, or
+  // (pair, chunk) lists of the FP64 tiles
   KnnClassInfo ci_merge = ci;
-  const double* merge_part = part;
+  const double* merge_part = nullptr;
+  bool scored = false;
   if (!items.empty() && use_filter) {
     const KnnItem* ditems = upload(items.data(), items.size());
-    FPLS_REQUIRE(items.size() < (1u << 31), "candidate-kNN: too many work items");
     const int slot = ctx.prof_begin("cknn_filter", ctx.stream);
     const int nvalid = cr.offs[C];
     const long long a_rows = (total_pairs + kFT - 1) / kFT * kFT + kFT;
     const long long b_rows = ((long long)nvalid + kFT - 1) / kFT * kFT + kFT;
     FPLS_REQUIRE(a_rows < (1ll << 31) && b_rows < (1ll << 31), "candidate-kNN: too many rows for the filter");
-    __nv_bfloat16* ah = ctx.arena.alloc_n<__nv_bfloat16>((size_t)a_rows * kFK);
-    __nv_bfloat16* al = ctx.arena.alloc_n<__nv_bfloat16>((size_t)a_rows * kFK);
-    __nv_bfloat16* bh = ctx.arena.alloc_n<__nv_bfloat16>((size_t)b_rows * kFK);
-    __nv_bfloat16* bl = ctx.arena.alloc_n<__nv_bfloat16>((size_t)b_rows * kFK);
-    const int gs = 8 * ctx.sm_count;
-    knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, ah, al);
-    ::fpls::note_launch();
-    knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, nullptr, 1, (int)b_rows, bh, bl);
-    ::fpls::note_launch();
+    const int kw = kdim <= 64 ? 64 : kFK;
     unsigned* ymax = ctx.arena.alloc_n<unsigned>(1);
     dzero(ymax, sizeof(unsigned));
+    const int gs = 8 * ctx.sm_count;
     if (nvalid > 0) {
-      knn_row_norm_max_kernel<<<ceil_div(nvalid, 256), 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, ymax);
+      knn_row_norm_max_kernel<<<std::min(gs, ceil_div(nvalid, 8)), 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, ymax);
       ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
     }
+    float* apart = ctx.arena.alloc_n<float>((size_t)std::max<long long>(part_total, 1));
+    float* barv = ctx.arena.alloc_n<float>((size_t)total_pairs);
+    float* slack = ctx.arena.alloc_n<float>((size_t)total_pairs);
+    int* ccount = ctx.arena.alloc_n<int>((size_t)total_pairs);
+    int* crow = ctx.arena.alloc_n<int>((size_t)total_pairs * kFCap);
+    double* plist = ctx.arena.alloc_n<double>((size_t)total_pairs * use_k);
+    uint16_t* aplane = ctx.arena.alloc_n<uint16_t>((size_t)a_rows * kw);
+    uint16_t* bplane = ctx.arena.alloc_n<uint16_t>((size_t)b_rows * kw);
+    int* ferr = ctx.d_status + 24;    // [0] a pipeline wait ran out, [1] the lists are not exact
+    const unsigned ng = (unsigned)items.size();
+    const unsigned bar_grid = (unsigned)ceil_div(total_pairs, 256);
+    const unsigned exact_grid = (unsigned)ceil_div(total_pairs * 32, 256);
+    // both passes, the bar and the exact scores with planes of one form;
+    // returns [1]: 0 when every list is exact, 1 when a pair had more rows
+    // within the error bar than its slots hold, 2 when a row's norm is not finite
+    auto passes = [&](auto planes, const CUtensorMap& mA0, const CUtensorMap& mA1, const CUtensorMap& mB0,
+                      const CUtensorMap& mB1) {
+      constexpr int PLANES = decltype(planes)::value;
+      static bool fattr = false;
+      if (!fattr) {
+        FPLS_CUDA(cudaFuncSetAttribute(knn_filter_kernel<1, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       FilterTile<PLANES>::kSmem));
+        FPLS_CUDA(cudaFuncSetAttribute(knn_filter_kernel<2, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       FilterTile<PLANES>::kSmem));
+        fattr = true;
+      }
+      dzero(ccount, (size_t)total_pairs * sizeof(int));
+      knn_filter_kernel<1, PLANES><<<ng, kFThreads, FilterTile<PLANES>::kSmem, ctx.stream>>>(
+          mA0, mA1, mB0, mB1, ditems, ci, kdim, use_k, apart, nullptr, nullptr, nullptr, ferr);
+      ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      pt.mark("filter pass 1");
+      knn_filter_bar_kernel<<<bar_grid, 256, 0, ctx.stream>>>(apart, ci, C, total_pairs, use_k, slack, barv);
+      ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      pt.mark("filter bar");
+      knn_filter_kernel<2, PLANES><<<ng, kFThreads, FilterTile<PLANES>::kSmem, ctx.stream>>>(
+          mA0, mA1, mB0, mB1, ditems, ci, kdim, use_k, nullptr, barv, ccount, crow, ferr);
+      ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      pt.mark("filter pass 2");
+      knn_exact_kernel<<<exact_grid, 256, 0, ctx.stream>>>(ccount, crow, pairs, total_pairs, ntest, Tq, cr.Ts, kdim,
+                                                          use_k, plist, ferr + 1);
+      ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      pt.mark("filter exact scores");
+      int flags[2] = {0, 0};
+      d2h(flags, ferr, 2 * sizeof(int));
+      ctx.sync();
+      if (flags[0]) throw Error(kErrCuda, "candidate-kNN: a filter tile's pipeline wait timed out");
+      return flags[1];
+    };
+    dzero(ferr, 2 * sizeof(int));
+    __half* a16 = reinterpret_cast<__half*>(aplane);
+    __half* b16 = reinterpret_cast<__half*>(bplane);
+    knn_half_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, kw, ymax,
+                                                     a16, slack, ferr + 1);
+    ::fpls::note_launch();
+    knn_half_rows_kernel<<<gs, 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, nullptr, 1, (int)b_rows, kw, ymax, b16,
+                                                     nullptr, ferr + 1);
+    ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     pt.mark("filter planes");
-    const CUtensorMap mAh = make_bf16_rows_map(ah, (int)a_rows), mAl = make_bf16_rows_map(al, (int)a_rows);
-    const CUtensorMap mBh = make_bf16_rows_map(bh, (int)b_rows), mBl = make_bf16_rows_map(bl, (int)b_rows);
-    float* apart = ctx.arena.alloc_n<float>((size_t)std::max<long long>(part_total, 1));
-    float* barv = ctx.arena.alloc_n<float>((size_t)std::max<long long>(total_pairs, 1));
-    int* ferr = ctx.d_status + 24;
-    dzero(ferr, sizeof(int));
-    int* ccount = ctx.arena.alloc_n<int>((size_t)std::max<long long>(total_pairs, 1));
-    int* crow = ctx.arena.alloc_n<int>((size_t)std::max<long long>(total_pairs, 1) * kFCap);
-    dzero(ccount, (size_t)std::max<long long>(total_pairs, 1) * sizeof(int));
-    static bool fattr = false;
-    if (!fattr) {
-      FPLS_CUDA(cudaFuncSetAttribute(knn_filter_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
-      FPLS_CUDA(cudaFuncSetAttribute(knn_filter_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
-      fattr = true;
+    const CUtensorMap mA = make_rows_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a16, (int)a_rows, kw);
+    const CUtensorMap mB = make_rows_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b16, (int)b_rows, kw);
+    int left = passes(std::integral_constant<int, 1>{}, mA, mA, mB, mB);
+    if (left == 1) {
+      // similarities crowd within the FP16 bar: a bar 17 times narrower
+      __nv_bfloat16* ah = reinterpret_cast<__nv_bfloat16*>(aplane);
+      __nv_bfloat16* bh = reinterpret_cast<__nv_bfloat16*>(bplane);
+      __nv_bfloat16* al = ctx.arena.alloc_n<__nv_bfloat16>((size_t)a_rows * kw);
+      __nv_bfloat16* bl = ctx.arena.alloc_n<__nv_bfloat16>((size_t)b_rows * kw);
+      dzero(ferr, 2 * sizeof(int));
+      knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, kw,
+                                                        ymax, ah, al, slack);
+      ::fpls::note_launch();
+      knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, nullptr, 1, (int)b_rows, kw, ymax, bh,
+                                                        bl, nullptr);
+      ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      pt.mark("filter planes");
+      const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+      left = passes(std::integral_constant<int, 2>{}, make_rows_map(bf, ah, (int)a_rows, kw),
+                    make_rows_map(bf, al, (int)a_rows, kw), make_rows_map(bf, bh, (int)b_rows, kw),
+                    make_rows_map(bf, bl, (int)b_rows, kw));
     }
-    const unsigned ng = (unsigned)items.size();
-    knn_filter_kernel<1><<<ng, kFThreads, kFSmem, ctx.stream>>>(mAh, mAl, mBh, mBl, ditems, ci, pairs, ntest, Tq,
-                                                               cr.Ts, kdim, use_k, apart, nullptr, nullptr, nullptr,
-                                                               ferr);
-    ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-    pt.mark("filter pass 1");
-    knn_filter_bar_kernel<<<(unsigned)ceil_div(total_pairs, 256), 256, 0, ctx.stream>>>(
-        apart, ci, C, pairs, total_pairs, ntest, Tq, kdim, use_k, ymax, barv);
-    ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-    pt.mark("filter bar");
-    knn_filter_kernel<2><<<ng, kFThreads, kFSmem, ctx.stream>>>(mAh, mAl, mBh, mBl, ditems, ci, pairs, ntest, Tq,
-                                                               cr.Ts, kdim, use_k, nullptr, barv, ccount, crow,
-                                                               ferr);
-    ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-    pt.mark("filter pass 2");
-    // exact scores of the candidates, one list per pair
-    double* plist = ctx.arena.alloc_n<double>((size_t)std::max<long long>(total_pairs, 1) * use_k);
-    int* fover = ctx.d_status + 25;
-    dzero(fover, sizeof(int));
-    knn_exact_kernel<<<(unsigned)ceil_div(total_pairs * 32, 256), 256, 0, ctx.stream>>>(
-        ccount, crow, pairs, total_pairs, ntest, Tq, cr.Ts, kdim, use_k, plist, fover);
-    ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-    pt.mark("filter exact scores");
-    std::vector<int> ones(C, 1);
-    std::vector<long long> pbase(C);
-    for (int c = 0; c < C; ++c) pbase[c] = (long long)poffs[c] * use_k;
-    ci_merge.nchunks = upload(ones.data(), C);
-    ci_merge.part_base = upload(pbase.data(), C);
-    merge_part = plist;
     if (slot >= 0) {
-      // algorithmic work: the three BF16 products of both passes over every
+      // algorithmic work: the FP16 products of both passes over every
       // (candidate pair, class row); bytes: the score planes of every class's
-      // training rows once per 128-pair tile and pass, the pair planes once
-      // (the class's time includes the planes, the bar and the exact scores)
-      double work = 0.0, bytes = 2.0 * 4.0 * kFK * (double)total_pairs;
+      // training rows once per 128-pair tile and pass, the pair planes once a
+      // pass (the class's time includes the planes, the bar, the exact scores
+      // and the split BF16 products where they run)
+      double work = 0.0, bytes = 2.0 * 2.0 * kw * (double)total_pairs;
       for (int c = 0; c < C; ++c) {
         const double rows = cr.offs[c + 1] - cr.offs[c];
         work += (double)hp[c] * rows;
-        bytes += 2.0 * 4.0 * kFK * rows * (double)ceil_div(hp[c], kFT);
+        bytes += 2.0 * 2.0 * kw * rows * (double)ceil_div(hp[c], kFT);
       }
-      ctx.prof_end(slot, ctx.stream, bytes, 2.0 * 3.0 * 2.0 * work * kdim);
+      ctx.prof_end(slot, ctx.stream, bytes, 2.0 * 2.0 * work * kdim);
     }
-    int flags[2] = {0, 0};
-    d2h(flags, ferr, 2 * sizeof(int));
-    ctx.sync();
-    if (flags[0]) throw Error(kErrCuda, "candidate-kNN: a filter tile's pipeline wait timed out");
-    if (flags[1]) {
-      // a pair had more rows within the error bar than its candidate slots
-      // hold: the call runs again on the FP64 tiles
-      candidate_knn_predict_device(dTt, ntest, dTr, ntrain, kdim, dy, dC, C, dbias, top_k, top_m, knn_k, tau,
-                                   alpha, d_ti, d_ts, false);
-      return;
+    if (left == 0) {
+      std::vector<int> ones(C, 1);
+      std::vector<long long> pbase(C);
+      for (int c = 0; c < C; ++c) pbase[c] = (long long)poffs[c] * use_k;
+      ci_merge.nchunks = upload(ones.data(), C);
+      ci_merge.part_base = upload(pbase.data(), C);
+      merge_part = plist;
+      scored = true;
+    } else {
+      // the FP64 tiles score every row
+      make_items(kTileM, kTileN);
+      upload_items();
+      ci_merge = ci;
     }
-  } else if (!items.empty()) {
+  }
+  if (!items.empty() && !scored) {
     const KnnItem* ditems = upload(items.data(), items.size());
-    FPLS_REQUIRE(items.size() < (1u << 31), "candidate-kNN: too many work items");
+    double* part = ctx.arena.alloc_n<double>((size_t)std::max<long long>(part_total, 1));
+    merge_part = part;
     const int slot = ctx.prof_begin("cknn_tiles", ctx.stream);
     // stride of the staged rows: K rounded up to 4, then to 4 mod 16
     const int KP = (kdim + 3) / 4 * 4;
