@@ -79,19 +79,76 @@ __global__ void row_l2_kernel(const double* __restrict__ A, int n, int k, double
   for (int j = 0; j < k; ++j) out[i + (size_t)j * n] = A[i + (size_t)j * n] / nr;
 }
 
-__global__ void class_hist_kernel(const int* __restrict__ codes, int n, int C, int* counts) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int c = codes[i];
-    if (c >= 1 && c <= C) atomicAdd(counts + (c - 1), 1);
+// Class counts and class-contiguous slots of integer codes 1..C (other codes
+// are dropped).  One atomic a code on its class's counter serialises the
+// frequent classes in L2: 1,200,000 codes, the most frequent of 1000 classes a
+// tenth of them, took 280 us for the counts and 280 us for the slots.  So a
+// block counts a range of codes in shared memory, where the count before each
+// code is also its rank, and takes one range of slots a class: 12 and 17 us.
+// More classes than the shared counters hold use the counters in L2 directly.
+constexpr int kHistClasses = 12288;       // 48 KB of shared counters
+constexpr int kSlotRows = 4096;           // codes a block ranks
+constexpr int kSlotThreads = 256;
+__global__ void __launch_bounds__(kSlotThreads)
+class_hist_kernel(const int* __restrict__ codes, int n, int C, int in_smem, int* counts) {
+  extern __shared__ int hist[];
+  if (in_smem) {
+    for (int c = threadIdx.x; c < C; c += kSlotThreads) hist[c] = 0;
+    __syncthreads();
+  }
+  const long long i0 = (long long)blockIdx.x * kSlotRows;
+#pragma unroll
+  for (int u = 0; u < kSlotRows / kSlotThreads; ++u) {
+    const long long i = i0 + u * kSlotThreads + threadIdx.x;
+    const int c = i < n ? codes[i] : 0;
+    if (c >= 1 && c <= C) atomicAdd((in_smem ? hist : counts) + (c - 1), 1);
+  }
+  if (in_smem) {
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += kSlotThreads)
+      if (hist[c]) atomicAdd(counts + c, hist[c]);
   }
 }
 
-// dest[i] = slot of row i in class-contiguous order (-1 for codes outside 1..C).
-__global__ void class_slot_kernel(const int* __restrict__ codes, int n, int C,
-                                  const int* __restrict__ offs, int* cursor, int* dest) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int c = codes[i];
-    dest[i] = (c >= 1 && c <= C) ? offs[c - 1] + atomicAdd(cursor + (c - 1), 1) : -1;
+// dest[i] = slot of code i in class-contiguous order (-1 when dropped), perm
+// its inverse, sorted[slot] the 0-based class; each may be null.  The order
+// within a class is not fixed.
+__global__ void __launch_bounds__(kSlotThreads)
+class_slot_kernel(const int* __restrict__ codes, int n, int C, const int* __restrict__ offs, int in_smem,
+                  int* cursor, int* __restrict__ dest, int* __restrict__ perm, int* __restrict__ sorted) {
+  extern __shared__ int hist[];
+  const long long i0 = (long long)blockIdx.x * kSlotRows;
+  int code[kSlotRows / kSlotThreads], rank[kSlotRows / kSlotThreads];
+#pragma unroll
+  for (int u = 0; u < kSlotRows / kSlotThreads; ++u) {
+    const long long i = i0 + u * kSlotThreads + threadIdx.x;
+    const int c = i < n ? codes[i] : 0;
+    code[u] = (c >= 1 && c <= C) ? c - 1 : -1;
+  }
+  if (in_smem) {
+    for (int c = threadIdx.x; c < C; c += kSlotThreads) hist[c] = 0;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < kSlotRows / kSlotThreads; ++u)
+    rank[u] = code[u] >= 0 ? atomicAdd((in_smem ? hist : cursor) + code[u], 1) : 0;
+  if (in_smem) {
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += kSlotThreads)
+      if (hist[c]) hist[c] = atomicAdd(cursor + c, hist[c]);   // becomes the block's first rank
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < kSlotRows / kSlotThreads; ++u) {
+    const long long i = i0 + u * kSlotThreads + threadIdx.x;
+    if (i >= n) continue;
+    int d = -1;
+    if (code[u] >= 0) {
+      d = offs[code[u]] + rank[u] + (in_smem ? hist[code[u]] : 0);
+      if (perm) perm[d] = static_cast<int>(i);
+      if (sorted) sorted[d] = code[u];
+    }
+    if (dest) dest[i] = d;
   }
 }
 
@@ -116,17 +173,59 @@ __global__ void transpose_scatter_kernel(const double* __restrict__ A, int n, in
   }
 }
 
+// row_l2 and the scatter above in one pass: out[dest[i] * k + j] = A[i, j] /
+// norm of row i, 32 rows a CTA held in shared memory (k + 1 doubles a row) from
+// the norm to the store, the sums in column order as row_l2_kernel's.  Bound by
+// its one read and one write; 1,200,000 x 100: 0.48 ms, against 1.05 ms for
+// the two kernels.
+constexpr int kL2Rows = 32;
+__global__ void __launch_bounds__(256)
+row_l2_scatter_kernel(const double* __restrict__ A, int n, int k, const int* __restrict__ dest,
+                      double* __restrict__ out) {
+  extern __shared__ double rows_s[];   // kL2Rows x (k + 1), then the norms
+  const int S = k + 1;
+  double* norms = rows_s + (size_t)kL2Rows * S;
+  const int i0 = blockIdx.x * kL2Rows;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = i0 + lane;
+#pragma unroll 8
+  for (int j = warp; j < k; j += 8) rows_s[lane * S + j] = i < n ? A[i + (size_t)j * n] : 0.0;
+  __syncthreads();
+  if (warp == 0) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < k; ++j) {
+      const double v = rows_s[lane * S + j];
+      s += v * v;
+    }
+    double nr = sqrt(s);
+    if (!isfinite(nr) || nr == 0.0) nr = 1.0;
+    norms[lane] = nr;
+  }
+  __syncthreads();
+  for (int r = warp; r < kL2Rows && i0 + r < n; r += 8) {
+    const int d = dest[i0 + r];
+    if (d < 0) continue;
+    const double nr = norms[r];
+    for (int j = lane; j < k; j += 32) out[(size_t)d * k + j] = rows_s[r * S + j] / nr;
+  }
+}
+
 // Class sums of class-contiguous row-major rows (R/main.R:686-698): each CTA
 // walks a fixed range of rows, locating its first class by binary search in
-// the class offsets; each thread keeps up to 4 column sums in registers and
-// flushes them (atomicAdd into sums, C x k column-major) at class boundaries,
-// so a very large class is spread over many CTAs.
-constexpr int kCentCols = 4;
+// the class offsets; each thread keeps a column sum in registers and flushes
+// it (atomicAdd into sums, C x k column-major) at class boundaries, so a very
+// large class is spread over many CTAs.  The next kCentRows rows are loaded
+// before they are added: a load a row, waited for, took 1.1 ms for 1,200,000
+// rows of 100 columns, this 0.16 ms (960 MB).
+constexpr int kCentRows = 16;
 __global__ void __launch_bounds__(128) class_rowsum_kernel(const double* __restrict__ Ts, int k, int nrows,
                                                            const int* __restrict__ offs, int C, int rows,
-                                                           int col0, double* __restrict__ sums) {
+                                                           double* __restrict__ sums) {
   const int s0 = blockIdx.x * rows;
   const int s1 = min(nrows, s0 + rows);
+  const int j = blockIdx.y * 128 + threadIdx.x;
+  if (j >= k) return;
   int lo = 0, hi = C - 1;  // last class with offs[c] <= s0
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -134,31 +233,24 @@ __global__ void __launch_bounds__(128) class_rowsum_kernel(const double* __restr
   }
   int c = lo;
   int cend = offs[c + 1];
-  int jc[kCentCols];
-  double acc[kCentCols];
+  double acc = 0.0;
+  for (int r0 = s0; r0 < s1; r0 += kCentRows) {
+    double v[kCentRows];
 #pragma unroll
-  for (int u = 0; u < kCentCols; ++u) {
-    jc[u] = col0 + threadIdx.x + u * blockDim.x;
-    acc[u] = 0.0;
-  }
-  for (int r = s0; r < s1; ++r) {
-    if (r >= cend) {
+    for (int u = 0; u < kCentRows; ++u) v[u] = r0 + u < s1 ? __ldg(Ts + (size_t)(r0 + u) * k + j) : 0.0;
 #pragma unroll
-      for (int u = 0; u < kCentCols; ++u) {
-        if (jc[u] < k) atomicAdd(sums + c + (size_t)jc[u] * C, acc[u]);
-        acc[u] = 0.0;
+    for (int u = 0; u < kCentRows; ++u) {
+      if (r0 + u >= s1) break;
+      if (r0 + u >= cend) {
+        atomicAdd(sums + c + (size_t)j * C, acc);
+        acc = 0.0;
+        while (r0 + u >= offs[c + 1]) ++c;
+        cend = offs[c + 1];
       }
-      while (r >= offs[c + 1]) ++c;
-      cend = offs[c + 1];
+      acc += v[u];
     }
-    const double* row = Ts + (size_t)r * k;
-#pragma unroll
-    for (int u = 0; u < kCentCols; ++u)
-      if (jc[u] < k) acc[u] += __ldg(row + jc[u]);
   }
-#pragma unroll
-  for (int u = 0; u < kCentCols; ++u)
-    if (jc[u] < k) atomicAdd(sums + c + (size_t)jc[u] * C, acc[u]);
+  atomicAdd(sums + c + (size_t)j * C, acc);
 }
 
 // centroid = row_l2(sums / max(count, 1)); one thread per class.
@@ -169,12 +261,14 @@ __global__ void centroid_finish_kernel(const double* __restrict__ sums, int k, c
   const int cnt = offs[c + 1] - offs[c];
   const double den = cnt > 0 ? (double)cnt : 1.0;
   double sq = 0.0;
+#pragma unroll 16
   for (int j = 0; j < k; ++j) {
     const double t = sums[c + (size_t)j * C] / den;
     sq += t * t;
   }
   double nr = sqrt(sq);
   if (!isfinite(nr) || nr == 0.0) nr = 1.0;
+#pragma unroll 16
   for (int j = 0; j < k; ++j) cent[c + (size_t)j * C] = (sums[c + (size_t)j * C] / den) / nr;
 }
 
@@ -194,24 +288,6 @@ __global__ void select_candidates_kernel(const double* __restrict__ base, int nt
   }
   for (int c = 0; c < C; ++c)
     insert_desc(vals, idx, top_m, (size_t)ntest, base[i + (size_t)c * ntest], c + 1);
-}
-
-__global__ void pair_hist_kernel(const int* __restrict__ cand, long long npairs, int C, int* counts) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npairs;
-       p += (long long)gridDim.x * blockDim.x) {
-    const int c = cand[p];
-    if (c >= 1 && c <= C) atomicAdd(counts + (c - 1), 1);
-  }
-}
-
-// pairs[slot] = flat (row + slot_j * ntest) index into the candidate matrix.
-__global__ void pair_scatter_kernel(const int* __restrict__ cand, long long npairs, int C,
-                                    const int* __restrict__ offs, int* cursor, int* pairs) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npairs;
-       p += (long long)gridDim.x * blockDim.x) {
-    const int c = cand[p];
-    if (c >= 1 && c <= C) pairs[offs[c - 1] + atomicAdd(cursor + (c - 1), 1)] = (int)p;
-  }
 }
 
 struct KnnItem {
@@ -873,7 +949,7 @@ knn_half_rows_kernel(const double* __restrict__ S, int rows, int K, const int* _
     }
     int e = ey;
     bool ok = y_ok;
-    if (pairs) {
+    if (pairs) {   // warp-uniform
       double s2 = 0.0;
 #pragma unroll
       for (int m = 0; m < 2; ++m)
@@ -893,10 +969,12 @@ knn_half_rows_kernel(const double* __restrict__ S, int rows, int K, const int* _
       }
     }
     if (!y_ok && i == 0 && lane == 0) atomicMax(flag, 2);
+    // 2^-e as two factors, each of which a double holds
+    const double f1 = ok ? ldexp(1.0, -(e / 2)) : 0.0, f2 = ok ? ldexp(1.0, -(e - e / 2)) : 0.0;
 #pragma unroll
     for (int m = 0; m < 2; ++m)
       if (m < nq) {
-        const __half2 v = ok ? __halves2half2(__double2half(ldexp(x[m][0], -e)), __double2half(ldexp(x[m][1], -e)))
+        const __half2 v = ok ? __halves2half2(__double2half(x[m][0] * f1 * f2), __double2half(x[m][1] * f1 * f2))
                              : __halves2half2(__half(0.0f), __half(0.0f));
         *reinterpret_cast<__half2*>(plane + (size_t)i * kw + m * 64 + lane * 2) = v;
       }
@@ -1154,49 +1232,52 @@ __global__ void knn_rerank_kernel(const int* __restrict__ cand, const double* __
   }
 }
 
-__global__ void fill_int_kernel(int* x, size_t n, int v) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    x[i] = v;
+void class_hist(const int* codes, int n, int C, int* counts) {
+  Context& ctx = Context::get();
+  FPLS_CUDA(cudaMemsetAsync(counts, 0, C * sizeof(int), ctx.stream));
+  if (n <= 0) return;
+  const int in_smem = C <= kHistClasses;
+  class_hist_kernel<<<ceil_div(n, kSlotRows), kSlotThreads, in_smem ? C * sizeof(int) : 0, ctx.stream>>>(
+      codes, n, C, in_smem, counts);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
 }
 
-// Class-contiguous, row-major copy of the rows of T (n x k, column-major) by
-// class code; returns the C + 1 row offsets on the host and device.
-struct ClassRows {
-  double* Ts = nullptr;       // rows in class order, row-major (nvalid x k)
-  int* d_offs = nullptr;      // C + 1
-  std::vector<int> offs;      // C + 1 (host)
-};
+}  // namespace
+
+void class_slots(const int* codes, int n, int C, const int* d_offs, int* dest, int* perm, int* sorted) {
+  Context& ctx = Context::get();
+  int* cursor = ctx.arena.alloc_n<int>(C);
+  FPLS_CUDA(cudaMemsetAsync(cursor, 0, C * sizeof(int), ctx.stream));
+  if (n <= 0) return;
+  const int in_smem = C <= kHistClasses;
+  class_slot_kernel<<<ceil_div(n, kSlotRows), kSlotThreads, in_smem ? C * sizeof(int) : 0, ctx.stream>>>(
+      codes, n, C, d_offs, in_smem, cursor, dest, perm, sorted);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+}
 
 ClassRows group_rows_by_class(const double* dT, int n, int k, const int* dcodes, int C) {
   Context& ctx = Context::get();
   ClassRows cr;
   int* counts = ctx.arena.alloc_n<int>(C);
-  int* cursor = ctx.arena.alloc_n<int>(C);
   int* dest = ctx.arena.alloc_n<int>(std::max(n, 1));
-  fill_int_kernel<<<ceil_div(C, 256), 256, 0, ctx.stream>>>(counts, C, 0); ::fpls::note_launch();
-  fill_int_kernel<<<ceil_div(C, 256), 256, 0, ctx.stream>>>(cursor, C, 0); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
-  const int g = std::max(1, std::min(ceil_div(n, 256), 8 * ctx.sm_count));
-  class_hist_kernel<<<g, 256, 0, ctx.stream>>>(dcodes, n, C, counts); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  class_hist(dcodes, n, C, counts);
   std::vector<int> h(C);
   d2h(h.data(), counts, C * sizeof(int));
   ctx.sync();
   cr.offs.assign(C + 1, 0);
   for (int c = 0; c < C; ++c) cr.offs[c + 1] = cr.offs[c] + h[c];
-  cr.d_offs = ctx.arena.alloc_n<int>(C + 1);
-  h2d(cr.d_offs, cr.offs.data(), (C + 1) * sizeof(int));
-  class_slot_kernel<<<g, 256, 0, ctx.stream>>>(dcodes, n, C, cr.d_offs, cursor, dest); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
-  const int nvalid = cr.offs[C];
-  cr.Ts = ctx.arena.alloc_n<double>((size_t)std::max(nvalid, 1) * k);
+  int* d_offs = ctx.arena.alloc_n<int>(C + 1);
+  h2d(d_offs, cr.offs.data(), (C + 1) * sizeof(int));
+  cr.d_offs = d_offs;
+  class_slots(dcodes, n, C, d_offs, dest, nullptr, nullptr);
+  cr.Ts = ctx.arena.alloc_n<double>((size_t)std::max(cr.offs[C], 1) * k);
   dim3 grid(ceil_div(n, 32), ceil_div(k, 32));
   transpose_scatter_kernel<<<grid, dim3(32, 8), 0, ctx.stream>>>(dT, n, k, dest, cr.Ts); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
   return cr;
 }
-
-}  // namespace
 
 using capi::upload;
 
@@ -1212,27 +1293,48 @@ void candidate_scores_device(const double* dT, int n, int k, const double* dCk, 
   FPLS_CHECK_LAUNCH();
 }
 
-void candidate_centroids_device(const double* dTn, int n, int k, const int* dy, int C, double* dCent) {
+void candidate_score_rows_device(const double* dT, int n, int k, const double* dCk, const int* dest, double* dTs) {
   Context& ctx = Context::get();
-  ClassRows cr = group_rows_by_class(dTn, n, k, dy, C);
+  double* prod = ctx.arena.alloc_n<double>((size_t)n * k);
+  gemm(false, false, n, k, k, 1.0, dT, n, dCk, k, 0.0, prod, n);
+  const size_t smem = sizeof(double) * kL2Rows * ((size_t)k + 2);
+  // two CTAs an SM still hide a row's norm behind the other's copies; wider
+  // rows go through memory between the two steps
+  if (smem <= 100 * 1024) {
+    static bool attr = false;
+    if (!attr) {
+      FPLS_CUDA(cudaFuncSetAttribute(row_l2_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+      attr = true;
+    }
+    row_l2_scatter_kernel<<<ceil_div(n, kL2Rows), 256, smem, ctx.stream>>>(prod, n, k, dest, dTs);
+  } else {
+    double* Tn = ctx.arena.alloc_n<double>((size_t)n * k);
+    row_l2_kernel<<<ceil_div(n, 128), 128, 0, ctx.stream>>>(prod, n, k, Tn); ::fpls::note_launch();
+    dim3 grid(ceil_div(n, 32), ceil_div(k, 32));
+    transpose_scatter_kernel<<<grid, dim3(32, 8), 0, ctx.stream>>>(Tn, n, k, dest, dTs);
+  }
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+}
+
+void candidate_centroids_device(const ClassRows& cr, int k, int C, double* dCent) {
+  Context& ctx = Context::get();
   const int nvalid = cr.offs[C];
   double* sums = ctx.arena.alloc_n<double>((size_t)C * k);
   fill(sums, (size_t)C * k, 0.0);
   if (nvalid > 0) {
-    const int rows = std::min(2048, std::max(64, ceil_div(nvalid, 4 * ctx.sm_count)));
-    for (int col0 = 0; col0 < k; col0 += 128 * kCentCols) {
-      class_rowsum_kernel<<<ceil_div(nvalid, rows), 128, 0, ctx.stream>>>(cr.Ts, k, nvalid, cr.d_offs, C, rows,
-                                                                         col0, sums); ::fpls::note_launch();
-      FPLS_CHECK_LAUNCH();
-    }
+    const int rows = std::min(2048, std::max(64, ceil_div(ceil_div(nvalid, 16 * ctx.sm_count), kCentRows) * kCentRows));
+    class_rowsum_kernel<<<dim3(ceil_div(nvalid, rows), ceil_div(k, 128)), 128, 0, ctx.stream>>>(
+        cr.Ts, k, nvalid, cr.d_offs, C, rows, sums); ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
   }
-  centroid_finish_kernel<<<ceil_div(C, 128), 128, 0, ctx.stream>>>(sums, k, cr.d_offs, C, dCent); ::fpls::note_launch();
+  centroid_finish_kernel<<<ceil_div(C, 32), 32, 0, ctx.stream>>>(sums, k, cr.d_offs, C, dCent); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 
-void candidate_knn_predict_device(const double* dTt, int ntest, const double* dTr, int ntrain, int kdim,
-                                  const int* dy, const double* dC, int C, const double* dbias, int top_k,
-                                  int top_m, int knn_k, double tau, double alpha, int* d_ti, double* d_ts) {
+void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows& cr, int kdim, const double* dC,
+                                  int C, const double* dbias, int top_k, int top_m, int knn_k, double tau,
+                                  double alpha, int* d_ti, double* d_ts) {
   Context& ctx = Context::get();
   const int tk = std::max(1, std::min(top_k, C));
   const int tm = std::max(tk, std::min(std::max(1, top_m), C));
@@ -1261,9 +1363,8 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const double* dT
     FPLS_CHECK_LAUNCH();
   }
 
-  // training rows grouped by class (row-major), test rows row-major
+  // test rows row-major, as the training rows are
   pt.mark("base scores + candidates");
-  ClassRows cr = group_rows_by_class(dTr, ntrain, kdim, dy, C);
   double* Tq = ctx.arena.alloc_n<double>((size_t)ntest * kdim);
   {
     dim3 grid(ceil_div(ntest, 32), ceil_div(kdim, 32));
@@ -1273,12 +1374,7 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const double* dT
 
   // (row, candidate) pairs grouped by class
   int* pcount = ctx.arena.alloc_n<int>(C);
-  int* pcursor = ctx.arena.alloc_n<int>(C);
-  fill_int_kernel<<<ceil_div(C, 256), 256, 0, ctx.stream>>>(pcount, C, 0); ::fpls::note_launch();
-  fill_int_kernel<<<ceil_div(C, 256), 256, 0, ctx.stream>>>(pcursor, C, 0); ::fpls::note_launch();
-  const int g = std::max(1, std::min(ceil_div(npairs, 256), 8 * ctx.sm_count));
-  pair_hist_kernel<<<g, 256, 0, ctx.stream>>>(cand, npairs, C, pcount); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  class_hist(cand, (int)npairs, C, pcount);
   std::vector<int> hp(C);
   d2h(hp.data(), pcount, C * sizeof(int));
   ctx.sync();
@@ -1330,8 +1426,7 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const double* dT
   int* pairs = ctx.arena.alloc_n<int>((size_t)std::max<long long>(total_pairs, 1));
   int* d_poffs = ctx.arena.alloc_n<int>(C + 1);
   h2d(d_poffs, poffs.data(), (C + 1) * sizeof(int));
-  pair_scatter_kernel<<<g, 256, 0, ctx.stream>>>(cand, npairs, C, d_poffs, pcursor, pairs); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  class_slots(cand, (int)npairs, C, d_poffs, nullptr, pairs, nullptr);
 
   KnnClassInfo ci;
   ci.row_offs = cr.d_offs;
@@ -1590,7 +1685,7 @@ int fpls_candidate_centroids(const double* Tn, int n, int k, const int* y_codes,
     const double* dT = upload(Tn, (size_t)n * k);
     const int* dy = upload(y_codes, n);
     double* dC = ctx.arena.alloc_n<double>((size_t)n_classes * k);
-    candidate_centroids_device(dT, n, k, dy, n_classes, dC);
+    candidate_centroids_device(group_rows_by_class(dT, n, k, dy, n_classes), k, n_classes, dC);
     d2h(centroids, dC, (size_t)n_classes * k * sizeof(double));
     ctx.sync();
   });
@@ -1615,8 +1710,8 @@ int fpls_candidate_knn_predict(const double* Ttest_norm, int ntest, const double
     const double* dbias = candidate_bias ? upload(candidate_bias, C) : nullptr;
     int* d_ti = ctx.arena.alloc_n<int>((size_t)ntest * tk);
     double* d_ts = ctx.arena.alloc_n<double>((size_t)ntest * tk);
-    candidate_knn_predict_device(dTt, ntest, dTr, ntrain, kdim, dy, dC, C, dbias, top_k, top_m, knn_k,
-                                 tau, alpha, d_ti, d_ts);
+    candidate_knn_predict_device(dTt, ntest, group_rows_by_class(dTr, ntrain, kdim, dy, C), kdim, dC, C, dbias, top_k,
+                                 top_m, knn_k, tau, alpha, d_ti, d_ts);
     d2h(top_index, d_ti, (size_t)ntest * tk * sizeof(int));
     d2h(top_score, d_ts, (size_t)ntest * tk * sizeof(double));
     ctx.sync();

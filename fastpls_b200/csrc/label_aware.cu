@@ -24,40 +24,61 @@
 #include "svd.cuh"
 
 namespace fpls {
+
+using capi::upload;
+
 namespace {
 
-// Column sums (and sums of squares) of the raw predictors, one CTA per column
-// (R/main.R:542-551).
+// Column sums (and sums of squares) of the raw predictors (R/main.R:542-551):
+// CTA (j, range) adds a range of column j, sixteen loads a thread in flight,
+// into sums[j + range * p]; la_stats_kernel adds the ranges in order.  One CTA
+// a column with a load at a time took 2.14 ms for 1,200,000 x 768 FP32
+// (3.7 GB), this 0.60 ms.
+constexpr int kSumAhead = 16;
+constexpr int kSumRanges = 16;      // at most
 template <typename T>
-__global__ void col_sums_kernel(const T* __restrict__ X, int n, int p, double* __restrict__ sums,
-                                double* __restrict__ sumsq) {
+__global__ void __launch_bounds__(256)
+col_sums_kernel(const T* __restrict__ X, int n, int p, int rows, double* __restrict__ sums,
+                double* __restrict__ sumsq) {
   __shared__ double scratch[32];
   const int j = blockIdx.x;
+  const int r0 = blockIdx.y * rows, r1 = min(n, r0 + rows);
   const T* col = X + (size_t)j * n;
   double s = 0.0, q = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double v = static_cast<double>(col[i]);
-    s += v;
-    q += v * v;
+  for (int i = r0 + threadIdx.x; i < r1; i += 256 * kSumAhead) {
+    T x[kSumAhead];
+#pragma unroll
+    for (int u = 0; u < kSumAhead; ++u) x[u] = i + u * 256 < r1 ? col[i + u * 256] : T(0);
+#pragma unroll
+    for (int u = 0; u < kSumAhead; ++u) {
+      const double v = static_cast<double>(x[u]);
+      s += v;
+      q += v * v;
+    }
   }
   s = block_sum(s, scratch);
   q = block_sum(q, scratch);
   if (threadIdx.x == 0) {
-    sums[j] = s;
-    sumsq[j] = q;
+    sums[j + (size_t)blockIdx.y * p] = s;
+    sumsq[j + (size_t)blockIdx.y * p] = q;
   }
 }
 
 // mX = sums / n (scaling < 3, else 0); vX = sqrt(max(sumsq - n mX^2, 0) / max(1, n - 1))
 // for scaling 2 with zero / non-finite -> 1 (R/main.R:552-558).
-__global__ void la_stats_kernel(const double* sums, const double* sumsq, int n, int p, int scaling,
+__global__ void la_stats_kernel(const double* sums, const double* sumsq, int ranges, int n, int p, int scaling,
                                 double* mX, double* vX) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p; j += gridDim.x * blockDim.x) {
-    const double m = scaling < 3 ? sums[j] / n : 0.0;
+    double s = 0.0, q = 0.0;
+    for (int r = 0; r < ranges; ++r) {
+      s += sums[j + (size_t)r * p];
+      q += sumsq[j + (size_t)r * p];
+    }
+    const double m = scaling < 3 ? s / n : 0.0;
     mX[j] = m;
     double v = 1.0;
     if (scaling == 2) {
-      const double css = fmax(sumsq[j] - n * m * m, 0.0);
+      const double css = fmax(q - n * m * m, 0.0);
       v = sqrt(css / (double)max(1, n - 1));
       if (!isfinite(v) || v == 0.0) v = 1.0;
     }
@@ -66,35 +87,39 @@ __global__ void la_stats_kernel(const double* sums, const double* sumsq, int n, 
 }
 
 // Xt[j + i * p] = (X[i + j * n] - mX[j]) / vX[j]  (column-major n x p -> row-major),
-// 32 x 32 tiles through shared memory.
+// 64 x 64 tiles through shared memory in X's own type, centred on the way out:
+// a thread stores one column of sixteen rows, so its mean stays in a register,
+// its sixteen loads are in flight together and each row segment is 512 bytes.
+// 1,200,000 x 768 FP32 (3.7 GB in, 7.4 GB out): 1.97 ms; 32 x 32 tiles with
+// four loads a thread took 2.77 ms.
+constexpr int kTT = 64;
 template <typename T>
-__global__ void transpose_center_kernel(const T* __restrict__ X, int n, int p, const double* __restrict__ mX,
-                                        const double* __restrict__ vX, int scaling, double* __restrict__ Xt) {
-  __shared__ double tile[32][33];
-  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int j = j0 + r, i = i0 + threadIdx.x;
-    if (i < n && j < p) {
-      double v = static_cast<double>(X[i + (size_t)j * n]);
-      if (scaling < 3) v -= mX[j];
-      if (scaling == 2) v /= vX[j];
-      tile[r][threadIdx.x] = v;
-    }
+__global__ void __launch_bounds__(256)
+transpose_center_kernel(const T* __restrict__ X, int n, int p, const double* __restrict__ mX,
+                        const double* __restrict__ vX, int scaling, double* __restrict__ Xt) {
+  __shared__ T tile[kTT][kTT + 1];   // [column][row]
+  const int i0 = blockIdx.x * kTT, j0 = blockIdx.y * kTT;
+  const int a = threadIdx.x & (kTT - 1), b = threadIdx.x / kTT;
+  T x[kTT / 4];
+#pragma unroll
+  for (int u = 0; u < kTT / 4; ++u) {
+    const int j = j0 + b + 4 * u;
+    x[u] = (i0 + a < n && j < p) ? X[i0 + a + (size_t)j * n] : T(0);
   }
+#pragma unroll
+  for (int u = 0; u < kTT / 4; ++u) tile[b + 4 * u][a] = x[u];
   __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int i = i0 + r, j = j0 + threadIdx.x;
-    if (i < n && j < p) Xt[j + (size_t)i * p] = tile[threadIdx.x][r];
-  }
-}
-
-__global__ void la_sort_kernel(const int* __restrict__ y, int n, const int* __restrict__ offs, int* cursor,
-                               int* __restrict__ perm, int* __restrict__ ysorted) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int c = y[i] - 1;
-    const int d = offs[c] + atomicAdd(cursor + c, 1);
-    perm[d] = i;
-    ysorted[d] = c;
+  const int j = j0 + a;
+  if (j >= p) return;
+  const double m = mX[j], v = vX[j];
+#pragma unroll
+  for (int u = 0; u < kTT / 4; ++u) {
+    const int i = i0 + b + 4 * u;
+    if (i >= n) break;
+    double y = static_cast<double>(tile[a][b + 4 * u]);
+    if (scaling < 3) y -= m;
+    if (scaling == 2) y /= v;
+    Xt[j + (size_t)i * p] = y;
   }
 }
 
@@ -158,16 +183,43 @@ __global__ void __launch_bounds__(256) class_sum_kernel(const double* __restrict
     if (jcol[u] < p) atomicAdd(cs + jcol[u] + (size_t)cur * p, acc[u]);
 }
 
-// S = cs - total mY^T with total_j = sum_c cs[j, c] (class order) and
-// mY = counts / n (R/main.R:560-592).
-__global__ void la_crosscov_kernel(double* cs, int p, int m, const int* counts, int n, double* mY) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p; j += gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (int c = 0; c < m; ++c) t += cs[j + (size_t)c * p];
-    for (int c = 0; c < m; ++c) cs[j + (size_t)c * p] -= t * ((double)counts[c] / n);
+// total_j = sum_c cs[j, c] (R/main.R:560-592): a CTA takes 32 columns, each of
+// its eight warps a range of the classes, sixteen loads in flight, and the
+// ranges are added in order; mY = counts / n.
+__global__ void __launch_bounds__(256)
+la_total_kernel(const double* __restrict__ cs, int p, int m, const int* __restrict__ counts, int n,
+                double* __restrict__ total, double* __restrict__ mY) {
+  constexpr int kAhead = 16;
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  const int len = (m + 7) / 8, c1 = min(m, (w + 1) * len);
+  double t = 0.0;
+  for (int c0 = w * len; c0 < c1; c0 += kAhead) {
+    double x[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) x[u] = (c0 + u < c1 && j < p) ? cs[j + (size_t)(c0 + u) * p] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) t += x[u];
+  }
+  part[w][lane] = t;
+  __syncthreads();
+  if (w == 0 && j < p) {
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += part[u][lane];
+    total[j] = s;
   }
   if (blockIdx.x == 0)
     for (int c = threadIdx.x; c < m; c += blockDim.x) mY[c] = (double)counts[c] / n;
+}
+
+// S = cs - total mY^T.
+__global__ void la_crosscov_kernel(double* cs, int p, int m, const double* __restrict__ total,
+                                   const double* __restrict__ mY) {
+  for (int c = blockIdx.y; c < m; c += gridDim.y)
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p; j += gridDim.x * blockDim.x)
+      cs[j + (size_t)c * p] -= total[j] * mY[c];
 }
 
 // out (n x p, column-major FP64) = (X - mX) / vX as the model's scaling.
@@ -200,8 +252,7 @@ std::vector<int> cap_plssvd_ncomp(const int* ncomp, int L, int n, int p, int m, 
   return out;
 }
 
-LabelAwareFit label_aware_fit(const void* dX, bool f32, int n, int p, const int* dy, const int* y_host,
-                              int m, const std::vector<int>& ncomp, int scaling, int svd_method,
+LabelAwareFit label_aware_fit(const void* dX, bool f32, int n, int p, const int* y_host, int m, const std::vector<int>& ncomp, int scaling, int svd_method,
                               int oversample, int power_iters, unsigned int seed) {
   Context& ctx = Context::get();
   FPLS_REQUIRE(n >= 1 && p >= 1 && m >= 2,
@@ -217,45 +268,52 @@ LabelAwareFit label_aware_fit(const void* dX, bool f32, int n, int p, const int*
   const int L = static_cast<int>(ncomp.size());
 
   // predictor statistics and the centred row-major copy
-  double* sums = ctx.arena.alloc_n<double>(p);
-  double* sumsq = ctx.arena.alloc_n<double>(p);
+  // (ranges of rows: four CTAs an SM when the columns alone are fewer, at least 4096 rows each)
+  const int ranges = std::max(1, std::min(kSumRanges, std::min(ceil_div(4 * ctx.sm_count, p), n / 4096)));
+  const int range_rows = ceil_div(n, ranges);
+  double* sums = ctx.arena.alloc_n<double>((size_t)p * kSumRanges);
+  double* sumsq = ctx.arena.alloc_n<double>((size_t)p * kSumRanges);
   f.mX = ctx.arena.alloc_n<double>(p);
   f.vX = ctx.arena.alloc_n<double>(p);
-  if (f32) col_sums_kernel<float><<<p, 256, 0, ctx.stream>>>(static_cast<const float*>(dX), n, p, sums, sumsq);
-  else col_sums_kernel<double><<<p, 256, 0, ctx.stream>>>(static_cast<const double*>(dX), n, p, sums, sumsq);
+  const dim3 sgrid(p, ranges);
+  if (f32)
+    col_sums_kernel<float><<<sgrid, 256, 0, ctx.stream>>>(static_cast<const float*>(dX), n, p, range_rows, sums, sumsq);
+  else
+    col_sums_kernel<double><<<sgrid, 256, 0, ctx.stream>>>(static_cast<const double*>(dX), n, p, range_rows, sums,
+                                                          sumsq);
   ::fpls::note_launch();
-  la_stats_kernel<<<ceil_div(p, 256), 256, 0, ctx.stream>>>(sums, sumsq, n, p, scaling, f.mX, f.vX); ::fpls::note_launch();
+  la_stats_kernel<<<ceil_div(p, 256), 256, 0, ctx.stream>>>(sums, sumsq, ranges, n, p, scaling, f.mX, f.vX);
+  ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
   f.Xt = ctx.arena.alloc_n<double>((size_t)n * p);
   {
-    dim3 grid(ceil_div(n, 32), ceil_div(p, 32));
+    dim3 grid(ceil_div(n, kTT), ceil_div(p, kTT));
     if (f32)
-      transpose_center_kernel<float><<<grid, dim3(32, 8), 0, ctx.stream>>>(static_cast<const float*>(dX), n, p,
-                                                                          f.mX, f.vX, scaling, f.Xt);
+      transpose_center_kernel<float><<<grid, 256, 0, ctx.stream>>>(static_cast<const float*>(dX), n, p, f.mX, f.vX,
+                                                                  scaling, f.Xt);
     else
-      transpose_center_kernel<double><<<grid, dim3(32, 8), 0, ctx.stream>>>(static_cast<const double*>(dX), n, p,
-                                                                           f.mX, f.vX, scaling, f.Xt);
+      transpose_center_kernel<double><<<grid, 256, 0, ctx.stream>>>(static_cast<const double*>(dX), n, p, f.mX, f.vX,
+                                                                   scaling, f.Xt);
     ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
   }
   pt.mark("stats + centred copy");
 
-  // class-sorted row order (counting sort of the labels)
+  // class-sorted row order (counting sort of the labels); the labels are
+  // counted on the host and cross the link while the passes above run
   std::vector<int> counts_h(m, 0);
   for (int i = 0; i < n; ++i) counts_h[y_host[i] - 1]++;
-  std::vector<int> offs(m + 1, 0);
-  for (int c = 0; c < m; ++c) offs[c + 1] = offs[c] + counts_h[c];
+  f.offs.assign(m + 1, 0);
+  for (int c = 0; c < m; ++c) f.offs[c + 1] = f.offs[c] + counts_h[c];
+  const int* dy = upload(y_host, n);
   int* counts = ctx.arena.alloc_n<int>(m);
-  int* d_offs = ctx.arena.alloc_n<int>(m + 1);
-  int* cursor = ctx.arena.alloc_n<int>(m);
   int* perm = ctx.arena.alloc_n<int>(n);
   int* ysorted = ctx.arena.alloc_n<int>(n);
+  f.d_offs = ctx.arena.alloc_n<int>(m + 1);
+  f.dest = ctx.arena.alloc_n<int>(n);
   h2d(counts, counts_h.data(), m * sizeof(int));
-  h2d(d_offs, offs.data(), (m + 1) * sizeof(int));
-  FPLS_CUDA(cudaMemsetAsync(cursor, 0, m * sizeof(int), ctx.stream));
-  const int g = std::max(1, std::min(ceil_div(n, 256), 8 * ctx.sm_count));
-  la_sort_kernel<<<g, 256, 0, ctx.stream>>>(dy, n, d_offs, cursor, perm, ysorted); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
+  h2d(f.d_offs, f.offs.data(), (m + 1) * sizeof(int));
+  class_slots(dy, n, m, f.d_offs, f.dest, perm, ysorted);
   pt.mark("class sort");
 
   // class sums -> S (p x m)
@@ -268,7 +326,11 @@ LabelAwareFit label_aware_fit(const void* dX, bool f32, int n, int p, const int*
     FPLS_CHECK_LAUNCH();
   }
   f.mY = ctx.arena.alloc_n<double>(m);
-  la_crosscov_kernel<<<ceil_div(p, 128), 128, 0, ctx.stream>>>(f.S, p, m, counts, n, f.mY); ::fpls::note_launch();
+  double* total = ctx.arena.alloc_n<double>(p);
+  la_total_kernel<<<ceil_div(p, 32), 256, 0, ctx.stream>>>(f.S, p, m, counts, n, total, f.mY); ::fpls::note_launch();
+  la_crosscov_kernel<<<dim3(std::min(ceil_div(p, 256), 64), std::min(m, 4096)), 256, 0, ctx.stream>>>(f.S, p, m, total,
+                                                                                              f.mY);
+  ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
   pt.mark("class sums");
 
@@ -323,20 +385,24 @@ LabelAwareFit label_aware_fit(const void* dX, bool f32, int n, int p, const int*
 // candidate-kNN prediction of the test rows (R/main.R:875-950), all on
 // device buffers.  d_ti / d_ts: ntest x max(1, min(top_k, m)).
 void label_aware_cknn_device(const void* dX, const void* dXtest, bool f32, int n, int ntest, int p,
-                             const int* dy, const int* y_host, int m, int ncomp, int scaling, int svd_method,
+                             const int* y_host, int m, int ncomp, int scaling, int svd_method,
                              int oversample, int power_iters, unsigned int seed, int knn_k, double tau,
                              double alpha, int top_m, int top_k, int* d_ti, double* d_ts,
                              capi::SideUpload* xtest_copy) {
   Context& ctx = Context::get();
   const std::vector<int> nc = cap_plssvd_ncomp(&ncomp, 1, n, p, m, nullptr);
-  LabelAwareFit f = label_aware_fit(dX, f32, n, p, dy, y_host, m, nc, scaling, svd_method, oversample,
+  LabelAwareFit f = label_aware_fit(dX, f32, n, p, y_host, m, nc, scaling, svd_method, oversample,
                                     power_iters, seed);
   PhaseTimer pt("candidate-kNN on label-aware scores");
   const int K = f.K;
-  double* Tn = ctx.arena.alloc_n<double>((size_t)n * K);
-  candidate_scores_device(f.T, n, K, f.C, Tn);
+  // the training score rows go straight into the class order of the fit's sort
+  ClassRows cr;
+  cr.offs = f.offs;
+  cr.d_offs = f.d_offs;
+  cr.Ts = ctx.arena.alloc_n<double>((size_t)n * K);
+  candidate_score_rows_device(f.T, n, K, f.C, f.dest, cr.Ts);
   double* cent = ctx.arena.alloc_n<double>((size_t)m * K);
-  candidate_centroids_device(Tn, n, K, dy, m, cent);
+  candidate_centroids_device(cr, K, m, cent);
   pt.mark("train scores + centroids");
   double* Xc = ctx.arena.alloc_n<double>((size_t)ntest * p);
   if (xtest_copy) xtest_copy->wait();
@@ -354,8 +420,7 @@ void label_aware_cknn_device(const void* dX, const void* dXtest, bool f32, int n
   double* Ttn = ctx.arena.alloc_n<double>((size_t)ntest * K);
   candidate_scores_device(Tt, ntest, K, f.C, Ttn);
   pt.mark("test scores");
-  candidate_knn_predict_device(Ttn, ntest, Tn, n, K, dy, cent, m, nullptr, top_k, top_m, knn_k, tau, alpha,
-                               d_ti, d_ts);
+  candidate_knn_predict_device(Ttn, ntest, cr, K, cent, m, nullptr, top_k, top_m, knn_k, tau, alpha, d_ti, d_ts);
   pt.mark("candidate-kNN predict");
   pt.report();
 }
@@ -363,7 +428,6 @@ void label_aware_cknn_device(const void* dX, const void* dXtest, bool f32, int n
 }  // namespace fpls
 
 using namespace fpls;
-using capi::upload;
 
 extern "C" {
 
@@ -388,8 +452,7 @@ int fpls_plssvd_label_aware(const void* X, int x_is_float32, int n, int p, const
     const size_t xbytes = (size_t)n * p * (x_is_float32 ? sizeof(float) : sizeof(double));
     void* dX = ctx.arena.alloc_n<char>(xbytes);
     h2d(dX, X, xbytes);
-    const int* dy = upload(y_codes, n);
-    LabelAwareFit f = label_aware_fit(dX, x_is_float32 != 0, n, p, dy, y_codes, m, nc, scaling,
+    LabelAwareFit f = label_aware_fit(dX, x_is_float32 != 0, n, p, y_codes, m, nc, scaling,
                                       svd_method, oversample, power_iters,
                                       static_cast<unsigned int>(seed));
     const int K = f.K;
@@ -429,13 +492,12 @@ int fpls_label_aware_cknn(const void* Xtrain, int x_is_float32, int n, int p, co
     const size_t es = x_is_float32 ? sizeof(float) : sizeof(double);
     void* dX = ctx.arena.alloc_n<char>((size_t)n * p * es);
     h2d(dX, Xtrain, (size_t)n * p * es);
-    const int* dy = upload(y_codes, n);
     // the test rows cross the link while the fit runs
     capi::SideUpload xt(Xtest, (size_t)ntest * p * es);
     const int tk = std::max(1, std::min(top_k, m));
     int* d_ti = ctx.arena.alloc_n<int>((size_t)ntest * tk);
     double* d_ts = ctx.arena.alloc_n<double>((size_t)ntest * tk);
-    label_aware_cknn_device(dX, xt.dst, x_is_float32 != 0, n, ntest, p, dy, y_codes, m, ncomp, scaling,
+    label_aware_cknn_device(dX, xt.dst, x_is_float32 != 0, n, ntest, p, y_codes, m, ncomp, scaling,
                             svd_method, oversample, power_iters, static_cast<unsigned int>(seed), knn_k,
                             tau, alpha, top_m, top_k, d_ti, d_ts, &xt);
     d2h(top_index, d_ti, (size_t)ntest * tk * sizeof(int));
@@ -468,11 +530,10 @@ int fpls_label_aware_cknn_resident(int xtrain_handle, const int* y_codes, int m,
     for (int i = 0; i < tr.n; ++i)
       FPLS_REQUIRE(y_codes[i] >= 1 && y_codes[i] <= m, "label-aware PLSSVD: class code outside 1..m");
     ctx.begin_call();
-    const int* dy = upload(y_codes, tr.n);
     const int tk = std::max(1, std::min(top_k, m));
     int* d_ti = ctx.arena.alloc_n<int>((size_t)te.n * tk);
     double* d_ts = ctx.arena.alloc_n<double>((size_t)te.n * tk);
-    label_aware_cknn_device(tr.ptr, te.ptr, tr.f32, tr.n, te.n, tr.p, dy, y_codes, m, ncomp, scaling,
+    label_aware_cknn_device(tr.ptr, te.ptr, tr.f32, tr.n, te.n, tr.p, y_codes, m, ncomp, scaling,
                             svd_method, oversample, power_iters, static_cast<unsigned int>(seed), knn_k,
                             tau, alpha, top_m, top_k, d_ti, d_ts, nullptr);
     d2h(top_index, d_ti, (size_t)te.n * tk * sizeof(int));
