@@ -382,12 +382,43 @@ int fpls_pls_model2_fast_xprod(const double* X, int n, int p, const double* Y, i
   });
 }
 
+// Device copies of what a fit's prediction needs (context arena).
+struct FitOnDevice {
+  double* R = nullptr;    // p x K
+  double* mX = nullptr;   // p
+  double* vX = nullptr;   // p
+};
+
+// Rp = R / vX by rows (a zero or non-finite scale counts as 1) and offset =
+// mX Rp (fastPLS.cpp:6321-6335), one CTA a column.  A pass over R, 8 us for
+// 20000 x 60; formed on the host, with R and Rp crossing the link for it, it
+// took 2.1 ms.
+__global__ void __launch_bounds__(1024)
+prediction_weights_kernel(const double* __restrict__ R, int p, const double* __restrict__ mX,
+                          const double* __restrict__ vX, double* __restrict__ Rp, double* __restrict__ offset) {
+  __shared__ double scratch[32];
+  const size_t col = (size_t)blockIdx.x * p;
+  double sum = 0.0;
+#pragma unroll 4
+  for (int j = threadIdx.x; j < p; j += blockDim.x) {
+    double sc = vX[j];
+    if (!isfinite(sc) || sc == 0.0) sc = 1.0;
+    const double v = R[col + j] / sc;
+    Rp[col + j] = v;
+    sum += mX[j] * v;
+  }
+  sum = block_sum(sum, scratch);
+  if (threadIdx.x == 0) offset[blockIdx.x] = sum;
+}
+
 // Fast SIMPLS (pls_model2_fast): centred / scaled copies of X (n x p) and Y
-// (n x m) go to dX and dYc; host outputs as fpls_pls_model2_fast.
+// (n x m) go to dX and dYc; host outputs as fpls_pls_model2_fast (R, mX, vX
+// may be null when `dev` takes their device copies).
 static void simpls_fast_on_device(const MatrixSource& sX, double* dX, int n, int p, const MatrixSource& sY, double* dYc,
                                   int m, const int* ncomp, int L,
                                   int scaling, int fit, int seed, double* R, double* Q, double* mX, double* vX,
-                                  double* mY, double* B, double* Yfit, double* R2Y, int* n_components) {
+                                  double* mY, double* B, double* Yfit, double* R2Y, int* n_components,
+                                  FitOnDevice* dev = nullptr) {
     FPLS_REQUIRE(n > 0 && p > 0 && m > 0, "pls_model2_fast requires non-empty X and Y");
     FPLS_REQUIRE(L >= 1 && ncomp, "ncomp must contain at least one value");
     FPLS_REQUIRE(!(fit && !Yfit), "fit = 1 requires a Yfit buffer");
@@ -470,11 +501,12 @@ static void simpls_fast_on_device(const MatrixSource& sX, double* dX, int n, int
         ++i_out;
       }
     }
-    download(R, b.R, (size_t)p * K);
-    download(Q, b.Q, (size_t)m * K);
-    download(mX, dmX, p);
-    download(vX, dvX, p);
-    download(mY, dmY, m);
+    if (dev) *dev = FitOnDevice{b.R, dmX, dvX};
+    if (R) download(R, b.R, (size_t)p * K);
+    if (Q) download(Q, b.Q, (size_t)m * K);
+    if (mX) download(mX, dmX, p);
+    if (vX) download(vX, dvX, p);
+    if (mY) download(mY, dmY, m);
     if (B) download(B, dB, (size_t)p * m * L);
     std::vector<double> hrq(2 * L, 0.0);
     if (fit) {
@@ -938,17 +970,19 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
     capi::SideUpload xt_up(Xtest, ntest > 0 ? (size_t)ntest * p * (f32 ? sizeof(float) : sizeof(double)) : 0);
     pt.mark("upload");
     int K0 = 0;
-    double* dR = nullptr;
+    FitOnDevice fd;
+    PlssvdOut o;
+    double* dmY = nullptr;
     double* dT = nullptr;   // training scores (X - mX) / vX R, n x K0
-    std::vector<double> hR, hmX(p), hvX(p);
+    std::vector<double> r2(L, 0.0);
     if (method == 1) {
       const int max_rank = std::min(n, std::min(p, m));
       for (int& c : nc) c = std::min(c, max_rank);
       K0 = std::min(max_of(nc.data(), L), max_rank);
-      double* dmX = ctx.arena.alloc_n<double>(p);
-      double* dvX = ctx.arena.alloc_n<double>(p);
-      double* dmY = ctx.arena.alloc_n<double>(m);
-      center_scale_xy(sX, dX, n, p, sY, dY, m, scaling, dmX, dvX, dmY);
+      fd.mX = ctx.arena.alloc_n<double>(p);
+      fd.vX = ctx.arena.alloc_n<double>(p);
+      dmY = ctx.arena.alloc_n<double>(m);
+      center_scale_xy(sX, dX, n, p, sY, dY, m, scaling, fd.mX, fd.vX, dmY);
       pt.mark("centre / scale");
       FitOptions opt;
       opt.scaling = scaling;
@@ -959,62 +993,32 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
       opt.svds_tol = std::max(svds_tol, 0.0);
       opt.seed = static_cast<unsigned int>(seed);
       opt.xprod = xprod != 0;
-      PlssvdOut o;
       o.C_latent = ctx.arena.alloc_n<double>((size_t)K0 * K0 * L);
       o.W_latent = ctx.arena.alloc_n<double>((size_t)K0 * m * L);
-      o.R = dR = ctx.arena.alloc_n<double>((size_t)p * K0);
+      o.R = fd.R = ctx.arena.alloc_n<double>((size_t)p * K0);
       o.Q = ctx.arena.alloc_n<double>((size_t)m * K0);
       o.T = dT = ctx.arena.alloc_n<double>((size_t)n * K0);
       o.s = ctx.arena.alloc_n<double>(K0);
       o.B = B ? ctx.arena.alloc_n<double>((size_t)p * m * L) : nullptr;
       o.Yfit = fit ? ctx.arena.alloc_n<double>((size_t)n * m * L) : nullptr;
-      std::vector<double> r2(L, 0.0);
       o.R2Y = r2.data();
       plssvd_fit_centered(dX, n, p, dY, m, nc.data(), L, K0, opt, dmY, o);
       pt.mark("PLSSVD fit");
-      download(Q, o.Q, (size_t)m * K0);
-      download(mY, dmY, m);
-      if (B) download(B, o.B, (size_t)p * m * L);
-      if (fit) download(Yfit, o.Yfit, (size_t)n * m * L);
-      hR.resize((size_t)p * K0);
-      download(hR.data(), dR, (size_t)p * K0);
-      download(hmX.data(), dmX, p);
-      download(hvX.data(), dvX, p);
-      ctx.sync();
-      pt.mark("fit outputs to host");
-      if (R2Y) std::copy(r2.begin(), r2.end(), R2Y);
     } else {
       K0 = max_of(nc.data(), L);
-      hR.resize((size_t)p * K0);
-      std::vector<double> hQ((size_t)m * K0), hmY(m);
       int done = 0;
       // centres / scales dX in place (the fit's own copy) and fits on it
-      simpls_fast_on_device(sX, dX, n, p, sY, dY, m, nc.data(), L, scaling, fit, seed, hR.data(), hQ.data(), hmX.data(),
-                            hvX.data(), hmY.data(), B, Yfit, R2Y, &done);
+      simpls_fast_on_device(sX, dX, n, p, sY, dY, m, nc.data(), L, scaling, fit, seed, nullptr, Q, nullptr, nullptr,
+                            mY, B, Yfit, R2Y, &done, &fd);
       if (done < K0) throw Error(FPLS_ERR_NUMERICAL, "pls_lda has invalid effective component count");
-      if (Q) std::copy(hQ.begin(), hQ.end(), Q);
-      if (mY) std::copy(hmY.begin(), hmY.end(), mY);
-      dR = upload(hR.data(), (size_t)p * K0);
       dT = ctx.arena.alloc_n<double>((size_t)n * K0);
-      xgemm(false, n, K0, p, dX, n, dR, p, dT, n);
+      xgemm(false, n, K0, p, dX, n, fd.R, p, dT, n);
     }
-    if (R) std::copy(hR.begin(), hR.end(), R);
-    if (mX) std::copy(hmX.begin(), hmX.end(), mX);
-    if (vX) std::copy(hvX.begin(), hvX.end(), vX);
+    double* dRp = ctx.arena.alloc_n<double>((size_t)p * K0);
+    double* doff = ctx.arena.alloc_n<double>(K0);
+    prediction_weights_kernel<<<K0, 1024, 0, ctx.stream>>>(fd.R, p, fd.mX, fd.vX, dRp, doff); ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
     if (ncomp_out) std::copy(nc.begin(), nc.end(), ncomp_out);
-    // R_predict = R / vX (rows; a zero or non-finite scale counts as 1) and
-    // offset = mX R_predict (fastPLS.cpp:6321-6335)
-    std::vector<double> hRp((size_t)p * K0), hoff(K0, 0.0);
-    for (int a = 0; a < K0; ++a)
-      for (int j = 0; j < p; ++j) {
-        double sc = hvX[j];
-        if (!std::isfinite(sc) || sc == 0.0) sc = 1.0;
-        const double v = hR[j + (size_t)a * p] / sc;
-        hRp[j + (size_t)a * p] = v;
-        hoff[a] += hmX[j] * v;
-      }
-    if (R_predict) std::copy(hRp.begin(), hRp.end(), R_predict);
-    if (R_offset) std::copy(hoff.begin(), hoff.end(), R_offset);
     // LDA on the fit's training scores, one model per distinct ncomp in
     // increasing order (arma::unique)
     std::vector<int> uq(nc);
@@ -1028,18 +1032,15 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
     d.priors = ctx.arena.alloc_n<double>(n_classes);
     std::vector<double> lam(U);
     d.lambda = lam.data();
-    pt.mark("prediction weights (host)");
+    pt.mark("prediction weights");
     lda_train_prefix(dT, n, K0, y, n_classes, uq.data(), U, lda_ridge, d);
     pt.mark("LDA train");
-    lda_outputs_to_host(d, n_classes, K0, U, lda_means, lda_linear, lda_constants, lda_priors);
-    pt.mark("LDA outputs to host");
+    int* dpred = nullptr;
     if (ntest > 0) {
       xt_up.wait();
       const double* dXt = f32 ? widen_on_device(static_cast<const float*>(xt_up.dst), ntest, p)
                               : static_cast<const double*>(xt_up.dst);
-      const double* dRp = upload(hRp.data(), (size_t)p * K0);
-      const double* doff = upload(hoff.data(), K0);
-      int* dpred = ctx.arena.alloc_n<int>((size_t)ntest * L);
+      dpred = ctx.arena.alloc_n<int>((size_t)ntest * L);
       double* dc = ctx.arena.alloc_n<double>(n_classes);
       for (int i = 0; i < L; ++i) {
         const int u = static_cast<int>(std::lower_bound(uq.begin(), uq.end(), nc[i]) - uq.begin());
@@ -1047,11 +1048,26 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
         lda_project_scores_device(dXt, ntest, p, dRp, p, nc[i], doff, d.linear + (size_t)u * n_classes * K0,
                                   n_classes, dc, n_classes, dpred + (size_t)i * ntest, nullptr);
       }
-      download(pred_codes, dpred, (size_t)ntest * L);
       pt.mark("test prediction");
     }
+    // the results leave once every kernel is queued
+    lda_outputs_to_host(d, n_classes, K0, U, lda_means, lda_linear, lda_constants, lda_priors);
+    if (R) download(R, fd.R, (size_t)p * K0);
+    if (mX) download(mX, fd.mX, p);
+    if (vX) download(vX, fd.vX, p);
+    if (R_predict) download(R_predict, dRp, (size_t)p * K0);
+    if (R_offset) download(R_offset, doff, K0);
+    if (method == 1) {
+      if (Q) download(Q, o.Q, (size_t)m * K0);
+      if (mY) download(mY, dmY, m);
+      if (B) download(B, o.B, (size_t)p * m * L);
+      if (fit) download(Yfit, o.Yfit, (size_t)n * m * L);
+    }
+    if (ntest > 0) download(pred_codes, dpred, (size_t)ntest * L);
     ctx.sync();
+    pt.mark("outputs to host");
     pt.report();
+    if (method == 1 && R2Y) std::copy(r2.begin(), r2.end(), R2Y);
     if (lda_lambda) std::copy(lam.begin(), lam.end(), lda_lambda);
     if (n_unique) *n_unique = U;
     if (unique_ncomp) std::copy(uq.begin(), uq.end(), unique_ncomp);
