@@ -222,6 +222,11 @@ def _out(*shape):
     return np.zeros(shape, dtype=np.float64, order="F")
 
 
+def _filled(*shape):
+    """An output that a successful call fills whole: clearing it first would write it twice."""
+    return np.empty(shape, dtype=np.float64, order="F")
+
+
 def _call(name, *args):
     err = ctypes.create_string_buffer(1024)
     rc = getattr(load(), name)(*args, err, ctypes.sizeof(err))
@@ -348,8 +353,8 @@ def pls_model2_fast(X, Y, ncomp, scaling=1, fit=False, seed=1, store_B=True, xpr
     nc = _i32(np.maximum(np.atleast_1d(ncomp), 1))
     L = nc.size
     K = int(nc.max())
-    out = dict(R=_out(p, K), Q=_out(m, K), mX=_out(1, p), vX=_out(1, p), mY=_out(1, m),
-               B=_out(p, m, L) if store_B else None, Yfit=_out(n, m, L) if fit else None,
+    out = dict(R=_filled(p, K), Q=_filled(m, K), mX=_filled(1, p), vX=_filled(1, p), mY=_filled(1, m),
+               B=_filled(p, m, L) if store_B else None, Yfit=_filled(n, m, L) if fit else None,
                R2Y=np.zeros(L))
     ncmp = ctypes.c_int(0)
     errors = []
@@ -431,8 +436,8 @@ def predict_lowrank(model, Xtest, proj=False):
     m = int(model["m"])
     nc = _i32(np.minimum(np.atleast_1d(model["ncomp"]), kmax))
     L = nc.size
-    Yp = _out(w, m, L)
-    T = _out(w, kmax) if proj else None
+    Yp = _filled(w, m, L)
+    T = _filled(w, kmax) if proj else None
     _call("fpls_predict_lowrank", _p(Xt), w, p, _p(_f64(model["mX"]).ravel()),
           _p(_f64(model["vX"]).ravel()), _p(_f64(model["mY"]).ravel()), m, _p(R), kmax, _p(W),
           _p(nc), L, _p(Yp), _p(T))
@@ -452,7 +457,7 @@ def predict_classes(model, Xtest, class_bias=None, top_k=1, return_scores=False)
     nc = _i32(np.minimum(np.atleast_1d(model["ncomp"]), kmax))
     L = nc.size
     idx = np.zeros((w, top_k, L), dtype=np.int32, order="F")
-    sc = _out(w, top_k, L) if return_scores else None
+    sc = _filled(w, top_k, L) if return_scores else None
     bias = None if class_bias is None else np.ascontiguousarray(class_bias, dtype=np.float64)
     _call("fpls_predict_classes", _p(Xt), w, p, _p(_f64(model["mX"]).ravel()),
           _p(_f64(model["vX"]).ravel()), _p(_f64(model["mY"]).ravel()), m, _p(R), kmax, _p(W),
@@ -748,11 +753,11 @@ def pls_lda(Xtrain, Ytrain, y, Xtest, ncomp, n_classes, method=1, scaling=1, xpr
     C = int(n_classes)
     K0 = int(nc.max()) if method == 3 else min(int(nc.max()), min(n, p, m))
     ntest = Xt.shape[0]
-    o = dict(ncomp=np.zeros(L, dtype=np.int32), R=_out(p, K0), Q=_out(m, K0), mX=_out(1, p), vX=_out(1, p),
-             mY=_out(1, m), B=_out(p, m, L) if store_B else None, Yfit=_out(n, m, L) if fit else None,
+    o = dict(ncomp=np.zeros(L, dtype=np.int32), R=_filled(p, K0), Q=_filled(m, K0), mX=_filled(1, p), vX=_filled(1, p),
+             mY=_filled(1, m), B=_filled(p, m, L) if store_B else None, Yfit=_filled(n, m, L) if fit else None,
              R2Y=np.zeros(L), unique_ncomp=np.zeros(L, dtype=np.int32), lda_means=_out(C, K0, L),
              lda_linear=_out(C, K0, L), lda_constants=_out(C, L), lda_priors=np.zeros(C), lda_lambda=np.zeros(L),
-             R_predict=_out(p, K0), R_offset=np.zeros(K0),
+             R_predict=_filled(p, K0), R_offset=np.zeros(K0),
              pred_codes=np.zeros((max(ntest, 1), L), dtype=np.int32, order="F"))
     U = ctypes.c_int(0)
     xa_ptr = Xa.ptr if isinstance(Xa, DeviceMatrix) else Xa.ctypes.data
@@ -908,7 +913,7 @@ def gaussian_y_encode(Y, projection):
     G = _f64(projection)
     n, q = Y.shape
     d = G.shape[1]
-    Z, mu, dec = _out(n, d), np.zeros(q), _out(d, q)
+    Z, mu, dec = _filled(n, d), np.zeros(q), _filled(d, q)
     _call("fpls_gaussian_y_encode", _p(Y), n, q, _p(G), d, _p(Z), _p(mu), _p(dec))
     return dict(Z=Z, y_center=mu, decoder=dec)
 
@@ -919,7 +924,7 @@ def gaussian_y_decode(Z, decoder, y_center, out=None):
     mu = np.ascontiguousarray(y_center, dtype=np.float64).ravel()
     w, d = Z.shape
     q = D.shape[1]
-    Y = _out(w, q) if out is None else _f64(out)
+    Y = _filled(w, q) if out is None else _f64(out)
     _call("fpls_gaussian_y_decode", _p(Z), w, d, _p(D), _p(mu), q, _p(Y))
     return Y
 
@@ -938,7 +943,7 @@ def opls_filter(X, Y, north, scaling=1, out=None):
     Y = _f64(Y)
     n, p = X.shape
     q = Y.shape[1]
-    Xf = _out(n, p) if out is None else _f64(out)
+    Xf = _filled(n, p) if out is None else _f64(out)
     mX, vX = np.zeros(p), np.zeros(p)
     W, P = _out(p, max(north, 1)), _out(p, max(north, 1))
     used = ctypes.c_int(0)
@@ -953,7 +958,7 @@ def opls_apply_filter(X, mX, vX, W_orth, P_orth, out=None):
     w, p = X.shape
     W = _f64(W_orth)
     P = _f64(P_orth)
-    out = _out(w, p) if out is None else _f64(out)
+    out = _filled(w, p) if out is None else _f64(out)
     _call("fpls_opls_apply_filter", _p(X), w, p, _p(np.ascontiguousarray(mX, dtype=np.float64).ravel()),
           _p(np.ascontiguousarray(vX, dtype=np.float64).ravel()), _p(W), _p(P), W.shape[1], _p(out))
     return out
