@@ -26,7 +26,6 @@ constexpr int kAhead = 16;    // loads of one thread that go out before they are
 
 struct Eng {
   int n, p, m, F, K, cp, cn, szp, szn;
-  int lds;         // leading dimension of S and V: p, or a chunk's own copy
   const double* Yg;
   const int* labels;
   const double* mY_all;
@@ -182,14 +181,14 @@ __device__ __forceinline__ void chunk_StY(const Eng& e, int f, int chunk, const 
     if (threadIdx.x == 0) e.npart[(size_t)f * e.cp + chunk] = s2;
     return;
   }
-  chunk_dots(Sf + b, e.lds, e.m, ys, en - b, zout + ((size_t)f * e.cp + chunk) * e.m, 1);
+  chunk_dots(Sf + b, e.p, e.m, ys, en - b, zout + ((size_t)f * e.cp + chunk) * e.m, 1);
 }
 
 // First component's refresh start: y = Omega (or the single column of S).
 __device__ __forceinline__ void refresh_start_chunk(const Eng& e, int f, int chunk, double* ys) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
-  const double* Sf = e.S + (size_t)f * e.lds * e.m;
+  const double* Sf = e.S + (size_t)f * e.p * e.m;
   const double* y0 = e.m1_mode ? Sf : e.omega + (size_t)f * e.p;
   double* yf = e.y + (size_t)f * e.p;
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
@@ -210,14 +209,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_refresh_start(Eng e) {
 __device__ __forceinline__ void refresh_apply_chunk(const Eng& e, const double* zin, double* zout, int last, int f, int chunk, double* zs, double* ys) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
-  const double* Sf = e.S + (size_t)f * e.lds * e.m;
+  const double* Sf = e.S + (size_t)f * e.p * e.m;
   double* yf = e.y + (size_t)f * e.p;
   // the first columns of this thread's row are on their way while z is summed
   double v[kAhead];
   {
     const int i = b + threadIdx.x;
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) v[u] = i < en && u < e.m ? Sf[i + (size_t)u * e.lds] : 0.0;
+    for (int u = 0; u < kAhead; ++u) v[u] = i < en && u < e.m ? Sf[i + (size_t)u * e.p] : 0.0;
   }
   for (int j = threadIdx.x; j < e.m; j += blockDim.x)
     zs[j] = sum_parts(zin + (size_t)f * e.cp * e.m + j, e.cp, e.m);
@@ -227,7 +226,7 @@ __device__ __forceinline__ void refresh_apply_chunk(const Eng& e, const double* 
     for (int j0 = 0; j0 < e.m; j0 += kAhead) {
       if (j0 > 0 || i >= b + (int)blockDim.x) {
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) v[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.lds] : 0.0;
+        for (int u = 0; u < kAhead; ++u) v[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.p] : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < kAhead; ++u)
@@ -374,7 +373,7 @@ __device__ __forceinline__ void loading_chunk(const Eng& e, int a, int f, int ch
   }
   __syncthreads();
   if (a > 0)
-    chunk_dots(e.V + (size_t)f * e.lds * e.K + b, e.lds, a, ps, en - b,
+    chunk_dots(e.V + (size_t)f * e.p * e.K + b, e.p, a, ps, en - b,
                e.wpart + ((size_t)f * e.cp + chunk) * e.K, 1);
 }
 
@@ -388,7 +387,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_loading(Eng e, int a) {
 __device__ __forceinline__ void orth_chunk(const Eng& e, int a, int f, int chunk, double* ws, double* vsh, double* scratch) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
-  const double* Vf = e.V + (size_t)f * e.lds * e.K;
+  const double* Vf = e.V + (size_t)f * e.p * e.K;
   const double* pf = e.pv + (size_t)f * e.p;
   double* vf = e.v + (size_t)f * e.p;
   // this thread's row is on its way while w is summed
@@ -397,7 +396,7 @@ __device__ __forceinline__ void orth_chunk(const Eng& e, int a, int f, int chunk
     const int i = b + threadIdx.x;
     if (i < en) x0 = pf[i];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) v[u] = i < en && u < a ? Vf[i + (size_t)u * e.lds] : 0.0;
+    for (int u = 0; u < kAhead; ++u) v[u] = i < en && u < a ? Vf[i + (size_t)u * e.p] : 0.0;
   }
   for (int l = threadIdx.x; l < a; l += blockDim.x)
     ws[l] = sum_parts(e.wpart + (size_t)f * e.cp * e.K + l, e.cp, e.K);
@@ -408,7 +407,7 @@ __device__ __forceinline__ void orth_chunk(const Eng& e, int a, int f, int chunk
     for (int l0 = 0; l0 < a; l0 += kAhead) {
       if (l0 > 0 || !first) {
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) v[u] = l0 + u < a ? Vf[i + (size_t)(l0 + u) * e.lds] : 0.0;
+        for (int u = 0; u < kAhead; ++u) v[u] = l0 + u < a ? Vf[i + (size_t)(l0 + u) * e.p] : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < kAhead; u += 4) {
@@ -430,7 +429,7 @@ __device__ __forceinline__ void orth_chunk(const Eng& e, int a, int f, int chunk
   const double s2 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + vsh[r] * vsh[r]; });
   if (threadIdx.x == 0) e.vpart[(size_t)f * e.cp + chunk] = s2;
   // S^T v (unnormalised) for the deflation.
-  chunk_dots(e.S + (size_t)f * e.lds * e.m + b, e.lds, e.m, vsh, en - b,
+  chunk_dots(e.S + (size_t)f * e.p * e.m + b, e.p, e.m, vsh, en - b,
              e.vSpart + ((size_t)f * e.cp + chunk) * e.m, 1);
 }
 
@@ -448,9 +447,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_orth(Eng e, int a) {
 __device__ __forceinline__ void deflate_chunk(const Eng& e, int a, int next, int f, int chunk, double* vs, double* ysh) {
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
-  double* Sf = e.S + (size_t)f * e.lds * e.m;
+  double* Sf = e.S + (size_t)f * e.p * e.m;
   double* vf = e.v + (size_t)f * e.p;
-  double* Vcol = e.V + ((size_t)f * e.K + a) * e.lds;
+  double* Vcol = e.V + ((size_t)f * e.K + a) * e.p;
   double* Rcol = e.R + ((size_t)f * e.K + a) * e.p;
   const double* rf = e.r + (size_t)f * e.p;
   double* yf = e.y + (size_t)f * e.p;
@@ -462,7 +461,7 @@ __device__ __forceinline__ void deflate_chunk(const Eng& e, int a, int next, int
   const double v0 = i0 < en ? vf[i0] : 0.0, r0 = i0 < en ? rf[i0] : 0.0;
   double x[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) x[u] = s0 < en && 8 * group + u < e.m ? Sf[s0 + (size_t)(8 * group + u) * e.lds] : 0.0;
+  for (int u = 0; u < 8; ++u) x[u] = s0 < en && 8 * group + u < e.m ? Sf[s0 + (size_t)(8 * group + u) * e.p] : 0.0;
   for (int j = threadIdx.x; j < e.m; j += blockDim.x) vs[j] = sum_parts(e.vSpart + (size_t)f * e.cp * e.m + j, e.cp, e.m);
   double tn, st;
   t_stats(e, f, tn, st);
@@ -485,11 +484,11 @@ __device__ __forceinline__ void deflate_chunk(const Eng& e, int a, int next, int
     for (int j0 = 8 * group; j0 < e.m; j0 += 8 * groups) {
       if (i > s0 || j0 > 8 * group) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) x[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.lds] : 0.0;
+        for (int u = 0; u < 8; ++u) x[u] = j0 + u < e.m ? Sf[i + (size_t)(j0 + u) * e.p] : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        if (j0 + u < e.m) Sf[i + (size_t)(j0 + u) * e.lds] = x[u] - vi * vs[j0 + u];
+        if (j0 + u < e.m) Sf[i + (size_t)(j0 + u) * e.p] = x[u] - vi * vs[j0 + u];
     }
   }
   __syncthreads();
@@ -530,20 +529,444 @@ __global__ void __launch_bounds__(kMaxThreads) k_deflate(Eng e, int a, int next)
   deflate_chunk(e, a, next, blockIdx.y, blockIdx.x, coef, vec);
 }
 
+// ---- The same bodies on a chunk of S in shared memory ---------------------------
+// The bodies above are bound by what they wait for in L2 and by their address
+// arithmetic.  These take a chunk of at most kTile rows whose S lies in shared
+// memory with that pitch, rows past the chunk zero: every offset is an immediate,
+// no load needs a bound, and each sum keeps the order of the body above it (a
+// zero row adds +0), so the results are the same bit for bit.  Sums of partials
+// that every block needs are loaded by one warp together instead of by every
+// thread in turn.
+constexpr int kTile = 256;
+constexpr int kTileStage = 1280;   // doubles staged at a time
+struct __align__(16) TileShared {   // stage is read as double2 too
+  double x[kTile];       // the phase's vector: p, v, y
+  double pv[kTile], v[kTile];
+  double stage[kTileStage];
+  double red[32];
+  double tn, st, nrm;
+};
+
+// s[0] + s[step] + ... (n of them) in order.
+__device__ __forceinline__ double in_order(const double* s, int n, int step) {
+  double t = 0.0;
+  int i = 0;
+  for (; i + 8 <= n; i += 8)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) t += s[(i + u) * step];
+  for (; i < n; ++i) t += s[i * step];
+  return t;
+}
+
+// One warp: the sum of `count` values in order, in every lane.
+__device__ __forceinline__ double warp_parts(const double* parts, int count, double* stage) {
+  const int lane = threadIdx.x & 31;
+  double t = 0.0;
+  for (int c0 = 0; c0 < count; c0 += 512) {
+    const int n = min(512, count - c0);
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = lane + 32 * u < n ? parts[c0 + lane + 32 * u] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (lane + 32 * u < n) stage[lane + 32 * u] = v[u];
+    __syncwarp();
+    for (int i = 0; i < n; ++i) t += stage[i];
+    __syncwarp();
+  }
+  return t;
+}
+
+// out[j] = parts[j] + parts[j + stride] + ... (`count` of them, in order) for
+// j < ncols: groups of threads take kAhead partials of every column each, so that
+// all loads are in flight at once, and add them in turn.  Ends with a barrier.
+template <int NT>
+__device__ __forceinline__ void column_sums(double* out, const double* parts, int ncols, int count, int stride) {
+  int shift = 5;
+  while ((1 << shift) < ncols && (1 << shift) < NT) ++shift;
+  const int width = 1 << shift, groups = NT >> shift, g = threadIdx.x >> shift, j0 = threadIdx.x & (width - 1);
+  for (int j = j0; j - j0 < ncols; j += width) {
+    for (int c0 = 0; c0 < count; c0 += groups * kAhead) {
+      const int c = c0 + g * kAhead;
+      const double* src = parts + j + (size_t)c * stride;
+      double v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        v[u] = j < ncols && c + u < count ? *src : 0.0;
+        src += stride;
+      }
+      const int turns = min(groups, (count - c0 + kAhead - 1) / kAhead);
+      for (int t = 0; t < turns; ++t) {
+        if (t == g && j < ncols) {
+          double s = c > 0 ? out[j] : 0.0;
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u)
+            if (c + u < count) s += v[u];
+          out[j] = s;
+        }
+        __syncthreads();
+      }
+    }
+  }
+}
+
+// out[j] = sum_r M[r + j ld] x[r] in the order of chunk_dots, for j < ncols.  M in
+// shared memory with zero rows (BOUND: in memory, rows read up to `rows` only).
+template <int NT, bool BOUND>
+__device__ __forceinline__ void tile_dots(const double* M, int ld, int ncols, TileShared& sh, int rows, double* out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (ncols >= kSumWarps) {
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = sh.x[lane + 32 * u];
+#pragma unroll 2
+    for (int j = warp; j < ncols; j += NT / 32) {
+      const double* col = M + (size_t)j * ld + lane;
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = !BOUND || lane + 32 * u < rows ? col[32 * u] : 0.0;
+      double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        a0 += v[u] * x[u];
+        a1 += v[u + 1] * x[u + 1];
+      }
+      const double acc = warp_sum(a0 + a1);
+      if (lane == 0) out[j] = acc;
+    }
+    return;
+  }
+  const int g = kSumWarps / max(ncols, 1);   // warps per column
+  const int j = warp / g, sub = warp - j * g;
+  if (warp < kSumWarps && j < ncols) {
+    const double* col = M + (size_t)j * ld;
+    double acc = 0.0;
+    for (int r = sub * 32 + lane; r < kTile; r += 32 * g) {
+      const double v = !BOUND || r < rows ? col[r] : 0.0;
+      acc += v * sh.x[r];
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) sh.red[warp] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x < ncols) {
+    double t = 0.0;
+    for (int u = 0; u < g; ++u) t += sh.red[threadIdx.x * g + u];
+    out[threadIdx.x] = t;
+  }
+  __syncthreads();
+}
+
+// Sum of x[r]^2 in chunk_sum's order, by the first kSumWarps warps; thread 0 stores it.
+__device__ __forceinline__ void tile_norm(TileShared& sh, double* out) {
+  if (threadIdx.x < kTile) {
+    const double x = sh.x[threadIdx.x];
+    const double s = warp_sum(x * x);
+    if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+#pragma unroll
+    for (int i = 0; i < kSumWarps; ++i) t += sh.red[i];
+    *out = t;
+  }
+}
+
+// Where a chunk lies: its rows b .. b + rows of the p, its S and V.
+struct TileView {
+  int b, rows;
+  double* S;          // shared, pitch kTile
+  const double* V;    // row b of V: shared with pitch kTile, or memory with pitch p
+  int ldv;
+};
+
+template <int NT, bool VMEM>
+__device__ __forceinline__ void tile_loading(const Eng& e, const TileView& w, int a, int f, int chunk, TileShared& sh) {
+  const int row = threadIdx.x & (kTile - 1), i = w.b + row;
+  const bool mine = threadIdx.x < kTile && row < w.rows;
+  double P = 0.0;
+  if (threadIdx.x >= NT - 32) {   // the last warp: ||t|| and sum(t)
+    const int lane = threadIdx.x & 31;
+    const double2* tp = reinterpret_cast<const double2*>(e.tpart) + (size_t)f * e.cn;
+    double2* st = reinterpret_cast<double2*>(sh.stage);
+    double s2 = 0.0, s1 = 0.0;
+    for (int c0 = 0; c0 < e.cn; c0 += 256) {
+      const int n = min(256, e.cn - c0);
+      double2 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = lane + 32 * u < n ? tp[c0 + lane + 32 * u] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (lane + 32 * u < n) st[lane + 32 * u] = v[u];
+      __syncwarp();
+#pragma unroll 4
+      for (int c = 0; c < n; ++c) {
+        s2 += st[c].x;
+        s1 += st[c].y;
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {
+      sh.tn = sqrt(s2);
+      sh.st = s1;
+    }
+  }
+  if (mine)
+    P = e.psplits > 1 ? sum_parts(e.ppart + (size_t)f * e.p + i, e.psplits, (size_t)e.p * e.F) : e.P[(size_t)f * e.p + i];
+  __syncthreads();
+  const double tn = sh.tn, st = sh.st;
+  if (!(tn > 0.0) || !isfinite(tn)) {
+    if (chunk == 0 && threadIdx.x == 0) e.status[f] = 1;
+    return;
+  }
+  if (threadIdx.x < kTile) {
+    double v = 0.0;
+    if (mine) {
+      v = P;
+      if (e.delta) v -= e.delta[(size_t)f * e.p + i] * st;
+      if (e.colscale) v *= e.colscale[(size_t)f * e.p + i];
+      v /= tn;
+    }
+    sh.pv[row] = v;
+    sh.x[row] = v;
+  }
+  __syncthreads();
+  if (a > 0) tile_dots<NT, VMEM>(w.V, VMEM ? w.ldv : kTile, a, sh, w.rows, e.wpart + ((size_t)f * e.cp + chunk) * e.K);
+}
+
+template <int NT, bool VMEM>
+__device__ __forceinline__ void tile_orth(const Eng& e, const TileView& w, int a, int f, int chunk, double* ws,
+                                          TileShared& sh) {
+  // Row r is thread r of every group of kTile threads: the groups take the columns
+  // of V four at a time in turn (a quad's sum of products is formed where its
+  // columns arrive) and the first group subtracts the quads' sums in order.
+  constexpr int groups = NT / kTile;
+  const int g = threadIdx.x / kTile, row = threadIdx.x % kTile;
+  const int quads = a / 4;
+  const int ld = VMEM ? w.ldv : kTile;
+  const bool in = !VMEM || row < w.rows;
+  const double* Vr = w.V + row;
+  double x = g == 0 ? sh.pv[row] : 0.0;
+  bool summed = false;
+  for (int q0 = 0; q0 < quads || q0 == 0; q0 += 4 * groups) {
+    double v[4][4];
+    const double* col = Vr + (size_t)(4 * (q0 + g)) * ld;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool have = in && q0 + g + u * groups < quads;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) v[u][c] = have ? col[(size_t)c * ld] : 0.0;
+      col += (size_t)(4 * groups) * ld;
+    }
+    if (!summed) {   // w, while the first columns are on their way
+      if (a > 0) column_sums<NT>(ws, e.wpart + (size_t)f * e.cp * e.K, a, e.cp, e.K);
+      summed = true;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int qu = q0 + u * groups;   // group 0's quad of this turn
+      if (qu >= quads) break;
+      const int q = qu + g, l = 4 * q;
+      double t = 0.0;
+      if (q < quads) t = v[u][0] * ws[l] + v[u][1] * ws[l + 1] + v[u][2] * ws[l + 2] + v[u][3] * ws[l + 3];
+      if (groups == 1) {
+        x -= t;
+      } else {
+        sh.stage[threadIdx.x] = t;
+        __syncthreads();
+        if (g == 0) {
+#pragma unroll
+          for (int h = 0; h < groups; ++h)
+            if (qu + h < quads) x -= sh.stage[h * kTile + row];
+        }
+        __syncthreads();
+      }
+    }
+  }
+  if (g == 0) {
+    for (int l = 4 * quads; l < a; ++l)   // the last one to three columns
+      if (in) x -= Vr[(size_t)l * ld] * ws[l];
+    sh.v[row] = x;
+    sh.x[row] = x;
+  }
+  __syncthreads();
+  tile_norm(sh, e.vpart + (size_t)f * e.cp + chunk);
+  // S^T v (unnormalised) for the deflation
+  tile_dots<NT, false>(w.S, kTile, e.m, sh, w.rows, e.vSpart + ((size_t)f * e.cp + chunk) * e.m);
+}
+
+// Partials of S^T x, or ||x||^2 (x in sh.x).
+template <int NT>
+__device__ __forceinline__ void tile_StY(const Eng& e, const TileView& w, int f, int chunk, TileShared& sh, double* zout,
+                                         bool norm_only) {
+  if (norm_only) tile_norm(sh, e.npart + (size_t)f * e.cp + chunk);
+  else tile_dots<NT, false>(w.S, kTile, e.m, sh, w.rows, zout + ((size_t)f * e.cp + chunk) * e.m);
+}
+
+// Vsh: V in shared memory (null: only memory's); Sg: memory's S, row b (null: not kept).
+template <int NT>
+__device__ __forceinline__ void tile_deflate(const Eng& e, const TileView& w, int a, int next, int f, int chunk, double* vs,
+                                             TileShared& sh, double* Vsh, double* Sg) {
+  constexpr int groups = NT / kTile;
+  const int g = threadIdx.x / kTile, row = threadIdx.x % kTile, i = w.b + row;
+  const bool in = row < w.rows;
+  const double r0 = g == 0 && in ? e.r[(size_t)f * e.p + i] : 0.0;
+  column_sums<NT>(vs, e.vSpart + (size_t)f * e.cp * e.m, e.m, e.cp, e.m);
+  if (threadIdx.x >= NT - 32) {
+    const double s = warp_parts(e.vpart + (size_t)f * e.cp, e.cp, sh.stage);
+    if ((threadIdx.x & 31) == 0) sh.nrm = sqrt(s);
+  }
+  __syncthreads();
+  const double vn = sh.nrm, tn = sh.tn, st = sh.st;
+  if (!(vn > 0.0) || !isfinite(vn)) {
+    if (chunk == 0 && threadIdx.x == 0) e.status[f] = 1;
+    return;
+  }
+  for (int j = threadIdx.x; j < e.m; j += NT) vs[j] /= vn;
+  if (g == 0) {
+    const double vi = sh.v[row] / vn;   // 0 past the chunk
+    sh.v[row] = vi;
+    if (Vsh) Vsh[a * kTile + row] = vi;
+    else if (in) e.V[((size_t)f * e.K + a) * e.p + i] = vi;
+  }
+  __syncthreads();
+  {   // the rank-1 update, elementwise
+    const double vi = sh.v[row];
+    double* col = w.S + row + g * kTile;
+    if (Sg) {
+      double* mem = Sg + row + (size_t)g * e.p;
+#pragma unroll 4
+      for (int j = g; j < e.m; j += groups) {
+        const double s = *col - vi * vs[j];
+        *col = s;
+        if (in) *mem = s;
+        col += groups * kTile;
+        mem += (size_t)groups * e.p;
+      }
+    } else {
+#pragma unroll 4
+      for (int j = g; j < e.m; j += groups) {
+        *col = *col - vi * vs[j];
+        col += groups * kTile;
+      }
+    }
+  }
+  __syncthreads();
+  if (g == 0) {
+    const double ri = r0 / tn;
+    if (in) e.R[((size_t)f * e.K + a) * e.p + i] = ri;
+    if (next) {
+      const double y0 = e.m1_mode ? w.S[row] : ri;
+      if (in) e.y[(size_t)f * e.p + i] = y0;
+      sh.x[row] = in ? y0 : 0.0;
+    }
+  }
+  // q: chunk c takes responses c, c + cp, ..., a thread a partial
+  {
+    double* Qcol = e.Q + ((size_t)f * e.K + a) * e.m;
+    const int cols = e.m > chunk ? (e.m - chunk + e.cp - 1) / e.cp : 0;   // of this chunk
+    const int fit = e.cn <= kTileStage ? kTileStage / e.cn : 0;           // columns staged at a time
+    for (int c0 = 0; c0 < cols; c0 += max(fit, 1)) {
+      const int nc = min(max(fit, 1), cols - c0);
+      for (int t = threadIdx.x; fit > 0 && t < nc * e.cn; t += NT) {
+        const int c = t / e.cn;
+        sh.stage[t] = e.qpart[((size_t)f * e.cn + (t - c * e.cn)) * e.m + chunk + (c0 + c) * e.cp];
+      }
+      __syncthreads();
+      for (int c = threadIdx.x; c < nc; c += NT) {
+        const int j = chunk + (c0 + c) * e.cp;
+        double q = fit > 0 ? in_order(sh.stage + c * e.cn, e.cn, 1)
+                           : sum_parts(e.qpart + (size_t)f * e.cn * e.m + j, e.cn, e.m);
+        double off = 0.0;
+        if (e.labels) off += e.mY_all[j];
+        if (e.dY) off += e.dY[(size_t)f * e.m + j];
+        q -= off * st;
+        Qcol[j] = q / tn;
+      }
+      __syncthreads();
+    }
+    if (chunk == 0 && threadIdx.x == 0) {
+      e.tnorm[(size_t)f * e.K + a] = tn;
+      e.ncomp_done[f] = a + 1;
+    }
+  }
+  if (next) {
+    __syncthreads();
+    tile_StY<NT>(e, w, f, chunk, sh, e.zA, e.iters == 0);
+  }
+}
+
+template <int NT>
+__device__ __forceinline__ void tile_start(const Eng& e, const TileView& w, int f, int chunk, TileShared& sh) {
+  if (threadIdx.x < kTile) {
+    const int row = threadIdx.x, i = w.b + row;
+    double y = 0.0;
+    if (row < w.rows) {
+      y = e.m1_mode ? w.S[row] : e.omega[(size_t)f * e.p + i];
+      e.y[(size_t)f * e.p + i] = y;
+    }
+    sh.x[row] = y;
+  }
+  __syncthreads();
+  tile_StY<NT>(e, w, f, chunk, sh, e.zA, e.iters == 0);
+}
+
+template <int NT>
+__device__ __forceinline__ void tile_apply(const Eng& e, const TileView& w, const double* zin, double* zout, int last, int f,
+                                           int chunk, double* zs, TileShared& sh) {
+  column_sums<NT>(zs, zin + (size_t)f * e.cp * e.m, e.m, e.cp, e.m);
+  if (threadIdx.x < kTile) {
+    const int row = threadIdx.x;
+    const double* s = w.S + row;
+    double acc = 0.0;
+    int j = 0;
+    for (; j + 8 <= e.m; j += 8, s += 8 * kTile)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += s[u * kTile] * zs[j + u];
+    for (; j < e.m; ++j, s += kTile) acc += *s * zs[j];
+    if (row < w.rows) e.y[(size_t)f * e.p + w.b + row] = acc;
+    sh.x[row] = acc;   // 0 past the chunk
+  }
+  __syncthreads();
+  tile_StY<NT>(e, w, f, chunk, sh, zout, last != 0);
+}
+
+// The chunk's S into shared memory, asynchronously, rows past the chunk zero;
+// tile_here() before it is read.
+template <int NT>
+__device__ __forceinline__ void tile_load(double* S, const double* src, size_t ld, int m, int rows) {
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(S));
+  const int row = threadIdx.x % kTile;
+  for (int j = threadIdx.x / kTile; j < m; j += NT / kTile) {
+    if (row < rows)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * static_cast<uint32_t>(j * kTile + row)),
+                   "l"(src + row + (size_t)j * ld)
+                   : "memory");
+    else S[j * kTile + row] = 0.0;
+  }
+}
+
+__device__ __forceinline__ void tile_here() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+}
+
 // ---- The component loop of one small fit in one launch -----------------------
 // A fit of a few hundred samples spends its time between kernels: eleven launches
 // a component, 5.2 us each inside a graph, for phases that move a few hundred
-// kilobytes of L2.  Here the phases are the same chunk bodies (sums in the same
+// kilobytes of L2.  Here the phases are the bodies above (sums in the same
 // order: the results are those of the launches bit for bit) with a grid barrier
 // between them, eight a component: the split sums of X r and the normalisation of
-// r are folded into the phases that read them, and a block keeps its chunk of S,
-// V and the p-vectors in shared memory.  400 x 2000, 5 responses: 57 us a component
-// as a graph of launches, 40 us now (1.2 us a barrier, about 3.5 us a phase).
+// r are folded into the phases that read them, and a block keeps its chunk of S
+// and V in shared memory.  400 x 2000, 5 responses: 57 us a component as a graph
+// of launches, 36 us now (1.2 us a barrier, about 3 us a phase).
 struct LoopArgs {
   Eng e;
   const double* X;    // n x p
   GemvRanges xr;      // ranges of X r
-  int coef_len;       // doubles of dynamic shared memory before the X tile
+  int coef_len;       // doubles of dynamic shared memory before the vector
+  int vec_len;        // and of the vector
   unsigned* barrier;  // zero at the start
   unsigned* stop;     // barrier after which a stopped fit leaves (all ones: none)
   int* fail;          // a barrier wait gave up
@@ -554,26 +977,26 @@ struct LoopArgs {
 // slots spent on predicated-off loads (1024 threads: 48 us a component).
 constexpr int kLoopThreads = 256;
 constexpr int kLoopWarps = kLoopThreads / 32;
-constexpr size_t kLoopSmem = 190 * 1024;             // beside the static arrays
+constexpr size_t kLoopSmem = 208 * 1024;             // beside the static arrays
 constexpr long long kBarrierClocks = 4000000000ll;   // about two seconds
 
-// Every CTA of the (cooperative) grid has arrived `count` times; false when a
-// wait ran out, in every thread of every CTA sooner or later.
-__device__ bool grid_barrier(const LoopArgs& g, unsigned count) {
+// `count` CTAs in all have arrived at *counter (CTAs of one cooperative launch);
+// false when a wait ran out, in every thread of every CTA sooner or later.
+__device__ bool counted_barrier(unsigned* counter, unsigned count, int* fail, int* host_fail) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(g.barrier, 1u);
+    atomicAdd(counter, 1u);
     const long long t0 = clock64();
     ok = 1;
     while (true) {
       unsigned seen;
-      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(g.barrier) : "memory");
-      if (seen >= count * gridDim.x) break;
-      if (*(volatile int*)g.fail || clock64() - t0 > kBarrierClocks) {
-        atomicExch(g.fail, 1);
-        *(volatile int*)g.host_fail = 1;
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+      if (seen >= count) break;
+      if (*(volatile int*)fail || clock64() - t0 > kBarrierClocks) {
+        atomicExch(fail, 1);
+        *(volatile int*)host_fail = 1;
         ok = 0;
         break;
       }
@@ -585,30 +1008,26 @@ __device__ bool grid_barrier(const LoopArgs& g, unsigned count) {
 }
 
 __global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
-  extern __shared__ double coef[];   // max(m, K)
-  __shared__ double vec[kMaxChunk];
+  extern __shared__ double coef[];   // max(m, K), a score chunk's vector, the X tile, S, V
   __shared__ double scratch[32];
+  __shared__ TileShared sh;
+  double* vec = coef + g.coef_len;
   const Eng& e = g.e;
   unsigned arrived = 0;
-  // The block's own chunk of S, V and the p-vectors stays in shared memory for the
-  // whole loop (a chunk a block): what a phase waits for in L2 is other blocks'
-  // partials only.
-  double* tile = coef + g.coef_len;            // [256][32]
-  double* own = tile + 256 * 32;
-  Eng l = e;
-  int b = 0, en = 0;
-  if (blockIdx.x < e.cp) chunk_range(blockIdx.x, e.szp, e.p, b, en);
-  l.lds = e.szp;
-  l.S = own - b;
-  l.V = own + (size_t)e.szp * e.m - b;
-  double* vecs = own + (size_t)e.szp * (e.m + e.K);
-  l.y = vecs - b;
-  l.r = vecs + e.szp - b;
-  l.pv = vecs + 2 * e.szp - b;
-  l.v = vecs + 3 * e.szp - b;
-  for (int j = threadIdx.x >> 5; j < e.m; j += kLoopThreads / 32)
-    for (int i = b + (threadIdx.x & 31); i < en; i += 32) l.S[i + (size_t)j * l.lds] = e.S[i + (size_t)j * e.p];
-  __syncthreads();
+  // The block's own chunk of S and V (a chunk a block) stays in shared memory for
+  // the whole loop: what a phase waits for in L2 is other blocks' partials only.
+  double* tile = vec + g.vec_len;              // [256][32]
+  TileView w{0, 0, tile + 256 * 32, nullptr, kTile};
+  double* Vsh = w.S + (size_t)e.m * kTile;
+  w.V = Vsh;
+  const int own = blockIdx.x;
+  if (own < e.cp) {
+    int en;
+    chunk_range(own, e.szp, e.p, w.b, en);
+    w.rows = en - w.b;
+    tile_load<kLoopThreads>(w.S, e.S + w.b, e.p, e.m, w.rows);
+    tile_here();
+  }
   // A phase over `count` chunks; false: leave (a wait gave up, or the fit stopped).
   // Block 0 has chunk 0, which raises the status: it names the barrier that ends
   // this phase, so that a block still on its way from the one before does not
@@ -620,24 +1039,15 @@ __global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
     }
     ++arrived;
     if (blockIdx.x == 0 && threadIdx.x == 0 && e.status[0] != 0) *(volatile unsigned*)g.stop = arrived;
-    if (!grid_barrier(g, arrived)) return false;
+    if (!counted_barrier(g.barrier, arrived * gridDim.x, g.fail, g.host_fail)) return false;
     return *(volatile unsigned*)g.stop > arrived;
   };
-  if (!phase(e.cp, [&](int c) { refresh_start_chunk(l, 0, c, vec);
-                             if (e.iters == 0)
-                               for (int i = b + threadIdx.x; i < en; i += blockDim.x) e.y[i] = l.y[i];
-                           }))
-    return;
+  if (!phase(e.cp, [&](int c) { tile_start<kLoopThreads>(e, w, 0, c, sh); })) return;
   for (int a = 0; a < e.K; ++a) {
     double *zin = e.zA, *zout = e.zB;
     for (int it = 0; it < e.iters; ++it) {
       const int last = it == e.iters - 1 ? 1 : 0;
-      if (!phase(e.cp, [&](int c) {
-            refresh_apply_chunk(l, zin, zout, last, 0, c, coef, vec);
-            if (last)   // every block reads it for X r
-              for (int i = b + threadIdx.x; i < en; i += blockDim.x) e.y[i] = l.y[i];
-          }))
-        return;
+      if (!phase(e.cp, [&](int c) { tile_apply<kLoopThreads>(e, w, zin, zout, last, 0, c, coef, sh); })) return;
       double* t = zin;
       zin = zout;
       zout = t;
@@ -653,7 +1063,7 @@ __global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
         const double sgn = (e.y[0] >= 0.0) ? -1.0 : 1.0;
         const int row_groups = (e.n + 31) / 32, items = row_groups * g.xr.splits;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (int i = b + threadIdx.x; i < en; i += blockDim.x) l.r[i] = sgn * l.y[i] / nrm;
+        for (int i = w.b + threadIdx.x; i < w.b + w.rows; i += blockDim.x) e.r[i] = sgn * e.y[i] / nrm;
         for (int item = blockIdx.x; item < items; item += gridDim.x) {
           const int rg = item % row_groups, z = item / row_groups, row = 32 * rg + lane;
           const int kbeg = z * g.xr.kps, kend = min(e.p, kbeg + g.xr.kps);
@@ -693,15 +1103,170 @@ __global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
       if ((threadIdx.x & 31) == 0) e.P[j] = acc;
     }
     if (!phase(0, [](int) {})) return;
-    if (!phase(e.cp, [&](int c) { loading_chunk(l, a, 0, c, vec); })) return;
-    if (!phase(e.cp, [&](int c) { orth_chunk(l, a, 0, c, coef, vec, scratch); })) return;
-    if (!phase(e.cp, [&](int c) {
-          deflate_chunk(l, a, a + 1 < e.K ? 1 : 0, 0, c, coef, vec);
-          if (e.iters == 0)
-            for (int i = b + threadIdx.x; i < en; i += blockDim.x) e.y[i] = l.y[i];
-        }))
+    if (!phase(e.cp, [&](int c) { tile_loading<kLoopThreads, false>(e, w, a, 0, c, sh); })) return;
+    if (!phase(e.cp, [&](int c) { tile_orth<kLoopThreads, false>(e, w, a, 0, c, coef, sh); })) return;
+    if (!phase(e.cp, [&](int c) { tile_deflate<kLoopThreads>(e, w, a, a + 1 < e.K ? 1 : 0, 0, c, coef, sh, Vsh, nullptr); }))
       return;
   }
+}
+
+// ---- From X^T t to the next r in one launch ------------------------------------
+// A larger fit, or a batch of fits, runs its two products as kernels of their
+// own; the phases between them (loading, orthogonalisation, deflation, the next
+// component's refresh) work on chunks of S that fit shared memory.  One launch
+// takes all of them: block (chunk, fit) loads its chunk of S once, the phases are
+// the chunk bodies above (sums in the same order: the results are those of the
+// separate launches bit for bit), and S is written back as it is deflated.  The
+// chunks of one fit meet between the phases: up to eight of them are a thread
+// block cluster and meet at its barrier, whatever the number of fits; more of them
+// need all blocks resident (a cooperative launch) and count arrivals in memory.
+// Bound by the latency of the phases' chains of sums and, at a few microseconds a
+// phase, by the instructions of a warp (a first form that called the bodies on
+// memory's layout executed four times as many and took as long as the launches).
+// A component's phases: 30 fits of 501 x 5, 2 chunks each: 50 -> 33 us; 8000 x
+// 100, 32 chunks: 105 -> 54 us; 1000 x 50, 4 chunks: 114 -> 57 us.
+constexpr int kClusterChunks = 8;
+constexpr size_t kUpdateSmem = 208 * 1024;   // dynamic, beside the static arrays
+struct UpdateArgs {
+  int coef_len;       // doubles before the chunk of S
+  unsigned arrived;   // barriers of the earlier launches of this fit
+  unsigned* counter;  // arrivals, 32 apart by fit
+  unsigned* stop;     // barrier after which a stopped fit leaves (all ones: none), 32 apart
+  int* fail;
+  int* host_fail;
+};
+
+// a: the component whose X^T t is in P, or -1 for the first refresh; next: refresh follows.
+template <int THREADS, bool CLUSTER>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng e, UpdateArgs g, int a, int next) {
+  extern __shared__ double coef[];   // max(m, K), then the chunk of S
+  __shared__ TileShared sh;
+  const int f = blockIdx.y, chunk = blockIdx.x;
+  if (e.status[f]) return;   // set by an earlier launch: the same for every block of the fit
+  int b, en;
+  chunk_range(chunk, e.szp, e.p, b, en);
+  double* Sg = e.S + (size_t)f * e.p * e.m + b;
+  const TileView w{b, en - b, coef + g.coef_len, e.V + (size_t)f * e.p * e.K + b, e.p};
+  tile_load<THREADS>(w.S, Sg, e.p, e.m, w.rows);
+  unsigned arrived = g.arrived;
+  // all chunks of the fit have finished the phase; false: the fit stopped, or a wait gave up
+  auto meet = [&]() {
+    if (CLUSTER) {
+      asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      // a block that sees the status of the phase after this one leaves early: in
+      // that phase every block of the fit finds the same sum and does nothing
+      return *(volatile int*)(e.status + f) == 0;
+    }
+    ++arrived;
+    __syncthreads();
+    if (chunk == 0 && threadIdx.x == 0 && e.status[f] != 0) *(volatile unsigned*)(g.stop + 32 * f) = arrived;
+    if (!counted_barrier(g.counter + 32 * f, arrived * gridDim.x, g.fail, g.host_fail)) return false;
+    return *(volatile unsigned*)(g.stop + 32 * f) > arrived;
+  };
+  if (a >= 0) {
+    tile_loading<THREADS, true>(e, w, a, f, chunk, sh);
+    tile_here();
+    if (!meet()) return;
+    tile_orth<THREADS, true>(e, w, a, f, chunk, coef, sh);
+    if (!meet()) return;
+    tile_deflate<THREADS>(e, w, a, next, f, chunk, coef, sh, nullptr, Sg);
+    if (!next) return;
+  } else {
+    tile_here();
+    tile_start<THREADS>(e, w, f, chunk, sh);
+  }
+  if (!meet()) return;
+  double *zin = e.zA, *zout = e.zB;
+  for (int it = 0; it < e.iters; ++it) {
+    tile_apply<THREADS>(e, w, zin, zout, it == e.iters - 1 ? 1 : 0, f, chunk, coef, sh);
+    if (!meet()) return;
+    double* t = zin;
+    zin = zout;
+    zout = t;
+  }
+  // r = -sign(y0) y / ||y||, Rhat and delta . Rhat as refresh_finish_chunk
+  if (threadIdx.x >= THREADS - 32) {
+    const double s = warp_parts(e.npart + (size_t)f * e.cp, e.cp, sh.stage);
+    if ((threadIdx.x & 31) == 0) sh.nrm = sqrt(s);
+  }
+  const int row = threadIdx.x;
+  const double* yf = e.y + (size_t)f * e.p;
+  const bool mine = row < w.rows;
+  const double y0 = yf[0], y = mine ? yf[b + row] : 0.0;
+  __syncthreads();
+  const double nrm = sh.nrm;
+  if (!(nrm > 0.0) || !isfinite(nrm)) {
+    if (chunk == 0 && threadIdx.x == 0) e.status[f] = 1;
+    return;
+  }
+  const double sgn = y0 >= 0.0 ? -1.0 : 1.0;
+  const size_t at = (size_t)f * e.p + b + row;
+  double rh = 0.0;
+  if (mine) {
+    const double ri = sgn * y / nrm;
+    e.r[at] = ri;
+    rh = e.colscale ? ri * e.colscale[at] : ri;
+    e.Rhat[at] = rh;
+  }
+  if (e.delta) {
+    double s = 0.0;
+    if (mine) s = s + e.delta[at] * rh;
+    s = warp_sum(s);
+    if ((row & 31) == 0) sh.red[row >> 5] = s;
+    __syncthreads();
+    if (row == 0) {
+      double t = 0.0;
+#pragma unroll
+      for (int i = 0; i < kSumWarps; ++i) t += sh.red[i];
+      e.cpart[(size_t)f * e.cp + chunk] = t;
+    }
+  }
+}
+
+// The launch of k_update for one engine: which kernel, and its shared memory.
+struct UpdateLaunch {
+  const void* kernel = nullptr;   // null: separate launches
+  bool cluster = false;
+  dim3 grid;
+  int threads = 0;
+  size_t smem = 0;
+  UpdateArgs args{};
+
+  void run(const Eng& e, int a, int next, cudaStream_t st) {
+    args.arrived = a < 0 ? 0u : (unsigned)(1 + e.iters) + (unsigned)a * (3 + e.iters);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (cluster) {
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = grid.x;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+    } else {
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    Eng ec = e;
+    void* argv[] = {&ec, &args, &a, &next};
+    FPLS_CUDA(cudaLaunchKernelExC(&cfg, kernel, argv));
+    ::fpls::note_launch();
+  }
+};
+
+template <int THREADS>
+const void* update_kernel(bool cluster) {
+  static const bool once = [] {
+    FPLS_CUDA(cudaFuncSetAttribute(k_update<THREADS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+    FPLS_CUDA(cudaFuncSetAttribute(k_update<THREADS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdateSmem));
+    return true;
+  }();
+  (void)once;
+  return cluster ? (const void*)k_update<THREADS, true> : (const void*)k_update<THREADS, false>;
 }
 
 __global__ void k_masked_response(Eng e, double* M) {
@@ -781,7 +1346,6 @@ __global__ void k_shard_unpack(Eng e, const double* __restrict__ red) {
 Eng make_eng(const SimplsBatch& b) {
   Eng e{};
   e.n = b.n; e.p = b.p; e.m = b.m; e.F = b.F; e.K = b.K;
-  e.lds = b.p;
   const int target = 4 * Context::get().sm_count;
   e.cp = std::max(1, std::min(ceil_div(target, b.F), ceil_div(b.p, 256)));
   e.cp = std::max(e.cp, ceil_div(b.p, kMaxChunk));
@@ -976,9 +1540,10 @@ void simpls_batch_run(const SimplsBatch& b) {
   // more loads in flight as kernels of their own.
   auto* op64 = dynamic_cast<XOperatorF64*>(b.X);
   const int coef_len = std::max(std::max(b.m, 1), std::max(b.K, 1));
-  const size_t loop_smem = (coef_len + 256 * 32 + (size_t)e.szp * (b.m + b.K + 4)) * sizeof(double);
+  const int vec_len = std::max(e.szn, kTile);
+  const size_t loop_smem = (coef_len + vec_len + 256 * 32 + (size_t)kTile * (b.m + b.K)) * sizeof(double);
   if (simpls_graph_enabled() && !trace && !ctx.profile && !shard_red && op64 && b.F == 1 && !b.labels && !b.mask &&
-      !b.delta && !b.colscale && !b.dY && (size_t)b.n * b.p <= ((size_t)1 << 22) && e.cp <= ctx.sm_count &&
+      !b.delta && !b.colscale && !b.dY && (size_t)b.n * b.p <= ((size_t)1 << 22) && e.cp <= ctx.sm_count && e.szp <= kTile &&
       loop_smem <= kLoopSmem) {
     LoopArgs g;
     g.xr = gemv_ranges(b.n, b.p, ctx.sm_count);
@@ -994,6 +1559,7 @@ void simpls_batch_run(const SimplsBatch& b) {
     g.stop = ctl + 64;
     g.host_fail = ctx.host_fail;
     g.coef_len = coef_len;
+    g.vec_len = vec_len;
     const int want = std::max({e.cp, e.cn, ceil_div(b.n, 32) * g.xr.splits, ceil_div(b.p, kLoopWarps)});
     static const bool once = [] {
       FPLS_CUDA(cudaFuncSetAttribute(simpls_loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLoopSmem));
@@ -1006,6 +1572,38 @@ void simpls_batch_run(const SimplsBatch& b) {
     ::fpls::note_launch();
     return;   // a wait that gave up ends the call with an error (Context::end_call)
   }
+  // The phases between the products in one launch, where a chunk's S fits shared
+  // memory and the chunks form a cluster or are all resident (the count of blocks
+  // an SM holds decides); else (wide responses, or many fits of many chunks) as
+  // launches of their own.
+  UpdateLaunch up;
+  {
+    up.cluster = e.cp <= kClusterChunks;
+    // few columns give a warp one or two, and 60 fits of a grid fill the SMs
+    up.threads = std::max(b.m, b.K) <= 32 ? 256 : 512;
+    up.grid = gp;
+    up.args.coef_len = coef_len;
+    up.smem = (coef_len + (size_t)b.m * kTile) * sizeof(double);
+    const void* k = up.threads == 256 ? update_kernel<256>(up.cluster) : update_kernel<512>(up.cluster);
+    bool fits = e.szp <= kTile && up.smem <= kUpdateSmem;
+    if (fits && !up.cluster) {
+      int per_sm = 0;
+      FPLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, up.threads, up.smem));
+      fits = (long long)e.cp * b.F <= (long long)per_sm * ctx.sm_count;
+    }
+    if (fits) {
+      up.kernel = k;
+      if (!up.cluster) {
+        unsigned* ctl = ar.alloc_n<unsigned>(32 * (2 * F + 1));   // each on a line of its own
+        FPLS_CUDA(cudaMemsetAsync(ctl, 0, 32 * (F + 1) * sizeof(unsigned), st));
+        FPLS_CUDA(cudaMemsetAsync(ctl + 32 * (F + 1), 0xff, 32 * F * sizeof(unsigned), st));
+        up.args.counter = ctl;
+        up.args.fail = reinterpret_cast<int*>(ctl + 32 * F);
+        up.args.stop = ctl + 32 * (F + 1);
+        up.args.host_fail = ctx.host_fail;
+      }
+    }
+  }
   // The component loop as one CUDA graph once its shape has run (not while a
   // trace or the kernel-class profiler records events, nor for row-sharded
   // fits, whose all-reduce callback is the caller's).
@@ -1014,24 +1612,30 @@ void simpls_batch_run(const SimplsBatch& b) {
   const bool eligible = simpls_graph_enabled() && !trace && !ctx.profile && !shard_red;
   const bool graph = eligible && simpls_seen().count(key) > 0;
   auto loop = [&]() {
-  k_refresh_start<<<gp, tm, 0, st>>>(e); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
-  for (int a = 0; a < b.K; ++a) {
-    // Refresh: y <- S (S^T y) `iters` times from the warm start, then normalise.
-    double* zin = e.zA;
-    double* zout = e.zB;
-    for (int it = 0; it < e.iters; ++it) {
-      const int last = (it == e.iters - 1) ? 1 : 0;
-      k_refresh_apply<<<gp, tm, sm_m, st>>>(e, zin, zout, last); ::fpls::note_launch();
-      FPLS_CHECK_LAUNCH();
-      std::swap(zin, zout);
-    }
-    k_refresh_finish<<<gp, kThreads, 0, st>>>(e); ::fpls::note_launch();
+  if (up.kernel) {
+    up.run(e, -1, 1, st);
+  } else {
+    k_refresh_start<<<gp, tm, 0, st>>>(e); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
-    mark("refresh");
-    const Partials up = b.X->times_partials(e.Rhat, b.F, e.U);
-    e.upart = const_cast<double*>(up.w);
-    e.usplits = up.splits;
+  }
+  for (int a = 0; a < b.K; ++a) {
+    if (!up.kernel) {
+      // Refresh: y <- S (S^T y) `iters` times from the warm start, then normalise.
+      double* zin = e.zA;
+      double* zout = e.zB;
+      for (int it = 0; it < e.iters; ++it) {
+        const int last = (it == e.iters - 1) ? 1 : 0;
+        k_refresh_apply<<<gp, tm, sm_m, st>>>(e, zin, zout, last); ::fpls::note_launch();
+        FPLS_CHECK_LAUNCH();
+        std::swap(zin, zout);
+      }
+      k_refresh_finish<<<gp, kThreads, 0, st>>>(e); ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      mark("refresh");
+    }
+    const Partials xr = b.X->times_partials(e.Rhat, b.F, e.U);
+    e.upart = const_cast<double*>(xr.w);
+    e.usplits = xr.splits;
     mark("X*R");
     k_scores<<<gn, tq, b.labels ? sm_m : 0, st>>>(e, a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
@@ -1051,6 +1655,11 @@ void simpls_batch_run(const SimplsBatch& b) {
       FPLS_CHECK_LAUNCH();
     }
     mark("X^T*T");
+    if (up.kernel) {
+      up.run(e, a, a + 1 < b.K ? 1 : 0, st);
+      mark("update");
+      continue;
+    }
     k_loading<<<gp, block(a), 0, st>>>(e, a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("loading");
