@@ -63,12 +63,16 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ W, int splits, l
   }
 }
 
-// y[n] = alpha * sum_k A[k + n*lda] x[k] + beta y[n] ; one warp per column.
+// y[n] = alpha * sum_k A[k + n*lda] x[k] + beta y[n]; one warp per column and
+// range of kps rows (blockIdx.y; its result at y + range * stride).
 __global__ void __launch_bounds__(128) gemv_t_kernel(int K, int N, double alpha, const double* __restrict__ A, int lda,
-                                                     const double* __restrict__ x, double beta, double* __restrict__ y) {
+                                                     const double* __restrict__ x, double beta, double* __restrict__ y,
+                                                     int kps, long long stride) {
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= N) return;
-  const double acc = gemv_column<kGemvAhead>(A + (size_t)n * lda, x, K);
+  const int k0 = blockIdx.y * kps;
+  const double acc = gemv_column<kGemvAhead>(A + (size_t)n * lda + k0, x + k0, min(kps, K - k0));
+  y += blockIdx.y * stride;
   if ((threadIdx.x & 31) == 0) y[n] = (beta == 0.0) ? alpha * acc : alpha * acc + beta * y[n];
 }
 
@@ -493,6 +497,33 @@ Partials gemv_partials(int rows, int cols, const double* A, int lda, const doubl
   return Partials{ws, gr.splits, (size_t)rows};
 }
 
+Partials gemv_t_partials(int rows, int cols, const double* A, int lda, const double* x, double* y) {
+  Context& ctx = Context::get();
+  const GemvRanges gr = gemv_t_ranges(rows, std::max(cols, 1), ctx.sm_count);
+  if (rows <= 0 || cols <= 0 || gr.splits == 1) {
+    gemv(true, rows, cols, 1.0, A, lda, x, 0.0, y);
+    return Partials{y, 1, 0};
+  }
+  cudaStream_t st = ctx.stream;
+  const int slot = ctx.prof_begin("gemv_f64", st);
+  double* ws = ctx.splitk_workspace(st, (size_t)gr.splits * cols);
+  gemv_t_kernel<<<dim3(ceil_div(cols, 4), gr.splits), 128, 0, st>>>(rows, cols, 1.0, A, lda, x, 0.0, ws, gr.kps,
+                                                                    (long long)cols);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+  ctx.prof_end(slot, st, 8.0 * ((double)rows * cols + rows + cols), 2.0 * (double)rows * cols);
+  return Partials{ws, gr.splits, (size_t)cols};
+}
+
+void gemv_t_ranged(int rows, int cols, const double* A, int lda, const double* x, double* y) {
+  const Partials p = gemv_t_partials(rows, cols, A, lda, x, y);
+  if (p.splits == 1) return;
+  splitk_reduce_kernel<<<grid_for(cols, 256), 256, 0, Context::get().stream>>>(p.w, p.splits, (long long)p.stride, cols, 1,
+                                                                              cols, 0.0, y, cols, nullptr);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
+}
+
 void gemv(bool trans, int rows, int cols, double alpha, const double* A, int lda, const double* x,
           double beta, double* y) {
   Context& ctx = Context::get();
@@ -521,7 +552,8 @@ void gemv(bool trans, int rows, int cols, double alpha, const double* A, int lda
     ::fpls::note_launch();
   } else {
     if (cols <= 0) return;
-    gemv_t_kernel<<<ceil_div(cols, 4), 128, 0, st>>>(rows, cols, alpha, A, lda, x, beta, y); ::fpls::note_launch();
+    gemv_t_kernel<<<ceil_div(cols, 4), 128, 0, st>>>(rows, cols, alpha, A, lda, x, beta, y, rows, 0ll);
+    ::fpls::note_launch();
   }
   FPLS_CHECK_LAUNCH();
   // algorithmic bytes: the matrix once plus both vectors

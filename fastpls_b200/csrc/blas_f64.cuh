@@ -28,6 +28,9 @@ Partials gemm_partials(bool transA, bool transB, int M, int N, int K, const doub
                        int ldb, double* C);
 // gemv (no transpose, alpha 1, beta 0) whose column ranges the reader adds up.
 Partials gemv_partials(int rows, int cols, const double* A, int lda, const double* x, double* y);
+// y = A^T x by gemv_t_ranges' row ranges, which the reader adds up (gemv_t_ranged: added here).
+Partials gemv_t_partials(int rows, int cols, const double* A, int lda, const double* x, double* y);
+void gemv_t_ranged(int rows, int cols, const double* A, int lda, const double* x, double* y);
 
 // K (n x n) = X X^T for X n x p: the upper-triangle tiles by FP64 tensor-core
 // MMA, the lower triangle mirrored (K exactly symmetric).

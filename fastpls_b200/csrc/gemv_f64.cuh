@@ -24,6 +24,23 @@ inline GemvRanges gemv_ranges(int rows, int cols, int sm_count) {
   return g;
 }
 
+// Row ranges of y = A^T x that SIMPLS takes for one fit: a warp a column leaves a
+// tall matrix of few columns with too few loads in flight (50000 x 1000: 214 us
+// for 400 MB, five ranges 66 us), so columns get ranges until there are 32 warps
+// an SM, each of at least 8192 rows.  One range up to 2^22 elements, where the
+// one-launch loop takes whole columns and the sums have to be its.
+inline GemvRanges gemv_t_ranges(int rows, int cols, int sm_count) {
+  GemvRanges g{cols, 1, rows};
+  if ((long long)rows * cols > (1ll << 22)) {
+    const int a = ceil_div(32 * sm_count, cols), b = rows / 8192;
+    g.splits = a < b ? a : b;
+    if (g.splits < 1) g.splits = 1;
+  }
+  g.kps = ceil_div(ceil_div(rows, g.splits), 32) * 32;
+  g.splits = ceil_div(rows, g.kps);
+  return g;
+}
+
 // acc += sum_k a[k * lda] xs[k], k < kn in order; AHEAD loads go out before they
 // are multiplied (one after another, a 400 x 2000 product waited 63 times for L2).
 template <int AHEAD>

@@ -1372,7 +1372,7 @@ void XOperatorF64::times(const double* Rhat, int F, double* U) {
 }
 
 void XOperatorF64::t_times(const double* T, int F, double* P) {
-  if (F == 1) gemv(true, n, p, 1.0, Xc, n, T, 0.0, P);
+  if (F == 1) gemv_t_ranged(n, p, Xc, n, T, P);
   else gemm(true, false, p, F, n, 1.0, Xc, n, T, n, 0.0, P, p);
 }
 
@@ -1382,10 +1382,7 @@ Partials XOperatorF64::times_partials(const double* Rhat, int F, double* U) {
 }
 
 Partials XOperatorF64::t_times_partials(const double* T, int F, double* P) {
-  if (F == 1) {
-    t_times(T, F, P);
-    return Partials{P, 1, 0};
-  }
+  if (F == 1) return gemv_t_partials(n, p, Xc, n, T, P);
   return gemm_partials(true, false, p, F, n, Xc, n, T, n, P);
 }
 

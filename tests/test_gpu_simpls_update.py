@@ -25,3 +25,19 @@ def test_update_matches_oracle(lib, p, m):
     # sums of 2^22 products in another order, amplified by the deflations' cancellation
     for key in ("R", "Q", "B"):
         assert np.linalg.norm(got[key] - ref[key]) <= 1e-9 * np.linalg.norm(ref[key]), key
+
+
+# X^T t of a tall matrix in row ranges: two, and four of unequal length; a row-sharded fit on one rank adds
+# the same ranges before its all-reduce
+@pytest.mark.parametrize("n,p,m", [(16385, 300, 2), (33001, 259, 9)])
+def test_row_ranges(lib, n, p, m):
+    rng = np.random.default_rng(n)
+    L = rng.standard_normal((n, 4))
+    X = L @ rng.standard_normal((4, p)) + 0.3 * rng.standard_normal((n, p))
+    Y = L @ rng.standard_normal((4, m)) + 0.1 * rng.standard_normal((n, m))
+    got = lib.pls_model2_fast(X, Y, [4], seed=1)
+    ref = opls.pls_model2_fast(X, Y, [4], seed=1)
+    one = lib.pls_model2_fast(X, Y, [4], seed=1, allreduce=lambda buf, count, stream: None)
+    for key in ("R", "Q", "B"):
+        assert np.linalg.norm(got[key] - ref[key]) <= 1e-9 * np.linalg.norm(ref[key]), key
+        assert np.array_equal(one[key], got[key]), key
