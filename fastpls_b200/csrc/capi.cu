@@ -901,28 +901,35 @@ int fpls_lda_predict(const double* T, int w, int k, const double* linear,
 
 namespace {
 
-// LDA scores of raw rows X (w x p, device) through the projection R (p x k, ld
-// ldr) and offset: S = (X R - offset) linear^T + constants, by the direct or
-// the latent route as lda_project_predict_labels_cpp chooses
-// (fastPLS.cpp:2100-2147, CPU rule with the 0.5 factor); labels (device, w) and,
-// when scores is set, the full score matrix (device, w x C).  dc is modified.
-void lda_project_scores_device(const double* dX, int w, int p, const double* dR, int ldr, int k,
-                               const double* doff, const double* dL, int ldl, double* dc, int C, int* dlab,
-                               double* dS_out) {
-  Context& ctx = Context::get();
-  double* dS = dS_out ? dS_out : ctx.arena.alloc_n<double>((size_t)w * C);
-  // constants_adj = constants - offset linear^T
-  if (doff) gemv(false, C, k, -1.0, dL, ldl, doff, 1.0, dc);
+// The route of lda_project_predict_labels_cpp (fastPLS.cpp:2100-2147, CPU rule
+// with the 0.5 factor): through the latent scores, or directly.
+bool lda_latent_path(int w, int p, int k, int C) {
   const double nn = w, pp = p, kk = k, cc = C;
   const double latent_ops = nn * kk * (pp + cc);
   const double direct_ops = nn * pp * cc;
-  if (direct_ops < 0.5 * latent_ops) {
+  return !(direct_ops < 0.5 * latent_ops);
+}
+
+// LDA scores of raw rows X (w x p, device) through the projection R (p x k, ld
+// ldr): S = X R linear^T + dc (the class constants, adjusted for an offset of
+// the scores); labels (device, w) and, when scores is set, the full score matrix
+// (device, w x C).  dT: the latent scores X R (w x k or wider), null to form
+// them here; the component counts of one call share them.
+void lda_project_scores_device(const double* dX, int w, int p, const double* dR, int ldr, int k,
+                               const double* dL, int ldl, const double* dc, int C, int* dlab, double* dS_out,
+                               const double* dT = nullptr) {
+  Context& ctx = Context::get();
+  double* dS = dS_out ? dS_out : ctx.arena.alloc_n<double>((size_t)w * C);
+  if (!lda_latent_path(w, p, k, C)) {
     double* dW = ctx.arena.alloc_n<double>((size_t)p * C);
     gemm(false, true, p, C, k, 1.0, dR, ldr, dL, ldl, 0.0, dW, p);
     xgemm(false, w, C, p, dX, w, dW, p, dS, w);
   } else {
-    double* dT = ctx.arena.alloc_n<double>((size_t)w * k);
-    gemm(false, false, w, k, p, 1.0, dX, w, dR, ldr, 0.0, dT, w);
+    if (!dT) {
+      double* T = ctx.arena.alloc_n<double>((size_t)w * k);
+      gemm(false, false, w, k, p, 1.0, dX, w, dR, ldr, 0.0, T, w);
+      dT = T;
+    }
     gemm(false, true, w, C, k, 1.0, dT, w, dL, ldl, 0.0, dS, w);
   }
   row_argmax(dS, w, C, dc, dlab);
@@ -1030,6 +1037,8 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
     d.linear = ctx.arena.alloc_n<double>((size_t)n_classes * K0 * U);
     d.constants = ctx.arena.alloc_n<double>((size_t)n_classes * U);
     d.priors = ctx.arena.alloc_n<double>(n_classes);
+    d.offset = doff;
+    d.adjusted = ctx.arena.alloc_n<double>((size_t)n_classes * U);
     std::vector<double> lam(U);
     d.lambda = lam.data();
     pt.mark("prediction weights");
@@ -1041,12 +1050,19 @@ int fpls_pls_lda(const void* Xtrain, int x_is_float32, int n, int p, const doubl
       const double* dXt = f32 ? widen_on_device(static_cast<const float*>(xt_up.dst), ntest, p)
                               : static_cast<const double*>(xt_up.dst);
       dpred = ctx.arena.alloc_n<int>((size_t)ntest * L);
-      double* dc = ctx.arena.alloc_n<double>(n_classes);
+      // the latent scores of the largest component count hold those of the others
+      double* dTt = nullptr;
+      int kt = 0;
+      for (int i = 0; i < L; ++i)
+        if (lda_latent_path(ntest, p, nc[i], n_classes)) kt = std::max(kt, nc[i]);
+      if (kt > 0) {
+        dTt = ctx.arena.alloc_n<double>((size_t)ntest * kt);
+        gemm(false, false, ntest, kt, p, 1.0, dXt, ntest, dRp, p, 0.0, dTt, ntest);
+      }
       for (int i = 0; i < L; ++i) {
         const int u = static_cast<int>(std::lower_bound(uq.begin(), uq.end(), nc[i]) - uq.begin());
-        d2d(dc, d.constants + (size_t)u * n_classes, n_classes * sizeof(double));
-        lda_project_scores_device(dXt, ntest, p, dRp, p, nc[i], doff, d.linear + (size_t)u * n_classes * K0,
-                                  n_classes, dc, n_classes, dpred + (size_t)i * ntest, nullptr);
+        lda_project_scores_device(dXt, ntest, p, dRp, p, nc[i], d.linear + (size_t)u * n_classes * K0, n_classes,
+                                  d.adjusted + (size_t)u * n_classes, n_classes, dpred + (size_t)i * ntest, nullptr, dTt);
       }
       pt.mark("test prediction");
     }
@@ -1090,7 +1106,9 @@ int fpls_lda_project_predict(const double* X, int w, int p, const double* R, int
     const double* doff = offset ? upload(offset, k) : nullptr;
     double* dS = scores ? ctx.arena.alloc_n<double>((size_t)w * n_classes) : nullptr;
     int* dlab = ctx.arena.alloc_n<int>(w);
-    lda_project_scores_device(dX, w, p, dR, p, k, doff, dL, n_classes, dc, n_classes, dlab, dS);
+    // constants_adj = constants - offset linear^T
+    if (doff) gemv(false, n_classes, k, -1.0, dL, n_classes, doff, 1.0, dc);
+    lda_project_scores_device(dX, w, p, dR, p, k, dL, n_classes, dc, n_classes, dlab, dS);
     download(labels, dlab, w);
     if (scores) download(scores, dS, (size_t)w * n_classes);
     ctx.sync();

@@ -15,7 +15,7 @@ namespace fpls {
 namespace {
 
 __global__ void diag_kernel(double* D, int k, const double* s) {
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < k * k; t += gridDim.x * blockDim.x) {
     const int i = t % k, j = t / k;
     D[t] = (i == j) ? s[i] : 0.0;
   }
@@ -239,25 +239,25 @@ int plssvd_fit_centered(const double* X, int n, int p, const double* Y, int m, c
   pt.mark("T = X R, G");
   dzero(out.C_latent, (size_t)K0 * K0 * L * sizeof(double));
   dzero(out.W_latent, (size_t)K0 * m * L * sizeof(double));
+  // diag(s); a component count's right-hand side is its leading block
   double* D = ctx.arena.alloc_n<double>((size_t)keff * keff);
-  double* Cw = ctx.arena.alloc_n<double>((size_t)keff * keff);
-  double* Wa = ctx.arena.alloc_n<double>((size_t)keff * m);
+  diag_kernel<<<std::max(1, std::min(ctx.sm_count, ceil_div(keff * keff, 256))), 256, 0, ctx.stream>>>(D, keff, out.s);
+  ::fpls::note_launch();
+  FPLS_CHECK_LAUNCH();
   double* Yf = opt.fit ? ctx.arena.alloc_n<double>((size_t)n * m) : nullptr;
   double* rq = ctx.arena.alloc_n<double>(2 * L);
   const double* rq_mu = opt.fit ? shard_rq_means(Y, n, m) : nullptr;
   for (int a = 0; a < L; ++a) {
     const int mc = std::min(ncomp[a], keff);
-    diag_kernel<<<1, 256, 0, ctx.stream>>>(D, mc, out.s); ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
     // G_a is the leading mc x mc block of G (leading dimension keff).
-    spd_solve(mc, G, keff, mc, D, mc, Cw, mc, ctx.d_status + 2);
-    copy_matrix(out.C_latent + (size_t)a * K0 * K0, K0, Cw, mc, mc, mc);
+    double* Cw = out.C_latent + (size_t)a * K0 * K0;
+    double* Wa = out.W_latent + (size_t)a * K0 * m;
+    spd_solve(mc, G, keff, mc, D, keff, Cw, K0, ctx.d_status + 2);
     // W_a = C V_a^T  (mc x m)
-    gemm(false, true, mc, m, mc, 1.0, Cw, mc, out.Q, m, 0.0, Wa, mc);
-    copy_matrix(out.W_latent + (size_t)a * K0 * m, K0, Wa, mc, mc, m);
-    if (out.B) gemm(false, false, p, m, mc, 1.0, out.R, p, Wa, mc, 0.0, out.B + (size_t)a * p * m, p);
+    gemm(false, true, mc, m, mc, 1.0, Cw, K0, out.Q, m, 0.0, Wa, K0);
+    if (out.B) gemm(false, false, p, m, mc, 1.0, out.R, p, Wa, K0, 0.0, out.B + (size_t)a * p * m, p);
     if (opt.fit) {
-      gemm(false, false, n, m, mc, 1.0, out.T, n, Wa, mc, 0.0, Yf, n);
+      gemm(false, false, n, m, mc, 1.0, out.T, n, Wa, K0, 0.0, Yf, n);
       rq_sums(Y, Yf, n, m, rq + 2 * a, rq_mu);
       add_row_vector(Yf, n, m, n, mY);
       d2d(out.Yfit + (size_t)a * n * m, Yf, (size_t)n * m * sizeof(double));

@@ -53,9 +53,12 @@ __global__ void symm_upper_scale_kernel(double* P, int k, double inv_df) {
   }
 }
 
-// Leading kk x kk block plus lambda I; lambda = ridge * trace/kk (reference ridge rule).
-__global__ void ridge_block_kernel(const double* P, int kmax, int kk, double ridge, double* out,
-                                   double* lambda_out) {
+// One component count's system: out = leading kk x kk block of P plus lambda I
+// with lambda = ridge * trace / kk (reference ridge rule), and Mt (kk x C) = the
+// transposed leading columns of the means.  Every block forms the trace itself.
+__global__ void __launch_bounds__(256)
+lda_system_kernel(const double* __restrict__ P, int kmax, int kk, double ridge, const double* __restrict__ M, int C,
+                  double* __restrict__ out, double* __restrict__ Mt, double* lambda_out) {
   __shared__ double scratch[32];
   __shared__ double lam;
   double tr = 0.0;
@@ -67,33 +70,50 @@ __global__ void ridge_block_kernel(const double* P, int kmax, int kk, double rid
     double l = ridge;
     if (!isfinite(l) || l < 0.0) l = 1e-8;
     lam = l * scale;
-    *lambda_out = lam;
+    if (blockIdx.x == 0) *lambda_out = lam;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < kk * kk; t += blockDim.x) {
+  const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int t = first; t < kk * kk; t += step) {
     const int i = t % kk, j = t / kk;
     out[t] = P[i + (size_t)j * kmax] + (i == j ? lam : 0.0);
   }
+  for (int t = first; t < kk * C; t += step) {
+    const int c = t % C, j = t / C;
+    Mt[j + (size_t)c * kk] = M[t];
+  }
 }
 
-__global__ void transpose_block_kernel(const double* A, int rows, int cols, int lda, double* B,
-                                       int ldb) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= rows * cols) return;
-  const int i = t % rows, j = t / rows;
-  B[j + (size_t)i * ldb] = A[i + (size_t)j * lda];
-}
-
-// constants[c] = -0.5 * means_c . linear_c + log(max(prior_c, DBL_MIN))
-__global__ void lda_constants_kernel(const double* M, const double* Lin, int C, int kk, int ldm,
-                                     const double* counts, int n, double* constants,
-                                     double* priors) {
+// One component count's model, a thread a class: the means' and the solution's
+// (Xs, kk x C) leading columns into means and linear (C x kmax, zero past kk),
+// constants[c] = -0.5 means_c . linear_c + log(max(prior_c, DBL_MIN)) and, with
+// an offset, adjusted[c] = constants[c] - linear_c . offset.  With the system
+// above this is two launches a component count beside the solve, where copies,
+// clears, transposes and the two sums of a class had been eight.
+__global__ void __launch_bounds__(32)
+lda_model_kernel(const double* __restrict__ M, const double* __restrict__ Xs, int C, int kk, int kmax,
+                 const double* __restrict__ counts, int n, const double* __restrict__ offset,
+                 double* __restrict__ means, double* __restrict__ linear, double* __restrict__ constants,
+                 double* __restrict__ adjusted, double* __restrict__ priors) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
-  double d = 0.0;
-  for (int j = 0; j < kk; ++j) d += M[c + (size_t)j * ldm] * Lin[c + (size_t)j * ldm];
+  double d = 0.0, off = 0.0;
+#pragma unroll 8
+  for (int j = 0; j < kk; ++j) {
+    const double mean = M[c + (size_t)j * C], x = Xs[j + (size_t)c * kk];
+    means[c + (size_t)j * C] = mean;
+    linear[c + (size_t)j * C] = x;
+    d += mean * x;
+    if (offset) off = fma(x, offset[j], off);
+  }
+  for (int j = kk; j < kmax; ++j) {
+    means[c + (size_t)j * C] = 0.0;
+    linear[c + (size_t)j * C] = 0.0;
+  }
   const double prior = counts[c] / static_cast<double>(n);
-  constants[c] = -0.5 * d + log(fmax(prior, DBL_MIN));
+  const double constant = -0.5 * d + log(fmax(prior, DBL_MIN));
+  constants[c] = constant;
+  if (offset) adjusted[c] = constant - off;
   if (priors) priors[c] = prior;
 }
 
@@ -172,18 +192,15 @@ void lda_train_prefix(const double* T, int n, int kmax, const int* y_host, int C
   double* lam = ctx.arena.alloc_n<double>(L);
   for (int a = 0; a < L; ++a) {
     const int kk = ncomp_host[a];
-    ridge_block_kernel<<<1, 256, 0, ctx.stream>>>(P, kmax, kk, ridge, Pk, lam + a); ::fpls::note_launch();
-    transpose_block_kernel<<<ceil_div(C * kk, 256), 256, 0, ctx.stream>>>(M, C, kk, C, Mt, kk); ::fpls::note_launch();
+    const int blocks = std::max(1, std::min(ctx.sm_count, ceil_div(kk * std::max(kk, C), 1024)));
+    lda_system_kernel<<<blocks, 256, 0, ctx.stream>>>(P, kmax, kk, ridge, M, C, Pk, Mt, lam + a); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     spd_solve(kk, Pk, kk, C, Mt, kk, Xs, kk, ctx.d_status + 5);
-    double* Ma = out.means + (size_t)a * C * kmax;
-    double* La = out.linear + (size_t)a * C * kmax;
-    dzero(Ma, (size_t)C * kmax * sizeof(double));
-    dzero(La, (size_t)C * kmax * sizeof(double));
-    copy_matrix(Ma, C, M, C, C, kk);
-    transpose_block_kernel<<<ceil_div(C * kk, 256), 256, 0, ctx.stream>>>(Xs, kk, C, kk, La, C); ::fpls::note_launch();
-    lda_constants_kernel<<<ceil_div(C, 128), 128, 0, ctx.stream>>>(
-        Ma, La, C, kk, C, counts, n, out.constants + (size_t)a * C, a == 0 ? out.priors : nullptr); ::fpls::note_launch();
+    lda_model_kernel<<<ceil_div(C, 32), 32, 0, ctx.stream>>>(
+        M, Xs, C, kk, kmax, counts, n, out.offset, out.means + (size_t)a * C * kmax, out.linear + (size_t)a * C * kmax,
+        out.constants + (size_t)a * C, out.offset ? out.adjusted + (size_t)a * C : nullptr,
+        a == 0 ? out.priors : nullptr);
+    ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
   }
   std::vector<double> hl(L);

@@ -24,6 +24,9 @@ struct LdaModelsDev {
   double* constants;  // C x L
   double* priors;     // C
   double* lambda;     // L (host)
+  // with an offset of the scores (kmax): adjusted (C x L) = constants - linear . offset
+  const double* offset = nullptr;
+  double* adjusted = nullptr;
 };
 
 // lda_train_prefix_cpp (src/fastPLS.cpp:1817-1927) on scores T (n x kmax, ld n)
