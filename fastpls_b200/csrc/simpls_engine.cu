@@ -1124,7 +1124,7 @@ __global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
 // phase, by the instructions of a warp (a first form that called the bodies on
 // memory's layout executed four times as many and took as long as the launches).
 // A component's phases: 30 fits of 501 x 5, 2 chunks each: 50 -> 33 us; 8000 x
-// 100, 32 chunks: 105 -> 54 us; 1000 x 50, 4 chunks: 114 -> 57 us.
+// 100, 32 chunks: 105 -> 54 us; 1000 x 100, 4 chunks: 114 -> 57 us.
 constexpr int kClusterChunks = 8;
 constexpr size_t kUpdateSmem = 208 * 1024;   // dynamic, beside the static arrays
 struct UpdateArgs {
