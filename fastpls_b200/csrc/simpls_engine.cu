@@ -123,6 +123,7 @@ __device__ void chunk_dots(const double* M, size_t ld, int ncols,
   __shared__ double red[kSumWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (ncols >= kSumWarps) {
+#pragma unroll 2
     for (int j = warp; j < ncols; j += blockDim.x >> 5) {
       const double* col = M + (size_t)j * ld;
       double a0 = 0.0, a1 = 0.0;
