@@ -283,7 +283,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_refresh_finish(Eng e) {
   refresh_finish_chunk(e, blockIdx.y, blockIdx.x, vec, scratch);
 }
 
-// t = mask * (U - delta.rhat); partial sums of t^2, t and q = Y^T t.
+// t = mask * (U - delta.rhat); partial sums of t^2, t and q = Y^T t (LABELS: Y is
+// the one-hot matrix of e.labels).
+template <bool LABELS>
 __device__ __forceinline__ void scores_chunk(const Eng& e, int a, int f, int chunk, double* qs, double* ts, double* scratch) {
   int b, en;
   chunk_range(chunk, e.szn, e.n, b, en);
@@ -292,7 +294,7 @@ __device__ __forceinline__ void scores_chunk(const Eng& e, int a, int f, int chu
   const double* Uf = e.U + (size_t)f * e.n;
   double* Tf = e.T + (size_t)f * e.n;
   double* keep = e.Tkeep ? e.Tkeep + ((size_t)f * e.K + a) * e.n : nullptr;
-  if (e.labels) {
+  if (LABELS) {
     for (int j = threadIdx.x; j < e.m; j += blockDim.x) qs[j] = 0.0;
     __syncthreads();
   }
@@ -302,7 +304,7 @@ __device__ __forceinline__ void scores_chunk(const Eng& e, int a, int f, int chu
     Tf[i] = t;
     ts[i - b] = t;
     if (keep) keep[i] = u;
-    if (e.labels && t != 0.0) atomicAdd(&qs[e.labels[i]], t);
+    if (LABELS && t != 0.0) atomicAdd(&qs[e.labels[i]], t);
   }
   __syncthreads();
   const double s2 = chunk_sum(en - b, scratch, [&](int r, double s) { return s + ts[r] * ts[r]; });
@@ -312,19 +314,20 @@ __device__ __forceinline__ void scores_chunk(const Eng& e, int a, int f, int chu
     e.tpart[((size_t)f * e.cn + chunk) * 2 + 1] = s1;
   }
   double* qp = e.qpart + ((size_t)f * e.cn + chunk) * e.m;
-  if (e.labels) {
+  if (LABELS) {
     for (int j = threadIdx.x; j < e.m; j += blockDim.x) qp[j] = qs[j];
-    return;
+  } else {
+    chunk_dots(e.Yg + b, e.n, e.m, ts, en - b, qp, 1);
   }
-  chunk_dots(e.Yg + b, e.n, e.m, ts, en - b, qp, 1);
 }
 
-__global__ void __launch_bounds__(kMaxThreads) k_scores(Eng e, int a) {
+template <bool LABELS>
+__global__ void __launch_bounds__(LABELS ? kSumThreads : kMaxThreads) k_scores(Eng e, int a) {
   extern __shared__ double coef[];
   __shared__ double vec[kMaxChunk];
   __shared__ double scratch[32];
   if (e.status[blockIdx.y]) return;
-  scores_chunk(e, a, blockIdx.y, blockIdx.x, coef, vec, scratch);
+  scores_chunk<LABELS>(e, a, blockIdx.y, blockIdx.x, coef, vec, scratch);
 }
 
 __device__ __forceinline__ void t_stats(const Eng& e, int f, double& tn, double& st) {
@@ -1098,7 +1101,7 @@ __global__ void __launch_bounds__(kLoopThreads) simpls_loop_kernel(LoopArgs g) {
       }
     }
     if (!phase(0, [](int) {})) return;
-    if (!phase(e.cn, [&](int c) { scores_chunk(e, a, 0, c, coef, vec, scratch); })) return;
+    if (!phase(e.cn, [&](int c) { scores_chunk<false>(e, a, 0, c, coef, vec, scratch); })) return;
     for (int j = blockIdx.x * (kLoopThreads / 32) + (threadIdx.x >> 5); j < e.p; j += gridDim.x * (kLoopThreads / 32)) {
       const double acc = gemv_column<32>(g.X + (size_t)j * e.n, e.T, e.n);
       if ((threadIdx.x & 31) == 0) e.P[j] = acc;
@@ -1508,7 +1511,7 @@ void simpls_batch_run(const SimplsBatch& b) {
   // it is, and 1024-thread ones took 35 us instead of 10 for their class scores),
   // then 512, then 1024.
   auto block = [](int cols) { return cols <= 32 ? 256 : cols <= 64 ? 512 : kMaxThreads; };
-  const int tm = block(b.m), tq = b.labels ? 256 : tm;
+  const int tm = block(b.m), tq = b.labels ? kSumThreads : tm;
   constexpr int kThreads = 256;   // elementwise kernels
   // all-reduce buffer of a row-sharded fit: [P (F x p) | t^T t, sum t (F x 2) | Y^T t (F x m)]
   const size_t shard_count = sharded() ? F * ((size_t)b.p + 2 + b.m) : 0;
@@ -1635,7 +1638,9 @@ void simpls_batch_run(const SimplsBatch& b) {
     e.upart = const_cast<double*>(xr.w);
     e.usplits = xr.splits;
     mark("X*R");
-    k_scores<<<gn, tq, b.labels ? sm_m : 0, st>>>(e, a); ::fpls::note_launch();
+    if (b.labels) k_scores<true><<<gn, tq, sm_m, st>>>(e, a);
+    else k_scores<false><<<gn, tq, 0, st>>>(e, a);
+    ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     mark("scores");
     if (shard_red) {
