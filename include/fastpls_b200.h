@@ -18,9 +18,9 @@
  *    fpls_predict_lowrank, fpls_lda_project_train_prefix,
  *    fpls_lda_project_predict, fpls_opls_filter, fpls_opls_apply_filter,
  *    fpls_gaussian_y_encode / _decode and fpls_x_upload) may instead be device
- *    memory of the library's device: unified addressing tells the two apart
- *    and the copy then stays in HBM (no counterpart in the reference, whose
- *    inputs are R objects in host memory).
+ *    memory of the library's device: unified addressing tells the two apart,
+ *    and inputs are read where they lie (fpls_x_upload copies; no counterpart
+ *    in the reference, whose inputs are R objects in host memory).
  *  - Every function returns 0 on success or a non-zero fpls_status; on failure a
  *    NUL-terminated message is written to err[0..errlen-1] (err may be NULL).
  *    No exception crosses this boundary and there is no CPU fallback: without
