@@ -548,6 +548,7 @@ struct __align__(16) TileShared {   // stage is read as double2 too
   double pv[kTile], v[kTile];
   double stage[kTileStage];
   double red[32];
+  double norm[kSumWarps];   // tile_norm's own: tile_dots follows it without a barrier
   double tn, st, nrm;
 };
 
@@ -661,18 +662,19 @@ __device__ __forceinline__ void tile_dots(const double* M, int ld, int ncols, Ti
   __syncthreads();
 }
 
-// Sum of x[r]^2 in chunk_sum's order, by the first kSumWarps warps; thread 0 stores it.
+// Sum of x[r]^2 in chunk_sum's order, by the first kSumWarps warps; thread 0 stores
+// it, after the last barrier: sh.norm may be written again behind a later one only.
 __device__ __forceinline__ void tile_norm(TileShared& sh, double* out) {
   if (threadIdx.x < kTile) {
     const double x = sh.x[threadIdx.x];
     const double s = warp_sum(x * x);
-    if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = s;
+    if ((threadIdx.x & 31) == 0) sh.norm[threadIdx.x >> 5] = s;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
 #pragma unroll
-    for (int i = 0; i < kSumWarps; ++i) t += sh.red[i];
+    for (int i = 0; i < kSumWarps; ++i) t += sh.norm[i];
     *out = t;
   }
 }
