@@ -1137,7 +1137,11 @@ struct UpdateArgs {
   int coef_len;       // doubles before the chunk of S
   unsigned arrived;   // barriers of the earlier launches of this fit
   unsigned* counter;  // arrivals, 32 apart by fit
-  unsigned* stop;     // barrier after which a stopped fit leaves (all ones: none), 32 apart
+  // Where a stopped fit leaves, 32 apart (all ones: nowhere): 2 b at barrier b, 2 b + 1
+  // at the end of the launch whose last barrier was b.  A launch begins on what earlier
+  // launches wrote here, never on the status, which chunk 0 may set before another block
+  // has started: that block would leave without arriving at the first barrier.
+  unsigned* stop;
   int* fail;
   int* host_fail;
 };
@@ -1148,7 +1152,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng 
   extern __shared__ double coef[];   // max(m, K), then the chunk of S
   __shared__ TileShared sh;
   const int f = blockIdx.y, chunk = blockIdx.x;
-  if (e.status[f]) return;   // set by an earlier launch: the same for every block of the fit
+  if (CLUSTER) {
+    if (e.status[f]) return;   // set by an earlier launch: the same for every block of the fit
+  } else if (*(volatile unsigned*)(g.stop + 32 * f) <= 2 * g.arrived + 1) {
+    return;
+  }
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
   double* Sg = e.S + (size_t)f * e.p * e.m + b;
@@ -1165,9 +1173,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng 
     }
     ++arrived;
     __syncthreads();
-    if (chunk == 0 && threadIdx.x == 0 && e.status[f] != 0) *(volatile unsigned*)(g.stop + 32 * f) = arrived;
+    if (chunk == 0 && threadIdx.x == 0 && e.status[f] != 0) *(volatile unsigned*)(g.stop + 32 * f) = 2 * arrived;
     if (!counted_barrier(g.counter + 32 * f, arrived * gridDim.x, g.fail, g.host_fail)) return false;
-    return *(volatile unsigned*)(g.stop + 32 * f) > arrived;
+    return *(volatile unsigned*)(g.stop + 32 * f) > 2 * arrived;
   };
   if (a >= 0) {
     tile_loading<THREADS, true>(e, w, a, f, chunk, sh);
@@ -1202,7 +1210,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng 
   __syncthreads();
   const double nrm = sh.nrm;
   if (!(nrm > 0.0) || !isfinite(nrm)) {
-    if (chunk == 0 && threadIdx.x == 0) e.status[f] = 1;
+    if (chunk == 0 && threadIdx.x == 0) {
+      e.status[f] = 1;
+      if (!CLUSTER) *(volatile unsigned*)(g.stop + 32 * f) = 2 * arrived + 1;
+    }
     return;
   }
   const double sgn = y0 >= 0.0 ? -1.0 : 1.0;
