@@ -1136,7 +1136,7 @@ constexpr size_t kUpdateSmem = 208 * 1024;   // dynamic, beside the static array
 struct UpdateArgs {
   int coef_len;       // doubles before the chunk of S
   unsigned arrived;   // barriers of the earlier launches of this fit
-  unsigned* counter;  // arrivals, 32 apart by fit
+  unsigned* counter;  // arrivals, 32 apart by fit (counted form)
   // Where a stopped fit leaves, 32 apart (all ones: nowhere): 2 b at barrier b, 2 b + 1
   // at the end of the launch whose last barrier was b.  A launch begins on what earlier
   // launches wrote here, never on the status, which chunk 0 may set before another block
@@ -1152,29 +1152,26 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng 
   extern __shared__ double coef[];   // max(m, K), then the chunk of S
   __shared__ TileShared sh;
   const int f = blockIdx.y, chunk = blockIdx.x;
-  if (CLUSTER) {
-    if (e.status[f]) return;   // set by an earlier launch: the same for every block of the fit
-  } else if (*(volatile unsigned*)(g.stop + 32 * f) <= 2 * g.arrived + 1) {
-    return;
-  }
+  if (*(volatile unsigned*)(g.stop + 32 * f) <= 2 * g.arrived + 1) return;
   int b, en;
   chunk_range(chunk, e.szp, e.p, b, en);
   double* Sg = e.S + (size_t)f * e.p * e.m + b;
   const TileView w{b, en - b, coef + g.coef_len, e.V + (size_t)f * e.p * e.K + b, e.p};
   tile_load<THREADS>(w.S, Sg, e.p, e.m, w.rows);
   unsigned arrived = g.arrived;
-  // all chunks of the fit have finished the phase; false: the fit stopped, or a wait gave up
+  // all chunks of the fit have finished the phase; false: the fit stopped, or a wait
+  // gave up.  Every thread of the fit decides alike, however late it reads: a value
+  // from a later phase is larger.
   auto meet = [&]() {
-    if (CLUSTER) {
-      asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-      // a block that sees the status of the phase after this one leaves early: in
-      // that phase every block of the fit finds the same sum and does nothing
-      return *(volatile int*)(e.status + f) == 0;
-    }
     ++arrived;
-    __syncthreads();
+    if (!CLUSTER) __syncthreads();
     if (chunk == 0 && threadIdx.x == 0 && e.status[f] != 0) *(volatile unsigned*)(g.stop + 32 * f) = 2 * arrived;
-    if (!counted_barrier(g.counter + 32 * f, arrived * gridDim.x, g.fail, g.host_fail)) return false;
+    if (CLUSTER) {
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else if (!counted_barrier(g.counter + 32 * f, arrived * gridDim.x, g.fail, g.host_fail)) {
+      return false;
+    }
     return *(volatile unsigned*)(g.stop + 32 * f) > 2 * arrived;
   };
   if (a >= 0) {
@@ -1212,7 +1209,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng 
   if (!(nrm > 0.0) || !isfinite(nrm)) {
     if (chunk == 0 && threadIdx.x == 0) {
       e.status[f] = 1;
-      if (!CLUSTER) *(volatile unsigned*)(g.stop + 32 * f) = 2 * arrived + 1;
+      *(volatile unsigned*)(g.stop + 32 * f) = 2 * arrived + 1;
     }
     return;
   }
@@ -1607,13 +1604,13 @@ void simpls_batch_run(const SimplsBatch& b) {
     }
     if (fits) {
       up.kernel = k;
+      unsigned* ctl = ar.alloc_n<unsigned>(32 * (2 * F + 1));   // each on a line of its own
+      FPLS_CUDA(cudaMemsetAsync(ctl, 0xff, 32 * F * sizeof(unsigned), st));
+      up.args.stop = ctl;
       if (!up.cluster) {
-        unsigned* ctl = ar.alloc_n<unsigned>(32 * (2 * F + 1));   // each on a line of its own
-        FPLS_CUDA(cudaMemsetAsync(ctl, 0, 32 * (F + 1) * sizeof(unsigned), st));
-        FPLS_CUDA(cudaMemsetAsync(ctl + 32 * (F + 1), 0xff, 32 * F * sizeof(unsigned), st));
-        up.args.counter = ctl;
-        up.args.fail = reinterpret_cast<int*>(ctl + 32 * F);
-        up.args.stop = ctl + 32 * (F + 1);
+        FPLS_CUDA(cudaMemsetAsync(ctl + 32 * F, 0, 32 * (F + 1) * sizeof(unsigned), st));
+        up.args.counter = ctl + 32 * F;
+        up.args.fail = reinterpret_cast<int*>(ctl + 32 * 2 * F);
         up.args.host_fail = ctx.host_fail;
       }
     }

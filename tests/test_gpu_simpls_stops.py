@@ -1,6 +1,6 @@
 """A fit that stops in the launch of the phases between the products: in the loading (||t|| overflows), in the
-deflation (||v|| overflows), and in the next refresh (nothing is left to fit), on chunks that count their
-arrivals in memory."""
+deflation (||v|| overflows), and in the next refresh (nothing is left to fit), on chunks that form a cluster and
+on chunks that count their arrivals in memory."""
 import numpy as np
 import pytest
 
@@ -34,7 +34,7 @@ def _one_direction(p):
 
 # the component count is known beforehand: none, none and one
 @pytest.mark.parametrize("make,count", [(_overflowing_scores, 0), (_overflowing_loading, 0), (_one_direction, 1)])
-@pytest.mark.parametrize("p", [2049, 5003])   # 9 and 20 chunks
+@pytest.mark.parametrize("p", [259, 2048, 2049, 5003])   # 2 and 8 chunks (clusters), 9 and 20
 def test_stopped_fit(lib, make, count, p):
     X, Y = make(p)
     for _ in range(3):   # launch by launch, then as a graph
