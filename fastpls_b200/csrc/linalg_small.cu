@@ -748,19 +748,25 @@ jacobi_apply_log_kernel(int l, const double2* __restrict__ log, const int* __res
 // The rotations of one-sided Jacobi depend on the columns' inner products only,
 // and those of A = Q R are those of R; so A is reduced to its c x c triangle by
 // Householder QR over row blocks (one CTA a block, the blocks' triangles stacked
-// and reduced again), the sweeps run on R, and U = A V / s is one product.
-// A sweep over A itself moves its columns three times through shared (or global)
-// memory: 375 x 22 took 340 us that way, 5000 x 22 several ms.
+// and reduced again) and the sweeps run on R.  A sweep over A itself moves its
+// columns three times through shared (or global) memory: 375 x 22 took 340 us
+// that way, 5000 x 22 several ms.  U = Q (R V / s): the rotated columns R V are
+// orthogonal to rounding whatever their lengths, and the reflectors keep them so.
+// (U = A V / s, one product, loses orthogonality as 1 / s, and a NaN of A reaches
+// every column.)
 constexpr int kThinMax = 96;
 
 // R (c x c, upper) of rows [b rb, b rb + rb) of A into rows [b c, b c + c) of
 // out.  Every warp works out the reflector of a column for itself and applies it
-// to its own columns, so a column costs one barrier.
+// to its own columns, so a column costs one barrier.  The reflectors I - tau v v^T
+// stay in F (rows x c, v from the diagonal down) and tau (c a block).
 __global__ void __launch_bounds__(512) qr_block_kernel(const double* __restrict__ A, int rows, int c, int lda, int rb,
-                                                       double* __restrict__ out, int ldo) {
+                                                       double* __restrict__ out, int ldo, double* __restrict__ F,
+                                                       double* __restrict__ tau) {
   extern __shared__ double sm[];
   double* X = sm;                       // [rb][c], column-major
   double* diag = sm + (size_t)rb * c;   // [c]
+  double* heads = diag + c;             // [c]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int r0 = blockIdx.x * rb, nr = min(rb, rows - r0), steps = min(c, nr);
   for (int j = warp; j < c; j += nw)
@@ -773,9 +779,13 @@ __global__ void __launch_bounds__(512) qr_block_kernel(const double* __restrict_
     sigma = warp_sum(sigma);
     const double alpha = x[j], norm = sqrt(alpha * alpha + sigma);
     const double beta = alpha >= 0.0 ? -norm : norm, head = alpha - beta;
-    if (threadIdx.x == 0) diag[j] = beta;
+    const double inv = norm > 0.0 ? 1.0 / (norm * (norm + fabs(alpha))) : 0.0;   // 2 / v.v, v = (head, x below)
+    if (threadIdx.x == 0) {
+      diag[j] = beta;
+      heads[j] = head;
+      tau[blockIdx.x * c + j] = inv;
+    }
     if (norm > 0.0) {
-      const double inv = 1.0 / (norm * (norm + fabs(alpha)));   // 2 / v.v, v = (head, x below)
       for (int col = j + 1 + warp; col < c; col += nw) {
         double* y = X + col * rb;
         double d = 0.0;
@@ -788,20 +798,75 @@ __global__ void __launch_bounds__(512) qr_block_kernel(const double* __restrict_
     }
     __syncthreads();
   }
-  for (int j = warp; j < c; j += nw)
+  for (int j = warp; j < c; j += nw) {
     for (int i = lane; i < c; i += 32) {
       const double v = i < j ? (i < nr ? X[i + j * rb] : 0.0) : i == j && j < steps ? diag[j] : 0.0;
       out[blockIdx.x * c + i + (size_t)j * ldo] = v;
     }
+    if (j < steps)
+      for (int i = j + lane; i < nr; i += 32) F[r0 + i + (size_t)j * rows] = i == j ? heads[j] : X[i + j * rb];
+  }
 }
 
+// Rows [b rb, b rb + rb) of Z (rows x need) = the block's reflectors applied to rows
+// [b c, b c + c) of Y, zero below.  One warp a column, its rows in registers and
+// the next reflector on its way, no barriers: a reflector is a load of L2 that is
+// there, a shuffle tree and two passes over the registers.
+constexpr int kApplyCols = 8;   // columns (warps) a CTA
+template <int NE>               // 32 NE rows at least
+__global__ void __launch_bounds__(32 * kApplyCols)
+qr_apply_kernel(const double* __restrict__ F, const double* __restrict__ tau, int rows, int c, int rb,
+                const double* __restrict__ Y, int ldy, int need, double* __restrict__ Z, int ldz) {
+  const int lane = threadIdx.x & 31, col = blockIdx.y * kApplyCols + (threadIdx.x >> 5);
+  if (col >= need) return;   // whole warps; no barrier below
+  const int b = blockIdx.x, r0 = b * rb, nr = min(rb, rows - r0), steps = min(c, nr);
+  double z[NE], v[NE], next[NE];
+#pragma unroll
+  for (int e = 0; e < NE; ++e) z[e] = lane + 32 * e < steps ? Y[(size_t)b * c + lane + 32 * e + (size_t)col * ldy] : 0.0;
+  auto fetch = [&](int j, double (&d)[NE]) {
+    const double* f = F + r0 + (size_t)max(j, 0) * rows;
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int i = lane + 32 * e;
+      d[e] = j >= 0 && i >= j && i < nr ? __ldg(f + i) : 0.0;
+    }
+  };
+  fetch(steps - 1, v);
+  for (int j = steps - 1; j >= 0; --j) {
+    fetch(j - 1, next);
+    const double t = __ldg(tau + (size_t)b * c + j);
+    double d = 0.0;
+#pragma unroll
+    for (int e = 0; e < NE; ++e) d = fma(v[e], z[e], d);
+    d = warp_sum(d) * t;
+    if (t != 0.0) {   // a column without a reflector (zero, or not a number)
+#pragma unroll
+      for (int e = 0; e < NE; ++e) z[e] -= d * v[e];
+    }
+#pragma unroll
+    for (int e = 0; e < NE; ++e) v[e] = next[e];
+  }
+#pragma unroll
+  for (int e = 0; e < NE; ++e)
+    if (lane + 32 * e < nr) Z[r0 + lane + 32 * e + (size_t)col * ldz] = z[e];
+}
+
+// A column whose norm is below this share of the columns' root mean square is a
+// null direction: its angle to the others is rounding, which no rotation removes,
+// so a rank-deficient matrix (every centred class response) would only stop when
+// the column has underflowed.  A sweep takes such a column down by about eps, so
+// it is there after two; values above this share are resolved.
+__host__ __device__ inline double null_share(int c) { return (4.0 * kEps * c) * (4.0 * kEps * c); }
+
 // One-sided Jacobi on R (c x c, column-major), one CTA, one warp a column pair,
-// the pairs turning as in the symmetric solver: singular values and V,
-// descending.  A column of R and the one of V below it sit in NE registers a
-// lane each while their rotation is worked out.
+// the pairs turning as in the symmetric solver: singular values, and of V and of
+// R V / s the first `need` columns, descending (R V / s: c x need; zero where s is
+// at most tol_rel of the largest).  A column of R and the one of V below it sit in
+// NE registers a lane each while their rotation is worked out.
 template <int NE>
-__global__ void __launch_bounds__(1024) jacobi_core_kernel(const double* __restrict__ R, int c, int max_sweeps, double null_rel,
-                                                           double* __restrict__ s_out, double* __restrict__ V_out) {
+__global__ void __launch_bounds__(1024)
+jacobi_core_kernel(const double* __restrict__ R, int c, int max_sweeps, double tol_rel, int need, double* __restrict__ s_out,
+                   double* __restrict__ V_out, int ldv, double* __restrict__ RV_out) {
   extern __shared__ double sm[];
   double* W = sm;                       // [c][c]
   double* V = W + c * c;
@@ -817,11 +882,7 @@ __global__ void __launch_bounds__(1024) jacobi_core_kernel(const double* __restr
     V[t] = t % c == t / c ? 1.0 : 0.0;
     fro += w * w;
   }
-  // A column below this squared norm is a null direction (U's column is
-  // replaced): its angle to the others is rounding, which no rotation removes,
-  // so a rank-deficient matrix (every centred class response) would never
-  // converge.
-  const double null2 = block_sum(fro, scratch) / c * null_rel * null_rel;
+  const double null2 = block_sum(fro, scratch) / c * null_share(c) * null_share(c);
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
@@ -874,27 +935,24 @@ __global__ void __launch_bounds__(1024) jacobi_core_kernel(const double* __restr
   }
   __syncthreads();
   for (int k = warp; k < c; k += nw) {   // rank of column k, then its place in the outputs
-    const double v = isnan(norms[k]) ? -INFINITY : norms[k];
+    const double sk = norms[k], v = isnan(sk) ? -INFINITY : sk;
     int rank = 0;
+    double top = -INFINITY;
     for (int j = lane; j < c; j += 32) {
       const double w = isnan(norms[j]) ? -INFINITY : norms[j];
       rank += (w > v) || (w == v && j < k);
+      top = fmax(top, w);
     }
     rank = __reduce_add_sync(0xffffffffu, rank);
-    if (lane == 0) s_out[rank] = norms[k];
-    for (int i = lane; i < c; i += 32) V_out[i + rank * c] = V[i + k * c];
-  }
-}
-
-// U[:, j] /= s[j] where s[j] is no null direction (else zero; completed below).
-__global__ void scale_left_kernel(double* U, int rows, int c, int ldu, const double* __restrict__ s, double tol_rel) {
-  const double tol = tol_rel * s[0];
-  const int j = blockIdx.y;
-  const double sj = s[j];
-  const bool ok = sj > tol && sj > 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
-    double* u = U + i + (size_t)j * ldu;
-    *u = ok ? *u / sj : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane == 0) s_out[rank] = sk;
+    if (rank >= need) continue;
+    const bool ok = sk > tol_rel * top && sk > 0.0;
+    for (int i = lane; i < c; i += 32) {
+      V_out[i + (size_t)rank * ldv] = V[i + k * c];
+      RV_out[i + rank * c] = ok ? W[i + k * c] / sk : 0.0;
+    }
   }
 }
 
@@ -916,7 +974,7 @@ __global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* 
   double null2 = 0.0;   // as in jacobi_core_kernel
   for (int j = warp; j < c; j += nwarps)
     for (int i = lane; i < r; i += 32) null2 += W[i + (size_t)j * r] * W[i + (size_t)j * r];
-  null2 = block_sum(null2, scratch0) / c * (kEps * r) * (kEps * r);
+  null2 = block_sum(null2, scratch0) / c * null_share(c) * null_share(c);
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
@@ -1144,24 +1202,49 @@ void eig_sym_desc(int l, const double* G, int ldg, double* evals, double* V, int
 
 namespace {
 
+// One level of the reduction: the reflectors of nb blocks of rb rows.
+struct QrLevel {
+  double *F, *tau;
+  int rows, rb, nb;
+};
+
 // R of A (rows x c, lda) by blocks of rows until one block holds it all.
-const double* reduce_to_triangle(const double* A, int rows, int c, int lda) {
+const double* reduce_to_triangle(const double* A, int rows, int c, int lda, std::vector<QrLevel>& levels) {
   Context& ctx = Context::get();
-  const int rb_max = std::min(512, static_cast<int>((200 * 1024 / sizeof(double) - c) / c));
-  static const bool once = (allow_smem(qr_block_kernel, 201 * 1024), true);
+  const int rb_max = std::min(512, static_cast<int>((200 * 1024 / sizeof(double) - 2 * c) / c));
+  static const bool once = (allow_smem(qr_block_kernel, 200 * 1024), true);
   (void)once;
   while (true) {
     // blocks of 256 rows (three times the columns, at least) keep the first pass on many SMs
     const int rb = rows <= rb_max ? rows : std::min(rb_max, std::max(256, 3 * c));
     const int nb = ceil_div(rows, rb);
     double* out = ctx.arena.alloc_n<double>((size_t)nb * c * c);
-    const size_t smem = ((size_t)rb * c + c) * sizeof(double);
-    qr_block_kernel<<<nb, 512, smem, ctx.stream>>>(A, rows, c, lda, rb, out, nb * c); ::fpls::note_launch();
+    const QrLevel level{ctx.arena.alloc_n<double>((size_t)rows * c), ctx.arena.alloc_n<double>((size_t)nb * c), rows, rb, nb};
+    const size_t smem = ((size_t)rb * c + 2 * c) * sizeof(double);
+    qr_block_kernel<<<nb, 512, smem, ctx.stream>>>(A, rows, c, lda, rb, out, nb * c, level.F, level.tau); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
+    levels.push_back(level);
     if (nb == 1) return out;
     A = out;
     rows = nb * c;
     lda = rows;
+  }
+}
+
+// Z (rows x need, ldz) = Q Y for the Q of the levels, Y c x need.
+void apply_reflectors(const std::vector<QrLevel>& levels, int c, const double* Y, int need, double* Z, int ldz) {
+  Context& ctx = Context::get();
+  int ldy = c;
+  for (size_t l = levels.size(); l-- > 0;) {
+    const QrLevel& q = levels[l];
+    double* out = l == 0 ? Z : ctx.arena.alloc_n<double>((size_t)q.rows * need);
+    const int ldo = l == 0 ? ldz : q.rows;
+    const dim3 grid(q.nb, ceil_div(need, kApplyCols));
+    auto kernel = q.rb <= 64 ? qr_apply_kernel<2> : q.rb <= 256 ? qr_apply_kernel<8> : qr_apply_kernel<16>;
+    kernel<<<grid, 32 * kApplyCols, 0, ctx.stream>>>(q.F, q.tau, q.rows, c, q.rb, Y, ldy, need, out, ldo); ::fpls::note_launch();
+    FPLS_CHECK_LAUNCH();
+    Y = out;
+    ldy = ldo;
   }
 }
 
@@ -1198,25 +1281,22 @@ void svd_thin(int rows, int cols, const double* A, int lda, double* U, int ldu, 
     FPLS_CHECK_LAUNCH();
     return;
   }
-  const double* R = reduce_to_triangle(M, r, c, ldm);
-  double* Vs = ctx.arena.alloc_n<double>((size_t)c * c);
-  const double tol_rel = kEps * static_cast<double>(r);
+  std::vector<QrLevel> levels;
+  const double* R = reduce_to_triangle(M, r, c, ldm, levels);
+  double* RV = ctx.arena.alloc_n<double>((size_t)c * need);
+  double* left = tall ? U : V;    // M's side
+  const int ldl = tall ? ldu : ldv;
   const size_t smem = (2 * (size_t)c * c + c) * sizeof(double);
   const int threads = 32 * std::min(32, std::max(4, (c + 1) / 2));
   auto core = c <= 32 ? jacobi_core_kernel<1> : c <= 64 ? jacobi_core_kernel<2> : jacobi_core_kernel<3>;
   static const bool once = (allow_smem(jacobi_core_kernel<1>, 160 * 1024), allow_smem(jacobi_core_kernel<2>, 160 * 1024),
                             allow_smem(jacobi_core_kernel<3>, 160 * 1024), true);
   (void)once;
-  core<<<1, threads, smem, ctx.stream>>>(R, c, 60, tol_rel, s, Vs); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
-  double* left = tall ? U : V;    // M's side
-  const int ldl = tall ? ldu : ldv;
-  copy_matrix(tall ? V : U, tall ? ldv : ldu, Vs, c, c, need);
-  gemm(false, false, r, need, c, 1.0, M, ldm, Vs, c, 0.0, left, ldl);
-  scale_left_kernel<<<dim3(std::min(ceil_div(r, 256), 64), need), 256, 0, ctx.stream>>>(left, r, need, ldl, s, tol_rel);
+  core<<<1, threads, smem, ctx.stream>>>(R, c, 60, kEps * static_cast<double>(r), need, s, tall ? V : U, tall ? ldv : ldu, RV);
   ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
-  complete_null_columns(r, need, s, 1e-4, left, ldl);
+  apply_reflectors(levels, c, RV, need, left, ldl);
+  complete_null_columns(r, need, s, left, ldl);
 }
 
 }  // namespace fpls

@@ -40,9 +40,8 @@ void svd_thin(int rows, int cols, const double* A, int lda, double* U, int ldu, 
               double* V, int ldv, int need);
 
 // Columns j < cols of U (L rows) whose s[j] is negligible against s[0]: unit
-// vectors made orthogonal to the columns before them; columns whose s[j] is
-// below weak_rel s[0]: made orthogonal to them as they are.
-void complete_null_columns(int L, int cols, const double* s, double weak_rel, double* U, int ldu);
+// vectors made orthogonal to the columns before them.
+void complete_null_columns(int L, int cols, const double* s, double* U, int ldu);
 
 // Same contract as svd_thin, computed by a cooperative one-sided Jacobi over
 // the whole GPU (one CTA per column pair, grid barrier per round); for

@@ -27,7 +27,6 @@ struct CoopJacobi {
   int* flag;           // set when a barrier wait gives up
   int* sweeps;         // sweeps run
   double tol;
-  const double* null2; // squared norm at and below which a column is a null direction
   int max_sweeps;
 };
 
@@ -102,7 +101,6 @@ __device__ __forceinline__ double block_sum3(double& a, double& b, double& c, do
 __global__ void __launch_bounds__(kCoopThreads) jacobi_coop_kernel(CoopJacobi J) {
   __shared__ double red[kCoopThreads / 32][3];
   const int npairs = J.ne / 2;
-  const double null2 = *J.null2;
   for (int sweep = 0; sweep < J.max_sweeps; ++sweep) {
     if (blockIdx.x == 0 && threadIdx.x == 0) J.rot[(sweep + 1) % 3] = 0u;
     for (int rd = 0; rd < J.ne - 1; ++rd) {
@@ -120,8 +118,6 @@ __global__ void __launch_bounds__(kCoopThreads) jacobi_coop_kernel(CoopJacobi J)
           ga += x * y;
         }
         block_sum3(al, be, ga, red);
-        // null directions (replaced at the end) only ever hold rounding
-        if (fmin(al, be) <= null2) continue;
         if (!(ga != 0.0) || !(fabs(ga) > J.tol * sqrt(al) * sqrt(be))) continue;
         const double zeta = (be - al) / (2.0 * ga);
         double t;
@@ -162,16 +158,6 @@ __global__ void identity_kernel(double* W, int r) {
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
        t += (size_t)gridDim.x * blockDim.x)
     W[t] = (t % r == t / r) ? 1.0 : 0.0;
-}
-
-// (eps L)^2 of the mean squared column norm of M (L x r); one CTA.
-__global__ void null_norm_kernel(const double* __restrict__ M, int L, int r, double* __restrict__ out) {
-  __shared__ double scratch[32];
-  double s = 0.0;
-  for (size_t t = threadIdx.x; t < (size_t)L * r; t += blockDim.x) s += M[t] * M[t];
-  s = block_sum(s, scratch);
-  const double e = 2.220446049250313e-16 * L;
-  if (threadIdx.x == 0) *out = s / r * e * e;
 }
 
 __global__ void transpose_into_kernel(const double* __restrict__ A, int rows, int cols, int lda,
@@ -253,35 +239,23 @@ __device__ double orthogonal_to_first(double* u, int L, const double* U, int ldu
 
 // Negligible singular values: complete the L-dimensional side with unit
 // vectors made orthogonal to the columns before them, as the single-CTA Jacobi
-// does.  Weak ones (below weak_rel of the largest, where U's column is a product
-// A v / s whose rounding grows by 1 / s) are made orthogonal as they are.  One
-// CTA; nothing to do when there are none.
-__global__ void complete_null_kernel(int L, int r, int cols, const double* __restrict__ s, double weak_rel, double* U,
-                                     int ldu) {
+// does.  One CTA; nothing to do when there are none.
+__global__ void complete_null_kernel(int L, int r, int cols, const double* __restrict__ s, double* U, int ldu) {
   __shared__ double scratch[32];
   const double smax = s[0];
   const double tol = 2.220446049250313e-16 * (double)(L > r ? L : r) * smax;
   for (int j = 0; j < cols; ++j) {
-    const bool null = !(s[j] > tol && s[j] > 0.0);
-    if (!null && s[j] >= weak_rel * smax) continue;
+    if (s[j] > tol && s[j] > 0.0) continue;
     double* uj = U + (size_t)j * ldu;
-    // candidates: the column as it is (when weak), the unit vectors that keep half
-    // their length, then any that keeps its share (one does: the squared lengths
-    // left of all unit vectors add up to the dimensions left)
-    bool done = false;
-    for (int e = null ? 0 : -1; e < 2 * L && !done; ++e) {
-      double nn = 0.0;
-      if (e < 0) {
-        for (int i = threadIdx.x; i < L; i += blockDim.x) nn += uj[i] * uj[i];
-        nn = sqrt(block_sum(nn, scratch));
-        if (!(nn > 0.0) || !isfinite(nn)) continue;
-        for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] /= nn;
-      } else {
-        for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] = (i == e % L) ? 1.0 : 0.0;
-      }
+    // candidates: the unit vectors that keep half their length, then any that
+    // keeps its share (one does: the squared lengths left of all unit vectors add
+    // up to the dimensions left)
+    for (int e = 0; e < 2 * L; ++e) {
+      for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] = (i == e % L) ? 1.0 : 0.0;
       __syncthreads();
-      nn = orthogonal_to_first(uj, L, U, ldu, j, scratch);
-      if (nn > (e < 0 ? 1e-4 : e < L ? 0.25 : 0.5 / L)) {
+      const double nn = orthogonal_to_first(uj, L, U, ldu, j, scratch);
+      if (!isfinite(nn)) break;   // a column before it is not finite, and none of the candidates would be
+      if (nn > (e < L ? 0.25 : 0.5 / L)) {
         const double inv = 1.0 / sqrt(nn);
         for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] *= inv;
         __syncthreads();
@@ -290,7 +264,7 @@ __global__ void complete_null_kernel(int L, int r, int cols, const double* __res
           for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] /= sqrt(n2);
           __syncthreads();
         }
-        done = true;
+        break;
       }
     }
   }
@@ -333,11 +307,7 @@ void svd_jacobi_coop(int rows, int cols, const double* A, int lda, double* U, in
   const int blocks_needed = ne / 2;
   const int grid = std::max(1, std::min(blocks_needed, max_blocks_per_sm * ctx.sm_count));
 
-  double* null2 = ctx.arena.alloc_n<double>(1);
-  null_norm_kernel<<<1, 1024, 0, ctx.stream>>>(M, L, r, null2); ::fpls::note_launch();
-  FPLS_CHECK_LAUNCH();
   CoopJacobi J;
-  J.null2 = null2;
   J.M = M;
   J.W = W;
   J.L = L;
@@ -365,12 +335,12 @@ void svd_jacobi_coop(int rows, int cols, const double* A, int lda, double* U, in
   rank_desc_kernel<<<ceil_div(r, 128), 128, 0, ctx.stream>>>(nrm, r, order); ::fpls::note_launch();
   write_svd_kernel<<<dim3(std::max(1, std::min(ceil_div(L, 256), 8)), r), 256, 0, ctx.stream>>>(
       M, W, L, r, nrm, order, tall, U, ldu, s, V, ldv); ::fpls::note_launch();
-  complete_null_kernel<<<1, 512, 0, ctx.stream>>>(L, r, r, s, 0.0, tall ? U : V, tall ? ldu : ldv); ::fpls::note_launch();
+  complete_null_kernel<<<1, 512, 0, ctx.stream>>>(L, r, r, s, tall ? U : V, tall ? ldu : ldv); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 
-void complete_null_columns(int L, int cols, const double* s, double weak_rel, double* U, int ldu) {
-  complete_null_kernel<<<1, 512, 0, Context::get().stream>>>(L, cols, cols, s, weak_rel, U, ldu); ::fpls::note_launch();
+void complete_null_columns(int L, int cols, const double* s, double* U, int ldu) {
+  complete_null_kernel<<<1, 512, 0, Context::get().stream>>>(L, cols, cols, s, U, ldu); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 
