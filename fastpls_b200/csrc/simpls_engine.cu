@@ -983,8 +983,11 @@ struct LoopArgs {
 // slots spent on predicated-off loads (1024 threads: 48 us a component).
 constexpr int kLoopThreads = 256;
 constexpr int kLoopWarps = kLoopThreads / 32;
-constexpr size_t kLoopSmem = 208 * 1024;             // beside the static arrays
-constexpr long long kBarrierClocks = 4000000000ll;   // about two seconds
+constexpr size_t kLoopSmem = 208 * 1024;   // beside the static arrays
+// Looks at a counter before a wait gives up: some seconds of a running grid.  Looks,
+// not clock cycles: a grid whose GPU is lent to another process for a while goes on
+// afterwards.
+constexpr int kBarrierLooks = 1 << 23;
 
 // `count` CTAs in all have arrived at *counter (CTAs of one cooperative launch);
 // false when a wait ran out, in every thread of every CTA sooner or later.
@@ -994,13 +997,12 @@ __device__ bool counted_barrier(unsigned* counter, unsigned count, int* fail, in
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(counter, 1u);
-    const long long t0 = clock64();
     ok = 1;
-    while (true) {
+    for (int looks = 0;; ++looks) {
       unsigned seen;
       asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
       if (seen >= count) break;
-      if (*(volatile int*)fail || clock64() - t0 > kBarrierClocks) {
+      if (*(volatile int*)fail || looks > kBarrierLooks) {
         atomicExch(fail, 1);
         *(volatile int*)host_fail = 1;
         ok = 0;
