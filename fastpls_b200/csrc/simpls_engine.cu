@@ -1239,6 +1239,21 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_update(Eng 
   }
 }
 
+// What the driver may refuse: a grid that has to be resident, or a cluster (another
+// process's share of the GPU, a partition of it).  FASTPLS_TEST_REFUSE_FROM=k (tests
+// only): from the k-th such launch of a fit on, none is made.
+bool launch_accepted(const cudaLaunchConfig_t& cfg, const void* kernel, void** args, int& made) {
+  const char* from = std::getenv("FASTPLS_TEST_REFUSE_FROM");
+  if (from && from[0] && made >= std::atoi(from)) return false;
+  if (cudaLaunchKernelExC(&cfg, kernel, args) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  ++made;
+  ::fpls::note_launch();
+  return true;
+}
+
 // The launch of k_update for one engine: which kernel, and its shared memory.
 struct UpdateLaunch {
   const void* kernel = nullptr;   // null: separate launches
@@ -1247,8 +1262,12 @@ struct UpdateLaunch {
   int threads = 0;
   size_t smem = 0;
   UpdateArgs args{};
+  int made = 0;
 
-  void run(const Eng& e, int a, int next, cudaStream_t st) {
+  // False, with nothing done, when the driver refuses it: separate launches from here
+  // on (S, V, R and the vectors between the phases are theirs in memory).
+  bool run(const Eng& e, int a, int next, cudaStream_t st) {
+    if (!kernel) return false;
     args.arrived = a < 0 ? 0u : (unsigned)(1 + e.iters) + (unsigned)a * (3 + e.iters);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -1269,8 +1288,8 @@ struct UpdateLaunch {
     cfg.numAttrs = 1;
     Eng ec = e;
     void* argv[] = {&ec, &args, &a, &next};
-    FPLS_CUDA(cudaLaunchKernelExC(&cfg, kernel, argv));
-    ::fpls::note_launch();
+    if (!launch_accepted(cfg, kernel, argv, made)) kernel = nullptr;
+    return kernel != nullptr;
   }
 };
 
@@ -1579,11 +1598,20 @@ void simpls_batch_run(const SimplsBatch& b) {
       return true;
     }();
     (void)once;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::min(std::max(want, e.cp), ctx.sm_count));
+    cfg.blockDim = dim3(kLoopThreads);
+    cfg.dynamicSmemBytes = loop_smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     void* args[] = {&g};
-    FPLS_CUDA(cudaLaunchCooperativeKernel((const void*)simpls_loop_kernel, dim3(std::min(std::max(want, e.cp), ctx.sm_count)),
-                                          dim3(kLoopThreads), args, loop_smem, st));
-    ::fpls::note_launch();
-    return;   // a wait that gave up ends the call with an error (Context::end_call)
+    int made = 0;
+    // a wait that gave up ends the call with an error (Context::end_call)
+    if (launch_accepted(cfg, (const void*)simpls_loop_kernel, args, made)) return;
   }
   // The phases between the products in one launch, where a chunk's S fits shared
   // memory and the chunks form a cluster or are all resident (the count of blocks
@@ -1625,14 +1653,13 @@ void simpls_batch_run(const SimplsBatch& b) {
   const bool eligible = simpls_graph_enabled() && !trace && !ctx.profile && !shard_red;
   const bool graph = eligible && simpls_seen().count(key) > 0;
   auto loop = [&]() {
-  if (up.kernel) {
-    up.run(e, -1, 1, st);
-  } else {
+  bool refreshed = up.run(e, -1, 1, st);
+  if (!refreshed) {
     k_refresh_start<<<gp, tm, 0, st>>>(e); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
   }
   for (int a = 0; a < b.K; ++a) {
-    if (!up.kernel) {
+    if (!refreshed) {
       // Refresh: y <- S (S^T y) `iters` times from the warm start, then normalise.
       double* zin = e.zA;
       double* zout = e.zB;
@@ -1670,8 +1697,8 @@ void simpls_batch_run(const SimplsBatch& b) {
       FPLS_CHECK_LAUNCH();
     }
     mark("X^T*T");
-    if (up.kernel) {
-      up.run(e, a, a + 1 < b.K ? 1 : 0, st);
+    refreshed = up.run(e, a, a + 1 < b.K ? 1 : 0, st);
+    if (refreshed) {
       mark("update");
       continue;
     }
