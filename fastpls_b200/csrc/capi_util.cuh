@@ -21,31 +21,21 @@ inline void set_err(char* err, size_t errlen, const char* msg) {
 template <typename Fn>
 int guarded(char* err, size_t errlen, Fn&& fn) {
   if (err && errlen) err[0] = '\0';
-  // Kernels of a call that leaves early may still read the caller's matrices:
-  // they end before the error is returned.
-  auto settle = [] {
-    try {
-      Context& ctx = Context::get();
-      cudaStreamSynchronize(ctx.stream);
-      cudaStreamSynchronize(ctx.side);
-    } catch (...) {   // no device
-    }
-  };
   try {
     fn();
     Context::get().end_call();
     return FPLS_OK;
   } catch (const Error& e) {
     set_err(err, errlen, e.what());
-    settle();
+    Context::settle();
     return e.code;
   } catch (const std::exception& e) {
     set_err(err, errlen, e.what());
-    settle();
+    Context::settle();
     return FPLS_ERR_INTERNAL;
   } catch (...) {
     set_err(err, errlen, "fastpls_b200: unknown internal error");
-    settle();
+    Context::settle();
     return FPLS_ERR_INTERNAL;
   }
 }

@@ -1,9 +1,11 @@
 #include "context.cuh"
 
 #include <algorithm>
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
+#include <thread>
 
 namespace fpls {
 
@@ -53,8 +55,13 @@ void Arena::release() {
   blocks_.clear();
 }
 
-Context& Context::get() {
+Context& Context::instance() {
   static Context ctx;
+  return ctx;
+}
+
+Context& Context::get() {
+  Context& ctx = instance();
   if (ctx.device < 0) {
     int n = 0;
     cudaError_t e = cudaGetDeviceCount(&n);
@@ -118,6 +125,17 @@ void Context::end_call() {
   FPLS_CUDA(cudaEventElapsedTime(&ms, call_start, call_stop));
   last_call_ms = ms;
   if (*static_cast<volatile int*>(host_fail)) throw Error(kErrCuda, "a grid barrier wait exceeded its limit");
+}
+
+void Context::settle() {
+  Context& ctx = instance();
+  if (!ctx.call_started) return;
+  ctx.call_started = false;
+  const auto limit = std::chrono::steady_clock::now() + std::chrono::seconds(2);
+  for (cudaStream_t st : {ctx.stream, ctx.side})
+    while (cudaStreamQuery(st) == cudaErrorNotReady && std::chrono::steady_clock::now() < limit)
+      std::this_thread::sleep_for(std::chrono::microseconds(20));
+  cudaGetLastError();
 }
 
 int Context::read_status() {

@@ -92,8 +92,13 @@ struct Context {
   RowShards* shards = nullptr;
 
   static Context& get();       // initialises the device on first use
+  static Context& instance();  // as it is
   void begin_call();           // resets the arena and the status flag, starts the call timer
   void end_call();             // stops the call timer (after the final synchronisation)
+  // A call that leaves early: waits for its kernels, which may still read the caller's
+  // matrices, but for two seconds at most (a collective of a row-sharded fit may never
+  // end).  Nothing when no call has begun.
+  static void settle();
   int read_status();           // synchronises the stream and reads the flag
   void sync();
   void release();
