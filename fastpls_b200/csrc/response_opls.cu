@@ -354,12 +354,14 @@ int fpls_opls_apply_filter(const double* X, int w, int p, const double* mX, cons
     ctx.begin_call();
     const MatrixSource sX(X, false, (size_t)w * p);
     double* dX = filtered_storage(Xf, sX, (size_t)w * p, sX, (size_t)w * p);
+    // every input is copied before the first write: dX may be the caller's output, and
+    // that may be memory that held one of them
     const double* dm = upload(mX, p);
     const double* dv = upload(vX, p);
+    const double* dW = upload(W_orth, (size_t)p * north);
+    const double* dP = upload(P_orth, (size_t)p * north);
     center_scale(sX.f64(), dX, w, p, dm, dv);
     if (north > 0) {
-      const double* dW = upload(W_orth, (size_t)p * north);
-      const double* dP = upload(P_orth, (size_t)p * north);
       double* t = ctx.arena.alloc_n<double>(w);
       for (int a = 0; a < north; ++a) {
         gemv(false, w, p, 1.0, dX, w, dW + (size_t)a * p, 0.0, t);

@@ -23,6 +23,9 @@
  *    in the reference, whose inputs are R objects in host memory).
  *  - Every function returns 0 on success or a non-zero fpls_status; on failure a
  *    NUL-terminated message is written to err[0..errlen-1] (err may be NULL).
+ *    The outputs of a failed call are not defined: some of them may have been
+ *    written, a filtered X in device memory in part.  Inputs are never written,
+ *    except where an output shares their memory.
  *    No exception crosses this boundary and there is no CPU fallback: without
  *    a B200 the calls return FPLS_ERR_NO_DEVICE.
  *  - The library keeps one device context per process (stream, scratch arena),
