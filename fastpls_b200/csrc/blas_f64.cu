@@ -71,7 +71,11 @@ __global__ void __launch_bounds__(128) gemv_t_kernel(int K, int N, double alpha,
   const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (n >= N) return;
   const int k0 = blockIdx.y * kps;
-  const double acc = gemv_column<kGemvAhead>(A + (size_t)n * lda + k0, x + k0, min(kps, K - k0));
+  const int rows = min(kps, K - k0);
+  const double* col = A + (size_t)n * lda + k0;
+  const double acc = rows <= 32 * 2   ? gemv_column<2>(col, x + k0, rows)
+                     : rows <= 32 * 8 ? gemv_column<8>(col, x + k0, rows)
+                                      : gemv_column<kGemvAhead>(col, x + k0, rows);
   y += blockIdx.y * stride;
   if ((threadIdx.x & 31) == 0) y[n] = (beta == 0.0) ? alpha * acc : alpha * acc + beta * y[n];
 }
@@ -84,20 +88,26 @@ __global__ void __launch_bounds__(128) gemv_t_kernel(int K, int N, double alpha,
 constexpr int kColWarps = 4;   // 768 columns fill the SMs in blocks of four
 constexpr int kColAhead = 48;
 
-template <typename T, typename F>
-__device__ __forceinline__ double lane_column_sum(const T* __restrict__ x, int n, F term) {
+template <int AHEAD, typename T, typename F>
+__device__ __forceinline__ double lane_sum_ahead(const T* __restrict__ x, int n, F term) {
   double s = 0.0;
   int i = threadIdx.x & 31;
-  for (; i < n; i += 32 * kColAhead) {
-    T v[kColAhead];
+  for (; i < n; i += 32 * AHEAD) {
+    T v[AHEAD];
 #pragma unroll
-    for (int u = 0; u < kColAhead; ++u)
+    for (int u = 0; u < AHEAD; ++u)
       if (i + 32 * u < n) v[u] = __ldg(x + i + 32 * u);
 #pragma unroll
-    for (int u = 0; u < kColAhead; ++u)
+    for (int u = 0; u < AHEAD; ++u)
       if (i + 32 * u < n) s += term(static_cast<double>(v[u]));
   }
   return warp_sum(s);
+}
+
+// A short column would pass 48 bounds for its one to eight loads.
+template <typename T, typename F>
+__device__ __forceinline__ double lane_column_sum(const T* __restrict__ x, int n, F term) {
+  return n <= 32 * 8 ? lane_sum_ahead<8>(x, n, term) : lane_sum_ahead<kColAhead>(x, n, term);
 }
 
 __device__ __forceinline__ int warp_column() { return blockIdx.x * kColWarps + (threadIdx.x >> 5); }
@@ -153,30 +163,30 @@ __global__ void div_vec_kernel(const double* __restrict__ in, size_t count, doub
 }
 
 // dst[:, j] = (src[:, j] - mean[j]) / scale[j] (mean or scale may be null), both
-// n x p with ld n, src FP32 or FP64 and possibly dst itself.  A block takes 2048
-// rows of a column, eight loads a thread in flight, no index divisions:
+// n x p with ld n, src FP32 or FP64 and possibly dst itself.  A thread takes eight
+// rows (RowTiles) of a column, its loads in flight together, no index divisions:
 // 20000 x 5000 from FP32 in one pass instead of a copy, a widening and a centring one.
-constexpr int kCenterRows = 2048;
 template <typename T>
-__global__ void __launch_bounds__(256) center_scale_kernel(const T* src, double* dst, int n, int p,
+__global__ void __launch_bounds__(256) center_scale_kernel(const T* src, double* dst, int n, int p, RowTiles tiles,
                                                            const double* __restrict__ mean,
                                                            const double* __restrict__ scale) {
-  const int i0 = blockIdx.x * kCenterRows + threadIdx.x;
-  for (int j = blockIdx.y; j < p; j += gridDim.y) {
+  const int tx = 1 << tiles.log_rows, i0 = blockIdx.x * 8 * tx + (threadIdx.x & (tx - 1));
+  const int cols = 256 >> tiles.log_rows;
+  for (int j = blockIdx.y * cols + (threadIdx.x >> tiles.log_rows); j < p; j += gridDim.y * cols) {
     const T* x = src + (size_t)j * n;
     double* y = dst + (size_t)j * n;
     T v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      if (i0 + 256 * u < n) v[u] = x[i0 + 256 * u];
+      if (i0 + tx * u < n) v[u] = x[i0 + tx * u];
     const double m = mean ? mean[j] : 0.0, sc = scale ? scale[j] : 1.0;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      if (i0 + 256 * u < n) {
+      if (i0 + tx * u < n) {
         double w = static_cast<double>(v[u]);
         if (mean) w -= m;
         if (scale) w /= sc;
-        y[i0 + 256 * u] = w;
+        y[i0 + tx * u] = w;
       }
     }
   }
@@ -600,8 +610,8 @@ namespace {
 template <typename T>
 void center_scale_run(const T* src, double* dst, int n, int p, const double* mean, const double* scale) {
   if ((size_t)n * p == 0) return;
-  const dim3 grid(ceil_div(n, kCenterRows), std::min(p, 65535));
-  center_scale_kernel<T><<<grid, 256, 0, Context::get().stream>>>(src, dst, n, p, mean, scale); ::fpls::note_launch();
+  const RowTiles t(n);
+  center_scale_kernel<T><<<t.grid(n, p), 256, 0, Context::get().stream>>>(src, dst, n, p, t, mean, scale); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 }  // namespace

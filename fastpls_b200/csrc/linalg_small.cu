@@ -1,6 +1,7 @@
 #include "blas_f64.cuh"
 #include "context.cuh"
 #include "linalg_small.cuh"
+#include "null_columns.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -956,8 +957,9 @@ jacobi_core_kernel(const double* __restrict__ R, int c, int max_sweeps, double t
   }
 }
 
-// More columns than kThinMax: W (r x c, r >= c) is overwritten in global memory,
-// V (c x c) accumulates the rotations; one CTA, one warp a pair.
+// More columns than kThinMax, or so few that the launches of the reduction are the
+// time (kDirect below): W (r x c, r >= c) is overwritten in global memory, V (c x c)
+// accumulates the rotations; one CTA, one warp a pair.
 __global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* W, double* V, int max_sweeps,
                                   double* U_out, int ldu, double* s_out, double* V_out, int ldv,
                                   int transpose_out) {
@@ -971,10 +973,13 @@ __global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int t = threadIdx.x; t < c * c; t += blockDim.x) V[t] = (t % c == t / c) ? 1.0 : 0.0;
   __syncthreads();
-  double null2 = 0.0;   // as in jacobi_core_kernel
-  for (int j = warp; j < c; j += nwarps)
-    for (int i = lane; i < r; i += 32) null2 += W[i + (size_t)j * r] * W[i + (size_t)j * r];
-  null2 = block_sum(null2, scratch0) / c * null_share(c) * null_share(c);
+  double null2 = -1.0;   // as in jacobi_core_kernel; four columns underflow in a few sweeps
+  if (c > 4) {
+    double fro = 0.0;
+    for (int j = warp; j < c; j += nwarps)
+      for (int i = lane; i < r; i += 32) fro += W[i + (size_t)j * r] * W[i + (size_t)j * r];
+    null2 = block_sum(fro, scratch0) / c * null_share(c) * null_share(c);
+  }
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
@@ -1044,32 +1049,7 @@ __global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* 
       for (int i = threadIdx.x; i < r; i += blockDim.x) uj[i] = W[i + (size_t)src * r] / sj;
       __syncthreads();
     } else {
-      // Complete with a unit vector orthogonal to the earlier columns.
-      for (int e = 0; e < r; ++e) {
-        for (int i = threadIdx.x; i < r; i += blockDim.x) uj[i] = (i == e) ? 1.0 : 0.0;
-        __syncthreads();
-        for (int pass = 0; pass < 2; ++pass) {
-          for (int jj = 0; jj < j; ++jj) {
-            const double* uo = transpose_out ? V_out + (size_t)jj * ldv : U_out + (size_t)jj * ldu;
-            __shared__ double scratch[32];
-            double d = 0.0;
-            for (int i = threadIdx.x; i < r; i += blockDim.x) d += uo[i] * uj[i];
-            d = block_sum(d, scratch);
-            for (int i = threadIdx.x; i < r; i += blockDim.x) uj[i] -= d * uo[i];
-            __syncthreads();
-          }
-        }
-        __shared__ double scratch2[32];
-        double nn = 0.0;
-        for (int i = threadIdx.x; i < r; i += blockDim.x) nn += uj[i] * uj[i];
-        nn = block_sum(nn, scratch2);
-        if (nn > 0.25) {
-          const double inv = 1.0 / sqrt(nn);
-          for (int i = threadIdx.x; i < r; i += blockDim.x) uj[i] *= inv;
-          __syncthreads();
-          break;
-        }
-      }
+      complete_null_column(r, j, transpose_out ? V_out : U_out, transpose_out ? ldv : ldu, scratch0);
     }
     for (int i = threadIdx.x; i < c; i += blockDim.x) vj[i] = V[i + (size_t)src * c];
     __syncthreads();
@@ -1259,8 +1239,13 @@ void svd_thin(int rows, int cols, const double* A, int lda, double* U, int ldu, 
   const int c = tall ? cols : rows;
   const double* M = A;   // the tall form, r x c
   int ldm = lda;
+  // up to four columns of little work a sweep in one launch, against four or six:
+  // 2000 x 1: 10 against 25 us, 2000 x 2: 24 against 30, 4000 x 2: 37 against 30,
+  // 512 x 4: 35 against 35
+  constexpr int kDirect = 8192;
+  const bool direct = c > kThinMax || (c <= 4 && (long long)r * c * c <= kDirect);
   double* W = nullptr;
-  if (!tall || c > kThinMax) {
+  if (!tall || direct) {
     W = ctx.arena.alloc_n<double>((size_t)r * c);
     if (tall) {
       copy_matrix(W, r, A, lda, rows, cols);
@@ -1273,7 +1258,7 @@ void svd_thin(int rows, int cols, const double* A, int lda, double* U, int ldu, 
   }
   // tall: U (rows x c) is M's side, V (cols x c) the rotations.
   // wide: A^T = U' S V'^T, so U (rows x c) <- V', V (cols x c) <- U'.
-  if (c > kThinMax) {
+  if (direct) {
     double* Vw = ctx.arena.alloc_n<double>((size_t)c * c);
     const size_t lists = (size_t)(c + (c + 1) / 2) * sizeof(double);
     jacobi_svd_kernel<<<1, 1024, lists, ctx.stream>>>(r, c, W, Vw, 60, U, ldu, s, V, ldv, tall ? 0 : 1);

@@ -5,6 +5,7 @@
 // cross-covariance of label-aware PLSSVD, which the reference hands to
 // LAPACK gesdd through R's svd()).
 #include "linalg_small.cuh"
+#include "null_columns.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -219,24 +220,6 @@ __global__ void write_svd_kernel(const double* __restrict__ M, const double* __r
     wdst[t] = W[t + (size_t)src * r];
 }
 
-// Makes u (L entries) orthogonal to the first j columns of U, two Gram-Schmidt
-// passes, and returns its squared norm; one CTA.
-__device__ double orthogonal_to_first(double* u, int L, const double* U, int ldu, int j, double* scratch) {
-  for (int pass = 0; pass < 2; ++pass) {
-    for (int jj = 0; jj < j; ++jj) {
-      const double* uo = U + (size_t)jj * ldu;
-      double d = 0.0;
-      for (int i = threadIdx.x; i < L; i += blockDim.x) d += uo[i] * u[i];
-      d = block_sum(d, scratch);
-      for (int i = threadIdx.x; i < L; i += blockDim.x) u[i] -= d * uo[i];
-      __syncthreads();
-    }
-  }
-  double nn = 0.0;
-  for (int i = threadIdx.x; i < L; i += blockDim.x) nn += u[i] * u[i];
-  return block_sum(nn, scratch);
-}
-
 // Negligible singular values: complete the L-dimensional side with unit
 // vectors made orthogonal to the columns before them, as the single-CTA Jacobi
 // does.  One CTA; nothing to do when there are none.
@@ -244,30 +227,8 @@ __global__ void complete_null_kernel(int L, int r, int cols, const double* __res
   __shared__ double scratch[32];
   const double smax = s[0];
   const double tol = 2.220446049250313e-16 * (double)(L > r ? L : r) * smax;
-  for (int j = 0; j < cols; ++j) {
-    if (s[j] > tol && s[j] > 0.0) continue;
-    double* uj = U + (size_t)j * ldu;
-    // candidates: the unit vectors that keep half their length, then any that
-    // keeps its share (one does: the squared lengths left of all unit vectors add
-    // up to the dimensions left)
-    for (int e = 0; e < 2 * L; ++e) {
-      for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] = (i == e % L) ? 1.0 : 0.0;
-      __syncthreads();
-      const double nn = orthogonal_to_first(uj, L, U, ldu, j, scratch);
-      if (!isfinite(nn)) break;   // a column before it is not finite, and none of the candidates would be
-      if (nn > (e < L ? 0.25 : 0.5 / L)) {
-        const double inv = 1.0 / sqrt(nn);
-        for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] *= inv;
-        __syncthreads();
-        if (nn <= 0.25) {   // more length was lost: once more
-          const double n2 = orthogonal_to_first(uj, L, U, ldu, j, scratch);
-          for (int i = threadIdx.x; i < L; i += blockDim.x) uj[i] /= sqrt(n2);
-          __syncthreads();
-        }
-        break;
-      }
-    }
-  }
+  for (int j = 0; j < cols; ++j)
+    if (!(s[j] > tol && s[j] > 0.0)) complete_null_column(L, j, U, ldu, scratch);
 }
 
 }  // namespace

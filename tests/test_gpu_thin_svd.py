@@ -8,7 +8,8 @@ EPS = np.finfo(np.float64).eps
 
 
 # one block of rows, several, and a last block of fewer rows than columns; columns per lane 1, 2 and 3; wide
-@pytest.mark.parametrize("rows,cols", [(30, 8), (375, 22), (8, 8), (515, 3), (22, 375), (70, 64), (2000, 90), (1000, 96)])
+@pytest.mark.parametrize("rows,cols", [(30, 8), (375, 22), (8, 8), (515, 3), (22, 375), (70, 64), (2000, 90), (1000, 96), (2048, 2), (2049, 2), (512, 4),
+                                       (4, 4), (3, 513), (8193, 1)])
 @pytest.mark.parametrize("decay", [0.8, 0.5, 0.1])
 def test_vectors_of_small_values_are_orthogonal(lib, rows, cols, decay):
     rng = np.random.default_rng(rows + cols)
@@ -36,3 +37,12 @@ def test_a_nan_stays_in_its_column(lib):
     assert np.isfinite(got["u"]).all() and np.max(np.abs(got["u"].T @ got["u"] - np.eye(12))) < 144 * EPS
     assert np.max(np.abs(got["d"][:11] - want)) < 144 * EPS * want[0]
     assert np.isnan(got["d"][11])
+
+
+@pytest.mark.parametrize("n", [2, 4, 5, 16])   # one launch, and QR first
+def test_null_direction_with_equal_entries(lib, n):
+    """The direction left over keeps 1 / n of every unit vector's squared length."""
+    P = np.eye(n) - np.full((n, n), 1.0 / n)
+    got = lib.truncated_svd(P, n, svd_method=3)
+    assert np.max(np.abs(got["u"].T @ got["u"] - np.eye(n))) < 12 * n * EPS
+    assert np.max(np.abs(got["d"] - np.r_[np.ones(n - 1), 0.0])) < 12 * n * EPS
