@@ -166,13 +166,13 @@ __global__ void div_vec_kernel(const double* __restrict__ in, size_t count, doub
 // n x p with ld n, src FP32 or FP64 and possibly dst itself.  A thread takes eight
 // rows (RowTiles) of a column, its loads in flight together, no index divisions:
 // 20000 x 5000 from FP32 in one pass instead of a copy, a widening and a centring one.
-template <typename T>
+template <typename T, int LOG>   // LOG: the tiles' log_rows, or -1
 __global__ void __launch_bounds__(256) center_scale_kernel(const T* src, double* dst, int n, int p, RowTiles tiles,
                                                            const double* __restrict__ mean,
                                                            const double* __restrict__ scale) {
-  const int tx = 1 << tiles.log_rows, i0 = blockIdx.x * 8 * tx + (threadIdx.x & (tx - 1));
-  const int cols = 256 >> tiles.log_rows;
-  for (int j = blockIdx.y * cols + (threadIdx.x >> tiles.log_rows); j < p; j += gridDim.y * cols) {
+  const int log_rows = LOG < 0 ? tiles.log_rows : LOG, tx = 1 << log_rows, cols = 256 >> log_rows;
+  const int i0 = blockIdx.x * 8 * tx + (threadIdx.x & (tx - 1));
+  for (int j = blockIdx.y * cols + (threadIdx.x >> log_rows); j < p; j += gridDim.y * cols) {
     const T* x = src + (size_t)j * n;
     double* y = dst + (size_t)j * n;
     T v[8];
@@ -295,48 +295,72 @@ int split_count(int tiles, int K, int sm_count) {
 
 struct GemmPlan { int nt, splits, kps; };
 
-// Tile width and K ranges by modelled time.  An SM's FP64 tensor pipe takes
-// 8 nt cycles a contraction step and tile whatever shares it, so the time is
-// that of the SM with the most tiles; the tiles' operands come from L2 at about
-// 2900 bytes a clock (all SMs), partials are written, read and summed once more.  Products below 2^28
-// multiply-adds keep the ranges of split_count (only their width is chosen):
-// they are over in tens of microseconds, and iterations that feed the split
-// precisions need their last bits unchanged.  50000 x 768 x 100 (S = X^T Y):
-// 551 us on 64 x 64 tiles in 13 ranges (312 tiles on 148 SMs).
-GemmPlan plan_gemm(int M, int N, int K, int sm_count) {
-  const double steps_min = 8 * kBK;
+// 16-byte copies need both operands' columns on 16-byte boundaries
+bool wide_copies(const double* A, int lda, const double* B, int ldb) {
+  auto aligned = [](const double* p, int ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 2 == 0; };
+  return aligned(A, lda) && aligned(B, ldb);
+}
+
+// Tile width and K ranges by modelled time: the time of the SM with the most tiles.  A
+// tile takes 8 nt cycles of the FP64 tensor pipe a contraction step; the tiles' operands
+// come from L2 at some 3000 bytes a clock (all SMs); partials are written, read and summed
+// once more.  Two estimates.  The plain one lets the pipe run at 95 per cent under
+// several CTAs and at 85 under one; the other takes the rates that CTAs of each width
+// and layout were measured to reach together (gemm64::kRate; one alone reaches half), in
+// rounds of the CTAs that an SM holds.  The plain choice stands unless the measured
+// rates put another one 7 per cent ahead: what they cannot tell apart, they rank by
+// their own error (208 products: 6 per cent faster on average than the plain choice, 4
+// of them more than 3 per cent slower; by the rates alone, 29).
+// Products below 2^28 multiply-adds keep the ranges of split_count (only their width is
+// chosen): they are over in tens of microseconds, and iterations that feed the split
+// precisions need their last bits unchanged.  50000 x 768 x 100 (S = X^T Y): 551 us
+// on 64 x 64 tiles in 13 ranges (312 tiles on 148 SMs), 361 us now; 20001 x 100 over
+// 1001, A transposed: 238 us on those tiles, 288 by the plain choice, 179 now.
+GemmPlan plan_gemm(bool ta, bool tb, bool wide, int M, int N, int K, int sm_count) {
   const bool large = static_cast<double>(M) * N * K >= 268435456.0;
   const int base = split_count(ceil_div(M, kBM) * ceil_div(N, 64), K, sm_count);
-  const int smax = large ? std::max(1, std::min(64, static_cast<int>(K / steps_min))) : base;
-  GemmPlan best{8, base, 0};
-  double best_cost = 1e300;
-  for (int nt : gemm64::kWidths) {
-    const long long tiles = (long long)ceil_div(M, kBM) * ceil_div(N, 8 * nt);
-    if (ceil_div(N, 8 * nt) > 65535) continue;
+  const int smax = large ? std::max(1, std::min(64, K / (8 * kBK))) : base;
+  GemmPlan plain{8, base, 0}, best{8, base, 0};
+  double plain_cost = 1e300, plain_measured = 0.0, best_measured = 1e300;
+  for (int i = 0; i < 9; ++i) {
+    const int nt = gemm64::kWidths[i], columns = nt == gemm64::kStaged ? 64 : 8 * nt;
+    if (ceil_div(N, columns) > 65535) continue;
+    const unsigned char* rate = gemm64::kRate[4 * ta + 2 * tb + !wide][i];
+    const double tiles = static_cast<double>(ceil_div(M, kBM)) * ceil_div(N, columns);
+    const int resident = gemm64::resident_ctas(ta, tb, nt);
     for (int want = large ? 1 : base; want <= smax; ++want) {
-      const int kps = ceil_div(ceil_div(K, want), kBK) * kBK, splits = ceil_div(K, kps);
-      const double units = static_cast<double>(tiles) * splits, waves = std::ceil(units / sm_count);
-      // a tile alone: its tensor time at the pace one warp a scheduler holds, plus
-      // its first loads and its stores, which the SM's other tiles hide
-      const double work = kps * 8.0 * nt, alone = work / 0.85 + 4000.0;
-      const double resident = std::min(waves, nt >= 13 ? 2.0 : nt >= 8 ? 3.0 : 4.0);
-      const double bytes = units * kps * (kBM + 8.0 * nt) * 8.0;
-      double cost = std::max(waves * std::max(work / 0.95, alone / resident), bytes / 2900.0);
-      if (splits > 1) cost += 3000.0 + (2.0 * splits + 1.0) * M * N * 8.0 / 2900.0;
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = GemmPlan{nt, splits, kps};
+      const GemmPlan plan{nt, 0, ceil_div(ceil_div(K, want), kBK) * kBK};
+      const int splits = ceil_div(K, plan.kps);
+      const double units = tiles * splits, waves = std::ceil(units / sm_count), work = static_cast<double>(plan.kps) * columns;
+      const double bytes = units * plan.kps * (kBM + columns) * 8.0, sums = (2.0 * splits + 1.0) * M * N * 8.0;
+      const int together = static_cast<int>(std::min<double>(waves, resident));
+      const double rounds = std::floor(waves / together);
+      const int rest = static_cast<int>(waves - rounds * together);
+      // 400 cycles a tile before its first products (the staged kernel has none to fill)
+      double measured = 100.0 * work * (rounds * together / rate[together - 1] + (rest ? static_cast<double>(rest) / rate[rest - 1] : 0.0));
+      measured = std::max(measured + (nt == gemm64::kStaged ? 0.0 : 400.0 * waves), bytes / 3800.0);
+      if (splits > 1) measured += 4500.0 + sums / 3600.0;
+      if (measured < best_measured) {
+        best_measured = measured;
+        best = GemmPlan{nt, splits, plan.kps};
+      }
+      if (nt == gemm64::kStaged) continue;
+      const double alone = work / 0.85 + 4000.0, held = std::min(waves, nt >= 13 ? 2.0 : nt >= 8 ? 3.0 : 4.0);
+      double cost = std::max(waves * std::max(work / 0.95, alone / held), bytes / 2900.0);
+      if (splits > 1) cost += 3000.0 + sums / 2900.0;
+      if (cost < plain_cost) {
+        plain_cost = cost;
+        plain_measured = measured;
+        plain = GemmPlan{nt, splits, plan.kps};
       }
     }
   }
-  return best;
+  return best_measured < 0.93 * plain_measured ? best : plain;
 }
 
 void gemm_run(bool transA, bool transB, int nt, const gemm64::Args& g, int splits, cudaStream_t st) {
-  const dim3 grid(ceil_div(g.M, kBM), ceil_div(g.N, 8 * nt), splits);
-  // 16-byte copies need both operands' columns on 16-byte boundaries
-  auto aligned = [](const double* p, int ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 2 == 0; };
-  const bool vec = aligned(g.A, g.lda) && aligned(g.B, g.ldb);
+  const dim3 grid(ceil_div(g.M, kBM), ceil_div(g.N, nt == gemm64::kStaged ? 64 : 8 * nt), splits);
+  const bool vec = wide_copies(g.A, g.lda, g.B, g.ldb);
   if (!transA && !transB) gemm64::launch<false, false>(g, nt, vec, grid, st);
   else if (transA && !transB) gemm64::launch<true, false>(g, nt, vec, grid, st);
   else if (!transA) gemm64::launch<false, true>(g, nt, vec, grid, st);
@@ -353,7 +377,7 @@ Partials gemm_tiles(bool transA, bool transB, int M, int N, int K, double alpha,
                     const double* B, int ldb, double beta, double* C, int ldc, const double* row_add) {
   Context& ctx = Context::get();
   cudaStream_t st = ctx.stream;
-  const GemmPlan plan = plan_gemm(M, N, K, ctx.sm_count);
+  const GemmPlan plan = plan_gemm(transA, transB, wide_copies(A, lda, B, ldb), M, N, K, ctx.sm_count);
   gemm64::Args g{M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, plan.kps, 0, 0, row_add};
   if (plan.splits > 1) {
     g.split_stride = (long long)M * N;
@@ -611,7 +635,8 @@ template <typename T>
 void center_scale_run(const T* src, double* dst, int n, int p, const double* mean, const double* scale) {
   if ((size_t)n * p == 0) return;
   const RowTiles t(n);
-  center_scale_kernel<T><<<t.grid(n, p), 256, 0, Context::get().stream>>>(src, dst, n, p, t, mean, scale); ::fpls::note_launch();
+  auto kernel = t.log_rows == 8 ? center_scale_kernel<T, 8> : center_scale_kernel<T, -1>;
+  kernel<<<t.grid(n, p), 256, 0, Context::get().stream>>>(src, dst, n, p, t, mean, scale); ::fpls::note_launch();
   FPLS_CHECK_LAUNCH();
 }
 }  // namespace

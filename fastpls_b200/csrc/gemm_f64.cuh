@@ -56,10 +56,45 @@ __device__ __forceinline__ void copy_async(double* dst, const double* src, int v
 }
 
 // Fills one tile (MN x kBK); elements outside the operand or the K range read as zero.
+// A thread's copies lie a fixed number of rows (KC) or, where the tile's width divides
+// the threads, of columns apart: one pointer moves on, instead of an address each (with
+// 8-byte copies, odd leading dimensions, the addresses were a third of all
+// instructions).
 template <bool KC, int MN, int V>   // V doubles a copy
 __device__ __forceinline__ void fill_tile(double* S, const double* __restrict__ P, int ld, int mn0, int k0, int limit,
                                           int kend) {
   constexpr int kChunks = MN * kBK / V;
+  if constexpr (!KC && kThreads % (MN / V) == 0 && kChunks >= kThreads) {
+    constexpr int kRow = MN / V, kStep = kThreads / kRow;
+    const int mn = (threadIdx.x % kRow) * V, k = threadIdx.x / kRow, left = limit - (mn0 + mn);
+    const int n = left < 0 ? 0 : left < V ? left : V;
+    const double* src = n ? P + mn0 + mn + (size_t)(k0 + k) * ld : P;
+    const size_t step = n ? (size_t)kStep * ld : 0;
+    double* dst = S + Tile<KC, MN>::at(mn, k);
+    if (k0 + kBK <= kend) {
+#pragma unroll
+      for (int u = 0; u < kBK / kStep; ++u, src += step) copy_async<8 * V>(dst + Tile<KC, MN>::at(0, u * kStep), src, 8 * n);
+    } else {
+#pragma unroll
+      for (int u = 0; u < kBK / kStep; ++u, src += step) {
+        const bool in = k0 + k + u * kStep < kend;
+        copy_async<8 * V>(dst + Tile<KC, MN>::at(0, u * kStep), in ? src : P, in ? 8 * n : 0);
+      }
+    }
+    return;
+  }
+  if (KC && mn0 + MN <= limit) {
+    constexpr int kRow = kBK / V, kStep = kThreads / kRow;
+    const int k = (threadIdx.x % kRow) * V, mn = threadIdx.x / kRow, left = kend - (k0 + k);
+    const int n = left < 0 ? 0 : left < V ? left : V;
+    const double* src = n ? P + (size_t)(mn0 + mn) * ld + k0 + k : P;
+    const size_t step = n ? (size_t)kStep * ld : 0;
+    double* dst = S + Tile<KC, MN>::at(mn, k);
+#pragma unroll
+    for (int u = 0; u < (MN + kStep - 1) / kStep; ++u, src += step)
+      if (MN % kStep == 0 || mn + u * kStep < MN) copy_async<8 * V>(dst + Tile<KC, MN>::at(u * kStep, 0), src, 8 * n);
+    return;
+  }
 #pragma unroll
   for (int t0 = 0; t0 < kChunks; t0 += kThreads) {
     const int t = t0 + threadIdx.x;
@@ -88,10 +123,30 @@ constexpr size_t smem_bytes() {
   return sizeof(double) * kStages<NT> * (Tile<TA, kBM>::kSize + Tile<!TB, 8 * NT>::kSize);
 }
 
+// Entries (m, n) and (m, n + 1) of the result.
+__device__ __forceinline__ void store_pair(const Args& g, int m, int n0, const double (&acc)[2]) {
+  if (m >= g.M) return;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int n = n0 + e;
+    if (n >= g.N) continue;
+    // split-K: each K range stores its own partial (summed in range order
+    // by splitk_reduce_kernel, so runs repeat bit for bit)
+    double* cp = g.C + (size_t)blockIdx.z * g.split_stride + m + (size_t)n * g.ldc;
+    double v = g.alpha * acc[e];
+    if (!g.split_stride && g.beta != 0.0) v += g.beta * *cp;
+    if (g.row_add) v += g.row_add[n];
+    *cp = v;
+  }
+}
+
 // op(A) (m,k): TA ? A[k + m*lda] : A[m + k*lda]   -> K-contiguous when TA
 // op(B) (k,n): TB ? B[n + k*ldb] : B[k + n*ldb]   -> K-contiguous when !TB
+template <int NT>
+constexpr int kResident = NT <= 8 ? 4 : NT <= 10 ? 3 : 2;   // CTAs of an SM, by registers
+
 template <bool TA, bool TB, int NT, int V>
-__global__ void __launch_bounds__(kThreads) gemm_f64_dmma(Args g) {
+__global__ void __launch_bounds__(kThreads, kResident<NT>) gemm_f64_dmma(Args g) {
   extern __shared__ __align__(16) double gemm_sm[];
   constexpr int BN = 8 * NT, S = kStages<NT>;
   using TileA = Tile<TA, kBM>;
@@ -158,29 +213,113 @@ __global__ void __launch_bounds__(kThreads) gemm_f64_dmma(Args g) {
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int m = bm + wm + i * 8 + gid;
-    if (m >= g.M) continue;
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
+    for (int j = 0; j < NT; ++j) store_pair(g, bm + wm + i * 8 + gid, bn + j * 8 + tig * 2, acc[i][j]);
+}
+
+// The same product on 64 x 64 tiles (warps of 32 x 32) whose loads are staged in
+// registers: 8 bytes an instruction whatever the alignment.  Where
+// 64 columns are no padding, above all where only 8-byte copies are allowed, it holds the
+// pace that the asynchronous copies lose (50001 x 60 x 769, A as it is: 198 us against
+// 258).  Sums in the same order.
+template <bool KC>
+__device__ __forceinline__ void staged_load(double (&r)[8], const double* __restrict__ P, int ld, int mn0, int k0, int limit,
+                                            int kend) {
+  const int t = threadIdx.x;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int n = bn + j * 8 + tig * 2 + e;
-        if (n >= g.N) continue;
-        // split-K: each K range stores its own partial (summed in range order
-        // by splitk_reduce_kernel, so runs repeat bit for bit)
-        double* cp = g.C + (size_t)blockIdx.z * g.split_stride + m + (size_t)n * g.ldc;
-        double v = g.alpha * acc[i][j][e];
-        if (!g.split_stride && g.beta != 0.0) v += g.beta * *cp;
-        if (g.row_add) v += g.row_add[n];
-        *cp = v;
-      }
-    }
+  for (int i = 0; i < 8; ++i) {
+    const int k = k0 + (KC ? (t & 15) : (t >> 6) + 2 * i), mn = mn0 + (KC ? (t >> 4) + 8 * i : (t & 63));
+    r[i] = mn < limit && k < kend ? __ldg(KC ? P + (size_t)mn * ld + k : P + mn + (size_t)k * ld) : 0.0;
   }
 }
 
-// Launches the tile kernel of (TA, TB) for 8 nt columns a tile (one of kWidths).
-constexpr int kWidths[] = {1, 2, 4, 5, 7, 8, 10, 13};
+template <bool KC>
+__device__ __forceinline__ void staged_store(double (*S)[kBM + 4], const double (&r)[8]) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) S[KC ? (t & 15) : (t >> 6) + 2 * i][KC ? (t >> 4) + 8 * i : (t & 63)] = r[i];
+}
+
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kThreads) gemm_f64_staged(Args g) {
+  __shared__ double As[2][kBK][kBM + 4], Bs[2][kBK][kBM + 4];
+  const int bm = blockIdx.x * kBM, bn = blockIdx.y * kBM;
+  if (g.upper && bm >= bn + kBM) return;
+  const int kbeg = blockIdx.z * g.k_per_split, kend = min(g.K, kbeg + g.k_per_split);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  double ra[8], rb[8];
+  if (kbeg < kend) {
+    staged_load<TA>(ra, g.A, g.lda, bm, kbeg, g.M, kend);
+    staged_load<!TB>(rb, g.B, g.ldb, bn, kbeg, g.N, kend);
+    staged_store<TA>(As[0], ra);
+    staged_store<!TB>(Bs[0], rb);
+  }
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = kbeg; k0 < kend; k0 += kBK, buf ^= 1) {
+    const bool more = k0 + kBK < kend;
+    if (more) {
+      staged_load<TA>(ra, g.A, g.lda, bm, k0 + kBK, g.M, kend);
+      staged_load<!TB>(rb, g.B, g.ldb, bn, k0 + kBK, g.N, kend);
+    }
+#pragma unroll
+    for (int kk = 0; kk < kBK; kk += 4) {
+      double a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk + tig][wm + i * 8 + gid];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk + tig][wn + j * 8 + gid];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    }
+    if (more) {
+      staged_store<TA>(As[buf ^ 1], ra);
+      staged_store<!TB>(Bs[buf ^ 1], rb);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) store_pair(g, bm + wm + i * 8 + gid, bn + wn + j * 8 + tig * 2, acc[i][j]);
+}
+
+// Tile widths, in 8 columns (kStaged: gemm_f64_staged, 64 columns), and the share of
+// the tensor pipe's rate, in per cent, that an SM reaches with 1, 2, 3 and 4 CTAs of
+// each, by the operands' layouts: A B, A B^T, A^T B, A^T B^T, each with 16-byte and with
+// 8-byte copies (a least-squares fit of 18400 timed products, 8 to 1000 columns, 60 to
+// 400000 rows and contractions, up to 64 K ranges; half of them within 2.5 per cent).
+constexpr int kStaged = 0;
+constexpr int kWidths[] = {kStaged, 1, 2, 4, 5, 7, 8, 10, 13};
+constexpr unsigned char kRate[8][9][4] = {
+    {{47, 74, 84, 80}, {21, 37, 39, 80}, {31, 51, 56, 80}, {44, 78, 76, 80}, {48, 86, 89, 80}, {49, 85, 83, 87}, {56, 81, 81, 87}, {60, 89, 93, 80}, {55, 84, 80, 80}},
+    {{47, 73, 84, 80}, {21, 33, 39, 80}, {29, 46, 49, 80}, {45, 71, 70, 73}, {51, 81, 85, 80}, {58, 87, 87, 93}, {53, 74, 73, 76}, {59, 87, 90, 80}, {63, 86, 80, 80}},
+    {{57, 84, 85, 91}, {22, 35, 37, 80}, {33, 54, 58, 80}, {44, 81, 79, 82}, {47, 81, 80, 84}, {51, 84, 88, 90}, {57, 88, 86, 90}, {60, 88, 92, 80}, {55, 83, 80, 80}},
+    {{57, 84, 85, 91}, {20, 32, 35, 80}, {30, 49, 51, 80}, {43, 77, 76, 77}, {50, 79, 81, 79}, {53, 81, 82, 88}, {56, 87, 83, 86}, {56, 82, 86, 80}, {60, 81, 80, 80}},
+    {{43, 66, 74, 80}, {16, 28, 32, 80}, {30, 53, 53, 80}, {41, 71, 83, 80}, {48, 82, 76, 80}, {52, 87, 92, 80}, {52, 83, 91, 80}, {61, 86, 82, 80}, {55, 85, 80, 80}},
+    {{43, 66, 74, 80}, {21, 24, 25, 80}, {33, 41, 41, 80}, {47, 80, 83, 80}, {47, 67, 66, 80}, {55, 85, 89, 80}, {58, 85, 88, 80}, {54, 72, 73, 80}, {63, 85, 80, 80}},
+    {{52, 74, 78, 86}, {19, 31, 34, 80}, {27, 48, 51, 80}, {40, 70, 83, 80}, {42, 71, 85, 80}, {48, 80, 78, 82}, {59, 89, 83, 85}, {62, 89, 91, 80}, {58, 84, 80, 80}},
+    {{52, 74, 78, 86}, {18, 26, 26, 80}, {31, 38, 40, 80}, {45, 80, 79, 80}, {49, 80, 83, 80}, {53, 80, 81, 87}, {54, 75, 73, 75}, {55, 82, 86, 80}, {59, 80, 80, 80}}};
+
+// CTAs of a width that an SM holds (four at most count), by shared memory and registers.
+inline int resident_ctas(bool ta, bool tb, int nt) {
+  if (nt == kStaged) return tb ? 4 : 3;
+  const int stages = nt <= 2 ? 6 : nt <= 5 ? 4 : 3;
+  const int a = ta ? kBM * (kBK + 4) : kBK * (kBM + 4), b = tb ? kBK * (8 * nt + 4) : 8 * nt * (kBK + 4);
+  const int by_smem = 228 * 1024 / (8 * stages * (a + b) + 1024), by_regs = nt >= 13 ? 2 : nt >= 10 ? 3 : 4;
+  return by_smem < by_regs ? by_smem : by_regs;
+}
+
+// Launches the tile kernel of (TA, TB) for 8 nt columns a tile (one of kWidths, or kStaged).
 template <bool TA, bool TB>
 void launch(const Args& g, int nt, bool vec, dim3 grid, cudaStream_t st);
 
@@ -203,6 +342,7 @@ void launch_width(const Args& g, bool vec, dim3 grid, cudaStream_t st) {
   template <>                                                                        \
   void launch<TA, TB>(const Args& g, int nt, bool vec, dim3 grid, cudaStream_t st) { \
     switch (nt) {                                                                    \
+      case kStaged: gemm_f64_staged<TA, TB><<<grid, kThreads, 0, st>>>(g); break;    \
       case 1: launch_width<TA, TB, 1>(g, vec, grid, st); break;                      \
       case 2: launch_width<TA, TB, 2>(g, vec, grid, st); break;                      \
       case 4: launch_width<TA, TB, 4>(g, vec, grid, st); break;                      \
