@@ -13,8 +13,9 @@
 namespace fpls {
 namespace {
 
-// A thread a row: the loads of a warp are coalesced and one maximum is little to
-// carry.  Bound by reading S (1,000,000 x 12: 15 us).
+// A thread a row: the loads of a warp are coalesced, those of the SM's other warps
+// hide their latency, and one maximum is little to carry.  Bound by reading S
+// (1,000,000 x 12: 15 us).
 __global__ void __launch_bounds__(256) argmax_kernel(const double* __restrict__ S, int w, int C,
                                                      const double* __restrict__ bias, int* __restrict__ labels) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -150,10 +151,11 @@ void lowrank_predict(const double* Xs, int w, int p, const double* R, int kmax, 
 
 void row_argmax(const double* S, int w, int C, const double* bias, int* labels) {
   if (w <= 0) return;
-  // Few classes, or rows enough to fill the GPU: a thread a row (1,000,000 x 3: 6.5 us
-  // against 42 in lists; 100000 x 100: 10.7 against 12.1).  Else several warps share a
-  // row's classes (20000 x 100: 6.6 against 8.5, 3000 x 1000: 8.6 against 53).
-  if (C <= 48 || (C <= 128 && w >= 65536)) {
+  // Rows enough to fill the GPU: a thread a row (1,000,000 x 3: 6.5 us against 42 in
+  // lists; 100000 x 100: 10.7 against 12.1).  Else several warps share a row's classes
+  // (125 x 22: 2.9 us against 4.6, 20000 x 100: 6.6 against 8.5, 3000 x 1000: 8.6
+  // against 53).
+  if (w >= 65536 ? C <= 128 : w >= 16384 ? C <= 48 : C <= 4) {
     argmax_kernel<<<ceil_div(w, 256), 256, 0, Context::get().stream>>>(S, w, C, bias, labels); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     return;

@@ -21,10 +21,9 @@ def _want(row, k):
     return idx, val
 
 
-# one warp a row group below 32 classes, two from there on, four from 64; a block of several groups from
-# 296 blocks on; the argmax by a thread a row up to 48 classes, and up to 128 from 65536 rows on
+# warps that share a row: as many as classes, or one for 8 of them where the rows fill the GPU; the argmax by a thread a row up to 4 classes, 48 from 16384 rows on and 128 from 65536 on
 @pytest.mark.parametrize("m", [2, 5, 15, 31, 32, 48, 49, 63, 64, 128, 129])
-@pytest.mark.parametrize("w", [33, 65535, 75777])
+@pytest.mark.parametrize("w", [33, 16383, 16384, 65535, 75777])
 def test_few_classes(lib, m, w):
     rng = np.random.default_rng(m)
     base = rng.integers(-3, 4, size=m).astype(np.float64)
