@@ -810,54 +810,54 @@ __global__ void __launch_bounds__(512) qr_block_kernel(const double* __restrict_
 }
 
 // Rows [b rb, b rb + rb) of Z (rows x need) = the block's reflectors applied to rows
-// [b c, b c + c) of Y, zero below.  One warp a column, its rows in registers and
-// the next reflector on its way, no barriers: a reflector is a load of L2 that is
-// there, a shuffle tree and two passes over the registers.
+// [b c, b c + c) of Y, zero below.  The reflectors come into shared memory once; one
+// warp a column then, its rows in registers, without barriers: a reflector is a shuffle
+// tree and two passes over the registers (375 x 22: 13 us with each reflector fetched
+// from L2 ahead of its turn).
 constexpr int kApplyCols = 8;   // columns (warps) a CTA
 template <int NE>               // 32 NE rows at least
 __global__ void __launch_bounds__(32 * kApplyCols)
 qr_apply_kernel(const double* __restrict__ F, const double* __restrict__ tau, int rows, int c, int rb,
                 const double* __restrict__ Y, int ldy, int need, double* __restrict__ Z, int ldz) {
-  const int lane = threadIdx.x & 31, col = blockIdx.y * kApplyCols + (threadIdx.x >> 5);
-  if (col >= need) return;   // whole warps; no barrier below
+  extern __shared__ double sm[];   // [rb][c] reflectors, [c] tau
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.y * kApplyCols + warp;
   const int b = blockIdx.x, r0 = b * rb, nr = min(rb, rows - r0), steps = min(c, nr);
-  double z[NE], v[NE], next[NE];
+  double* taus = sm + (size_t)rb * c;
+  for (int j = warp; j < steps; j += kApplyCols) {
+#pragma unroll 8
+    for (int i = lane; i < nr; i += 32) sm[i + j * rb] = i >= j ? F[r0 + i + (size_t)j * rows] : 0.0;
+    if (lane == 0) taus[j] = tau[(size_t)b * c + j];
+  }
+  double z[NE];
 #pragma unroll
-  for (int e = 0; e < NE; ++e) z[e] = lane + 32 * e < steps ? Y[(size_t)b * c + lane + 32 * e + (size_t)col * ldy] : 0.0;
-  auto fetch = [&](int j, double (&d)[NE]) {
-    const double* f = F + r0 + (size_t)max(j, 0) * rows;
-#pragma unroll
-    for (int e = 0; e < NE; ++e) {
-      const int i = lane + 32 * e;
-      d[e] = j >= 0 && i >= j && i < nr ? __ldg(f + i) : 0.0;
-    }
-  };
-  fetch(steps - 1, v);
+  for (int e = 0; e < NE; ++e)
+    z[e] = lane + 32 * e < steps && col < need ? Y[(size_t)b * c + lane + 32 * e + (size_t)col * ldy] : 0.0;
+  __syncthreads();
+  if (col >= need) return;
   for (int j = steps - 1; j >= 0; --j) {
-    fetch(j - 1, next);
-    const double t = __ldg(tau + (size_t)b * c + j);
-    double d = 0.0;
+    const double t = taus[j];
+    double v[NE], part[2] = {0.0, 0.0};   // two chains: a multiply-add waits 16 cycles for the one before
 #pragma unroll
-    for (int e = 0; e < NE; ++e) d = fma(v[e], z[e], d);
-    d = warp_sum(d) * t;
-    if (t != 0.0) {   // a column without a reflector (zero, or not a number)
+    for (int e = 0; e < NE; ++e) v[e] = lane + 32 * e < nr ? sm[lane + 32 * e + j * rb] : 0.0;
 #pragma unroll
-      for (int e = 0; e < NE; ++e) z[e] -= d * v[e];
-    }
+    for (int e = 0; e < NE; ++e) part[e & 1] = fma(v[e], z[e], part[e & 1]);
+    const double d = warp_sum(part[0] + part[1]) * t;
+    if (t == 0.0) continue;   // a column without a reflector (zero, or not a number)
 #pragma unroll
-    for (int e = 0; e < NE; ++e) v[e] = next[e];
+    for (int e = 0; e < NE; ++e) z[e] -= d * v[e];
   }
 #pragma unroll
   for (int e = 0; e < NE; ++e)
     if (lane + 32 * e < nr) Z[r0 + lane + 32 * e + (size_t)col * ldz] = z[e];
 }
 
-// A column whose norm is below this share of the columns' root mean square is a
-// null direction: its angle to the others is rounding, which no rotation removes,
-// so a rank-deficient matrix (every centred class response) would only stop when
-// the column has underflowed.  A sweep takes such a column down by about eps, so
-// it is there after two; values above this share are resolved.
-__host__ __device__ inline double null_share(int c) { return (4.0 * kEps * c) * (4.0 * kEps * c); }
+// A column whose norm is below 4 eps c of the columns' root mean square may be a null
+// direction: its angle to the others is rounding, which no rotation removes, so a
+// rank-deficient matrix (every centred class response) would only stop when the column
+// has underflowed.  Such a column is rotated, which resolves a small singular value and
+// takes a null direction down by eps a sweep, but asks for no further sweep, and is left
+// alone below the square of this share.
+__device__ inline double null_share(int c) { return 4.0 * kEps * c; }
 
 // One-sided Jacobi on R (c x c, column-major), one CTA, one warp a column pair,
 // the pairs turning as in the symmetric solver: singular values, and of V and of
@@ -883,7 +883,8 @@ jacobi_core_kernel(const double* __restrict__ R, int c, int max_sweeps, double t
     V[t] = t % c == t / c ? 1.0 : 0.0;
     fro += w * w;
   }
-  const double null2 = block_sum(fro, scratch) / c * null_share(c) * null_share(c);
+  const double weak2 = block_sum(fro, scratch) / c * null_share(c) * null_share(c);
+  const double null2 = weak2 * null_share(c) * null_share(c);
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
     __syncthreads();
@@ -921,7 +922,7 @@ jacobi_core_kernel(const double* __restrict__ R, int c, int max_sweeps, double t
             V[i + q * c] = t.s * vx[e] + t.c * vy[e];
           }
         }
-        if (lane == 0) rotated = 1;
+        if (lane == 0 && !(fmin(a, b) <= weak2)) rotated = 1;
       }
       __syncthreads();
     }
@@ -973,12 +974,13 @@ __global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int t = threadIdx.x; t < c * c; t += blockDim.x) V[t] = (t % c == t / c) ? 1.0 : 0.0;
   __syncthreads();
-  double null2 = -1.0;   // as in jacobi_core_kernel; four columns underflow in a few sweeps
+  double weak2 = -1.0, null2 = -1.0;   // as in jacobi_core_kernel; four columns underflow in a few sweeps
   if (c > 4) {
     double fro = 0.0;
     for (int j = warp; j < c; j += nwarps)
       for (int i = lane; i < r; i += 32) fro += W[i + (size_t)j * r] * W[i + (size_t)j * r];
-    null2 = block_sum(fro, scratch0) / c * null_share(c) * null_share(c);
+    weak2 = block_sum(fro, scratch0) / c * null_share(c) * null_share(c);
+    null2 = weak2 * null_share(c) * null_share(c);
   }
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     if (threadIdx.x == 0) rotated = 0;
@@ -1010,7 +1012,7 @@ __global__ void __launch_bounds__(1024) jacobi_svd_kernel(int r, int c, double* 
             V[i + (size_t)p * c] = t.c * x - t.s * y;
             V[i + (size_t)q * c] = t.s * x + t.c * y;
           }
-          if (lane == 0) rotated = 1;
+          if (lane == 0 && !(fmin(a, b) <= weak2)) rotated = 1;
         }
       }
       __syncthreads();
@@ -1214,6 +1216,9 @@ const double* reduce_to_triangle(const double* A, int rows, int c, int lda, std:
 // Z (rows x need, ldz) = Q Y for the Q of the levels, Y c x need.
 void apply_reflectors(const std::vector<QrLevel>& levels, int c, const double* Y, int need, double* Z, int ldz) {
   Context& ctx = Context::get();
+  static const bool once = (allow_smem(qr_apply_kernel<2>, 200 * 1024), allow_smem(qr_apply_kernel<8>, 200 * 1024),
+                            allow_smem(qr_apply_kernel<16>, 200 * 1024), true);
+  (void)once;
   int ldy = c;
   for (size_t l = levels.size(); l-- > 0;) {
     const QrLevel& q = levels[l];
@@ -1221,7 +1226,7 @@ void apply_reflectors(const std::vector<QrLevel>& levels, int c, const double* Y
     const int ldo = l == 0 ? ldz : q.rows;
     const dim3 grid(q.nb, ceil_div(need, kApplyCols));
     auto kernel = q.rb <= 64 ? qr_apply_kernel<2> : q.rb <= 256 ? qr_apply_kernel<8> : qr_apply_kernel<16>;
-    kernel<<<grid, 32 * kApplyCols, 0, ctx.stream>>>(q.F, q.tau, q.rows, c, q.rb, Y, ldy, need, out, ldo); ::fpls::note_launch();
+    kernel<<<grid, 32 * kApplyCols, ((size_t)q.rb * c + c) * sizeof(double), ctx.stream>>>(q.F, q.tau, q.rows, c, q.rb, Y, ldy, need, out, ldo); ::fpls::note_launch();
     FPLS_CHECK_LAUNCH();
     Y = out;
     ldy = ldo;
