@@ -602,9 +602,11 @@ knn_tile_kernel_v2(const KnnItem* __restrict__ items, KnnClassInfo ci, const int
 //      5.7e-5 < eps = 2^-14 |x| max|y|.
 // The FP16 form runs first: a third of the MMA work, half the bytes through L2
 // and shared memory, and two CTAs on an SM.  Its wider bar costs a few more
-// exact scores; a class whose similarities to a test row crowd within it fills
-// the candidate slots of a pair, and then the products run again as split BF16,
-// and after that on the FP64 tiles.
+// exact scores.  Where the similarities of a class to a test row crowd within it, the
+// candidate slots of that pair fill up, and then all products of the call run again
+// as split BF16, and after that on the FP64 tiles: 100 scores, 20 classes of 15000
+// rows, spread 0.005: 23.3 ms so, 25.5 with split BF16 first (and 10.7 -> 3.1 ms
+// where the FP16 slots hold).
 // What bounds it: a 128 x 128 tile brings 32 KB out of L2, 16384 values out of
 // TMEM, one max or compare a value, and 128 x 128 x 112 products, each a third
 // to a half of the tile's time; two CTAs overlap them.  1,200,000 training rows
@@ -612,8 +614,8 @@ knn_tile_kernel_v2(const KnnItem* __restrict__ items, KnnClassInfo ci, const int
 // 1.64 ms (1.06 ms is the MMA work of one pass at the measured 1670 TFLOP/s);
 // with split BF16 throughout, a search of the maxima in shared memory and an
 // atomic a hit, one CTA an SM: 5.65 and 7.55 ms.
-// Score rows up to 128 wide, neighbour lists up to 16 long, up to 2^24
-// training rows.  Warp 0 loads (TMA, SWIZZLE_128B boxes of 64 x 128 values:
+// Score rows up to 128 wide, neighbour lists up to 16 long, less than 2^31 padded
+// training rows and pairs.  Warp 0 loads (TMA, SWIZZLE_128B boxes of 64 x 128 values:
 // the A tile once, the B tiles through two stages), warp 1 issues the MMAs,
 // warps 2..9 are the epilogue (two per TMEM lane quarter).  Every mbarrier
 // wait is bounded; no cluster multicast.
@@ -811,8 +813,8 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant
 #pragma unroll
     for (int e = 0; e < kFBuckets; ++e) M[e] = -INFINITY;
     // the rows past np are other pairs' or padding: their maxima are not
-    // written, and no finite value reaches their bar
-    const float thr = (PASS == 2 && row_ok) ? bar[p0 + r] : INFINITY;
+    // written, and nothing reaches a bar that is not a number
+    const float thr = (PASS == 2 && row_ok) ? bar[p0 + r] : __int_as_float(0x7fffffff);
     uint32_t held[2] = {0u, 0u};   // the last tile's hits, not yet written
     int slot = 0, hbase = 0;
     auto write_hits = [&]() {
@@ -984,11 +986,12 @@ knn_half_rows_kernel(const double* __restrict__ S, int rows, int K, const int* _
 // Row i of the BF16 planes (rows_pad x kw, zero padded) = the hi / lo split
 // of row src(i) of S (row-major, K doubles per row): src(i) = pairs[i] % ntest
 // when pairs is given (the test row of class-sorted pair i; slack[i] = 2 eps,
-// rounded up), else i.
+// rounded up), else i.  These planes are not scaled: where |x| max|y| may leave the
+// range of FP32, *flag becomes 2 (the FP64 tiles).
 __global__ void __launch_bounds__(256)
 knn_split_rows_kernel(const double* __restrict__ S, int rows, int K, const int* __restrict__ pairs, int ntest,
                       int rows_pad, int kw, const unsigned* __restrict__ ymax_bits, __nv_bfloat16* __restrict__ hi,
-                      __nv_bfloat16* __restrict__ lo, float* __restrict__ slack) {
+                      __nv_bfloat16* __restrict__ lo, float* __restrict__ slack, int* flag) {
   const int lane = threadIdx.x & 31;
   for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < rows_pad; i += gridDim.x * 8) {
     const double* row = S + (size_t)(i < rows ? (pairs ? pairs[i] % ntest : i) : 0) * K;
@@ -1002,8 +1005,11 @@ knn_split_rows_kernel(const double* __restrict__ S, int rows, int K, const int* 
     }
     if (pairs && i < rows) {
       for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      if (lane == 0)
-        slack[i] = __double2float_ru(ldexp(sqrt(s2) * static_cast<double>(__uint_as_float(*ymax_bits)), -13));
+      if (lane == 0) {
+        const double largest = sqrt(s2) * static_cast<double>(__uint_as_float(*ymax_bits));
+        slack[i] = __double2float_ru(ldexp(largest, -13));
+        if (largest > 1e38) atomicMax(flag, 2);
+      }
     }
   }
 }
@@ -1072,9 +1078,9 @@ knn_filter_bar_kernel(const float* __restrict__ apart, KnnClassInfo ci, int C, l
 #pragma unroll
   for (int e = 1; e < kFList; ++e)
     if (e == use_k - 1) theta = lst[e];
-  // a slack of -inf marks a test row with a NaN: no row reaches its bar
+  // a slack of -inf marks a test row with a NaN: nothing reaches its bar, not a number
   const float sl = slack[P];
-  bar[P] = sl == -INFINITY ? INFINITY : (theta == -INFINITY ? -INFINITY : __fadd_rd(theta, -sl));
+  bar[P] = sl == -INFINITY ? __int_as_float(0x7fffffff) : (theta == -INFINITY ? -INFINITY : __fadd_rd(theta, -sl));
 }
 
 // Exact scores of the candidates of every pair (one warp per class-sorted
@@ -1534,10 +1540,10 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
       __nv_bfloat16* bl = ctx.arena.alloc_n<__nv_bfloat16>((size_t)b_rows * kw);
       dzero(ferr, 2 * sizeof(int));
       knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, kw,
-                                                        ymax, ah, al, slack);
+                                                        ymax, ah, al, slack, ferr + 1);
       ::fpls::note_launch();
       knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, nullptr, 1, (int)b_rows, kw, ymax, bh,
-                                                        bl, nullptr);
+                                                        bl, nullptr, nullptr);
       ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
       pt.mark("filter planes");
