@@ -167,9 +167,9 @@ class DeviceMatrix:
     """A column-major FP64 matrix already in device memory, taken from any
     object exposing __cuda_array_interface__ (for instance the transpose of a
     contiguous torch CUDA tensor).  The matrix entry points accept it for X, Y,
-    Xtest, the response and the filtered-X output: the library then copies
-    within HBM instead of across PCIe (the C ABI tells host and device
-    pointers apart by unified addressing)."""
+    Xtest, the response and the filtered-X output: the library then reads it
+    where it lies, and never writes to an input (the C ABI tells host and
+    device pointers apart by unified addressing)."""
 
     def __init__(self, obj, allow_f32=False):
         cai = obj.__cuda_array_interface__
