@@ -600,13 +600,14 @@ knn_tile_kernel_v2(const KnnItem* __restrict__ items, KnnClassInfo ci, const int
 //      2^-18 |x| and drops terms below 3 2^-18 |x||y| in all (1.2e-5 |x||y|),
 //      the accumulation of 3 x 128 products loses at most 4.6e-5 |x||y|;
 //      5.7e-5 < eps = 2^-14 |x| max|y|.
-// The FP16 form runs first: a third of the MMA work, half the bytes through L2
-// and shared memory, and two CTAs on an SM.  Its wider bar costs a few more
+// In large calls the FP16 form runs first: a third of the MMA work, half the bytes
+// through L2 and shared memory, and two CTAs on an SM.  Its wider bar costs more
 // exact scores.  Where the similarities of a class to a test row crowd within it, the
-// candidate slots of that pair fill up, and then all products of the call run again
-// as split BF16, and after that on the FP64 tiles: 100 scores, 20 classes of 15000
-// rows, spread 0.005: 23.3 ms so, 25.5 with split BF16 first (and 10.7 -> 3.1 ms
-// where the FP16 slots hold).
+// candidate slots of that pair fill up: pass 2 raises a flag, at which the CTAs that
+// start later and the exact scores return at once, and all products of the call run
+// again as split BF16, and after that on the FP64 tiles.  2 classes of 15000 rows of
+// 128 scores, spread 0.01, 5000 test rows: 1455 us with every FP16 candidate scored,
+// 665 with the flag.
 // What bounds it: a 128 x 128 tile brings 32 KB out of L2, 16384 values out of
 // TMEM, one max or compare a value, and 128 x 128 x 112 products, each a third
 // to a half of the tile's time; two CTAs overlap them.  1,200,000 training rows
@@ -687,7 +688,8 @@ __global__ void __launch_bounds__(kFThreads, FilterTile<PLANES>::kCtas)
 knn_filter_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ CUtensorMap mA1,
                   const __grid_constant__ CUtensorMap mB0, const __grid_constant__ CUtensorMap mB1,
                   const KnnItem* __restrict__ items, KnnClassInfo ci, int K, int use_k, float* __restrict__ apart,
-                  const float* __restrict__ bar, int* __restrict__ ccount, int* __restrict__ crow, int* err) {
+                  const float* __restrict__ bar, int* __restrict__ ccount, int* __restrict__ crow, int* err,
+                  int* inexact) {
   using Tile = FilterTile<PLANES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -709,6 +711,8 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant
   const int r0 = ci.row_offs[c] + it.chunk * ci.chunk_rows[c];
   const int r1 = min(ci.row_offs[c + 1], r0 + ci.chunk_rows[c]);
   const int ntiles = (r1 - r0 + kFT - 1) / kFT;
+  // the lists of this form are known not to be exact: another form follows
+  if (PASS == 2 && __syncthreads_or(threadIdx.x == 0 && *(volatile int*)inexact != 0)) return;
   const int nbox = (K + 63) / 64;        // 64-wide boxes a plane holds
   const int ksteps = (K + 15) / 16;      // columns past K are zero: their steps add nothing
 
@@ -814,7 +818,7 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant
     for (int e = 0; e < kFBuckets; ++e) M[e] = -INFINITY;
     // the rows past np are other pairs' or padding: their maxima are not
     // written, and nothing reaches a bar that is not a number
-    const float thr = (PASS == 2 && row_ok) ? bar[p0 + r] : __int_as_float(0x7fffffff);
+    float thr = (PASS == 2 && row_ok) ? bar[p0 + r] : __int_as_float(0x7fffffff);
     uint32_t held[2] = {0u, 0u};   // the last tile's hits, not yet written
     int slot = 0, hbase = 0;
     auto write_hits = [&]() {
@@ -823,7 +827,12 @@ knn_filter_kernel(const __grid_constant__ CUtensorMap mA0, const __grid_constant
         while (held[x]) {
           const int i = __ffs(held[x]) - 1;
           held[x] &= held[x] - 1;
-          if (slot < kFCap) crow[(size_t)(p0 + r) * kFCap + slot] = hbase + 32 * x + i;
+          if (slot < kFCap) {
+            crow[(size_t)(p0 + r) * kFCap + slot] = hbase + 32 * x + i;
+          } else if (thr == thr) {   // more candidates than slots: the pair looks for no more
+            atomicMax(inexact, 1);
+            thr = __int_as_float(0x7fffffff);
+          }
           ++slot;
         }
       }
@@ -986,8 +995,9 @@ knn_half_rows_kernel(const double* __restrict__ S, int rows, int K, const int* _
 // Row i of the BF16 planes (rows_pad x kw, zero padded) = the hi / lo split
 // of row src(i) of S (row-major, K doubles per row): src(i) = pairs[i] % ntest
 // when pairs is given (the test row of class-sorted pair i; slack[i] = 2 eps,
-// rounded up), else i.  These planes are not scaled: where |x| max|y| may leave the
-// range of FP32, *flag becomes 2 (the FP64 tiles).
+// rounded up; a row with a NaN, as above), else i.  These planes are not scaled:
+// where the products may leave the range of FP32, or a factor that of BF16, far
+// enough that the error is no longer below eps, *flag becomes 2 (the FP64 tiles).
 __global__ void __launch_bounds__(256)
 knn_split_rows_kernel(const double* __restrict__ S, int rows, int K, const int* __restrict__ pairs, int ntest,
                       int rows_pad, int kw, const unsigned* __restrict__ ymax_bits, __nv_bfloat16* __restrict__ hi,
@@ -1006,9 +1016,14 @@ knn_split_rows_kernel(const double* __restrict__ S, int rows, int K, const int* 
     if (pairs && i < rows) {
       for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
       if (lane == 0) {
-        const double largest = sqrt(s2) * static_cast<double>(__uint_as_float(*ymax_bits));
-        slack[i] = __double2float_ru(ldexp(largest, -13));
-        if (largest > 1e38) atomicMax(flag, 2);
+        const double norm = sqrt(s2), ymax = static_cast<double>(__uint_as_float(*ymax_bits));
+        const double largest = norm * ymax;
+        slack[i] = norm != norm ? -INFINITY : __double2float_ru(ldexp(largest, -13));
+        // lo rounds to a multiple of 2^-133: at most sqrt(128) 2^-134 of a row, 5.3e-7 of
+        // 1e-33, in both factors; products below 2^-126 add at most 3 128 2^-126, 4.6e-7 of
+        // 1e-29.  With these, 5.9e-5 < eps = 6.1e-5.
+        const bool in_range = norm >= 1e-33 && ymax >= 1e-33 && largest >= 1e-29 && largest <= 1e38;
+        if (!isfinite(ymax) || (norm > 0.0 && ymax > 0.0 && !in_range)) atomicMax(flag, 2);
       }
     }
   }
@@ -1083,38 +1098,38 @@ knn_filter_bar_kernel(const float* __restrict__ apart, KnnClassInfo ci, int C, l
   bar[P] = sl == -INFINITY ? __int_as_float(0x7fffffff) : (theta == -INFINITY ? -INFINITY : __fadd_rd(theta, -sl));
 }
 
-// Exact scores of the candidates of every pair (one warp per class-sorted
-// pair): up to 32 candidates, the lanes split each FP64 dot; more, each lane
-// takes candidates lane, lane + 32, ... and forms their dots (k in order).  The
-// use_k largest go to plist[P * use_k ..] in descending order (-inf when there
-// are fewer).  A pair with more than kFCap
-// candidates raises *overflow to 1 (its list would be incomplete).
+// Exact scores of the candidates of every pair, one warp per class-sorted pair:
+// the lanes split every FP64 dot (four candidates at a time, the test row loaded
+// once) and lane c keeps the values of candidates c, c + 32, ...  The use_k
+// largest go to plist[P * use_k ..] in descending order (-inf when there are
+// fewer).  Nothing is scored where a pair has more candidates than its slots
+// hold (*inexact, raised by pass 2): another form of the products follows.
+// What bounds it: the candidates' rows, 8 K bytes each, out of L2.  A lane
+// a candidate past 32 of them took 32 lines a load: 100,000 pairs with 50 candidates
+// of 128 scores, the call 808 us so, 358 with the dots split.
 __global__ void knn_exact_kernel(const int* __restrict__ ccount, const int* __restrict__ crow,
                                  const int* __restrict__ pairs, long long total_pairs, int ntest,
                                  const double* __restrict__ Tq, const double* __restrict__ Ts, int K, int use_k,
-                                 double* __restrict__ plist, int* overflow) {
+                                 double* __restrict__ plist, const int* __restrict__ inexact) {
   const long long P = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (P >= total_pairs) return;   // whole warps
-  int cnt = ccount[P];
-  if (cnt > kFCap) {
-    if (lane == 0) atomicMax(overflow, 1);
-    cnt = kFCap;
-  }
+  if (*inexact != 0) return;
+  const int cnt = ccount[P];   // at most kFCap
   const double* xr = Tq + (size_t)(pairs[P] % ntest) * K;
-  if (cnt <= 32) {
-    // The common case: the warp's lanes split every dot (four candidates at a
-    // time, the test row loaded once), lane c keeps candidate c's value, and
-    // each value goes to its rank in the descending list (ties by lane).
-    double xv[kFK / 32];
+  double xv[kFK / 32];
 #pragma unroll
-    for (int m = 0; m < kFK / 32; ++m) xv[m] = (lane + 32 * m < K) ? xr[lane + 32 * m] : 0.0;
-    double mine = -INFINITY;
-    for (int c0 = 0; c0 < cnt; c0 += 4) {
+  for (int m = 0; m < kFK / 32; ++m) xv[m] = (lane + 32 * m < K) ? xr[lane + 32 * m] : 0.0;
+  double v[kFCap / 32];
+#pragma unroll
+  for (int u = 0; u < kFCap / 32; ++u) {
+    v[u] = -INFINITY;
+    const int end = min(cnt, 32 * u + 32);
+    for (int c0 = 32 * u; c0 < end; c0 += 4) {
       double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        if (c0 + c < cnt) {
+        if (c0 + c < end) {
           const double* yr = Ts + (size_t)crow[(size_t)P * kFCap + c0 + c] * K;
 #pragma unroll
           for (int m = 0; m < kFK / 32; ++m)
@@ -1126,29 +1141,19 @@ __global__ void knn_exact_kernel(const int* __restrict__ ccount, const int* __re
         for (int c = 0; c < 4; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        if (lane == c0 + c && c0 + c < cnt) mine = acc[c];
+        if (32 * u + lane == c0 + c && c0 + c < end) v[u] = acc[c];
     }
-    if (!(mine == mine)) mine = -INFINITY;   // a NaN never enters a list
+    if (!(v[u] == v[u])) v[u] = -INFINITY;   // a NaN never enters a list
+  }
+  if (cnt <= 32) {
+    // each value goes to its rank in the descending list (ties by lane)
     int rank = 0;
     for (int j = 0; j < 32; ++j) {
-      const double vj = __shfl_sync(0xffffffffu, mine, j);
-      rank += (vj > mine || (vj == mine && j < lane)) ? 1 : 0;
+      const double vj = __shfl_sync(0xffffffffu, v[0], j);
+      rank += (vj > v[0] || (vj == v[0] && j < lane)) ? 1 : 0;
     }
-    if (rank < use_k) plist[P * use_k + rank] = mine;
+    if (rank < use_k) plist[P * use_k + rank] = v[0];
     return;
-  }
-  double v[kFCap / 32];
-#pragma unroll
-  for (int u = 0; u < kFCap / 32; ++u) {
-    v[u] = -INFINITY;
-    const int idx = lane + 32 * u;
-    if (idx < cnt) {
-      const double* yr = Ts + (size_t)crow[(size_t)P * kFCap + idx] * K;
-      double d = 0.0;
-#pragma unroll 4
-      for (int k = 0; k < K; ++k) d = fma(xr[k], yr[k], d);
-      v[u] = d;
-    }
   }
   for (int e = 0; e < use_k; ++e) {
     // the warp's largest remaining value; the lowest lane holding it gives it up
@@ -1385,11 +1390,12 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
   d2h(hp.data(), pcount, C * sizeof(int));
   ctx.sync();
   // Tile kernel (FASTPLS_CKNN_TILES): 4 or unset the tensor-core filter with
-  // exact FP64 rescoring (score rows up to 128 wide), 1 the 16-wide k-step FP64
+  // exact FP64 rescoring (score rows up to 128 wide), 5 / 6 the filter with the
+  // FP16 / the split BF16 products first at any size, 1 the 16-wide k-step FP64
   // kernel, 2 / 3 the staged FP64 kernels with two / one training-row buffers.
   const char* tv = std::getenv("FASTPLS_CKNN_TILES");
   const char sel = (tv && tv[0]) ? tv[0] : '4';
-  const bool use_filter = sel == '4' && kdim <= kFK && use_k <= kFList;
+  const bool use_filter = sel >= '4' && kdim <= kFK && use_k <= kFList;
   std::vector<int> poffs(C + 1, 0);
   for (int c = 0; c < C; ++c) poffs[c + 1] = poffs[c] + hp[c];
   // the (class, pair tile, row chunk) items of a tile kernel and the places of
@@ -1423,9 +1429,9 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
   };
   make_items(use_filter ? kFT : kTileM, use_filter ? kFT : kTileN);
   const long long total_pairs = poffs[C];
+  double work = 0.0;   // (pair, training row) products
+  for (int c = 0; c < C; ++c) work += (double)hp[c] * (cr.offs[c + 1] - cr.offs[c]);
   if (pt.enabled()) {
-    double work = 0.0;
-    for (int c = 0; c < C; ++c) work += (double)hp[c] * (cr.offs[c + 1] - cr.offs[c]);
     std::fprintf(stderr, "[fastpls trace] candidate-kNN: %lld pairs, %.3e pair-rows (%.3e flop), %zu items\n",
                  total_pairs, work, 2.0 * work * kdim, items.size());
   }
@@ -1494,7 +1500,7 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
       }
       dzero(ccount, (size_t)total_pairs * sizeof(int));
       knn_filter_kernel<1, PLANES><<<ng, kFThreads, FilterTile<PLANES>::kSmem, ctx.stream>>>(
-          mA0, mA1, mB0, mB1, ditems, ci, kdim, use_k, apart, nullptr, nullptr, nullptr, ferr);
+          mA0, mA1, mB0, mB1, ditems, ci, kdim, use_k, apart, nullptr, nullptr, nullptr, ferr, ferr + 1);
       ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
       pt.mark("filter pass 1");
@@ -1503,7 +1509,7 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
       FPLS_CHECK_LAUNCH();
       pt.mark("filter bar");
       knn_filter_kernel<2, PLANES><<<ng, kFThreads, FilterTile<PLANES>::kSmem, ctx.stream>>>(
-          mA0, mA1, mB0, mB1, ditems, ci, kdim, use_k, nullptr, barv, ccount, crow, ferr);
+          mA0, mA1, mB0, mB1, ditems, ci, kdim, use_k, nullptr, barv, ccount, crow, ferr, ferr + 1);
       ::fpls::note_launch();
       FPLS_CHECK_LAUNCH();
       pt.mark("filter pass 2");
@@ -1519,26 +1525,40 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
       return flags[1];
     };
     dzero(ferr, 2 * sizeof(int));
-    __half* a16 = reinterpret_cast<__half*>(aplane);
-    __half* b16 = reinterpret_cast<__half*>(bplane);
-    knn_half_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, kw, ymax,
-                                                     a16, slack, ferr + 1);
-    ::fpls::note_launch();
-    knn_half_rows_kernel<<<gs, 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, nullptr, 1, (int)b_rows, kw, ymax, b16,
-                                                     nullptr, ferr + 1);
-    ::fpls::note_launch();
-    FPLS_CHECK_LAUNCH();
-    pt.mark("filter planes");
-    const CUtensorMap mA = make_rows_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a16, (int)a_rows, kw);
-    const CUtensorMap mB = make_rows_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b16, (int)b_rows, kw);
-    int left = passes(std::integral_constant<int, 1>{}, mA, mA, mB, mB);
+    // FP16 products first only where they are most of the call and a crowded pair's
+    // exact scores little of it.  Measured, us, FP16 first / split BF16 first, where
+    // the FP16 slots hold and where similarities crowd (unit-norm rows, 5 candidate
+    // classes, or both of 2):
+    //   2 x 15000 rows, 64 scores, 5000 test rows (1.9e10): 354 / 408, 568 / 419
+    //   2 x 3000, 110, 5000 (6.6e9): 281 / 303, 435 / 329
+    //   20 x 50, 100, 10000 (1e8 and less): 3 % apart at most, 1.1 to 2 times
+    //   200 x 100, 128, 100000 (1.3e10): 1704 / 1828, 4467 / 1883 (every row of a
+    //   class within the FP16 bar, and its slots hold them)
+    const bool half_first =
+        sel == '5' || (sel == '4' && 2.0 * work * kdim >= 1e10 && work >= 2048.0 * (double)total_pairs);
+    int left = 1;
+    if (half_first) {
+      __half* a16 = reinterpret_cast<__half*>(aplane);
+      __half* b16 = reinterpret_cast<__half*>(bplane);
+      knn_half_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, kw,
+                                                       ymax, a16, slack, ferr + 1);
+      ::fpls::note_launch();
+      knn_half_rows_kernel<<<gs, 256, 0, ctx.stream>>>(cr.Ts, nvalid, kdim, nullptr, 1, (int)b_rows, kw, ymax, b16,
+                                                       nullptr, ferr + 1);
+      ::fpls::note_launch();
+      FPLS_CHECK_LAUNCH();
+      pt.mark("filter planes");
+      const CUtensorMap mA = make_rows_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a16, (int)a_rows, kw);
+      const CUtensorMap mB = make_rows_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, b16, (int)b_rows, kw);
+      left = passes(std::integral_constant<int, 1>{}, mA, mA, mB, mB);
+      if (left == 1) dzero(ferr, 2 * sizeof(int));
+    }
     if (left == 1) {
-      // similarities crowd within the FP16 bar: a bar 17 times narrower
+      // the first form, or similarities crowd within the FP16 bar: this one is 17 times narrower
       __nv_bfloat16* ah = reinterpret_cast<__nv_bfloat16*>(aplane);
       __nv_bfloat16* bh = reinterpret_cast<__nv_bfloat16*>(bplane);
       __nv_bfloat16* al = ctx.arena.alloc_n<__nv_bfloat16>((size_t)a_rows * kw);
       __nv_bfloat16* bl = ctx.arena.alloc_n<__nv_bfloat16>((size_t)b_rows * kw);
-      dzero(ferr, 2 * sizeof(int));
       knn_split_rows_kernel<<<gs, 256, 0, ctx.stream>>>(Tq, (int)total_pairs, kdim, pairs, ntest, (int)a_rows, kw,
                                                         ymax, ah, al, slack, ferr + 1);
       ::fpls::note_launch();
@@ -1558,12 +1578,9 @@ void candidate_knn_predict_device(const double* dTt, int ntest, const ClassRows&
       // training rows once per 128-pair tile and pass, the pair planes once a
       // pass (the class's time includes the planes, the bar, the exact scores
       // and the split BF16 products where they run)
-      double work = 0.0, bytes = 2.0 * 2.0 * kw * (double)total_pairs;
-      for (int c = 0; c < C; ++c) {
-        const double rows = cr.offs[c + 1] - cr.offs[c];
-        work += (double)hp[c] * rows;
-        bytes += 2.0 * 2.0 * kw * rows * (double)ceil_div(hp[c], kFT);
-      }
+      double bytes = 2.0 * 2.0 * kw * (double)total_pairs;
+      for (int c = 0; c < C; ++c)
+        bytes += 2.0 * 2.0 * kw * (double)(cr.offs[c + 1] - cr.offs[c]) * (double)ceil_div(hp[c], kFT);
       ctx.prof_end(slot, ctx.stream, bytes, 2.0 * 2.0 * work * kdim);
     }
     if (left == 0) {
